@@ -1,7 +1,8 @@
 """Cache of prepared (split / packed) weight forms for the tensor-core kernels, shared by the SO3Linear,
 dense and radial-chain front-ends.  Keyed on the weight tensors' storage address and version, so an in-place
-update or a new tensor invalidates the entry; an entry keeps its weight tensors alive so the address cannot
-be reused while it exists.  An entry remembers the stream it was built on and an event recorded behind the
+update or a new tensor invalidates the entry; an entry keeps the weights' storages alive (through detached
+aliases: a parameter object can be given another storage, ``module.double()`` or ``p.data = ...``) so the
+address cannot be reused while it exists.  An entry remembers the stream it was built on and an event recorded behind the
 build: a later call on another stream waits for that event (and tells the allocator about the new reader)
 before it uses the entry.  Plays the part of the reference's plan LRU
 (fasteq/ops/auto_schedule/eqlinear_plan.py:38-41, :81-100, :167-187).
@@ -82,6 +83,6 @@ def get(weights: Sequence[torch.Tensor], tag: Tuple, build: Callable[[], Optiona
     while _CACHE and _BYTES[0] + nbytes > _BUDGET[0]:
         _, old = _CACHE.popitem(last=False)
         _BYTES[0] -= old[1].numel() * old[1].element_size()
-    _CACHE[key] = (tuple(weights), val, done, {cur.cuda_stream})
+    _CACHE[key] = (tuple(w.detach() for w in weights), val, done, {cur.cuda_stream})
     _BYTES[0] += nbytes
     return val

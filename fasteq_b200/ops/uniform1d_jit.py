@@ -178,7 +178,7 @@ def graph_plan(dst: torch.Tensor, n_rows: int) -> GraphPlan:
     plan = _PLANS.get(key)
     if plan is None:
         plan = GraphPlan(dst, n_rows)
-        plan._keepalive = dst  # the key is the storage address: keep it from being recycled
+        plan._keepalive = dst.detach()  # the key is the storage address: keep the storage from being recycled
         _insert_plan(key, plan)
     else:
         _PLANS.move_to_end(key)
@@ -197,7 +197,7 @@ def register_sorted_plan(dst: torch.Tensor, n_rows: int, seg_ptr: torch.Tensor, 
         _OWNED[owner] = key
     _PLANS.pop(key, None)
     plan = GraphPlan(dst, n_rows, seg_ptr)
-    plan._keepalive = dst
+    plan._keepalive = dst.detach()
     _insert_plan(key, plan)
     return plan
 
@@ -342,7 +342,7 @@ _META_CACHE: Dict[Tuple, Tuple[torch.Tensor, np.ndarray]] = {}
 
 
 def _np(t, is_float=False) -> np.ndarray:
-    """Host copy of a meta tensor.  Cached by storage identity; the cache keeps the tensor alive,
+    """Host copy of a meta tensor.  Cached by storage identity; the cache keeps the storage alive,
     so its address cannot be handed to another tensor while the entry exists."""
     if isinstance(t, torch.Tensor):
         key = (t.data_ptr(), t.numel(), t._version, t.dtype, str(t.device))
@@ -351,7 +351,7 @@ def _np(t, is_float=False) -> np.ndarray:
             a = t.detach().cpu().numpy().astype(np.float64 if is_float else np.int64)
             if len(_META_CACHE) > 512:
                 _META_CACHE.clear()
-            _META_CACHE[key] = (t, a)
+            _META_CACHE[key] = (t.detach(), a)
             return a
         return hit[1]
     return np.asarray(t, dtype=np.float64 if is_float else np.int64)

@@ -119,3 +119,17 @@ def test_misaligned_float32_operand_takes_the_fma_kernel():
     w = (torch.randn(N, K, generator=g) / 8).cuda()
     out = dense(x, w)
     assert _rel(out.cpu(), x.cpu().double() @ w.cpu().double().t()) <= 2e-6
+
+
+def test_prepared_weights_survive_a_storage_swap():
+    """A parameter given another storage (``module.double()``) frees the address its prepared form was keyed on: the next
+    weight the allocator puts there must not be taken for it."""
+    from fasteq_b200.ops.dense import dense
+    g = torch.Generator().manual_seed(6)
+    x = torch.randn(256, 64, generator=g).cuda()
+    for _ in range(6):
+        w = torch.nn.Parameter((torch.randn(64, 64, generator=g) / 8).cuda())
+        out = dense(x, w)
+        assert _rel(out.detach().cpu(), x.cpu().double() @ w.detach().cpu().double().t()) <= 2e-6
+        w.data = w.data.double()
+        del w, out
