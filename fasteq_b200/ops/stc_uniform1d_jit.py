@@ -20,7 +20,7 @@ from .. import _build, _cabi
 from ..codegen import stc as _emit
 
 STC_PAD_VALUE = -1
-_EMITTER_VERSION = "stc-v2"
+_EMITTER_VERSION = "stc-v3"
 _lock = threading.Lock()
 
 
