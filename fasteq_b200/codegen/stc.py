@@ -303,6 +303,124 @@ extern "C" int fasteq_stc_double_backward(const void* go, const void* x1, const 
     return L
 
 
+def _emit_summed_backward(spec: STCSpec, groups, dt: str) -> List[str]:
+    """Backward with the weight gradient already summed over nodes of equal species.
+
+    Bound: FP32 issue (``_emit_grad_body``).  Writing ``[batch, D, U]`` per-node weight gradients and adding them up by
+    species afterwards cost twice the arithmetic: 3 GB out, 3 GB back in and one atomic per value at 200 k nodes.  Here the
+    nodes come in species order (``order``, a stable sort), a CTA walks one contiguous share of it and keeps the D sums of its
+    channel in registers; they go out once per (CTA, species) pair.  Along the order either the CTA or the species grows from
+    one pair to the next, so ``CTA + species`` is a slot of its own and ``n_parts + n_species`` rows of partial sums do.  A
+    second kernel adds each species' slots in a fixed order: the result does not depend on scheduling."""
+    L: List[str] = [f"""
+__global__ void __launch_bounds__(NT) fasteq_stc_bwd_sum_kernel(const T* __restrict__ go, const T* __restrict__ x1,
+    const T* __restrict__ x0, const long long* __restrict__ order, const int* __restrict__ species, long long batch,
+    long long n_species, T* __restrict__ gx1, T* __restrict__ partial, int* status) {{
+  const long long lo = batch * blockIdx.x / gridDim.x, hi = batch * (blockIdx.x + 1) / gridDim.x;
+  for (int u = threadIdx.x; u < U; u += NT) {{
+    int cur = -1;                                      // species whose sums are in the registers"""]
+    L += [f"    T gw{d} = T(0);" for d in range(spec.x0_segs)]
+    L.append("    for (long long i = lo; i <= hi; ++i) {")
+    L.append("      const int sp = i < hi ? species[i] : -1;")
+    L.append("      if (sp != cur) {")
+    L.append("        if (cur >= 0 && cur < n_species) {")
+    L.append("          T* pp = partial + ((size_t)blockIdx.x + cur) * D * U + u;")
+    L += [f"          pp[{d} * U] = gw{d};" for d in range(spec.x0_segs)]
+    L.append("        }")
+    L += [f"        gw{d} = T(0);" for d in range(spec.x0_segs)]
+    L.append("        cur = sp;")
+    L.append("      }")
+    L.append("      if (i == hi) break;")
+    L.append("      // a species out of range is reported, differentiates as species 0 and adds to no weight gradient")
+    L.append("      if (sp < 0 || sp >= n_species) atomicExch(status, 2);")
+    L.append("      const size_t b = (size_t)order[i];")
+    L.append("      const T* xp = x1 + b * A * U + u;")
+    L.append("      const T* wp = x0 + (size_t)(sp < 0 || sp >= n_species ? 0 : sp) * D * U + u;")
+    L.append("      const T* gp = go + b * V * U + u;")
+    L += [f"      const T x{a} = xp[{a} * U];" for a in range(spec.x1_segs)]
+    L += [f"      const T go{v} = gp[{v} * U];" for v in range(spec.out_segs)]
+    L += [f"      T ga{a} = T(0);" for a in range(spec.x1_segs)]
+    L += _emit_grad_body(groups, dt, "      ", True)
+    L.append("      T* gxp = gx1 + b * A * U + u;")
+    L += [f"      gxp[{a} * U] = ga{a};" for a in range(spec.x1_segs)]
+    L.append("    }\n  }\n}")
+    L.append(r"""
+// gx0[s][d][u] = sum of the partial sums of species s: 32 channels by 8 interleaved shares of its CTAs, both in a fixed order
+__global__ void __launch_bounds__(256) fasteq_stc_sum_parts_kernel(const int* __restrict__ species, const T* __restrict__ partial,
+    long long batch, int n_parts, T* __restrict__ gx0) {
+  __shared__ T share[8][33];
+  const int s = blockIdx.x / D, d = blockIdx.x % D, u = blockIdx.y * 32 + threadIdx.x;
+  long long bound[2];                                  // first positions of species s and s + 1 in the order
+  for (int e = 0; e < 2; ++e) {
+    long long a = e ? bound[0] : 0, b = batch;
+    while (a < b) {
+      const long long mid = (a + b) >> 1;
+      if (species[mid] < s + e) a = mid + 1; else b = mid;
+    }
+    bound[e] = a;
+  }
+  T sum = T(0);
+  if (bound[0] < bound[1] && u < U) {
+    // the CTA of position i is the largest c with floor(batch * c / n_parts) <= i
+    const long long first = ((bound[0] + 1) * n_parts - 1) / batch, last = (bound[1] * n_parts - 1) / batch;
+    for (long long c = first + threadIdx.y; c <= last; c += 8) sum += partial[((size_t)(c + s) * D + d) * U + u];
+  }
+  share[threadIdx.y][threadIdx.x] = sum;
+  __syncthreads();
+  if (threadIdx.y == 0 && u < U) {
+#pragma unroll
+    for (int k = 1; k < 8; ++k) sum += share[k][threadIdx.x];
+    gx0[((size_t)s * D + d) * U + u] = sum;
+  }
+}
+
+extern "C" int fasteq_stc_forward(const void*, const void*, const int32_t*, int64_t, int64_t, void*, fasteq_stream_t) {
+  return FASTEQ_UNSUPPORTED;  // summed-backward module
+}
+extern "C" int fasteq_stc_backward(const void*, const void*, const void*, const int32_t*, int64_t, int64_t, void*, void*, fasteq_stream_t) {
+  return FASTEQ_UNSUPPORTED;  // summed-backward module
+}
+extern "C" int fasteq_stc_double_backward(const void*, const void*, const void*, const int32_t*, const void*, const void*, int64_t,
+                                          int64_t, void*, void*, void*, fasteq_stream_t) {
+  return FASTEQ_UNSUPPORTED;  // this module holds another direction
+}
+// the CTAs one wave holds: every share of the order then runs at once
+extern "C" int fasteq_stc_backward_summed_parts(int64_t batch, int32_t* n_parts) {
+  if (batch < 0 || !n_parts) return FASTEQ_INVALID;
+  int dev = 0, sms = 0, per = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fasteq_stc_bwd_sum_kernel, NT, 0);
+  if (e != cudaSuccess) return cuda_fail(e);
+  const int64_t wave = (int64_t)sms * (per > 0 ? per : 1);
+  *n_parts = (int32_t)(batch < wave ? (batch < 1 ? 1 : batch) : wave);
+  return FASTEQ_OK;
+}
+extern "C" int fasteq_stc_backward_summed(const void* go, const void* x1, const void* x0, const int64_t* order,
+                                          const int32_t* species_sorted, int64_t batch, int64_t n_species, int32_t n_parts,
+                                          void* partial, void* gx1, void* gx0, fasteq_stream_t stream) {
+  if (batch < 0 || n_species < 0 || n_parts < 1 || n_species > 0x7fffffffLL / D) return FASTEQ_INVALID;
+  cudaStream_t s = (cudaStream_t)stream;
+  if (batch == 0) {
+    if (n_species > 0 && !gx0) return FASTEQ_INVALID;
+    cudaError_t e = n_species > 0 ? cudaMemsetAsync(gx0, 0, (size_t)n_species * D * U * sizeof(T), s) : cudaSuccess;
+    return e == cudaSuccess ? FASTEQ_OK : cuda_fail(e);
+  }
+  if (n_species == 0 || !go || !x1 || !x0 || !order || !species_sorted || !partial || !gx1 || !gx0) return FASTEQ_INVALID;
+  int* st = nullptr;
+  cudaError_t e = cudaGetSymbolAddress((void**)&st, g_status_word);
+  if (e != cudaSuccess) return cuda_fail(e);
+  fasteq_stc_bwd_sum_kernel<<<(unsigned)n_parts, NT, 0, s>>>((const T*)go, (const T*)x1, (const T*)x0, (const long long*)order,
+                                                             species_sorted, batch, n_species, (T*)gx1, (T*)partial, st);
+  fasteq_stc_sum_parts_kernel<<<dim3((unsigned)(n_species * D), (U + 31) / 32), dim3(32, 8), 0, s>>>(species_sorted, (const T*)partial,
+                                                                                                  batch, n_parts, (T*)gx0);
+  e = cudaGetLastError();
+  return e == cudaSuccess ? FASTEQ_OK : cuda_fail(e);
+}
+""")
+    return L
+
+
 def emit_stc(spec: STCSpec, direction: str, need_gx0: bool = False) -> str:
     dt = spec.dtype
     groups = _groups(spec)
@@ -318,7 +436,7 @@ constexpr int U = {spec.u}, A = {spec.x1_segs}, D = {spec.x0_segs}, V = {spec.ou
 extern "C" int fasteq_stc_describe(fasteq_stc_desc* d) {{
   if (!d) return FASTEQ_INVALID;
   d->abi_version = FASTEQ_ABI_VERSION; d->dtype = {0 if dt == 'f32' else 1}; d->u = U; d->x1_segs = A; d->x0_segs = D;
-  d->out_segs = V; d->num_paths = {len(spec.paths)}; d->direction = {dict(fwd=0, bwd=1, dbwd=2)[direction]}; d->need_gx0 = {int(need_gx0)};
+  d->out_segs = V; d->num_paths = {len(spec.paths)}; d->direction = {dict(fwd=0, bwd=1, dbwd=2, bwdsum=3)[direction]}; d->need_gx0 = {int(need_gx0)};
   return FASTEQ_OK;
 }}
 """
@@ -363,6 +481,8 @@ extern "C" int fasteq_stc_double_backward(const void*, const void*, const void*,
 """)
     elif direction == "dbwd":
         body += _emit_double_backward(spec, groups, dt)
+    elif direction == "bwdsum":
+        body += _emit_summed_backward(spec, groups, dt)
     else:
         body.append(f"""
 constexpr bool NEED_GX0 = {str(need_gx0).lower()};

@@ -38,6 +38,9 @@ class STCModule:
         lib.fasteq_stc_backward.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64, C.c_int64,
                                             C.c_void_p, C.c_void_p, C.c_void_p]
         lib.fasteq_stc_double_backward.argtypes = [C.c_void_p] * 6 + [C.c_int64, C.c_int64] + [C.c_void_p] * 4
+        if hasattr(lib, "fasteq_stc_backward_summed"):
+            lib.fasteq_stc_backward_summed_parts.argtypes = [C.c_int64, C.POINTER(C.c_int32)]
+            lib.fasteq_stc_backward_summed.argtypes = [C.c_void_p] * 5 + [C.c_int64, C.c_int64, C.c_int32] + [C.c_void_p] * 4
         lib.fasteq_stc_device_status.argtypes = [C.POINTER(C.c_int32)]
         lib.fasteq_last_cuda_error.restype = C.c_char_p
         self.lib = lib
@@ -132,12 +135,32 @@ class FastSymmetricTensorContractionUniform1dFunction(torch.autograd.Function):
         need_x1, need_x0 = ctx.needs_input_grad[0], ctx.needs_input_grad[1]
         if not (need_x1 or need_x0):
             return (None,) * 8
+        if need_x0 and not torch.is_grad_enabled():
+            # a first-order backward: nothing differentiates the per-node weight gradients, so they never exist
+            gx1, gx0 = _backward_summed(grad_out.contiguous(), x1.contiguous(), x0.contiguous(), i32, spec)
+            return (gx1 if need_x1 else None), gx0, None, None, None, None, None, None
         gx1, gx0n = FastSTCBackwardFunction.apply(grad_out.contiguous(), x1.contiguous(), x0.contiguous(), i32, spec, bool(need_x0))
         gx0 = None
         if need_x0:
             # summed over nodes of equal species here (differentiable torch op; the kernel writes per-node rows)
             gx0 = torch.zeros_like(x0).index_add(0, i32.long(), gx0n)
         return (gx1 if need_x1 else None), gx0, None, None, None, None, None, None
+
+
+def _backward_summed(go, x1, x0, i32, spec):
+    """``(grad_x1, grad_x0)`` with the weight gradient summed by species in the kernel (see ``_emit_summed_backward``)."""
+    B, S = x1.shape[0], x0.shape[0]
+    gx1, gx0 = torch.empty_like(x1), torch.empty_like(x0)
+    lib = get_module(spec, "bwdsum", True).lib
+    with torch.cuda.device(x1.device):
+        parts = C.c_int32(0)
+        _cabi.check(lib.fasteq_stc_backward_summed_parts(B, C.byref(parts)), lib, "fasteq_stc_backward_summed_parts")
+        species, order = torch.sort(i32.view(-1), stable=True)
+        partial = torch.empty((parts.value + S, spec.x0_segs, spec.u), dtype=x1.dtype, device=x1.device)
+        _cabi.check(lib.fasteq_stc_backward_summed(go.data_ptr(), x1.data_ptr(), x0.data_ptr(), order.data_ptr(), species.data_ptr(),
+                                                   B, S, parts.value, partial.data_ptr(), gx1.data_ptr(), gx0.data_ptr(),
+                                                   torch.cuda.current_stream(x1.device).cuda_stream), lib, "fasteq_stc_backward_summed")
+    return gx1, gx0
 
 
 class FastSTCBackwardFunction(torch.autograd.Function):

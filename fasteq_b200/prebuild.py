@@ -92,7 +92,7 @@ def build_standard_modules(verbose: bool = False) -> None:
     for a, b, dtypes in STANDARD_STC:
         for dt in dtypes:
             sp = stc_spec(a, b, dt)
-            stc_jobs += [(sp, "fwd", False), (sp, "bwd", False), (sp, "bwd", True)]
+            stc_jobs += [(sp, "fwd", False), (sp, "bwd", False), (sp, "bwd", True), (sp, "bwdsum", True)]
     import torch
     from .ops import spherical_harmonics as shmod
     sh_jobs = []

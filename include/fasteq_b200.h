@@ -124,7 +124,7 @@ int fasteq_u1d_device_status(int32_t* code /* host */);
  * ------------------------------------------------------------------------- */
 typedef struct fasteq_stc_desc {
   int32_t abi_version, dtype, u, x1_segs, x0_segs, out_segs, num_paths;
-  int32_t direction;   /* 0 forward module, 1 backward module */
+  int32_t direction;   /* 0 forward, 1 backward, 2 double backward, 3 backward with the weight gradient summed by species */
   int32_t need_gx0;    /* backward: also writes the per-node weight gradient */
 } fasteq_stc_desc;
 
@@ -136,6 +136,14 @@ int fasteq_stc_forward(const void* x1, const void* x0, const int32_t* i0, int64_
  * species (the reference does the same with index_add_, stc_uniform1d_jit.py:883-886). */
 int fasteq_stc_backward(const void* grad_out, const void* x1, const void* x0, const int32_t* i0, int64_t batch,
                         int64_t n_species, void* grad_x1, void* grad_x0_per_node, fasteq_stream_t stream);
+/* The same gradients with the weight gradient summed over nodes of equal species (modules built for direction 3; others do not
+ * export it): grad_x0 [n_species, x0_segs, u] is fully overwritten, in an order of additions that depends on the batch and
+ * the GPU's size alone.  `order` int64 [batch] lists the nodes by species, `species_sorted` int32 [batch] their species in
+ * that order.  `partial` is scratch of (n_parts + n_species) * x0_segs * u values with n_parts from the query. */
+int fasteq_stc_backward_summed_parts(int64_t batch, int32_t* n_parts /* host */);
+int fasteq_stc_backward_summed(const void* grad_out, const void* x1, const void* x0, const int64_t* order, const int32_t* species_sorted,
+                               int64_t batch, int64_t n_species, int32_t n_parts, void* partial, void* grad_x1, void* grad_x0,
+                               fasteq_stream_t stream);
 /* Second order (modules built for direction 2; others return FASTEQ_UNSUPPORTED): with ggx1 [batch, x1_segs, u] and
  * ggx0_per_node [batch, x0_segs, u] the cotangents of grad_x1 and of the per-node grad_x0, writes the
  * gradients of <ggx1, grad_x1> + <ggx0, grad_x0> with respect to grad_out, x1 and (per node) x0.
