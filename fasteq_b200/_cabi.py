@@ -53,6 +53,7 @@ def core():
         lib.fasteq_graph_check_sorted.argtypes = [C.c_void_p, C.c_int64, C.c_void_p, C.c_void_p]
         lib.fasteq_graph_build_csr.argtypes = [C.c_void_p, C.c_int64, C.c_int64, C.c_void_p, C.c_void_p]
         lib.fasteq_graph_partition.argtypes = [C.c_void_p, C.c_int64, C.c_int64, C.c_int32, C.c_void_p, C.c_void_p]
+        lib.fasteq_graph_partition_edges.argtypes = [C.c_void_p, C.c_int64, C.c_int64, C.c_int32, C.c_void_p, C.c_void_p, C.c_void_p]
         _core = lib
     return _core
 
@@ -66,6 +67,10 @@ class U1DModule:
         lib.fasteq_u1d_describe.argtypes = [C.POINTER(U1DDesc)]
         lib.fasteq_u1d_forward.argtypes = [C.POINTER(U1DGraph)] + [C.c_void_p] * 5
         lib.fasteq_u1d_backward.argtypes = [C.POINTER(U1DGraph)] + [C.c_void_p] * 8
+        if hasattr(lib, "fasteq_u1d_forward_split"):
+            lib.fasteq_u1d_forward_split.argtypes = [C.POINTER(U1DGraph)] + [C.c_void_p] * 7
+        if hasattr(lib, "fasteq_u1d_backward_split"):
+            lib.fasteq_u1d_backward_split.argtypes = [C.POINTER(U1DGraph)] + [C.c_void_p] * 9
         lib.fasteq_u1d_device_status.argtypes = [C.POINTER(C.c_int32)]
         lib.fasteq_last_cuda_error.restype = C.c_char_p
         if hasattr(lib, "fasteq_u1d_forward_noalloc"):   # forward modules only
@@ -79,6 +84,9 @@ class U1DModule:
     def forward(self, graph: U1DGraph, w: int, x: int, y: int, out: int, stream: int) -> None:
         check(self.lib.fasteq_u1d_forward(C.byref(graph), w, x, y, out, stream), self.lib, "fasteq_u1d_forward")
 
+    def forward_split(self, graph: U1DGraph, part_edge: int, carry: int, w: int, x: int, y: int, out: int, stream: int) -> None:
+        check(self.lib.fasteq_u1d_forward_split(C.byref(graph), part_edge, carry, w, x, y, out, stream), self.lib, "fasteq_u1d_forward_split")
+
     def forward_noalloc(self, dst_sorted: int, x_index, n_edges: int, n_out_rows: int, x_rows: int,
                         w: int, x: int, y: int, out: int, stream: int) -> int:
         """Raw status of fasteq_u1d_forward_noalloc (the caller decides how to treat a refusal)."""
@@ -90,6 +98,10 @@ class U1DModule:
     def backward(self, graph: U1DGraph, go: int, w: int, x: int, y: int, gw, gx, gy, stream: int) -> None:
         check(self.lib.fasteq_u1d_backward(C.byref(graph), go, w, x, y, gw, gx, gy, stream), self.lib,
               "fasteq_u1d_backward")
+
+    def backward_split(self, graph: U1DGraph, part_edge: int, go: int, w: int, x: int, y: int, gw, gx, gy, stream: int) -> None:
+        check(self.lib.fasteq_u1d_backward_split(C.byref(graph), part_edge, go, w, x, y, gw, gx, gy, stream), self.lib,
+              "fasteq_u1d_backward_split")
 
     def device_status(self) -> int:
         v = C.c_int32(0)

@@ -119,22 +119,22 @@ def _emit_forward_body(groups, dt: str, ind: str) -> List[str]:
                 if len(a) == 2:
                     pairs[a] = None
         L.append(_segment_scope(ind, v))
-        L += [f"{ind}  const T p{a}_{b} = x{a} * x{b};" for a, b in sorted(pairs)]
+        L += [f"{ind}  const V p{a}_{b} = x{a} * x{b};" for a, b in sorted(pairs)]
         for d, mono, singles in plan:
-            L.append(f"{ind}  {{ T r;")
+            L.append(f"{ind}  {{ V r;")
             first = True
             for a, c in sorted(mono.items()):
                 if len(a) < 3:
                     L.append(_axpy(ind + "    ", "r", lit(c, dt), f"x{a[0]}" if len(a) == 1 else f"p{a[0]}_{a[1]}", first))
                     first = False
             for (c1,), ms in singles.items():
-                L.append(f"{ind}    {{ T s;")
+                L.append(f"{ind}    {{ V s;")
                 for n, m in enumerate(ms):
                     a, b = _rest(m, (c1,))
                     L.append(_axpy(ind + "      ", "s", lit(mono[m], dt), f"p{a}_{b}", n == 0))
                 L.append(_axpy(ind + "      ", "r", f"x{c1}", "s", first) + " }")
                 first = False
-            L.append(f"{ind}    o{v} = fma(wp[{d} * U], r, o{v}); }}")
+            L.append(f"{ind}    o{v} = fma(LD(wp + {d} * U), r, o{v}); }}")
         L.append(f"{ind}}}")
     return L
 
@@ -160,12 +160,12 @@ def _emit_grad_body(groups, dt: str, ind: str, need_gw: bool) -> List[str]:
         for a in quads:
             pairs.setdefault(a, [])
         L.append(_segment_scope(ind, v))
-        L += [f"{ind}  const T g{d} = wp[{d} * U] * go{v};" for d in ds]
+        L += [f"{ind}  const V g{d} = LD(wp + {d} * U) * go{v};" for d in ds]
         if need_gw:
-            L += [f"{ind}  T P{d} = T(0);" for d in ds]
+            L += [f"{ind}  V P{d} = ZERO;" for d in ds]
 
         def coefficient(a, ind2):
-            return [_axpy(ind2, "C", lit(c, dt), f"g{d}", n == 0, "T " if n == 0 else "") for n, (d, c) in enumerate(mono[a])]
+            return [_axpy(ind2, "C", lit(c, dt), f"g{d}", n == 0, "V " if n == 0 else "") for n, (d, c) in enumerate(mono[a])]
 
         def value(a, name, ind2):
             return [f"{ind2}P{d} = fma({lit(c, dt)}, {name}, P{d});" for d, c in mono[a]] if need_gw else []
@@ -175,7 +175,7 @@ def _emit_grad_body(groups, dt: str, ind: str, need_gw: bool) -> List[str]:
             L += coefficient(a, ind + "    ") + value(a, f"x{a[0]}", ind + "    ")
             L.append(f"{ind}    ga{a[0]} += C; }}")
         for (a, b), ms in sorted(pairs.items()):
-            L.append(f"{ind}  {{ const T p = x{a} * x{b}; T S;")
+            L.append(f"{ind}  {{ const V p = x{a} * x{b}; V S;")
             first = True
             if (a, b) in mono:
                 L += [f"{ind}    {{"] + coefficient((a, b), ind + "      ") + value((a, b), "p", ind + "      ")
@@ -185,7 +185,7 @@ def _emit_grad_body(groups, dt: str, ind: str, need_gw: bool) -> List[str]:
                 (c1,) = _rest(m, (a, b))
                 L += [f"{ind}    {{"] + coefficient(m, ind + "      ")
                 if need_gw:
-                    L.append(f"{ind}      const T m = p * x{c1};")
+                    L.append(f"{ind}      const V m = p * x{c1};")
                     L += value(m, "m", ind + "      ")
                 L.append(_axpy(ind + "      ", "S", "C", f"x{c1}", first))
                 L.append(f"{ind}      ga{c1} = fma(C, p, ga{c1}); }}")
@@ -238,7 +238,7 @@ __global__ void __launch_bounds__(NT) fasteq_stc_dbwd_kernel(const T* __restrict
       const T* tp = ggx1 + (size_t)b * A * U + u;
       const T* wp = x0 + (size_t)sp * D * U + u;
       const T* twp = ggx0n + (size_t)b * D * U + u;
-      const T* gp = go + (size_t)b * V * U + u;"""]
+      const T* gp = go + (size_t)b * OSEG * U + u;"""]
     L += [f"      const T x{a} = xp[{a} * U], t{a} = tp[{a} * U];" for a in range(spec.x1_segs)]
     L += [f"      const T go{v} = gp[{v} * U];" for v in range(spec.out_segs)]
     L += [f"      T dx{a} = T(0);" for a in range(spec.x1_segs)]
@@ -275,7 +275,7 @@ __global__ void __launch_bounds__(NT) fasteq_stc_dbwd_kernel(const T* __restrict
             L.append(f"      d_x0n[((size_t)b * D + {d}) * U + u] = T(0);")
     L.append("      T* dxp = d_x1 + (size_t)b * A * U + u;")
     L += [f"      dxp[{a} * U] = dx{a};" for a in range(spec.x1_segs)]
-    L.append("      T* dgp = d_go + (size_t)b * V * U + u;")
+    L.append("      T* dgp = d_go + (size_t)b * OSEG * U + u;")
     L += [f"      dgp[{v} * U] = dg{v};" for v in range(spec.out_segs)]
     L.append("    }\n  }\n}")
     L.append("""
@@ -317,17 +317,17 @@ __global__ void __launch_bounds__(NT) fasteq_stc_bwd_sum_kernel(const T* __restr
     const T* __restrict__ x0, const long long* __restrict__ order, const int* __restrict__ species, long long batch,
     long long n_species, T* __restrict__ gx1, T* __restrict__ partial, int* status) {{
   const long long lo = batch * blockIdx.x / gridDim.x, hi = batch * (blockIdx.x + 1) / gridDim.x;
-  for (int u = threadIdx.x; u < U; u += NT) {{
+  for (int u = threadIdx.x * VEC; u < U; u += NT * VEC) {{
     int cur = -1;                                      // species whose sums are in the registers"""]
-    L += [f"    T gw{d} = T(0);" for d in range(spec.x0_segs)]
+    L += [f"    V gw{d} = ZERO;" for d in range(spec.x0_segs)]
     L.append("    for (long long i = lo; i <= hi; ++i) {")
     L.append("      const int sp = i < hi ? species[i] : -1;")
     L.append("      if (sp != cur) {")
     L.append("        if (cur >= 0 && cur < n_species) {")
     L.append("          T* pp = partial + ((size_t)blockIdx.x + cur) * D * U + u;")
-    L += [f"          pp[{d} * U] = gw{d};" for d in range(spec.x0_segs)]
+    L += [f"          ST(pp + {d} * U, gw{d});" for d in range(spec.x0_segs)]
     L.append("        }")
-    L += [f"        gw{d} = T(0);" for d in range(spec.x0_segs)]
+    L += [f"        gw{d} = ZERO;" for d in range(spec.x0_segs)]
     L.append("        cur = sp;")
     L.append("      }")
     L.append("      if (i == hi) break;")
@@ -336,13 +336,13 @@ __global__ void __launch_bounds__(NT) fasteq_stc_bwd_sum_kernel(const T* __restr
     L.append("      const size_t b = (size_t)order[i];")
     L.append("      const T* xp = x1 + b * A * U + u;")
     L.append("      const T* wp = x0 + (size_t)(sp < 0 || sp >= n_species ? 0 : sp) * D * U + u;")
-    L.append("      const T* gp = go + b * V * U + u;")
-    L += [f"      const T x{a} = xp[{a} * U];" for a in range(spec.x1_segs)]
-    L += [f"      const T go{v} = gp[{v} * U];" for v in range(spec.out_segs)]
-    L += [f"      T ga{a} = T(0);" for a in range(spec.x1_segs)]
+    L.append("      const T* gp = go + b * OSEG * U + u;")
+    L += [f"      const V x{a} = LD(xp + {a} * U);" for a in range(spec.x1_segs)]
+    L += [f"      const V go{v} = LD(gp + {v} * U);" for v in range(spec.out_segs)]
+    L += [f"      V ga{a} = ZERO;" for a in range(spec.x1_segs)]
     L += _emit_grad_body(groups, dt, "      ", True)
     L.append("      T* gxp = gx1 + b * A * U + u;")
-    L += [f"      gxp[{a} * U] = ga{a};" for a in range(spec.x1_segs)]
+    L += [f"      ST(gxp + {a} * U, ga{a});" for a in range(spec.x1_segs)]
     L.append("    }\n  }\n}")
     L.append(r"""
 // gx0[s][d][u] = sum of the partial sums of species s: 32 channels by 8 interleaved shares of its CTAs, both in a fixed order
@@ -407,6 +407,7 @@ extern "C" int fasteq_stc_backward_summed(const void* go, const void* x1, const 
     return e == cudaSuccess ? FASTEQ_OK : cuda_fail(e);
   }
   if (n_species == 0 || !go || !x1 || !x0 || !order || !species_sorted || !partial || !gx1 || !gx0) return FASTEQ_INVALID;
+  if (misaligned(go, x1, x0, partial, gx1)) return FASTEQ_INVALID;
   int* st = nullptr;
   cudaError_t e = cudaGetSymbolAddress((void**)&st, g_status_word);
   if (e != cudaSuccess) return cuda_fail(e);
@@ -421,22 +422,54 @@ extern "C" int fasteq_stc_backward_summed(const void* go, const void* x1, const 
     return L
 
 
-def emit_stc(spec: STCSpec, direction: str, need_gx0: bool = False) -> str:
+def packed_ok(spec: STCSpec, direction: str) -> bool:
+    """Whether a thread may carry two channels in packed FP32 arithmetic (full warps of pairs; operands 8-byte aligned).  The
+    scalar kernels issued in 84 % (forward) and 67 % (backward with the weight gradient, whose 42 KB of straight-line code also
+    waits for instructions) of their cycles; packed ones need half the slots and half the code per channel."""
+    return spec.dtype == "f32" and spec.u % 64 == 0 and direction != "dbwd"
+
+
+_SCALAR = """typedef T V;             // what a thread carries per segment
+constexpr int VEC = 1;
+#define LD(p) (*(p))
+#define ST(p, v) (*(p) = (v))
+#define ZERO T(0)
+template <typename... P> static bool misaligned(P...) { return false; }
+"""
+
+_PACKED = """#include "fasteq_device.cuh"
+typedef float2 V;        // what a thread carries per segment: two channels
+constexpr int VEC = 2;
+#define LD(p) (*reinterpret_cast<const float2*>(p))
+#define ST(p, v) (*reinterpret_cast<float2*>(p) = (v))
+#define ZERO make_float2(0.f, 0.f)
+__device__ __forceinline__ V operator*(V a, V b) { return fasteq::vmul(a, b); }
+__device__ __forceinline__ V operator*(float c, V b) { return fasteq::vmul(make_float2(c, c), b); }
+__device__ __forceinline__ V fma(V a, V b, V c) { return fasteq::vfma(a, b, c); }
+__device__ __forceinline__ V fma(float a, V b, V c) { return fasteq::vfma(make_float2(a, a), b, c); }
+__device__ __forceinline__ void operator+=(V& a, V b) { a = fasteq::vadd(a, b); }
+template <typename... P> static bool misaligned(P... p) { return ((reinterpret_cast<uintptr_t>(p) | ...) & 7u) != 0; }
+"""
+
+
+def emit_stc(spec: STCSpec, direction: str, need_gx0: bool = False, packed: bool = False) -> str:
     dt = spec.dtype
     groups = _groups(spec)
-    threads = min((spec.u + 31) // 32 * 32, 128)
+    if packed and not packed_ok(spec, direction):
+        raise ValueError("packed arithmetic needs FP32, a multiple of 64 channels and a first-order kernel")
+    threads = min(((spec.u // 2 if packed else spec.u) + 31) // 32 * 32, 128)
     head = f"""// Generated by fasteq_b200.codegen.stc -- do not edit.
 #include <cstdio>
 #include <cstdint>
 #include <cuda_runtime.h>
 #include "fasteq_b200.h"
 typedef {spec.ctype} T;
-constexpr int U = {spec.u}, A = {spec.x1_segs}, D = {spec.x0_segs}, V = {spec.out_segs}, NT = {threads};
-{_COMMON}
+constexpr int U = {spec.u}, A = {spec.x1_segs}, D = {spec.x0_segs}, OSEG = {spec.out_segs}, NT = {threads};
+{_PACKED if packed else _SCALAR}{_COMMON}
 extern "C" int fasteq_stc_describe(fasteq_stc_desc* d) {{
   if (!d) return FASTEQ_INVALID;
   d->abi_version = FASTEQ_ABI_VERSION; d->dtype = {0 if dt == 'f32' else 1}; d->u = U; d->x1_segs = A; d->x0_segs = D;
-  d->out_segs = V; d->num_paths = {len(spec.paths)}; d->direction = {dict(fwd=0, bwd=1, dbwd=2, bwdsum=3)[direction]}; d->need_gx0 = {int(need_gx0)};
+  d->out_segs = OSEG; d->num_paths = {len(spec.paths)}; d->direction = {dict(fwd=0, bwd=1, dbwd=2, bwdsum=3)[direction]}; d->need_gx0 = {int(need_gx0)};
   return FASTEQ_OK;
 }}
 """
@@ -448,21 +481,21 @@ __global__ void __launch_bounds__(NT) fasteq_stc_fwd_kernel(const T* __restrict_
   for (long long b = blockIdx.x; b < batch; b += gridDim.x) {{
     int sp = i0[b];
     if (sp < 0 || sp >= n_species) {{ atomicExch(status, 2); sp = 0; }}
-    for (int u = threadIdx.x; u < U; u += NT) {{
+    for (int u = threadIdx.x * VEC; u < U; u += NT * VEC) {{
       const T* xp = x1 + (size_t)b * A * U + u;
       const T* wp = x0 + (size_t)sp * D * U + u;""")
-        body += [f"      const T x{a} = xp[{a} * U];" for a in range(spec.x1_segs)]
-        body += [f"      T o{v} = T(0);" for v in range(spec.out_segs)]
+        body += [f"      const V x{a} = LD(xp + {a} * U);" for a in range(spec.x1_segs)]
+        body += [f"      V o{v} = ZERO;" for v in range(spec.out_segs)]
         body += _emit_forward_body(groups, dt, "      ")
-        body.append("      T* op = out + (size_t)b * V * U + u;")
-        body += [f"      op[{v} * U] = o{v};" for v in range(spec.out_segs)]
+        body.append("      T* op = out + (size_t)b * OSEG * U + u;")
+        body += [f"      ST(op + {v} * U, o{v});" for v in range(spec.out_segs)]
         body.append("    }\n  }\n}")
         body.append("""
 extern "C" int fasteq_stc_forward(const void* x1, const void* x0, const int32_t* i0, int64_t batch, int64_t n_species,
                                   void* out, fasteq_stream_t stream) {
   if (batch < 0 || n_species < 0) return FASTEQ_INVALID;
   if (batch == 0) return FASTEQ_OK;
-  if (!x1 || !x0 || !i0 || !out) return FASTEQ_INVALID;
+  if (!x1 || !x0 || !i0 || !out || misaligned(x1, x0, out)) return FASTEQ_INVALID;
   int* st = nullptr;
   cudaError_t e = cudaGetSymbolAddress((void**)&st, g_status_word);
   if (e != cudaSuccess) return cuda_fail(e);
@@ -492,20 +525,20 @@ __global__ void __launch_bounds__(NT) fasteq_stc_bwd_kernel(const T* __restrict_
   for (long long b = blockIdx.x; b < batch; b += gridDim.x) {{
     int sp = i0[b];
     if (sp < 0 || sp >= n_species) {{ atomicExch(status, 2); sp = 0; }}
-    for (int u = threadIdx.x; u < U; u += NT) {{
+    for (int u = threadIdx.x * VEC; u < U; u += NT * VEC) {{
       const T* xp = x1 + (size_t)b * A * U + u;
       const T* wp = x0 + (size_t)sp * D * U + u;
-      const T* gp = go + (size_t)b * V * U + u;""")
-        body += [f"      const T x{a} = xp[{a} * U];" for a in range(spec.x1_segs)]
-        body += [f"      const T go{v} = gp[{v} * U];" for v in range(spec.out_segs)]
-        body += [f"      T ga{a} = T(0);" for a in range(spec.x1_segs)]
+      const T* gp = go + (size_t)b * OSEG * U + u;""")
+        body += [f"      const V x{a} = LD(xp + {a} * U);" for a in range(spec.x1_segs)]
+        body += [f"      const V go{v} = LD(gp + {v} * U);" for v in range(spec.out_segs)]
+        body += [f"      V ga{a} = ZERO;" for a in range(spec.x1_segs)]
         if need_gx0:
-            body += [f"      T gw{d} = T(0);" for d in range(spec.x0_segs)]
+            body += [f"      V gw{d} = ZERO;" for d in range(spec.x0_segs)]
         body += _emit_grad_body(groups, dt, "      ", need_gx0)
         if need_gx0:
-            body += [f"      gx0n[((size_t)b * D + {d}) * U + u] = gw{d};" for d in range(spec.x0_segs)]
+            body += [f"      ST(gx0n + ((size_t)b * D + {d}) * U + u, gw{d});" for d in range(spec.x0_segs)]
         body.append("      T* gxp = gx1 + (size_t)b * A * U + u;")
-        body += [f"      gxp[{a} * U] = ga{a};" for a in range(spec.x1_segs)]
+        body += [f"      ST(gxp + {a} * U, ga{a});" for a in range(spec.x1_segs)]
         body.append("    }\n  }\n}")
         body.append("""
 extern "C" int fasteq_stc_forward(const void*, const void*, const int32_t*, int64_t, int64_t, void*, fasteq_stream_t) {
@@ -516,6 +549,7 @@ extern "C" int fasteq_stc_backward(const void* go, const void* x1, const void* x
   if (batch < 0 || n_species < 0) return FASTEQ_INVALID;
   if (batch == 0) return FASTEQ_OK;
   if (!go || !x1 || !x0 || !i0 || !gx1 || (NEED_GX0 && !gx0_per_node)) return FASTEQ_INVALID;
+  if (misaligned(go, x1, x0, gx1, gx0_per_node)) return FASTEQ_INVALID;
   int* st = nullptr;
   cudaError_t e = cudaGetSymbolAddress((void**)&st, g_status_word);
   if (e != cudaSuccess) return cuda_fail(e);
@@ -543,6 +577,7 @@ def arith_ops(spec: STCSpec, direction: str, need_gx0: bool = False) -> Dict[str
     end = body.find('extern "C"')
     body = body[:end if end > 0 else len(body)]
     body = re.sub(r"//[^\n]*", "", body)
+    body = re.sub(r"\b(LD|ST)\([^,;]*?\* U", r"\1(", body)                     # address arithmetic
     body = re.sub(r"\[[^\]]*\]", "[]", body)                                   # subscripts hold index arithmetic only
     body = "\n".join(ln for ln in body.splitlines() if "size_t" not in ln and "const T*" not in ln)
     fma = len(re.findall(r"\bfma\(", body))

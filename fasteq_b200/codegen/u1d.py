@@ -156,6 +156,7 @@ static int fill_graph(const fasteq_u1d_graph* g, fasteq::u1d::Graph* o, int* gri
   if (g->n_edges > 0x7fffffffLL || g->n_out_rows > 0x7fffffffLL) return FASTEQ_UNSUPPORTED;
   o->n_edges = g->n_edges; o->n_out_rows = g->n_out_rows; o->x_rows = g->x_rows; o->y_rows = g->y_rows;
   o->x_index = g->x_index; o->y_index = g->y_index; o->seg_ptr = g->seg_ptr; o->perm = g->perm; o->part_ptr = g->part_ptr;
+  o->part_edge = nullptr;
   o->status = status_ptr();
   int dev = 0, sms = 0;
   cudaError_t e = cudaGetDevice(&dev);
@@ -442,7 +443,7 @@ constexpr int SMEM_BYTES = cfg::PIPES * PIPE_BYTES;
 
 __global__ void __launch_bounds__(NTHREADS, {tun.min_blocks})
 fasteq_u1d_fwd_kernel(const Graph g, const T* __restrict__ w, const T* __restrict__ x, const T* __restrict__ y,
-                      T* __restrict__ out) {{
+                      T* __restrict__ out, T* __restrict__ carry) {{
   extern __shared__ __align__(128) unsigned char smem_all[];
   if (threadIdx.x == 0) {{
     for (int p = 0; p < cfg::PIPES; ++p) {{
@@ -497,7 +498,7 @@ fasteq_u1d_fwd_kernel(const Graph g, const T* __restrict__ w, const T* __restric
     body.append("    }")
     body.append("    if (m.flags & F_LAST) {")
     body.append("      if (live) {")
-    body.append("        T* o = out + (size_t)m.row * OSEG * U + (size_t)m.ct * CT + ch;")
+    body.append("        T* o = (m.carry ? carry + (size_t)(m.carry - 1) * OSEG * U : out + (size_t)m.row * OSEG * U) + (size_t)m.ct * CT + ch;")
     for gi in range(G):
         body.append(f"        if (grp == {gi}) {{" if G > 1 else "        {")
         for s, v in enumerate(owners[gi]):
@@ -516,22 +517,54 @@ fasteq_u1d_fwd_kernel(const Graph g, const T* __restrict__ w, const T* __restric
     src.append(_HOST_COMMON)
     src.append(_describe(spec, tun, 0, threads=threads))
     src.append(f"""
-extern "C" int fasteq_u1d_forward(const fasteq_u1d_graph* gh, const void* w, const void* x, const void* y, void* out,
-                                  fasteq_stream_t stream) {{
+// Receivers whose edges several pipelines shared: the pipeline that began one stored its sum, every later one left its own in
+// its carry row; they are added in pipeline order.  One CTA column per pipeline, working only where the first carry of a
+// receiver sits.
+__global__ void __launch_bounds__(256) fasteq_u1d_carry_kernel(const int* __restrict__ seg_ptr, const int* __restrict__ part_ptr,
+    const int* __restrict__ part_edge, int n_parts, long long n_out_rows, const T* __restrict__ carry, T* __restrict__ out) {{
+  const int p = blockIdx.x, row = part_ptr[p];
+  if (row >= n_out_rows || part_edge[p] <= seg_ptr[row]) return;                                   // starts at a receiver's first edge
+  if (p > 0 && part_ptr[p - 1] == row && part_edge[p - 1] > seg_ptr[row]) return;                  // an earlier pipeline is the first
+  const int i = blockIdx.y * 256 + threadIdx.x;
+  if (i >= OSEG * U) return;
+  T sum = out[(size_t)row * OSEG * U + i];
+  for (int q = p; q < n_parts && part_ptr[q] == row; ++q)
+    if (part_edge[q + 1] > part_edge[q]) sum += carry[(size_t)q * OSEG * U + i];
+  out[(size_t)row * OSEG * U + i] = sum;
+}}
+
+static int run_forward(const fasteq_u1d_graph* gh, const int32_t* part_edge, void* carry, const void* w, const void* x, const void* y,
+                       void* out, fasteq_stream_t stream) {{
   Graph g; int grid = 1;
   int rc = fill_graph(gh, &g, &grid, {tun.min_blocks});
   if (rc != FASTEQ_OK) return rc;
   if (gh->n_out_rows == 0 && gh->n_edges == 0) return FASTEQ_OK;
   if (!out || (gh->n_edges > 0 && (!w || !x || !y))) return FASTEQ_INVALID;
+  g.part_edge = part_edge;
   g.bulk_ok = aligned16(w) && aligned16(x) && aligned16(y) && ((U * sizeof(T)) % 16 == 0) && ((CT * sizeof(T)) % 16 == 0);
-  if (VEC == 2 && ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(w)) & 7u)) return FASTEQ_INVALID;
+  if (VEC == 2 && ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(carry)) & 7u)) return FASTEQ_INVALID;
   cudaError_t e = cudaFuncSetAttribute(fasteq_u1d_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
   if (e != cudaSuccess) return cuda_fail(e);
   fasteq_u1d_fwd_kernel<<<grid, NTHREADS, SMEM_BYTES, (cudaStream_t)stream>>>(
-      g, (const T*)w, (const T*)x, (const T*)y, (T*)out);
+      g, (const T*)w, (const T*)x, (const T*)y, (T*)out, (T*)carry);
+  if (part_edge)
+    fasteq_u1d_carry_kernel<<<dim3((unsigned)gh->n_parts, (OSEG * U + 255) / 256), 256, 0, (cudaStream_t)stream>>>(
+        gh->seg_ptr, gh->part_ptr, part_edge, gh->n_parts, gh->n_out_rows, (const T*)carry, (T*)out);
   e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e);
   return FASTEQ_OK;
+}}
+
+extern "C" int fasteq_u1d_forward(const fasteq_u1d_graph* gh, const void* w, const void* x, const void* y, void* out,
+                                  fasteq_stream_t stream) {{
+  return run_forward(gh, nullptr, nullptr, w, x, y, out, stream);
+}}
+
+extern "C" int fasteq_u1d_forward_split(const fasteq_u1d_graph* gh, const int32_t* part_edge, void* carry, const void* w, const void* x,
+                                        const void* y, void* out, fasteq_stream_t stream) {{
+  if (!cfg::SCATTERED) return FASTEQ_UNSUPPORTED;
+  if (!gh || !gh->part_ptr || gh->n_parts < 1 || !part_edge || !carry) return FASTEQ_INVALID;
+  return run_forward(gh, part_edge, carry, w, x, y, out, stream);
 }}
 
 extern "C" int fasteq_u1d_backward(const fasteq_u1d_graph*, const void*, const void*, const void*, const void*, void*,
@@ -949,8 +982,8 @@ extern "C" int fasteq_u1d_forward(const fasteq_u1d_graph*, const void*, const vo
   return FASTEQ_UNSUPPORTED;  // this module holds the backward kernel only
 }}
 
-extern "C" int fasteq_u1d_backward(const fasteq_u1d_graph* gh, const void* go, const void* w, const void* x,
-                                   const void* y, void* gw, void* gx, void* gy, fasteq_stream_t stream) {{
+static int run_backward(const fasteq_u1d_graph* gh, const int32_t* part_edge, const void* go, const void* w, const void* x,
+                        const void* y, void* gw, void* gx, void* gy, fasteq_stream_t stream) {{
   Graph g; int grid = 1;
   int rc = fill_graph(gh, &g, &grid, {tun.min_blocks});
   if (rc != FASTEQ_OK) return rc;
@@ -960,6 +993,7 @@ extern "C" int fasteq_u1d_backward(const fasteq_u1d_graph* gh, const void* go, c
   if (gh->n_edges == 0) return FASTEQ_OK;          // per-edge buffers are empty (and may be null); the rest is zeroed
   if ((NEED_GW && !gw) || (NEED_GX && !gx) || (NEED_GY && !gy)) return FASTEQ_INVALID;
   if (!go || !w || !x || !y) return FASTEQ_INVALID;
+  g.part_edge = part_edge;
   g.bulk_ok = aligned16(w) && aligned16(x) && aligned16(y) && aligned16(go) && ((U * sizeof(T)) % 16 == 0) &&
               ((CT * sizeof(T)) % 16 == 0);
   if (VEC == 2 && ((reinterpret_cast<uintptr_t>(gw) | reinterpret_cast<uintptr_t>(gx) | reinterpret_cast<uintptr_t>(gy)) & 7u))
@@ -971,6 +1005,18 @@ extern "C" int fasteq_u1d_backward(const fasteq_u1d_graph* gh, const void* go, c
   e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e);
   return FASTEQ_OK;
+}}
+
+extern "C" int fasteq_u1d_backward(const fasteq_u1d_graph* gh, const void* go, const void* w, const void* x,
+                                   const void* y, void* gw, void* gx, void* gy, fasteq_stream_t stream) {{
+  return run_backward(gh, nullptr, go, w, x, y, gw, gx, gy, stream);
+}}
+
+extern "C" int fasteq_u1d_backward_split(const fasteq_u1d_graph* gh, const int32_t* part_edge, const void* go, const void* w, const void* x,
+                                         const void* y, void* gw, void* gx, void* gy, fasteq_stream_t stream) {{
+  if (!cfg::SCATTERED) return FASTEQ_UNSUPPORTED;
+  if (!gh || !gh->part_ptr || gh->n_parts < 1 || !part_edge) return FASTEQ_INVALID;
+  return run_backward(gh, part_edge, go, w, x, y, gw, gx, gy, stream);
 }}
 """)
     return "\n".join(src)

@@ -103,3 +103,31 @@ extern "C" int fasteq_graph_partition(const int32_t* seg_ptr, int64_t n_rows, in
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? FASTEQ_OK : cuda_fail(e);
 }
+
+// The same shares cut between edges: boundary p lies `target` units along the rows laid out as (edges, 1), inside a row's
+// edges where it falls there.  part_ptr[p] is the row it falls in, part_edge[p] the edge.
+__global__ void partition_edges_kernel(const int* __restrict__ seg_ptr, long long n_rows, long long n_edges, int n_parts,
+                                       int* __restrict__ part_ptr, int* __restrict__ part_edge) {
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p > n_parts) return;
+  if (p == n_parts) { part_ptr[p] = (int)n_rows; part_edge[p] = (int)n_edges; return; }
+  const long long target = (n_edges + n_rows) * p / n_parts;
+  long long lo = 0, hi = n_rows;                       // the first row that ends beyond the target
+  while (lo < hi) {
+    const long long mid = (lo + hi) >> 1;
+    if ((long long)seg_ptr[mid + 1] + mid + 1 <= target) lo = mid + 1; else hi = mid;
+  }
+  if (lo == n_rows) { part_ptr[p] = (int)n_rows; part_edge[p] = (int)n_edges; return; }
+  const long long first = seg_ptr[lo], end = seg_ptr[lo + 1], edge = first + (target - first - lo);
+  const bool done = end > first && edge >= end;        // only the row's own unit is left of it
+  part_ptr[p] = (int)(done ? lo + 1 : lo);
+  part_edge[p] = (int)(done ? end : edge);
+}
+
+extern "C" int fasteq_graph_partition_edges(const int32_t* seg_ptr, int64_t n_rows, int64_t n_edges, int32_t n_parts,
+                                            int32_t* part_ptr, int32_t* part_edge, fasteq_stream_t stream) {
+  if (!seg_ptr || !part_ptr || !part_edge || n_parts < 1 || n_rows < 0 || n_edges < 0) return FASTEQ_INVALID;
+  partition_edges_kernel<<<(n_parts + 1 + 255) / 256, 256, 0, (cudaStream_t)stream>>>(seg_ptr, n_rows, n_edges, n_parts, part_ptr, part_edge);
+  cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? FASTEQ_OK : cuda_fail(e);
+}

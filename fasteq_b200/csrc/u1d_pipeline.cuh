@@ -25,7 +25,7 @@ constexpr bool FULL_ROW = (CT == U);             // a tile is the whole contiguo
 
 constexpr int round_up(int a, int b) { return (a + b - 1) / b * b; }
 
-struct Meta { int row; int flags; int ct; int e; int xr; int yr; int pad0; int pad1; };
+struct Meta { int row; int flags; int ct; int e; int xr; int yr; int carry; int pad; };   // carry: see Producer::carry
 enum : int { F_DATA = 1, F_LAST = 2, F_DONE = 4, F_FIRST = 8 };
 
 constexpr int W_TILE_BYTES = cfg::W_SHARED ? 0 : WSEG * CT * (int)sizeof(T);
@@ -43,6 +43,7 @@ static_assert(STAGES * 16 + 32 <= BAR_BYTES, "too many stages for the barrier bl
 struct Graph {
   long long n_edges, n_out_rows, x_rows, y_rows;
   const int* x_index; const int* y_index; const int* seg_ptr; const int* perm; const int* part_ptr;
+  const int* part_edge;   // first edge of each pipeline's share, which may begin and end inside a receiver's edges; or null
   int bulk_ok;      // rows may travel as bulk copies
   int n_vblocks;    // pipelines that have work (grid * pipelines per CTA may exceed it)
   int* status;
@@ -78,6 +79,9 @@ __device__ __forceinline__ void copy_tile(unsigned char* sdst, const T* grow, in
 struct Producer {
   const Graph& g; const T* w; const T* x; const T* y;
   unsigned char* stages; uint64_t* full; uint64_t* empty; int lane; uint32_t it; int vblock;
+  // pipeline index + 1 while the edges being staged continue a receiver that an earlier pipeline began (its sum then goes to
+  // this pipeline's carry row instead of the output), else 0
+  int carry = 0;
   bool failed = false;   // a wait of this lane gave up: the warp stops issuing copies and reductions (see dead())
 
   static __device__ __forceinline__ int valid_of(int ct) { return (U - ct * CT) < CT ? (U - ct * CT) : CT; }
@@ -102,7 +106,7 @@ struct Producer {
     unsigned char* st = stages + (size_t)stage * STAGE_BYTES;
     if (myit >= (uint32_t)STAGES) flush(st);
     const int valid = valid_of(ct);
-    Meta m; m.row = row; m.flags = flags; m.ct = ct; m.e = e; m.xr = xr; m.yr = yr; m.pad0 = 0; m.pad1 = 0;
+    Meta m; m.row = row; m.flags = flags; m.ct = ct; m.e = e; m.xr = xr; m.yr = yr; m.carry = carry; m.pad = 0;
     *reinterpret_cast<Meta*>(st + OFF_META) = m;
     const bool data = (flags & F_DATA) != 0;
     if (cfg::Y_SH && data) sh_row(st, yr);     // plain stores, published by the arrive below
@@ -183,7 +187,7 @@ struct Producer {
     unsigned char* st = stages + (size_t)stage * STAGE_BYTES;
     if (lane == 0) {
       if (it >= (uint32_t)STAGES) flush(st);
-      Meta m; m.row = row; m.flags = flags; m.ct = ct; m.e = e; m.xr = xr; m.yr = yr; m.pad0 = 0; m.pad1 = 0;
+      Meta m; m.row = row; m.flags = flags; m.ct = ct; m.e = e; m.xr = xr; m.yr = yr; m.carry = carry; m.pad = 0;
       *reinterpret_cast<Meta*>(st + OFF_META) = m;
       if (cfg::Y_SH && (flags & F_DATA)) sh_row(st, yr);
       mbar_arrive_expect_tx(&full[stage], 0u);
@@ -267,6 +271,11 @@ struct Producer {
     if (vblock >= g.n_vblocks) { s0 = 0; s1 = 0; }
     else if (g.part_ptr) { s0 = g.part_ptr[vblock]; s1 = g.part_ptr[vblock + 1]; }
     else { s0 = n_units * vblock / g.n_vblocks; s1 = n_units * (vblock + 1) / g.n_vblocks; }
+    int ea = 0, eb = 0x7fffffff;                       // the share's edges when receivers are split
+    if (cfg::SCATTERED && g.part_edge && vblock < g.n_vblocks) {
+      ea = g.part_edge[vblock]; eb = g.part_edge[vblock + 1];
+      if (s1 < g.n_out_rows && eb > g.seg_ptr[s1]) ++s1;   // the share ends inside this receiver
+    }
     for (int ct = 0; ct < NCT; ++ct) {
       if (cfg::SCATTERED) {
         for (long long sb = s0; sb < s1; sb += 32) {
@@ -274,12 +283,14 @@ struct Producer {
           int rp0 = 0, rp1 = 0;
           if (lane < n) { rp0 = g.seg_ptr[sb + lane]; rp1 = g.seg_ptr[sb + lane + 1]; }
           for (int i = 0; i < n; ++i) {
-            const int e0 = __shfl_sync(0xffffffffu, rp0, i), e1 = __shfl_sync(0xffffffffu, rp1, i);
-            const int row = (int)(sb + i);
+            const int r0 = __shfl_sync(0xffffffffu, rp0, i), r1 = __shfl_sync(0xffffffffu, rp1, i);
+            const int row = (int)(sb + i), e0 = r0 > ea ? r0 : ea, e1 = r1 < eb ? r1 : eb;
+            carry = 0;
             if (e0 >= e1) {
-              if (cfg::EMIT_EMPTY_ROWS) { fill_special(F_LAST, row, ct, flush); if (dead()) { settle(); return; } }
+              if (cfg::EMIT_EMPTY_ROWS && r0 >= r1) { fill_special(F_LAST, row, ct, flush); if (dead()) { settle(); return; } }
               continue;
             }
+            carry = e0 > r0 ? vblock + 1 : 0;
             begin(row, ct, lane);
             if (dead()) { settle(); return; }
             for (int pb = e0; pb < e1; pb += 32) {
@@ -310,6 +321,7 @@ struct Producer {
         }
       }
     }
+    carry = 0;
     fill_special(F_DONE, 0, 0, flush);
     if (dead()) { settle(); return; }
     // drain: every stage still holding a finished edge gets its flush

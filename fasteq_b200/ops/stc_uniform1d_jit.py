@@ -20,7 +20,7 @@ from .. import _build, _cabi
 from ..codegen import stc as _emit
 
 STC_PAD_VALUE = -1
-_EMITTER_VERSION = "stc-v3"
+_EMITTER_VERSION = "stc-v4"
 _lock = threading.Lock()
 
 
@@ -57,13 +57,16 @@ _MODULES: Dict[Tuple, STCModule] = {}
 _SPECS: Dict[Tuple, Tuple] = {}
 
 
-def get_module(spec: _emit.STCSpec, direction: str, need_gx0: bool = False) -> STCModule:
-    key = (spec, direction, need_gx0)
+def get_module(spec: _emit.STCSpec, direction: str, need_gx0: bool = False, operands=()) -> STCModule:
+    """``operands``: the tensors of the call; packed modules read pairs of channels, so one at an odd 4-byte offset (a view
+    into a larger buffer) gets the scalar module."""
+    packed = _emit.packed_ok(spec, direction) and not any(t.data_ptr() % 8 for t in operands)
+    key = (spec, direction, need_gx0, packed)
     with _lock:
         mod = _MODULES.get(key)
     if mod is None:
-        tag = spec.key(f"{_EMITTER_VERSION}|{direction}|{need_gx0}")
-        so = _build.build_generated(f"stc_{direction}_{tag}", _emit.emit_stc(spec, direction, need_gx0))
+        tag = spec.key(f"{_EMITTER_VERSION}|{direction}|{need_gx0}|{packed}")
+        so = _build.build_generated(f"stc_{direction}_{tag}", _emit.emit_stc(spec, direction, need_gx0, packed))
         with _lock:
             mod = _MODULES.get(key)
             if mod is None:
@@ -120,7 +123,7 @@ class FastSymmetricTensorContractionUniform1dFunction(torch.autograd.Function):
         i32 = i0.to(torch.int32).contiguous()
         B = x1c.shape[0]
         out = torch.empty((B, spec.out_segs, spec.u), dtype=x1.dtype, device=x1.device)
-        mod = get_module(spec, "fwd")
+        mod = get_module(spec, "fwd", operands=(x1c, x0c))
         with torch.cuda.device(x1.device):
             _cabi.check(mod.lib.fasteq_stc_forward(x1c.data_ptr(), x0c.data_ptr(), i32.data_ptr(), B, x0c.shape[0], out.data_ptr(),
                                                    torch.cuda.current_stream(x1.device).cuda_stream), mod.lib, "fasteq_stc_forward")
@@ -151,7 +154,7 @@ def _backward_summed(go, x1, x0, i32, spec):
     """``(grad_x1, grad_x0)`` with the weight gradient summed by species in the kernel (see ``_emit_summed_backward``)."""
     B, S = x1.shape[0], x0.shape[0]
     gx1, gx0 = torch.empty_like(x1), torch.empty_like(x0)
-    lib = get_module(spec, "bwdsum", True).lib
+    lib = get_module(spec, "bwdsum", True, (go, x1, x0)).lib
     with torch.cuda.device(x1.device):
         parts = C.c_int32(0)
         _cabi.check(lib.fasteq_stc_backward_summed_parts(B, C.byref(parts)), lib, "fasteq_stc_backward_summed_parts")
@@ -172,7 +175,7 @@ class FastSTCBackwardFunction(torch.autograd.Function):
         B = x1.shape[0]
         gx1 = torch.empty_like(x1)
         gx0n = torch.empty((B, spec.x0_segs, spec.u), dtype=x1.dtype, device=x1.device) if need_x0 else None
-        mod = get_module(spec, "bwd", bool(need_x0))
+        mod = get_module(spec, "bwd", bool(need_x0), (go, x1, x0))
         with torch.cuda.device(x1.device):
             _cabi.check(mod.lib.fasteq_stc_backward(go.data_ptr(), x1.data_ptr(), x0.data_ptr(), i32.data_ptr(), B, x0.shape[0],
                                                     gx1.data_ptr(), gx0n.data_ptr() if need_x0 else None,

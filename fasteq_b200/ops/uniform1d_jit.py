@@ -29,7 +29,7 @@ from .. import tuning as _tuning
 from ..codegen import u1d as _emit
 from ..codegen.u1d_common import U1DSpec, make_spec
 
-_EMITTER_VERSION = "u1d-v2"
+_EMITTER_VERSION = "u1d-v3"
 _MODULES: Dict[Tuple, _cabi.U1DModule] = {}
 _TUNING_OVERRIDE: Dict[str, _emit.Tuning] = {}
 _lock = threading.Lock()
@@ -80,7 +80,7 @@ class GraphPlan:
         self.n_rows = int(n_rows)
         self.n_edges = int(dst.numel())
         dev = dst.device
-        self._parts: Dict[int, torch.Tensor] = {}
+        self._parts: Dict[Tuple[int, bool], torch.Tensor] = {}
         self._ready: List[Tuple[int, torch.cuda.Event]] = []
         self._waited: Set[int] = set()          # streams already ordered behind every event in _ready
         self.device = dev
@@ -139,16 +139,22 @@ class GraphPlan:
                     t.record_stream(cur)
         self._waited.add(cur.cuda_stream)
 
-    def partition(self, n_parts: int) -> torch.Tensor:
-        p = self._parts.get(n_parts)
+    def partition(self, n_parts: int, split: bool = False) -> torch.Tensor:
+        """First row of each share (``[1, n_parts + 1]``); with ``split`` shares are cut between edges and a second row holds
+        their first edges."""
+        p = self._parts.get((n_parts, split))
         if p is None:
             core = _cabi.core()
-            p = torch.empty(n_parts + 1, dtype=torch.int32, device=self.device)
+            p = torch.empty((2 if split else 1, n_parts + 1), dtype=torch.int32, device=self.device)
             with torch.cuda.device(self.device):
                 stream = torch.cuda.current_stream(self.device).cuda_stream
-                _cabi.check(core.fasteq_graph_partition(self.seg_ptr.data_ptr(), self.n_rows, self.n_edges, n_parts,
-                                                        p.data_ptr(), stream), core, "fasteq_graph_partition")
-            self._parts[n_parts] = p
+                if split:
+                    _cabi.check(core.fasteq_graph_partition_edges(self.seg_ptr.data_ptr(), self.n_rows, self.n_edges, n_parts, p[0].data_ptr(),
+                                                                  p[1].data_ptr(), stream), core, "fasteq_graph_partition_edges")
+                else:
+                    _cabi.check(core.fasteq_graph_partition(self.seg_ptr.data_ptr(), self.n_rows, self.n_edges, n_parts,
+                                                            p.data_ptr(), stream), core, "fasteq_graph_partition")
+            self._parts[(n_parts, split)] = p
             self._mark_built()
         return p
 
@@ -320,22 +326,35 @@ class _Call:
             _SPEC_CACHE[skey] = hit
         self.spec = hit[0]
 
-    def graph(self, mod: _cabi.U1DModule, dev) -> _cabi.U1DGraph:
-        g = _cabi.U1DGraph()
+    def graph(self, mod: _cabi.U1DModule, dev) -> Tuple[_cabi.U1DGraph, Optional[int]]:
+        """The launch's graph record and, when the shares of its pipelines split receivers, the address of their first edges."""
+        g, part_edge = _cabi.U1DGraph(), None
         g.n_edges, g.n_out_rows, g.x_rows, g.y_rows = self.n_edges, self.n_out_rows, self.x_rows, self.y_rows
         g.x_index = self.src.data_ptr() if self.x_indexed else None
         g.y_index = self.src.data_ptr() if self.y_indexed else None
         if self.plan is not None:
             g.seg_ptr = self.plan.seg_ptr.data_ptr()
             g.perm = self.plan.perm.data_ptr() if self.plan.perm is not None else None
-            n_parts = max(1, min(_sm_count(dev) * int(mod.desc.ctas_per_sm), self.n_out_rows))
-            g.part_ptr = self.plan.partition(n_parts).data_ptr()
-            g.n_parts = n_parts
+            pipelines = _sm_count(dev) * int(mod.desc.ctas_per_sm)
+            if 0 < self.n_edges and self.n_out_rows < SPLIT_ROWS_PER_PIPELINE * pipelines:
+                g.n_parts = max(1, min(pipelines, max(self.n_out_rows, (self.n_edges + 3) // 4)))
+                part = self.plan.partition(g.n_parts, split=True)
+                part_edge = part[1].data_ptr()
+            else:
+                g.n_parts = max(1, min(pipelines, self.n_out_rows))
+                part = self.plan.partition(g.n_parts)
+            g.part_ptr = part.data_ptr()
             self.plan.ready_on_current_stream()
             for rec in _RECORDERS:
                 if not any(p is self.plan for p in rec):
                     rec.append(self.plan)
-        return g
+        return g, part_edge
+
+
+# Below this many receivers per pipeline the shares are cut between edges: a share of whole receivers is up to one receiver
+# longer than the mean (the whole kernel, when there are fewer receivers than pipelines), while a split costs the forward one
+# output row per pipeline written, read and added.  Beyond it the two are within noise of each other.
+SPLIT_ROWS_PER_PIPELINE = 32
 
 
 _META_CACHE: Dict[Tuple, Tuple[torch.Tensor, np.ndarray]] = {}
@@ -376,8 +395,13 @@ def _run_fwd(call: _Call, w, x, y) -> torch.Tensor:
     out = torch.empty((call.n_out_rows, call.out_segs * call.u), dtype=x.dtype, device=dev)
     mod = get_module(call.spec, "fwd", tuning=_tuning_for(call.spec, "fwd", (w, x, y, out)))
     with torch.cuda.device(dev):
-        g = call.graph(mod, dev)
-        mod.forward(g, w.data_ptr(), x.data_ptr(), y.data_ptr(), out.data_ptr(), torch.cuda.current_stream(dev).cuda_stream)
+        g, part_edge = call.graph(mod, dev)
+        stream = torch.cuda.current_stream(dev).cuda_stream
+        if part_edge is not None:
+            carry = torch.empty((g.n_parts, call.out_segs * call.u), dtype=x.dtype, device=dev)
+            mod.forward_split(g, part_edge, carry.data_ptr(), w.data_ptr(), x.data_ptr(), y.data_ptr(), out.data_ptr(), stream)
+        else:
+            mod.forward(g, w.data_ptr(), x.data_ptr(), y.data_ptr(), out.data_ptr(), stream)
     return out
 
 
@@ -389,9 +413,13 @@ def _run_bwd(call: _Call, grad_out, w, x, y, needs):
     mod = get_module(call.spec, "bwd", needs, tuning=_tuning_for(call.spec, "bwd", (grad_out, w, x, y, gw, gx, gy), needs))
     ptr = lambda t: t.data_ptr() if t is not None else None
     with torch.cuda.device(dev):
-        g = call.graph(mod, dev)
-        mod.backward(g, grad_out.data_ptr(), w.data_ptr(), x.data_ptr(), y.data_ptr(), ptr(gw), ptr(gx), ptr(gy),
-                     torch.cuda.current_stream(dev).cuda_stream)
+        g, part_edge = call.graph(mod, dev)
+        args = (grad_out.data_ptr(), w.data_ptr(), x.data_ptr(), y.data_ptr(), ptr(gw), ptr(gx), ptr(gy),
+                torch.cuda.current_stream(dev).cuda_stream)
+        if part_edge is not None:
+            mod.backward_split(g, part_edge, *args)
+        else:
+            mod.backward(g, *args)
     return gw, gx, gy
 
 

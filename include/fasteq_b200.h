@@ -84,6 +84,13 @@ int fasteq_u1d_describe(fasteq_u1d_desc* out /* host */);
 int fasteq_u1d_forward(const fasteq_u1d_graph* g /* host */, const void* w, const void* x, const void* y,
                        void* out, fasteq_stream_t stream);
 
+/* The same with receivers split: the shares of `g->part_ptr` begin and end at the edges `part_edge` [n_parts + 1]
+ * (fasteq_graph_partition_edges makes both), so that a graph of few or uneven receivers keeps every pipeline busy.  `carry` is
+ * scratch of n_parts * out_segs * u values for the sums of receivers that an earlier share began; a second launch adds them
+ * in a fixed order.  Scattered signatures only. */
+int fasteq_u1d_forward_split(const fasteq_u1d_graph* g /* host */, const int32_t* part_edge, void* carry, const void* w, const void* x,
+                             const void* y, void* out, fasteq_stream_t stream);
+
 /* Forward without any allocation (forward modules only).  No counterpart in the reference, whose
  * entry points allocate their outputs and leave scatter to atomics.  For callers that cannot
  * allocate device memory when they need the operator -- a plug-in of a simulation engine that
@@ -108,6 +115,10 @@ int fasteq_u1d_forward_noalloc(const int32_t* dst_sorted, const int32_t* x_index
  * shared, grad_y when u is tiled) are zero-filled by this call on `stream` before the kernel. */
 int fasteq_u1d_backward(const fasteq_u1d_graph* g /* host */, const void* grad_out, const void* w, const void* x,
                         const void* y, void* grad_w, void* grad_x, void* grad_y, fasteq_stream_t stream);
+
+/* The same over shares that begin and end at the edges `part_edge` (see fasteq_u1d_forward_split; no scratch). */
+int fasteq_u1d_backward_split(const fasteq_u1d_graph* g /* host */, const int32_t* part_edge, const void* grad_out, const void* w,
+                              const void* x, const void* y, void* grad_w, void* grad_x, void* grad_y, fasteq_stream_t stream);
 
 /* Reads and clears the device-side status word of this module (synchronises the device).
  * 0 = no fault; otherwise the code of the first fault (1 wait timeout, 2 index out of range). */
@@ -192,6 +203,10 @@ int fasteq_graph_build_csr(const int32_t* dst_sorted, int64_t n_edges, int64_t n
  * seg_ptr[s] + s >= p * (n_edges + n_rows) / n_parts, part_ptr[n_parts] = n_rows. */
 int fasteq_graph_partition(const int32_t* seg_ptr, int64_t n_rows, int64_t n_edges, int32_t n_parts,
                            int32_t* part_ptr, fasteq_stream_t stream);
+/* The same balance with shares cut between edges: share p begins at edge part_edge[p], which belongs to row part_ptr[p]
+ * (its first edge, or one inside it).  Both [n_parts + 1]. */
+int fasteq_graph_partition_edges(const int32_t* seg_ptr, int64_t n_rows, int64_t n_edges, int32_t n_parts, int32_t* part_ptr,
+                                 int32_t* part_edge, fasteq_stream_t stream);
 
 /* ------------------------------------------------------------------------- *
  * Periodic radius graph on the GPU (a neighbour of the hot path; the reference's callers bring edge
