@@ -518,19 +518,31 @@ fasteq_u1d_fwd_kernel(const Graph g, const T* __restrict__ w, const T* __restric
     src.append(_describe(spec, tun, 0, threads=threads))
     src.append(f"""
 // Receivers whose edges several pipelines shared: the pipeline that began one stored its sum, every later one left its own in
-// its carry row; they are added in pipeline order.  One CTA column per pipeline, working only where the first carry of a
-// receiver sits.
+// its carry row; they are added in pipeline order.  One CTA per pipeline, working where the first carry of a receiver sits.
+// Bound by latency (two dependent index loads, then the rows): the indices a CTA may need come in one go.
 __global__ void __launch_bounds__(256) fasteq_u1d_carry_kernel(const int* __restrict__ seg_ptr, const int* __restrict__ part_ptr,
-    const int* __restrict__ part_edge, int n_parts, long long n_out_rows, const T* __restrict__ carry, T* __restrict__ out) {{
-  const int p = blockIdx.x, row = part_ptr[p];
-  if (row >= n_out_rows || part_edge[p] <= seg_ptr[row]) return;                                   // starts at a receiver's first edge
-  if (p > 0 && part_ptr[p - 1] == row && part_edge[p - 1] > seg_ptr[row]) return;                  // an earlier pipeline is the first
-  const int i = blockIdx.y * 256 + threadIdx.x;
-  if (i >= OSEG * U) return;
-  T sum = out[(size_t)row * OSEG * U + i];
-  for (int q = p; q < n_parts && part_ptr[q] == row; ++q)
-    if (part_edge[q + 1] > part_edge[q]) sum += carry[(size_t)q * OSEG * U + i];
-  out[(size_t)row * OSEG * U + i] = sum;
+    const int* __restrict__ part_edge, int n_parts, int n_out_rows, const T* __restrict__ carry, T* __restrict__ out) {{
+  const int p = blockIdx.x, before = p > 0 ? p - 1 : 0;
+  const int row = part_ptr[p], row_before = part_ptr[before], row_after = part_ptr[p + 1];
+  const int edge = part_edge[p], edge_before = part_edge[before], edge_after = part_edge[p + 1];
+  if (row >= n_out_rows) return;
+  const int first = seg_ptr[row];
+  if (edge <= first) return;                                                     // starts at a receiver's first edge
+  if (p > 0 && row_before == row && edge_before > first) return;                 // an earlier pipeline holds the first carry
+  T* o = out + (size_t)row * OSEG * U;
+  const T* c = carry + (size_t)p * OSEG * U;
+  if (row_after != row) {{                                                        // the usual case: one carry
+#pragma unroll 4
+    for (int i = threadIdx.x * VEC; i < OSEG * U; i += 256 * VEC) VS::st(o + i, vadd(VS::ld(o + i), VS::ld(c + i)));
+    return;
+  }}
+  for (int i = threadIdx.x * VEC; i < OSEG * U; i += 256 * VEC) {{
+    V sum = VS::ld(o + i);
+    if (edge_after > edge) sum = vadd(sum, VS::ld(c + i));
+    for (int q = p + 1; q < n_parts && part_ptr[q] == row; ++q)
+      if (part_edge[q + 1] > part_edge[q]) sum = vadd(sum, VS::ld(carry + (size_t)q * OSEG * U + i));
+    VS::st(o + i, sum);
+  }}
 }}
 
 static int run_forward(const fasteq_u1d_graph* gh, const int32_t* part_edge, void* carry, const void* w, const void* x, const void* y,
@@ -548,8 +560,8 @@ static int run_forward(const fasteq_u1d_graph* gh, const int32_t* part_edge, voi
   fasteq_u1d_fwd_kernel<<<grid, NTHREADS, SMEM_BYTES, (cudaStream_t)stream>>>(
       g, (const T*)w, (const T*)x, (const T*)y, (T*)out, (T*)carry);
   if (part_edge)
-    fasteq_u1d_carry_kernel<<<dim3((unsigned)gh->n_parts, (OSEG * U + 255) / 256), 256, 0, (cudaStream_t)stream>>>(
-        gh->seg_ptr, gh->part_ptr, part_edge, gh->n_parts, gh->n_out_rows, (const T*)carry, (T*)out);
+    fasteq_u1d_carry_kernel<<<(unsigned)gh->n_parts, 256, 0, (cudaStream_t)stream>>>(
+        gh->seg_ptr, gh->part_ptr, part_edge, gh->n_parts, (int)gh->n_out_rows, (const T*)carry, (T*)out);
   e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e);
   return FASTEQ_OK;
