@@ -1,9 +1,12 @@
 """ctypes bindings for the C ABI declared in include/fasteq_b200.h."""
 from __future__ import annotations
 
+import contextlib
 import ctypes as C
 import os
 from typing import Dict, Optional
+
+import torch
 
 from . import _build
 
@@ -25,6 +28,20 @@ class U1DGraph(C.Structure):
     _fields_ = [("n_edges", C.c_int64), ("n_out_rows", C.c_int64), ("x_rows", C.c_int64), ("y_rows", C.c_int64),
                 ("x_index", C.c_void_p), ("y_index", C.c_void_p), ("seg_ptr", C.c_void_p), ("perm", C.c_void_p),
                 ("part_ptr", C.c_void_p), ("n_parts", C.c_int32)]
+
+
+_NOTHING = contextlib.nullcontext()
+
+
+def on_device(dev: torch.device):
+    """Context in which a tensor's device is the current one: nothing to do when it is already, which is the usual case and
+    saves ``torch.cuda.device`` its three device-index conversions."""
+    return _NOTHING if dev.index == torch._C._cuda_getDevice() else torch.cuda.device(dev)
+
+
+def stream(dev: torch.device) -> int:
+    """Handle of torch's current stream on a tensor's device, without the Stream object around it."""
+    return torch._C._cuda_getCurrentRawStream(dev.index)
 
 
 def check(rc: int, lib=None, what: str = "") -> None:

@@ -31,6 +31,14 @@ class STCSpec:
     u: int
     dtype: str = "f32"
 
+    def __hash__(self) -> int:
+        # hashed once per object: the specification keys the module cache on every call and holds hundreds of paths
+        h = self.__dict__.get("_hash")
+        if h is None:
+            h = hash((self.paths, self.x1_segs, self.x0_segs, self.out_segs, self.u, self.dtype))
+            object.__setattr__(self, "_hash", h)
+        return h
+
     @property
     def ctype(self) -> str:
         return "float" if self.dtype == "f32" else "double"

@@ -64,8 +64,8 @@ def radius_graph(pos: torch.Tensor, atom_struct: torch.Tensor, box, cutoff: floa
     work = torch.empty(int(nbytes.value), dtype=torch.uint8, device=dev)
     seg_ptr = torch.empty(N + 1, dtype=torch.int32, device=dev)
     head = torch.zeros(1, dtype=torch.int32, device=dev)
-    with torch.cuda.device(dev):
-        stream = torch.cuda.current_stream(dev).cuda_stream
+    with _cabi.on_device(dev):
+        stream = _cabi.stream(dev)
         _cabi.check(lib.fasteq_neighbors_count(C.byref(prob), work.data_ptr(), nbytes.value, seg_ptr.data_ptr(), head.data_ptr(), stream),
                     lib, "fasteq_neighbors_count")
         n_edges, max_deg = (int(v) for v in torch.stack([seg_ptr[N], head[0]]).tolist())

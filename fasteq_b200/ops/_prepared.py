@@ -17,6 +17,8 @@ from typing import Callable, Optional, Sequence, Tuple
 
 import torch
 
+from .. import _cabi
+
 # key -> (weights kept alive, prepared tensor, event recorded after the build, ids of the streams ordered behind it)
 _CACHE: "OrderedDict[Tuple, Tuple[tuple, torch.Tensor, torch.cuda.Event, set]]" = OrderedDict()
 _BYTES = [0]
@@ -65,8 +67,8 @@ def get(weights: Sequence[torch.Tensor], tag: Tuple, build: Callable[[], Optiona
         _CACHE.move_to_end(key)
         val = hit[1]
         if not capturing:
-            cur = torch.cuda.current_stream(val.device)
-            if cur.cuda_stream not in hit[3]:
+            if _cabi.stream(val.device) not in hit[3]:
+                cur = torch.cuda.current_stream(val.device)
                 cur.wait_event(hit[2])
                 val.record_stream(cur)
                 hit[3].add(cur.cuda_stream)

@@ -52,8 +52,8 @@ def _fma_problem(M: int, K: int, N: int, dtype):
 def _fma_call(name: str, prob, p0, p1, out) -> None:
     from .eqlinear import _core
     lib = _core()
-    with torch.cuda.device(out.device):
-        rc = getattr(lib, name)(C.byref(prob), p0.data_ptr(), p1.data_ptr(), out.data_ptr(), torch.cuda.current_stream(out.device).cuda_stream)
+    with _cabi.on_device(out.device):
+        rc = getattr(lib, name)(C.byref(prob), p0.data_ptr(), p1.data_ptr(), out.data_ptr(), _cabi.stream(out.device))
     _cabi.check(rc, lib, name)
 
 
@@ -109,8 +109,8 @@ def _gemm(a: torch.Tensor, bt: torch.Tensor, weight: torch.Tensor = None, transp
     N = bt.shape[0]
     out = torch.empty((M, N), dtype=a.dtype, device=a.device)
     lib = _lib()
-    with torch.cuda.device(a.device):
-        stream = torch.cuda.current_stream(a.device).cuda_stream
+    with _cabi.on_device(a.device):
+        stream = _cabi.stream(a.device)
         split = None
         if weight is not None:
             def build():

@@ -39,9 +39,9 @@ class _EdgeGeometry(torch.autograd.Function):
         basis = torch.empty((E, n_basis), dtype=pos.dtype, device=pos.device)
         code = 0 if pos.dtype == torch.float32 else 1
         lib = _lib()
-        with torch.cuda.device(pos.device):
+        with _cabi.on_device(pos.device):
             rc = lib.fasteq_edge_geometry_forward(code, pos.data_ptr(), src.data_ptr(), dst.data_ptr(), shift.data_ptr(), E, pos.shape[0], float(r_max),
-                                                  n_basis, p, vec.data_ptr(), basis.data_ptr(), torch.cuda.current_stream(pos.device).cuda_stream)
+                                                  n_basis, p, vec.data_ptr(), basis.data_ptr(), _cabi.stream(pos.device))
         _cabi.check(rc, lib, "fasteq_edge_geometry_forward")
         ctx.save_for_backward(pos, src, dst, shift)
         ctx.cfg = (float(r_max), n_basis, p, code)
@@ -60,10 +60,10 @@ class _EdgeGeometry(torch.autograd.Function):
         g_pos = torch.empty_like(pos)
         lib = _lib()
         ptr = lambda t: t.data_ptr() if t is not None else None
-        with torch.cuda.device(pos.device):
+        with _cabi.on_device(pos.device):
             rc = lib.fasteq_edge_geometry_backward(code, pos.data_ptr(), src.data_ptr(), dst.data_ptr(), shift.data_ptr(), ptr(gv), ptr(gb),
                                                    src.numel(), pos.shape[0], r_max, n_basis, p, g_pos.data_ptr(),
-                                                   torch.cuda.current_stream(pos.device).cuda_stream)
+                                                   _cabi.stream(pos.device))
         _cabi.check(rc, lib, "fasteq_edge_geometry_backward")
         return g_pos, None, None, None, None, None, None
 

@@ -210,18 +210,18 @@ class _Plan:
         mapping, coeff, u, v, I, J = self.geom
         x3 = x.reshape(self.batch, I, u).contiguous()
         out = torch.empty((self.batch, J, v), dtype=x.dtype, device=x.device)
-        with torch.cuda.device(x.device):
+        with _cabi.on_device(x.device):
             _run(_core(), self._problem(), w, self._w3(w), x3, out, self.key, self.precision, False,
-                 torch.cuda.current_stream(x.device).cuda_stream)
+                 _cabi.stream(x.device))
         return out.reshape(self.batch, J * v)
 
     def dgrad(self, w, g):
         mapping, coeff, u, v, I, J = self.geom
         g3 = g.reshape(self.batch, J, v).contiguous()
         dx = torch.empty((self.batch, I, u), dtype=g3.dtype, device=g3.device)
-        with torch.cuda.device(g3.device):
+        with _cabi.on_device(g3.device):
             _run(_core(), self._problem(), w, self._w3(w), g3, dx, self.key, self.precision, True,
-                 torch.cuda.current_stream(g3.device).cuda_stream)
+                 _cabi.stream(g3.device))
         return dx.reshape(self.batch, I * u)
 
     def wgrad(self, x, g):
@@ -230,9 +230,9 @@ class _Plan:
         g3 = g.reshape(self.batch, J, v).contiguous()
         dw = torch.empty((len(mapping), u, v), dtype=g3.dtype, device=g3.device)
         lib = _core()
-        with torch.cuda.device(g3.device):
+        with _cabi.on_device(g3.device):
             _cabi.check(lib.fasteq_eqlinear_wgrad(C.byref(self._problem()), x3.data_ptr(), g3.data_ptr(), dw.data_ptr(),
-                                                  torch.cuda.current_stream(g3.device).cuda_stream), lib, "fasteq_eqlinear_wgrad")
+                                                  _cabi.stream(g3.device)), lib, "fasteq_eqlinear_wgrad")
         wps = [m[2] for m in mapping]
         if wps != list(range(len(wps))):      # block q of the table is block wps[q] of the caller's tensor
             full = torch.empty_like(dw)

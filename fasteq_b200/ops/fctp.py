@@ -119,8 +119,8 @@ class FastFullyConnectedTensorProductPathFused(torch.autograd.Function):
         outs = torch.empty((B, K, W), dtype=x.dtype, device=x.device)
         lib = _core()
         ws, start = {}, 0
-        with torch.cuda.device(x.device):
-            stream = torch.cuda.current_stream(x.device).cuda_stream
+        with _cabi.on_device(x.device):
+            stream = _cabi.stream(x.device)
             for s, n in enumerate(counts):
                 if n == 0:
                     continue
@@ -149,8 +149,8 @@ class FastFullyConnectedTensorProductPathFused(torch.autograd.Function):
         gxs = torch.empty((B, I, U), dtype=gs.dtype, device=gs.device) if need_x else None
         gw4 = torch.zeros((P, U, V, W), dtype=gs.dtype, device=gs.device) if need_w else None
         start, wi = 0, 0
-        with torch.cuda.device(gs.device):
-            stream = torch.cuda.current_stream(gs.device).cuda_stream
+        with _cabi.on_device(gs.device):
+            stream = _cabi.stream(gs.device)
             for s, n in enumerate(counts):
                 if n == 0:
                     continue

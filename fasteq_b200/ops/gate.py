@@ -79,8 +79,8 @@ class _Gate(torch.autograd.Function):
         out = torch.empty((B, spec.n_out * spec.u), dtype=x.dtype, device=x.device)
         lib = _lib()
         prob = spec.problem(B, x.dtype)
-        with torch.cuda.device(x.device):
-            _cabi.check(lib.fasteq_gate_forward(C.byref(prob), xc.data_ptr(), out.data_ptr(), torch.cuda.current_stream(x.device).cuda_stream),
+        with _cabi.on_device(x.device):
+            _cabi.check(lib.fasteq_gate_forward(C.byref(prob), xc.data_ptr(), out.data_ptr(), _cabi.stream(x.device)),
                         lib, "fasteq_gate_forward")
         ctx.save_for_backward(x)       # the input itself, so that a second backward reaches it
         ctx.spec = spec
@@ -101,9 +101,9 @@ class _GateBackward(torch.autograd.Function):
         B = xc.numel() // (spec.n_in * spec.u)
         lib = _lib()
         prob = spec.problem(B, xc.dtype)
-        with torch.cuda.device(xc.device):
+        with _cabi.on_device(xc.device):
             _cabi.check(lib.fasteq_gate_backward(C.byref(prob), xc.data_ptr(), go.data_ptr(), gx.data_ptr(),
-                                                 torch.cuda.current_stream(xc.device).cuda_stream), lib, "fasteq_gate_backward")
+                                                 _cabi.stream(xc.device)), lib, "fasteq_gate_backward")
         ctx.save_for_backward(go, xc)
         ctx.spec = spec
         return gx
@@ -118,9 +118,9 @@ class _GateBackward(torch.autograd.Function):
         B = xc.numel() // (spec.n_in * spec.u)
         lib = _lib()
         prob = spec.problem(B, xc.dtype)
-        with torch.cuda.device(xc.device):
+        with _cabi.on_device(xc.device):
             _cabi.check(lib.fasteq_gate_double_backward(C.byref(prob), xc.data_ptr(), go.data_ptr(), t.data_ptr(), d_go.data_ptr(),
-                                                        d_x.data_ptr(), torch.cuda.current_stream(xc.device).cuda_stream),
+                                                        d_x.data_ptr(), _cabi.stream(xc.device)),
                         lib, "fasteq_gate_double_backward")
         return d_go, d_x, None
 

@@ -64,8 +64,8 @@ class _RadialChain(torch.autograd.Function):
         out = torch.empty((E, WIDTH), dtype=torch.float32, device=basis.device)
         deriv = torch.empty((max(n_hidden - 1, 1), E, WIDTH), dtype=torch.float32, device=basis.device)
         lib = _lib()
-        with torch.cuda.device(basis.device):
-            stream = torch.cuda.current_stream(basis.device).cuda_stream
+        with _cabi.on_device(basis.device):
+            stream = _cabi.stream(basis.device)
             prep = _prepared_hidden(ws, False, lib, stream)
             rc = lib.fasteq_radial_chain_forward(basis.data_ptr(), E, nb, ws[0].data_ptr(), _hidden_array(ws[1:]),
                                                  prep.data_ptr() if prep is not None else None, n_hidden,
@@ -83,8 +83,8 @@ class _RadialChain(torch.autograd.Function):
         g = grad_out.contiguous()
         gb = torch.empty((E, nb), dtype=torch.float32, device=basis.device)
         lib = _lib()
-        with torch.cuda.device(basis.device):
-            stream = torch.cuda.current_stream(basis.device).cuda_stream
+        with _cabi.on_device(basis.device):
+            stream = _cabi.stream(basis.device)
             prep = _prepared_hidden(ws, True, lib, stream)
             rc = lib.fasteq_radial_chain_backward(g.data_ptr(), deriv.data_ptr(), basis.data_ptr(), E, nb, ws[0].data_ptr(),
                                                   _hidden_array(ws[1:]), prep.data_ptr() if prep is not None else None, len(ws),

@@ -49,8 +49,8 @@ class _SH(torch.autograd.Function):
         nout = sum(2 * l + 1 for l in ls)
         out = torch.empty((n, nout), dtype=x.dtype, device=x.device)
         lib = _module(ls, x.dtype, normalize, normalization)
-        with torch.cuda.device(x.device):
-            _cabi.check(lib.fasteq_sh_forward(flat.data_ptr(), n, out.data_ptr(), torch.cuda.current_stream(x.device).cuda_stream),
+        with _cabi.on_device(x.device):
+            _cabi.check(lib.fasteq_sh_forward(flat.data_ptr(), n, out.data_ptr(), _cabi.stream(x.device)),
                         lib, "fasteq_sh_forward")
         ctx.save_for_backward(x)       # the input itself: a view made here would be cut off from its autograd history
         ctx.cfg = (ls, normalize, normalization, x.shape)
@@ -72,9 +72,9 @@ class _SHBackward(torch.autograd.Function):
     def forward(ctx, g, flat, ls, normalize, normalization):
         gv = torch.empty_like(flat)
         lib = _module(ls, flat.dtype, normalize, normalization)
-        with torch.cuda.device(flat.device):
+        with _cabi.on_device(flat.device):
             _cabi.check(lib.fasteq_sh_backward(flat.data_ptr(), g.data_ptr(), flat.shape[0], gv.data_ptr(),
-                                               torch.cuda.current_stream(flat.device).cuda_stream), lib, "fasteq_sh_backward")
+                                               _cabi.stream(flat.device)), lib, "fasteq_sh_backward")
         ctx.save_for_backward(g, flat)
         ctx.cfg = (ls, normalize, normalization)
         return gv
@@ -87,9 +87,9 @@ class _SHBackward(torch.autograd.Function):
         t = ggv.reshape(flat.shape).contiguous()
         d_g, d_v = torch.empty_like(g), torch.empty_like(flat)
         lib = _module(ls, flat.dtype, normalize, normalization)
-        with torch.cuda.device(flat.device):
+        with _cabi.on_device(flat.device):
             _cabi.check(lib.fasteq_sh_double_backward(flat.data_ptr(), g.data_ptr(), t.data_ptr(), flat.shape[0], d_g.data_ptr(),
-                                                      d_v.data_ptr(), torch.cuda.current_stream(flat.device).cuda_stream),
+                                                      d_v.data_ptr(), _cabi.stream(flat.device)),
                         lib, "fasteq_sh_double_backward")
         return d_g, d_v, None, None, None
 

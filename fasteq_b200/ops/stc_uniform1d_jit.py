@@ -124,9 +124,9 @@ class FastSymmetricTensorContractionUniform1dFunction(torch.autograd.Function):
         B = x1c.shape[0]
         out = torch.empty((B, spec.out_segs, spec.u), dtype=x1.dtype, device=x1.device)
         mod = get_module(spec, "fwd", operands=(x1c, x0c))
-        with torch.cuda.device(x1.device):
+        with _cabi.on_device(x1.device):
             _cabi.check(mod.lib.fasteq_stc_forward(x1c.data_ptr(), x0c.data_ptr(), i32.data_ptr(), B, x0c.shape[0], out.data_ptr(),
-                                                   torch.cuda.current_stream(x1.device).cuda_stream), mod.lib, "fasteq_stc_forward")
+                                                   _cabi.stream(x1.device)), mod.lib, "fasteq_stc_forward")
         ctx.save_for_backward(x1, x0, i32)      # the inputs themselves, so that a second backward reaches them
         ctx.spec = spec
         return out.view(B, spec.out_segs * spec.u)
@@ -155,14 +155,14 @@ def _backward_summed(go, x1, x0, i32, spec):
     B, S = x1.shape[0], x0.shape[0]
     gx1, gx0 = torch.empty_like(x1), torch.empty_like(x0)
     lib = get_module(spec, "bwdsum", True, (go, x1, x0)).lib
-    with torch.cuda.device(x1.device):
+    with _cabi.on_device(x1.device):
         parts = C.c_int32(0)
         _cabi.check(lib.fasteq_stc_backward_summed_parts(B, C.byref(parts)), lib, "fasteq_stc_backward_summed_parts")
         species, order = torch.sort(i32.view(-1), stable=True)
         partial = torch.empty((parts.value + S, spec.x0_segs, spec.u), dtype=x1.dtype, device=x1.device)
         _cabi.check(lib.fasteq_stc_backward_summed(go.data_ptr(), x1.data_ptr(), x0.data_ptr(), order.data_ptr(), species.data_ptr(),
                                                    B, S, parts.value, partial.data_ptr(), gx1.data_ptr(), gx0.data_ptr(),
-                                                   torch.cuda.current_stream(x1.device).cuda_stream), lib, "fasteq_stc_backward_summed")
+                                                   _cabi.stream(x1.device)), lib, "fasteq_stc_backward_summed")
     return gx1, gx0
 
 
@@ -176,10 +176,10 @@ class FastSTCBackwardFunction(torch.autograd.Function):
         gx1 = torch.empty_like(x1)
         gx0n = torch.empty((B, spec.x0_segs, spec.u), dtype=x1.dtype, device=x1.device) if need_x0 else None
         mod = get_module(spec, "bwd", bool(need_x0), (go, x1, x0))
-        with torch.cuda.device(x1.device):
+        with _cabi.on_device(x1.device):
             _cabi.check(mod.lib.fasteq_stc_backward(go.data_ptr(), x1.data_ptr(), x0.data_ptr(), i32.data_ptr(), B, x0.shape[0],
                                                     gx1.data_ptr(), gx0n.data_ptr() if need_x0 else None,
-                                                    torch.cuda.current_stream(x1.device).cuda_stream), mod.lib, "fasteq_stc_backward")
+                                                    _cabi.stream(x1.device)), mod.lib, "fasteq_stc_backward")
         ctx.save_for_backward(go, x1, x0, i32)
         ctx.spec, ctx.need_x0 = spec, need_x0
         return gx1, (gx0n if need_x0 else x1.new_empty((0,)))
@@ -199,10 +199,10 @@ class FastSTCBackwardFunction(torch.autograd.Function):
         d_x1 = torch.empty_like(x1)
         d_x0n = torch.empty((B, spec.x0_segs, spec.u), dtype=x1.dtype, device=x1.device)
         mod = get_module(spec, "dbwd")
-        with torch.cuda.device(x1.device):
+        with _cabi.on_device(x1.device):
             _cabi.check(mod.lib.fasteq_stc_double_backward(go.data_ptr(), x1.data_ptr(), x0.data_ptr(), i32.data_ptr(), ggx1.data_ptr(),
                                                            ggx0n.data_ptr(), B, x0.shape[0], d_go.data_ptr(), d_x1.data_ptr(),
-                                                           d_x0n.data_ptr(), torch.cuda.current_stream(x1.device).cuda_stream),
+                                                           d_x0n.data_ptr(), _cabi.stream(x1.device)),
                         mod.lib, "fasteq_stc_double_backward")
         want = ctx.needs_input_grad
         d_x0 = torch.zeros_like(x0).index_add_(0, i32.long(), d_x0n) if want[2] else None

@@ -91,10 +91,10 @@ class GraphPlan:
                 raise ValueError("seg_ptr must be an int32 tensor of n_rows + 1 offsets on the index's device")
             self.sorted, self.perm, self.seg_ptr = True, None, seg_ptr.contiguous()
             return
-        stream = torch.cuda.current_stream(dev).cuda_stream
+        stream = _cabi.stream(dev)
         dst32 = dst.to(torch.int32).contiguous()
         flag = torch.empty(1, dtype=torch.int32, device=dev)
-        with torch.cuda.device(dev):
+        with _cabi.on_device(dev):
             _cabi.check(core.fasteq_graph_check_sorted(dst32.data_ptr(), self.n_edges, flag.data_ptr(), stream), core,
                         "fasteq_graph_check_sorted")
             self.sorted = bool(flag.item())
@@ -123,9 +123,9 @@ class GraphPlan:
         """Order the current stream behind the kernels that built this plan on other streams."""
         if not self._ready or torch.cuda.is_current_stream_capturing():
             return
-        cur = torch.cuda.current_stream(self.device)
-        if cur.cuda_stream in self._waited:
+        if _cabi.stream(self.device) in self._waited:
             return
+        cur = torch.cuda.current_stream(self.device)
         foreign = False
         for sid, ev in self._ready:
             if sid != cur.cuda_stream:
@@ -146,8 +146,8 @@ class GraphPlan:
         if p is None:
             core = _cabi.core()
             p = torch.empty((2 if split else 1, n_parts + 1), dtype=torch.int32, device=self.device)
-            with torch.cuda.device(self.device):
-                stream = torch.cuda.current_stream(self.device).cuda_stream
+            with _cabi.on_device(self.device):
+                stream = _cabi.stream(self.device)
                 if split:
                     _cabi.check(core.fasteq_graph_partition_edges(self.seg_ptr.data_ptr(), self.n_rows, self.n_edges, n_parts, p[0].data_ptr(),
                                                                   p[1].data_ptr(), stream), core, "fasteq_graph_partition_edges")
@@ -394,9 +394,9 @@ def _run_fwd(call: _Call, w, x, y) -> torch.Tensor:
     dev = x.device
     out = torch.empty((call.n_out_rows, call.out_segs * call.u), dtype=x.dtype, device=dev)
     mod = get_module(call.spec, "fwd", tuning=_tuning_for(call.spec, "fwd", (w, x, y, out)))
-    with torch.cuda.device(dev):
+    with _cabi.on_device(dev):
         g, part_edge = call.graph(mod, dev)
-        stream = torch.cuda.current_stream(dev).cuda_stream
+        stream = _cabi.stream(dev)
         if part_edge is not None:
             carry = torch.empty((g.n_parts, call.out_segs * call.u), dtype=x.dtype, device=dev)
             mod.forward_split(g, part_edge, carry.data_ptr(), w.data_ptr(), x.data_ptr(), y.data_ptr(), out.data_ptr(), stream)
@@ -412,10 +412,10 @@ def _run_bwd(call: _Call, grad_out, w, x, y, needs):
     gy = torch.empty_like(y) if needs[2] else None
     mod = get_module(call.spec, "bwd", needs, tuning=_tuning_for(call.spec, "bwd", (grad_out, w, x, y, gw, gx, gy), needs))
     ptr = lambda t: t.data_ptr() if t is not None else None
-    with torch.cuda.device(dev):
+    with _cabi.on_device(dev):
         g, part_edge = call.graph(mod, dev)
         args = (grad_out.data_ptr(), w.data_ptr(), x.data_ptr(), y.data_ptr(), ptr(gw), ptr(gx), ptr(gy),
-                torch.cuda.current_stream(dev).cuda_stream)
+                _cabi.stream(dev))
         if part_edge is not None:
             mod.backward_split(g, part_edge, *args)
         else:
