@@ -17,6 +17,7 @@ import torch
 
 from .. import _cabi
 from . import _prepared
+from ._needs import wanted
 
 _ready = False
 
@@ -139,7 +140,7 @@ class _Dense(torch.autograd.Function):
     @staticmethod
     def backward(ctx, grad_out):
         x, weight = ctx.saved_tensors
-        need_x, need_w = ctx.needs_input_grad
+        need_x, need_w = ctx.needs_input_grad[0], wanted(ctx, 1)
         if not (need_x or need_w):
             return None, None
         gx, gw = _DenseBackward.apply(grad_out.contiguous(), x, weight, need_x, need_w)

@@ -19,6 +19,7 @@ import torch
 
 from .. import _cabi
 from . import _prepared
+from ._needs import wanted
 
 __all__ = ["fast_equi_linear", "eqlinear_clear_plan_cache", "eqlinear_set_plan_cache", "eqlinear_debug_info"]
 
@@ -254,7 +255,7 @@ class _EqLinearFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, grad_out):
         w, x = ctx.saved_tensors
-        need_w, need_x = ctx.needs_input_grad[0], ctx.needs_input_grad[1]
+        need_w, need_x = wanted(ctx, 0), ctx.needs_input_grad[1]
         if not (need_w or need_x):
             return None, None, None, None
         dw, dx = _EqLinearBackwardFn.apply(grad_out.contiguous(), w, x, ctx.plan, need_w, need_x)

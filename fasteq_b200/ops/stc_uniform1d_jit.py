@@ -18,6 +18,7 @@ import torch
 
 from .. import _build, _cabi
 from ..codegen import stc as _emit
+from ._needs import wanted
 
 STC_PAD_VALUE = -1
 _EMITTER_VERSION = "stc-v4"
@@ -135,7 +136,7 @@ class FastSymmetricTensorContractionUniform1dFunction(torch.autograd.Function):
     def backward(ctx, grad_out):
         x1, x0, i32 = ctx.saved_tensors
         spec = ctx.spec
-        need_x1, need_x0 = ctx.needs_input_grad[0], ctx.needs_input_grad[1]
+        need_x1, need_x0 = ctx.needs_input_grad[0], wanted(ctx, 1)
         if not (need_x1 or need_x0):
             return (None,) * 8
         if need_x0 and not torch.is_grad_enabled():
