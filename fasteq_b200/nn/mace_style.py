@@ -22,6 +22,7 @@ from ..irreps import Irreps
 from ..ops.dense import dense
 from ..ops.edge_geometry import edge_geometry, edge_geometry_usable
 from ..ops.radial_chain import radial_chain
+from ..ops.silu import silu
 from ..ops.spherical_harmonics import SphericalHarmonics
 from .modules import ChannelwiseTensorProduct, SO3Linear, SymmetricContraction
 
@@ -53,7 +54,7 @@ class RadialMLP(torch.nn.Module):
         for i, lin in enumerate(self.layers):
             x = dense(x, lin.weight)
             if i + 1 < len(self.layers):
-                x = torch.nn.functional.silu(x)
+                x = silu(x)
         return x
 
 
@@ -125,7 +126,8 @@ class MACEStyleModel(torch.nn.Module):
         if self.fuse_geometry and not second_order and edge_geometry_usable(pos, self.num_basis):
             vec, radial = edge_geometry(pos, edge_src, edge_dst, edge_shift, self.r_max, self.num_basis, self.envelope_p)
         else:
-            vec = pos[edge_src] + edge_shift - pos[edge_dst]
+            # index_select: its gradient is one scatter launch, that of advanced indexing sorts the index first
+            vec = pos.index_select(0, edge_src) + edge_shift - pos.index_select(0, edge_dst)
             r = vec.norm(dim=-1)
             radial = bessel_basis(r, self.r_max, self.num_basis) * polynomial_cutoff(r, self.r_max, self.envelope_p).unsqueeze(-1)
         if self.fuse_sh and not second_order and vec.is_cuda:
@@ -137,7 +139,7 @@ class MACEStyleModel(torch.nn.Module):
         ``species`` then hold the owned nodes only and the edge indices are local ids."""
         pos_ext = pos if halo is None else halo(pos)
         edge_sh, edge_radial, edge_vec = self.edge_features(pos_ext, edge_src, edge_dst, edge_shift, second_order)
-        h = self.embedding[species]
+        h = self.embedding.index_select(0, species)
         e = pos.new_zeros(pos.shape[0])
         for layer, ro in zip(self.layers, self.readouts):
             h = layer(h, species, edge_sh, edge_radial, edge_dst, edge_src, halo, edge_vec)

@@ -400,6 +400,11 @@ int fasteq_edge_geometry_device_status(int32_t* code /* host */);
 /* Reads and clears the status word of the tensor-core kernels (synchronises). */
 int fasteq_tensorcore_device_status(int32_t* code /* host */);
 
+/* SiLU and its derivatives over n values (dtype 0 FP32, 1 FP64): order 0 out0 = silu(z); order 1 out0 = g silu'(z); order 2, for a
+ * cotangent h of that product, out0 = h silu'(z) and out1 = h g silu''(z).  Unused operands may be NULL. */
+int fasteq_silu(int32_t dtype, int32_t order, const void* z, const void* g, const void* h, void* out0, void* out1, int64_t n,
+                fasteq_stream_t stream);
+
 #ifdef __cplusplus
 }
 #endif
