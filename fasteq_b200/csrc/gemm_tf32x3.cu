@@ -57,14 +57,27 @@ struct Tile {
   long long m0;
 };
 
-__device__ __forceinline__ Tile decode_tile(const TcTable& tab, long long tile, int m_tiles, int n_tiles, int kb_per_seg, int BN) {
+// Every role of the CTA decodes every tile, in line with its other work: a short tile (K = 64: two k-blocks) spent more on three
+// 64-bit divisions and a walk over up to 64 groups than on its MMAs.  Hence 32-bit divisions where the tile count allows
+// and a shared-memory table from item to group (`item_g`, null when there are more items than it holds).
+constexpr int ITEM_TABLE = 768;
+
+__device__ __forceinline__ Tile decode_tile(const TcTable& tab, const unsigned char* item_g, long long tile, int m_tiles, int n_tiles,
+                                            int kb_per_seg, int BN) {
   Tile r;
-  const int mx = (int)(tile % m_tiles);
-  const long long rest = tile / m_tiles;
-  const int ny = (int)(rest % n_tiles);
-  const int z = (int)(rest / n_tiles);
+  int mx, ny, z;
+  if (tile <= 0xffffffffLL) {
+    const unsigned t32 = (unsigned)tile, rest = t32 / (unsigned)m_tiles;
+    mx = (int)(t32 - rest * (unsigned)m_tiles);
+    z = (int)(rest / (unsigned)n_tiles);
+    ny = (int)(rest - (unsigned)z * (unsigned)n_tiles);
+  } else {
+    const long long rest = tile / m_tiles;
+    mx = (int)(tile % m_tiles); ny = (int)(rest % n_tiles); z = (int)(rest / n_tiles);
+  }
   int g = 0;
-  while (g + 1 < tab.n_groups && z >= tab.item_first[g + 1]) ++g;
+  if (item_g) g = item_g[z];
+  else while (g + 1 < tab.n_groups && z >= tab.item_first[g + 1]) ++g;
   r.g = g; r.t = z - tab.item_first[g];
   r.seg0 = tab.group_first[g];
   r.n_kb = (tab.group_first[g + 1] - r.seg0) * kb_per_seg;
@@ -98,6 +111,15 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
   uint64_t* acc_empty = acc_full + 2;        // [2] accumulator read back by the four epilogue warps
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
 
+  unsigned char* item_table = reinterpret_cast<unsigned char*>(bars) + 1024 - ITEM_TABLE;   // behind the barriers
+  const unsigned char* item_g = tab.n_items <= ITEM_TABLE ? item_table : nullptr;
+  if (item_g) {
+    for (int z = threadIdx.x; z < tab.n_items; z += NT_P) {
+      int g = 0;
+      while (g + 1 < tab.n_groups && z >= tab.item_first[g + 1]) ++g;
+      item_table[z] = (unsigned char)g;
+    }
+  }
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int kb_per_seg = (K + BK - 1) / BK;
 
@@ -121,7 +143,7 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
     if (lane == 0) {
       int it = 0;
       for (long long tile = blockIdx.x; tile < n_tiles_total; tile += gridDim.x) {
-        const Tile tl = decode_tile(tab, tile, m_tiles, n_tiles, kb_per_seg, BN);
+        const Tile tl = decode_tile(tab, item_g, tile, m_tiles, n_tiles, kb_per_seg, BN);
         // each tile starts its walk over the k-blocks at a different one, so that the CTAs do not all fetch the same
         // weight lines from L2 at the same moment (the terms of a sum are the same, their order depends on the tile)
         const int kb_start = (int)(tile % tl.n_kb);
@@ -148,7 +170,7 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
       int it = 0;
       uint32_t lt = 0;
       for (long long tile = blockIdx.x; tile < n_tiles_total; tile += gridDim.x, ++lt) {
-        const Tile tl = decode_tile(tab, tile, m_tiles, n_tiles, kb_per_seg, BN);
+        const Tile tl = decode_tile(tab, item_g, tile, m_tiles, n_tiles, kb_per_seg, BN);
         const uint32_t buf = lt & 1u;
         mbar_wait(&acc_empty[buf], ((lt >> 1) & 1u) ^ 1u, status);
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -184,7 +206,7 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
     const int tid = threadIdx.x - 64;     // 0..127
     int it = 0;
     for (long long tile = blockIdx.x; tile < n_tiles_total; tile += gridDim.x) {
-      const Tile tl = decode_tile(tab, tile, m_tiles, n_tiles, kb_per_seg, BN);
+      const Tile tl = decode_tile(tab, item_g, tile, m_tiles, n_tiles, kb_per_seg, BN);
       for (int kb = 0; kb < tl.n_kb; ++kb, ++it) {
         const int s = it % STAGES;
         mbar_wait(&full_raw[s], (it / STAGES) & 1u, status);
@@ -234,7 +256,7 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
     uint32_t lt = 0;
     int chunk_no = 0;
     for (long long tile = blockIdx.x; tile < n_tiles_total; tile += gridDim.x, ++lt) {
-      const Tile tl = decode_tile(tab, tile, m_tiles, n_tiles, kb_per_seg, BN);
+      const Tile tl = decode_tile(tab, item_g, tile, m_tiles, n_tiles, kb_per_seg, BN);
       const uint32_t buf = lt & 1u;
       mbar_wait(&acc_full[buf], (lt >> 1) & 1u, status);
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
