@@ -524,7 +524,7 @@ __global__ void __launch_bounds__(256) fasteq_u1d_carry_kernel(const int* __rest
     const int* __restrict__ part_edge, int n_parts, int n_out_rows, const T* __restrict__ carry, T* __restrict__ out) {{
   const int p = blockIdx.x, before = p > 0 ? p - 1 : 0;
   const int row = part_ptr[p], row_before = part_ptr[before], row_after = part_ptr[p + 1];
-  const int edge = part_edge[p], edge_before = part_edge[before], edge_after = part_edge[p + 1];
+  const int edge = part_edge[p], edge_before = part_edge[before];
   if (row >= n_out_rows) return;
   const int first = seg_ptr[row];
   if (edge <= first) return;                                                     // starts at a receiver's first edge
@@ -536,11 +536,16 @@ __global__ void __launch_bounds__(256) fasteq_u1d_carry_kernel(const int* __rest
     for (int i = threadIdx.x * VEC; i < OSEG * U; i += 256 * VEC) VS::st(o + i, vadd(VS::ld(o + i), VS::ld(c + i)));
     return;
   }}
+  // several carries in a row of pipelines: count them together, then add their rows without a lookup in between
+  int n = 1;
+  for (int q = p + 1, hit = 256; hit == 256; q += 256) {{
+    hit = __syncthreads_count(q + (int)threadIdx.x < n_parts && part_ptr[q + threadIdx.x < n_parts ? q + threadIdx.x : p] == row);
+    n += hit;
+  }}
   for (int i = threadIdx.x * VEC; i < OSEG * U; i += 256 * VEC) {{
     V sum = VS::ld(o + i);
-    if (edge_after > edge) sum = vadd(sum, VS::ld(c + i));
-    for (int q = p + 1; q < n_parts && part_ptr[q] == row; ++q)
-      if (part_edge[q + 1] > part_edge[q]) sum = vadd(sum, VS::ld(carry + (size_t)q * OSEG * U + i));
+#pragma unroll 4
+    for (int q = 0; q < n; ++q) sum = vadd(sum, VS::ld(c + (size_t)q * OSEG * U + i));
     VS::st(o + i, sum);
   }}
 }}
@@ -576,6 +581,7 @@ extern "C" int fasteq_u1d_forward_split(const fasteq_u1d_graph* gh, const int32_
                                         const void* y, void* out, fasteq_stream_t stream) {{
   if (!cfg::SCATTERED) return FASTEQ_UNSUPPORTED;
   if (!gh || !gh->part_ptr || gh->n_parts < 1 || !part_edge || !carry) return FASTEQ_INVALID;
+  if (gh->n_parts > gh->n_edges + gh->n_out_rows) return FASTEQ_INVALID;      // every share holds something, so every carry is written
   return run_forward(gh, part_edge, carry, w, x, y, out, stream);
 }}
 

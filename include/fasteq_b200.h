@@ -87,7 +87,7 @@ int fasteq_u1d_forward(const fasteq_u1d_graph* g /* host */, const void* w, cons
 /* The same with receivers split: the shares of `g->part_ptr` begin and end at the edges `part_edge` [n_parts + 1]
  * (fasteq_graph_partition_edges makes both), so that a graph of few or uneven receivers keeps every pipeline busy.  `carry` is
  * scratch of n_parts * out_segs * u values for the sums of receivers that an earlier share began; a second launch adds them
- * in a fixed order.  Scattered signatures only. */
+ * in a fixed order.  n_parts may not exceed n_edges + n_out_rows.  Scattered signatures only. */
 int fasteq_u1d_forward_split(const fasteq_u1d_graph* g /* host */, const int32_t* part_edge, void* carry, const void* w, const void* x,
                              const void* y, void* out, fasteq_stream_t stream);
 
