@@ -84,10 +84,8 @@ class U1DModule:
         lib.fasteq_u1d_describe.argtypes = [C.POINTER(U1DDesc)]
         lib.fasteq_u1d_forward.argtypes = [C.POINTER(U1DGraph)] + [C.c_void_p] * 5
         lib.fasteq_u1d_backward.argtypes = [C.POINTER(U1DGraph)] + [C.c_void_p] * 8
-        if hasattr(lib, "fasteq_u1d_forward_split"):
-            lib.fasteq_u1d_forward_split.argtypes = [C.POINTER(U1DGraph)] + [C.c_void_p] * 7
-        if hasattr(lib, "fasteq_u1d_backward_split"):
-            lib.fasteq_u1d_backward_split.argtypes = [C.POINTER(U1DGraph)] + [C.c_void_p] * 9
+        lib.fasteq_u1d_forward_split.argtypes = [C.POINTER(U1DGraph)] + [C.c_void_p] * 7
+        lib.fasteq_u1d_backward_split.argtypes = [C.POINTER(U1DGraph)] + [C.c_void_p] * 9
         lib.fasteq_u1d_device_status.argtypes = [C.POINTER(C.c_int32)]
         lib.fasteq_last_cuda_error.restype = C.c_char_p
         if hasattr(lib, "fasteq_u1d_forward_noalloc"):   # forward modules only

@@ -459,6 +459,14 @@ __device__ __forceinline__ void operator+=(V& a, V b) { a = fasteq::vadd(a, b); 
 template <typename... P> static bool misaligned(P... p) { return ((reinterpret_cast<uintptr_t>(p) | ...) & 7u) != 0; }
 """
 
+_NOT_SUMMED = r"""
+extern "C" int fasteq_stc_backward_summed_parts(int64_t, int32_t*) { return FASTEQ_UNSUPPORTED; }
+extern "C" int fasteq_stc_backward_summed(const void*, const void*, const void*, const int64_t*, const int32_t*, int64_t, int64_t, int32_t,
+                                          void*, void*, void*, fasteq_stream_t) {
+  return FASTEQ_UNSUPPORTED;  // the module of direction 3 holds these
+}
+"""
+
 
 def emit_stc(spec: STCSpec, direction: str, need_gx0: bool = False, packed: bool = False) -> str:
     dt = spec.dtype
@@ -572,7 +580,7 @@ extern "C" int fasteq_stc_double_backward(const void*, const void*, const void*,
   return FASTEQ_UNSUPPORTED;  // this module holds another direction
 }
 """)
-    return head + "\n".join(body) + "\n"
+    return head + "\n".join(body) + "\n" + (_NOT_SUMMED if direction != "bwdsum" else "")
 
 
 def arith_ops(spec: STCSpec, direction: str, need_gx0: bool = False) -> Dict[str, int]:

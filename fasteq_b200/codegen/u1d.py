@@ -77,17 +77,30 @@ def default_tuning(spec: U1DSpec, direction: str) -> Tuning:
                 stages = 10
         elif packed and big and ct == 128:                     # two thread groups per pipeline: two pipelines, shorter rings
             pipes, stages = 2, 5
+        # two CTAs of four 64-channel pipelines leave a thread 128 registers: enough for its two accumulators per output segment
+        # up to about 40 segments (160,000 edges: 109 us, one CTA of six pipelines 116 us), spills beyond (55 segments, 80,533
+        # edges: 128 us, and 84 us for one CTA of six pipelines at 168 registers)
+        one_cta = packed and ct == 64 and not big and 2 * spec.out_segs + 46 > 128
+        if one_cta:
+            pipes = 6
         per_pipe = 256 + stages * _stage_bytes(spec, ct, 0)
         fit = max(1, _SMEM_BUDGET // per_pipe)                 # pipelines one SM can hold
         if fit < pipes:
             pipes = fit
         if packed:
-            residency = 1 if (big or (wide and not small)) else 2
+            residency = 1 if (big or one_cta or (wide and not small)) else 2
         else:
             residency = 2 if (big or not f32) else 3
         return Tuning(ct=ct, groups=groups, stages=stages, pipes=pipes, vec=vec, min_blocks=max(1, min(residency, fit // pipes)))
     pipes = 4 if wide else max(1, 4 // wpg)
     extra = wpg * spec.y_segs * e
+    if packed and ct == 64 and spec.scattered and 32 <= spec.out_segs <= 64:
+        # 64-channel rows of medium length: one CTA of eight one-warp pipelines with the gradient rows in tensor memory (220 of
+        # 512 columns at 55 segments) instead of two CTAs of four with 14 KB tiles each: 40 segments, 160,000 edges 218 -> 208 us;
+        # 55 segments, 80,533 edges 146 -> 140 us; shorter rows have small tiles already
+        fit = (_SMEM_BUDGET // 8 - 256) // _stage_bytes(spec, ct, extra)
+        if fit >= 2:
+            return Tuning(ct=ct, groups=1, stages=min(4, fit), pipes=8, vec=vec, min_blocks=1, go_smem=False, go_tmem=True)
     go_bytes = (spec.out_segs * ct * e + 127) // 128 * 128
     stages = 4 if (wide and small) else 3
     per_pipe = 256 + stages * _stage_bytes(spec, ct, extra) + go_bytes
@@ -589,6 +602,10 @@ extern "C" int fasteq_u1d_backward(const fasteq_u1d_graph*, const void*, const v
                                    void*, void*, fasteq_stream_t) {{
   return FASTEQ_UNSUPPORTED;  // this module holds the forward kernel only
 }}
+extern "C" int fasteq_u1d_backward_split(const fasteq_u1d_graph*, const int32_t*, const void*, const void*, const void*, const void*, void*,
+                                         void*, void*, fasteq_stream_t) {{
+  return FASTEQ_UNSUPPORTED;
+}}
 """)
     src.append(_NOALLOC_FORWARD.replace("@MINB@", str(tun.min_blocks)))
     return "\n".join(src)
@@ -998,6 +1015,10 @@ fasteq_u1d_bwd_kernel(const Graph g, const T* __restrict__ go, const T* __restri
     src.append(f"""
 extern "C" int fasteq_u1d_forward(const fasteq_u1d_graph*, const void*, const void*, const void*, void*, fasteq_stream_t) {{
   return FASTEQ_UNSUPPORTED;  // this module holds the backward kernel only
+}}
+extern "C" int fasteq_u1d_forward_split(const fasteq_u1d_graph*, const int32_t*, void*, const void*, const void*, const void*, void*,
+                                        fasteq_stream_t) {{
+  return FASTEQ_UNSUPPORTED;
 }}
 
 static int run_backward(const fasteq_u1d_graph* gh, const int32_t* part_edge, const void* go, const void* w, const void* x,

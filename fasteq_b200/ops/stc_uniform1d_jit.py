@@ -21,7 +21,7 @@ from ..codegen import stc as _emit
 from ._needs import wanted
 
 STC_PAD_VALUE = -1
-_EMITTER_VERSION = "stc-v4"
+_EMITTER_VERSION = "stc-v5"
 _lock = threading.Lock()
 
 
@@ -39,9 +39,8 @@ class STCModule:
         lib.fasteq_stc_backward.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64, C.c_int64,
                                             C.c_void_p, C.c_void_p, C.c_void_p]
         lib.fasteq_stc_double_backward.argtypes = [C.c_void_p] * 6 + [C.c_int64, C.c_int64] + [C.c_void_p] * 4
-        if hasattr(lib, "fasteq_stc_backward_summed"):
-            lib.fasteq_stc_backward_summed_parts.argtypes = [C.c_int64, C.POINTER(C.c_int32)]
-            lib.fasteq_stc_backward_summed.argtypes = [C.c_void_p] * 5 + [C.c_int64, C.c_int64, C.c_int32] + [C.c_void_p] * 4
+        lib.fasteq_stc_backward_summed_parts.argtypes = [C.c_int64, C.POINTER(C.c_int32)]
+        lib.fasteq_stc_backward_summed.argtypes = [C.c_void_p] * 5 + [C.c_int64, C.c_int64, C.c_int32] + [C.c_void_p] * 4
         lib.fasteq_stc_device_status.argtypes = [C.POINTER(C.c_int32)]
         lib.fasteq_last_cuda_error.restype = C.c_char_p
         self.lib = lib

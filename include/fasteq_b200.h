@@ -147,8 +147,8 @@ int fasteq_stc_forward(const void* x1, const void* x0, const int32_t* i0, int64_
  * species (the reference does the same with index_add_, stc_uniform1d_jit.py:883-886). */
 int fasteq_stc_backward(const void* grad_out, const void* x1, const void* x0, const int32_t* i0, int64_t batch,
                         int64_t n_species, void* grad_x1, void* grad_x0_per_node, fasteq_stream_t stream);
-/* The same gradients with the weight gradient summed over nodes of equal species (modules built for direction 3; others do not
- * export it): grad_x0 [n_species, x0_segs, u] is fully overwritten, in an order of additions that depends on the batch and
+/* The same gradients with the weight gradient summed over nodes of equal species (modules built for direction 3; others
+ * return FASTEQ_UNSUPPORTED): grad_x0 [n_species, x0_segs, u] is fully overwritten, in an order of additions that depends on the batch and
  * the GPU's size alone.  `order` int64 [batch] lists the nodes by species, `species_sorted` int32 [batch] their species in
  * that order.  `partial` is scratch of (n_parts + n_species) * x0_segs * u values with n_parts from the query. */
 int fasteq_stc_backward_summed_parts(int64_t batch, int32_t* n_parts /* host */);

@@ -21,12 +21,12 @@ def _degrees(kind, rng):
 
 @pytest.mark.parametrize("dtype,tol", [("f32", 1e-5), ("f64", 1e-11)])
 @pytest.mark.parametrize("kind", ["one", "few", "ragged"])
-@pytest.mark.parametrize("u,presorted", [(64, True), (33, False)])
-def test_split_receivers_match_oracle(dtype, tol, kind, u, presorted):
+@pytest.mark.parametrize("u,lmax,presorted", [(64, 2, True), (33, 2, False), (64, 3, False)])     # 64, 3: 55 output segments
+def test_split_receivers_match_oracle(dtype, tol, kind, u, lmax, presorted):
     from fasteq_b200.ops import fast_uniform1d_jit
     from fasteq_b200.ops import uniform1d_jit as u1d
-    sh = Irreps.spherical_harmonics(2)
-    io, ins = full_channelwise_instructions(f"{u}x0e+{u}x1o", sh, 2)
+    sh = Irreps.spherical_harmonics(lmax)
+    io, ins = full_channelwise_instructions(f"{u}x0e+{u}x1o", sh, lmax)
     d = channelwise_tensor_product(f"{u}x0e+{u}x1o", sh, io, ins)
     rng = np.random.default_rng(u)
     deg = _degrees(kind, rng)
