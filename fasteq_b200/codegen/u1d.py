@@ -18,7 +18,7 @@ uniform1d_backward.py:256-888 backward), with a different execution model:
 """
 from __future__ import annotations
 
-from dataclasses import dataclass
+from dataclasses import dataclass, replace
 from typing import Dict, List, Tuple
 
 from .u1d_common import U1DSpec, Block, build_blocks, lit, restrict_blocks, split_out_segments, split_w_segments
@@ -94,13 +94,6 @@ def default_tuning(spec: U1DSpec, direction: str) -> Tuning:
         return Tuning(ct=ct, groups=groups, stages=stages, pipes=pipes, vec=vec, min_blocks=max(1, min(residency, fit // pipes)))
     pipes = 4 if wide else max(1, 4 // wpg)
     extra = wpg * spec.y_segs * e
-    if packed and ct == 64 and spec.scattered and 32 <= spec.out_segs <= 64:
-        # 64-channel rows of medium length: one CTA of eight one-warp pipelines with the gradient rows in tensor memory (220 of
-        # 512 columns at 55 segments) instead of two CTAs of four with 14 KB tiles each: 40 segments, 160,000 edges 218 -> 208 us;
-        # 55 segments, 80,533 edges 146 -> 140 us; shorter rows have small tiles already
-        fit = (_SMEM_BUDGET // 8 - 256) // _stage_bytes(spec, ct, extra)
-        if fit >= 2:
-            return Tuning(ct=ct, groups=1, stages=min(4, fit), pipes=8, vec=vec, min_blocks=1, go_smem=False, go_tmem=True)
     go_bytes = (spec.out_segs * ct * e + 127) // 128 * 128
     stages = 4 if (wide and small) else 3
     per_pipe = 256 + stages * _stage_bytes(spec, ct, extra) + go_bytes
@@ -115,6 +108,20 @@ def default_tuning(spec: U1DSpec, direction: str) -> Tuning:
     else:
         residency = 1 if big else (3 if f32 else 2)
     return Tuning(ct=ct, groups=1, stages=stages, pipes=pipes, vec=vec, min_blocks=max(1, min(residency, fit // pipes)))
+
+
+def untuned(spec: U1DSpec, direction: str) -> Tuning:
+    """The configuration of a signature the tuning database does not hold: the heuristic default, and for the backward of
+    64-channel rows of medium length one CTA of eight one-warp pipelines with the gradient rows in tensor memory (220 of 512
+    columns at 55 segments) instead of two CTAs of four with 14 KB tiles each.  40 segments, 160,000 edges: 218 -> 208 us;
+    55 segments, 80,533 edges: 146 -> 140 us.  Shorter rows have small tiles already, longer ones do not fit the columns."""
+    base = default_tuning(spec, direction)
+    if direction != "bwd" or not (spec.scattered and base.vec == 2 and base.ct == 64 and 32 <= spec.out_segs <= 64):
+        return base
+    fit = (_SMEM_BUDGET // 8 - 256) // _stage_bytes(spec, 64, spec.y_segs * spec.elem_bytes)
+    if fit < 2:
+        return base
+    return replace(base, stages=min(4, fit), pipes=8, min_blocks=1, go_smem=False, go_tmem=True)
 
 
 _SMEM_BUDGET = 220 * 1024

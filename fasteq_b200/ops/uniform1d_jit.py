@@ -45,7 +45,7 @@ def _dtype_str(t: torch.Tensor) -> str:
 
 def get_module(spec: U1DSpec, direction: str, needs=(False, False, False), tuning: Optional[_emit.Tuning] = None) -> _cabi.U1DModule:
     """Build (or load from the in-tree cache) the module of one signature."""
-    tun = tuning or _TUNING_OVERRIDE.get(direction) or _tuning.lookup(spec, direction, needs) or _emit.default_tuning(spec, direction)
+    tun = tuning or _TUNING_OVERRIDE.get(direction) or _tuning.lookup(spec, direction, needs) or _emit.untuned(spec, direction)
     key = (spec, direction, tuple(needs), tun)
     with _lock:
         mod = _MODULES.get(key)
@@ -383,7 +383,7 @@ def _tuning_for(spec: U1DSpec, direction: str, tensors, needs=(False, False, Fal
     """The launch configuration of this call: the measured winner of the signature when the tuning database has one,
     else the heuristic default.  Packed two-channel modules read and write 8-byte pairs; operands at an odd 4-byte
     offset (a contiguous view into a larger buffer) get the one-channel-per-thread module instead."""
-    tun = _TUNING_OVERRIDE.get(direction) or _tuning.lookup(spec, direction, needs) or _emit.default_tuning(spec, direction)
+    tun = _TUNING_OVERRIDE.get(direction) or _tuning.lookup(spec, direction, needs) or _emit.untuned(spec, direction)
     if tun.vec == 2 and any(t is not None and t.data_ptr() % 8 for t in tensors):
         import dataclasses
         return dataclasses.replace(tun, vec=1, pipes=1, groups=max(tun.groups, 1), min_blocks=min(tun.min_blocks + 1, 3))
