@@ -22,6 +22,7 @@ from ..irreps import Irreps
 from ..ops.dense import dense
 from ..ops.edge_geometry import edge_geometry, edge_geometry_usable
 from ..ops.radial_chain import radial_chain
+from ..ops.readout import scalar_readout
 from ..ops.silu import silu
 from ..ops.spherical_harmonics import SphericalHarmonics
 from .modules import ChannelwiseTensorProduct, SO3Linear, SymmetricContraction
@@ -140,11 +141,11 @@ class MACEStyleModel(torch.nn.Module):
         pos_ext = pos if halo is None else halo(pos)
         edge_sh, edge_radial, edge_vec = self.edge_features(pos_ext, edge_src, edge_dst, edge_shift, second_order)
         h = self.embedding.index_select(0, species)
-        e = pos.new_zeros(pos.shape[0])
+        e = None
         for layer, ro in zip(self.layers, self.readouts):
             h = layer(h, species, edge_sh, edge_radial, edge_dst, edge_src, halo, edge_vec)
-            e = e + (h[:, : self.channels] * ro).sum(dim=-1)     # scalars are the first segment of the ir_mul row
-        return e
+            e = scalar_readout(h, ro, e)     # scalars are the first segment of the ir_mul row
+        return pos.new_zeros(pos.shape[0]) if e is None else e
 
     def forward(self, pos, species, edge_src, edge_dst, edge_shift, node_graph=None, n_graphs: int = 1, forces: bool = True,
                 halo=None, create_graph: bool = False):
@@ -159,6 +160,6 @@ class MACEStyleModel(torch.nn.Module):
             energy = torch.zeros(n_graphs, dtype=e_node.dtype, device=e_node.device).index_add(0, node_graph, e_node)
         out = {"energy": energy}
         if forces:
-            (g,) = torch.autograd.grad(e_node.sum(), pos, create_graph=create_graph)
+            (g,) = torch.autograd.grad(e_node, pos, torch.ones_like(e_node), create_graph=create_graph)
             out["forces"] = -g
         return out

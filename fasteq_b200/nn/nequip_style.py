@@ -18,6 +18,7 @@ import torch
 from ..descriptors import full_channelwise_instructions
 from ..irreps import Irreps
 from ..ops.gate import GateSpec, gate
+from ..ops.readout import scalar_readout
 from ..ops.spherical_harmonics import SphericalHarmonics
 from ..ops.edge_geometry import edge_geometry, edge_geometry_usable
 from .mace_style import RadialMLP, bessel_basis, polynomial_cutoff
@@ -97,7 +98,7 @@ class NequIPStyleModel(torch.nn.Module):
         h = self.embedding[species]
         for layer in self.layers:
             h = layer(h, edge_sh, radial, edge_dst, edge_src, halo, vec if fused else None)
-        return (h[:, : self.channels] * self.readout).sum(dim=-1)     # per-atom scalar readout: elementwise + row sum
+        return scalar_readout(h, self.readout)
 
     def forward(self, pos, species, edge_src, edge_dst, edge_shift, forces: bool = True, halo=None, create_graph: bool = False):
         """``create_graph``: keep the forces differentiable, for a force loss."""
@@ -106,6 +107,6 @@ class NequIPStyleModel(torch.nn.Module):
         e_node = self.node_energies(pos, species, edge_src, edge_dst, edge_shift, halo, second_order=create_graph)
         out = {"energy": e_node.sum().reshape(1)}
         if forces:
-            (g,) = torch.autograd.grad(e_node.sum(), pos, create_graph=create_graph)
+            (g,) = torch.autograd.grad(e_node, pos, torch.ones_like(e_node), create_graph=create_graph)
             out["forces"] = -g
         return out

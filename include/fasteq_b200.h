@@ -405,6 +405,13 @@ int fasteq_tensorcore_device_status(int32_t* code /* host */);
 int fasteq_silu(int32_t dtype, int32_t order, const void* z, const void* g, const void* h, void* out0, void* out1, int64_t n,
                 fasteq_stream_t stream);
 
+/* Per-atom scalar readout over the first c_count of d columns: e[n] = e_in[n] + sum_c h[n, c] w[c] (e_in may be NULL), and its
+ * gradient gh[n, c] = g[n] w[c], zero beyond c_count. */
+int fasteq_readout_forward(int32_t dtype, const void* h, const void* w, const void* e_in, void* e, int64_t n, int32_t c_count, int64_t d,
+                           fasteq_stream_t stream);
+int fasteq_readout_backward(int32_t dtype, const void* g, const void* w, void* gh, int64_t n, int32_t c_count, int64_t d,
+                            fasteq_stream_t stream);
+
 #ifdef __cplusplus
 }
 #endif
