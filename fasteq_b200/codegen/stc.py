@@ -433,7 +433,8 @@ extern "C" int fasteq_stc_backward_summed(const void* go, const void* x1, const 
 def packed_ok(spec: STCSpec, direction: str) -> bool:
     """Whether a thread may carry two channels in packed FP32 arithmetic (full warps of pairs; operands 8-byte aligned).  The
     scalar kernels issued in 84 % (forward) and 67 % (backward with the weight gradient, whose 42 KB of straight-line code also
-    waits for instructions) of their cycles; packed ones need half the slots and half the code per channel."""
+    waits for instructions) of their cycles; packed ones need half the slots and half the code per channel: 128-channel product
+    basis on 200,000 nodes, forward 0.96 -> 0.81 ms, backward 2.79 -> 2.49 ms."""
     return spec.dtype == "f32" and spec.u % 64 == 0 and direction != "dbwd"
 
 

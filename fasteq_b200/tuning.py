@@ -11,7 +11,7 @@ receiver's grad_out row (shared memory, L1, tensor memory) -- and the procedure 
   receiver-sorted graph of the benchmark's density, then time the fastest and the heuristic default again in five
   alternating bursts; the challenger replaces the default only if it wins that alternation by more than the margin;
 * the winners live in ``tuning_db.json`` beside this file (tracked, so that a fresh checkout starts tuned); the
-  operator front-end asks ``lookup`` before it falls back to the heuristic ``codegen.u1d.default_tuning``.
+  operator front-end asks ``lookup`` before it falls back to ``codegen.u1d.untuned`` (the heuristic default and one rule).
 
 ``python -m fasteq_b200.tuning`` sweeps the standard signatures and rewrites the file.
 """
@@ -199,19 +199,31 @@ def sweep(spec: U1DSpec, direction: str, needs=(True, True, True), n_boxes: int 
         gph = _cabi.U1DGraph()
         gph.n_edges, gph.n_out_rows, gph.x_rows, gph.y_rows = E, N, N, E
         gph.x_index, gph.y_index, gph.seg_ptr, gph.perm = src.data_ptr(), None, plan.seg_ptr.data_ptr(), None
-        n_parts = max(1, min(u1d._sm_count(dev) * int(mod.desc.ctas_per_sm), N))
-        gph.part_ptr, gph.n_parts = plan.partition(n_parts).data_ptr(), n_parts
+        pipelines = u1d._sm_count(dev) * int(mod.desc.ctas_per_sm)
+        split = N < u1d.SPLIT_ROWS_PER_PIPELINE * pipelines                 # shares as the operator cuts them
+        n_parts = max(1, min(pipelines, N))
+        part = plan.partition(n_parts, split)
+        gph.part_ptr, gph.n_parts = part.data_ptr(), n_parts
         stream = torch.cuda.current_stream(dev).cuda_stream
         # (the closures bind this candidate's module and graph record: they are called again in the confirmation phase)
         if direction == "fwd":
             out = bufs.setdefault("out", torch.empty(N, spec.out_segs * spec.u, dtype=x.dtype, device=dev))
-            run = lambda mod=mod, gph=gph: mod.forward(gph, w.data_ptr(), x.data_ptr(), y.data_ptr(), out.data_ptr(), stream)
+            carry = torch.empty(n_parts, spec.out_segs * spec.u, dtype=x.dtype, device=dev) if split else None
+            if split:
+                run = lambda mod=mod, gph=gph, part=part, carry=carry: mod.forward_split(gph, part[1].data_ptr(), carry.data_ptr(), w.data_ptr(),
+                                                                                         x.data_ptr(), y.data_ptr(), out.data_ptr(), stream)
+            else:
+                run = lambda mod=mod, gph=gph: mod.forward(gph, w.data_ptr(), x.data_ptr(), y.data_ptr(), out.data_ptr(), stream)
         else:
             gw = bufs.setdefault("gw", torch.empty_like(w)) if needs[0] else None
             gx = bufs.setdefault("gx", torch.empty_like(x)) if needs[1] else None
             gy = bufs.setdefault("gy", torch.empty_like(y)) if needs[2] else None
             ptr = lambda t: t.data_ptr() if t is not None else None
-            run = lambda mod=mod, gph=gph: mod.backward(gph, r.data_ptr(), w.data_ptr(), x.data_ptr(), y.data_ptr(), ptr(gw), ptr(gx), ptr(gy), stream)
+            ops = (r.data_ptr(), w.data_ptr(), x.data_ptr(), y.data_ptr(), ptr(gw), ptr(gx), ptr(gy), stream)
+            if split:
+                run = lambda mod=mod, gph=gph, part=part, ops=ops: mod.backward_split(gph, part[1].data_ptr(), *ops)
+            else:
+                run = lambda mod=mod, gph=gph, ops=ops: mod.backward(gph, *ops)
         try:
             run(); run(); torch.cuda.synchronize()
             ms = min(burst(run) for _ in range(repeats))
