@@ -98,7 +98,7 @@ def _matmul_nt(a: torch.Tensor, bt: torch.Tensor) -> torch.Tensor:
 def _matmul_tn(g: torch.Tensor, x: torch.Tensor) -> torch.Tensor:
     """``g [M, N]^T @ x [M, K] -> [N, K]``."""
     if g.is_cuda and g.dtype in (torch.float32, torch.float64) and g.dtype == x.dtype:
-        return _fma_wgrad(x, g).t().contiguous()
+        return _fma_wgrad(g, x)
     return g.t() @ x
 
 
