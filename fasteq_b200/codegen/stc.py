@@ -66,12 +66,14 @@ def make_stc_spec(paths, coeffs, *, x1_segs, x0_segs, out_segs, u, dtype, pad_va
 
 
 def _groups(spec: STCSpec):
-    """{(d, v): {sorted index tuple: coefficient}} with duplicates merged."""
+    """{(d, v): {sorted index tuple: coefficient}} with duplicates merged.  Terms that cancel or have a zero coefficient are dropped,
+    and with its last term the pair itself: the emitters start a pair's sum from its first term."""
     g: Dict[Tuple[int, int], Dict[Tuple[int, ...], float]] = {}
     for a, d, v, c in spec.paths:
         m = g.setdefault((d, v), {})
         m[a] = m.get(a, 0.0) + c
-    return {k: {a: c for a, c in m.items() if c != 0.0} for k, m in sorted(g.items())}
+    live = {k: {a: c for a, c in m.items() if c != 0.0} for k, m in sorted(g.items())}
+    return {k: m for k, m in live.items() if m}
 
 
 def _cover(cubics, k: int, prefer=()):
