@@ -53,10 +53,17 @@ class _Readout(torch.autograd.Function):
         return gh, gw, (g if ctx.needs_input_grad[2] else None)
 
 
+def _one_launch(h: torch.Tensor, w: torch.Tensor, e: Optional[torch.Tensor]) -> bool:
+    """Whether the kernel's view of the operands is theirs: rows of one matrix, a weight per column, a running sum per row, all
+    dense, of one type and on one device.  Everything else is left to the expression below, which broadcasts it or raises."""
+    return (h.dim() == 2 and h.is_contiguous() and h.dtype in (torch.float32, torch.float64)
+            and w.dim() == 1 and w.is_contiguous() and w.dtype == h.dtype and w.device == h.device and w.numel() <= h.shape[1]
+            and (e is None or (e.shape == h.shape[:1] and e.is_contiguous() and e.dtype == h.dtype and e.device == h.device)))
+
+
 def scalar_readout(h: torch.Tensor, w: torch.Tensor, e: Optional[torch.Tensor] = None) -> torch.Tensor:
     """``e + (h[:, : len(w)] * w).sum(-1)`` (``e`` omitted: without it)."""
-    if (h.is_cuda and h.dim() == 2 and h.is_contiguous() and w.is_contiguous() and h.dtype in (torch.float32, torch.float64)
-            and w.dtype == h.dtype and w.numel() <= h.shape[1] and (e is None or (e.is_contiguous() and e.dtype == h.dtype))):
+    if h.is_cuda and _one_launch(h, w, e):
         return _Readout.apply(h, w, e)
     s = (h[:, : w.numel()] * w).sum(dim=-1)
     return s if e is None else e + s
