@@ -39,6 +39,10 @@ class STCSpec:
             object.__setattr__(self, "_hash", h)
         return h
 
+    def __getstate__(self):
+        # another process hashes texts differently: a pickled copy computes its own
+        return {k: v for k, v in self.__dict__.items() if k != "_hash"}
+
     @property
     def ctype(self) -> str:
         return "float" if self.dtype == "f32" else "double"

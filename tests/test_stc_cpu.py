@@ -119,3 +119,20 @@ def test_table_spans_the_space_e3nn_reduces_to(golden, case, irr_out):
             dim = Irreps(irr_out)[ob].ir.dim
             assert len(rows) == dim and all(abs(c - dim ** -0.5) < 1e-12 for _, _, c in rows)
             assert sorted(v for _, v, _ in rows) == list(range(Irreps(irr_out).segment_offsets()[ob], Irreps(irr_out).segment_offsets()[ob] + dim))
+
+
+def test_specification_hash_is_not_carried_to_another_process():
+    """The hash kept on a specification depends on the process (texts hash differently in each): a pickled copy has none."""
+    import os
+    import pickle
+    import subprocess
+    import sys
+    from fasteq_b200.codegen.stc import make_stc_spec
+    make = "make_stc_spec([[0, 0, 0]], [1.0], x1_segs=1, x0_segs=1, out_segs=1, u=4, dtype='f32')"
+    spec = eval(make)
+    hash(spec)
+    code = ("import sys, pickle; from fasteq_b200.codegen.stc import make_stc_spec\n"
+            f"a = pickle.load(sys.stdin.buffer); b = {make}\n"
+            "assert a == b and hash(a) == hash(b) and len({a, b}) == 1")
+    for seed in ("1", "2"):
+        subprocess.run([sys.executable, "-c", code], input=pickle.dumps(spec), check=True, env={**os.environ, "PYTHONHASHSEED": seed})
