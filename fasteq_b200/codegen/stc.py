@@ -421,6 +421,7 @@ extern "C" int fasteq_stc_backward_summed(const void* go, const void* x1, const 
     return e == cudaSuccess ? FASTEQ_OK : cuda_fail(e);
   }
   if (n_species == 0 || !go || !x1 || !x0 || !order || !species_sorted || !partial || !gx1 || !gx0) return FASTEQ_INVALID;
+  if (n_parts > batch) return FASTEQ_INVALID;        // an empty share writes no slot, but the second kernel would add it
   if (misaligned(go, x1, x0, partial, gx1)) return FASTEQ_INVALID;
   int* st = nullptr;
   cudaError_t e = cudaGetSymbolAddress((void**)&st, g_status_word);

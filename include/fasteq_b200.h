@@ -150,7 +150,8 @@ int fasteq_stc_backward(const void* grad_out, const void* x1, const void* x0, co
 /* The same gradients with the weight gradient summed over nodes of equal species (modules built for direction 3; others
  * return FASTEQ_UNSUPPORTED): grad_x0 [n_species, x0_segs, u] is fully overwritten, in an order of additions that depends on the batch and
  * the GPU's size alone.  `order` int64 [batch] lists the nodes by species, `species_sorted` int32 [batch] their species in
- * that order.  `partial` is scratch of (n_parts + n_species) * x0_segs * u values with n_parts from the query. */
+ * that order.  `partial` is scratch of (n_parts + n_species) * x0_segs * u values with n_parts from the query for this
+ * batch: more parts than nodes are refused. */
 int fasteq_stc_backward_summed_parts(int64_t batch, int32_t* n_parts /* host */);
 int fasteq_stc_backward_summed(const void* grad_out, const void* x1, const void* x0, const int64_t* order, const int32_t* species_sorted,
                                int64_t batch, int64_t n_species, int32_t n_parts, void* partial, void* grad_x1, void* grad_x0,
