@@ -539,7 +539,8 @@ int run_packed(const fasteq_eqlinear_problem* p, bool dgrad, const void* packed,
 
 // ------------------------------------------------------------------------------------------------
 // Weight gradient: per path a [u, v] = X^T G product reduced over R = batch * rows GEMM rows.
-// grid = (splits of all paths back to back, u tiles * v tiles); a CTA reduces its share of R into one tile (chunks of
+// grid = splits of all paths back to back for the first tile, then for the next (a second grid dimension would hold 65,535
+// tiles); a CTA reduces its share of R into one tile (chunks of
 // rows summed on their own first, like the forward), writes it to partial[split] and a second kernel adds a path's
 // splits in a fixed order and applies the coefficient.
 struct WgradTable {
@@ -547,6 +548,13 @@ struct WgradTable {
   int split_first[kMaxPaths + 1];   // splits of path q: [split_first[q], split_first[q + 1])
   double coeff[kMaxPaths];
 };
+
+// split and tile of a CTA
+__device__ __forceinline__ void decode_cta(const WgradTable& tab, int num_paths, int* split, int* tile) {
+  const unsigned n = (unsigned)tab.split_first[num_paths];
+  *tile = (int)(blockIdx.x / n);
+  *split = (int)(blockIdx.x - (unsigned)*tile * n);
+}
 
 __device__ __forceinline__ int path_of_split(const WgradTable& tab, int num_paths, int split) {
   int q = 0;
@@ -579,9 +587,11 @@ __global__ void __launch_bounds__(wg_threads(TM, TN)) eqlinear_wgrad_f32_kernel(
   extern __shared__ __align__(16) float wg_ring[];
   float* sX = wg_ring;                                // [WG_STAGES][WG_BK][TM]
   float* sG = wg_ring + WG_STAGES * WG_BK * TM;       // [WG_STAGES][WG_BK][TN]
-  const int split = blockIdx.x, q = path_of_split(tab, num_paths, split);
+  int split, tile;
+  decode_cta(tab, num_paths, &split, &tile);
+  const int q = path_of_split(tab, num_paths, split);
   const int v_tiles = (v + TN - 1) / TN;
-  const int m0 = (blockIdx.y / v_tiles) * TM, n0 = (blockIdx.y % v_tiles) * TN;
+  const int m0 = (tile / v_tiles) * TM, n0 = (tile % v_tiles) * TN;
   const int gi = tab.rows[q], inv = 65536 / gi + 1;
   const long long R = batch * gi, r_begin = (long long)(split - tab.split_first[q]) * rows_per_split;
   const long long r_end = r_begin + rows_per_split < R ? r_begin + rows_per_split : R;
@@ -670,9 +680,11 @@ __global__ void __launch_bounds__(NT) eqlinear_wgrad_kernel(const __grid_constan
                                                             long long rows_per_split) {
   __shared__ T sX[BK][BM + 4];
   __shared__ T sG[BK][BN + 4];
-  const int split = blockIdx.x, q = path_of_split(tab, num_paths, split);
+  int split, tile;
+  decode_cta(tab, num_paths, &split, &tile);
+  const int q = path_of_split(tab, num_paths, split);
   const int v_tiles = (v + BN - 1) / BN;
-  const int m0 = (blockIdx.y / v_tiles) * BM, n0 = (blockIdx.y % v_tiles) * BN;
+  const int m0 = (tile / v_tiles) * BM, n0 = (tile % v_tiles) * BN;
   const int gi = tab.rows[q];
   const long long R = batch * gi;
   const long long r_begin = (long long)(split - tab.split_first[q]) * rows_per_split;
@@ -796,7 +808,7 @@ cudaError_t launch_wgrad_f32(const fasteq_eqlinear_problem* p, WgradTable* tab, 
   const long long rps = plan_splits(p, tiles, (long long)sms * std::max(per_sm, 1), tab);
   e = cudaMallocAsync((void**)partial, (size_t)tab->split_first[p->num_paths] * p->u * p->v * sizeof(float), s);
   if (e != cudaSuccess) return e;
-  kernel<<<dim3((unsigned)tab->split_first[p->num_paths], (unsigned)tiles), wg_threads(TM, TN), wg_smem(TM, TN), s>>>(
+  kernel<<<(unsigned)tab->split_first[p->num_paths] * (unsigned)tiles, wg_threads(TM, TN), wg_smem(TM, TN), s>>>(
       *tab, x, go, *partial, p->batch, p->in_rows, p->out_rows, p->u, p->v, p->num_paths, rps);
   return cudaGetLastError();
 }
@@ -836,7 +848,7 @@ int launch_wgrad(const fasteq_eqlinear_problem* p, const void* x, const void* go
     const long long rps = plan_splits(p, tiles, (long long)sms * 4, &tab);
     e = cudaMallocAsync((void**)&partial, (size_t)tab.split_first[p->num_paths] * uv * sizeof(T), s);
     if (e == cudaSuccess) {
-      eqlinear_wgrad_kernel<T><<<dim3((unsigned)tab.split_first[p->num_paths], (unsigned)tiles), NT, 0, s>>>(
+      eqlinear_wgrad_kernel<T><<<(unsigned)tab.split_first[p->num_paths] * (unsigned)tiles, NT, 0, s>>>(
           tab, (const T*)x, (const T*)go, partial, p->batch, p->in_rows, p->out_rows, p->u, p->v, p->num_paths, rps);
       e = cudaGetLastError();
     }
