@@ -747,25 +747,28 @@ __global__ void __launch_bounds__(NT) eqlinear_wgrad_kernel(const __grid_constan
   }
 }
 
-// 32 outputs by 8 interleaved shares of their path's splits, both added in a fixed order.  Bound by the latency of the
-// loads: one thread per output walked hundreds of splits one after the other (28 us for a [64, 64] gradient in 313 splits).
-template <typename T>
+// 256 / Y outputs by Y interleaved shares of their path's splits, both added in a fixed order.  Bound by the latency of the
+// loads: one thread per output walked hundreds of splits one after the other (28 us for a [64, 64] gradient in 313 splits), hence
+// Y = 8; a few rows make one split per path, and seven of eight threads would have none of it (ten-path SO3Linear of 128
+// channels, one node: 10.2 us with Y = 8, 6.9 with 1; general kernel in FP64 12.3 and 8.9).
+template <typename T, int Y>
 __global__ void __launch_bounds__(256) eqlinear_wgrad_reduce_kernel(const __grid_constant__ WgradTable tab, const T* __restrict__ partial,
                                                                     T* __restrict__ gw, int num_paths, long long uv) {
-  __shared__ T share[8][33];
-  const long long i = (long long)blockIdx.x * 32 + threadIdx.x, total = (long long)num_paths * uv;
+  constexpr int X = 256 / Y;
+  __shared__ T share[Y][X + 1];
+  const long long i = (long long)blockIdx.x * X + threadIdx.x, total = (long long)num_paths * uv;
   const int q = i < total ? (int)(i / uv) : 0;
   T sum = T(0);
   if (i < total) {
     const T* p = partial + (i - (long long)q * uv);
 #pragma unroll 4
-    for (int z = tab.split_first[q] + threadIdx.y; z < tab.split_first[q + 1]; z += 8) sum += p[(size_t)z * uv];
+    for (int z = tab.split_first[q] + threadIdx.y; z < tab.split_first[q + 1]; z += Y) sum += p[(size_t)z * uv];
   }
   share[threadIdx.y][threadIdx.x] = sum;
   __syncthreads();
   if (threadIdx.y == 0 && i < total) {
 #pragma unroll
-    for (int k = 1; k < 8; ++k) sum += share[k][threadIdx.x];
+    for (int k = 1; k < Y; ++k) sum += share[k][threadIdx.x];
     gw[i] = (T)tab.coeff[q] * sum;
   }
 }
@@ -841,8 +844,11 @@ int launch_wgrad(const fasteq_eqlinear_problem* p, const void* x, const void* go
       ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(go)) & 15u) == 0) {   // 16-byte row pieces
     const float *xf = (const float*)x, *gf = (const float*)go;
     float** pf = (float**)&partial;
-    if (p->u <= 64) e = p->v <= 64 ? launch_wgrad_f32<64, 64>(p, &tab, sms, xf, gf, pf, s) : launch_wgrad_f32<64, 128>(p, &tab, sms, xf, gf, pf, s);
-    else            e = p->v <= 64 ? launch_wgrad_f32<128, 64>(p, &tab, sms, xf, gf, pf, s) : launch_wgrad_f32<128, 128>(p, &tab, sms, xf, gf, pf, s);
+    // up to 128 rows every path is one share, and what counts is how many CTAs start and how little each stores: 64 x 64 tiles
+    // whatever the extents (that SO3Linear 6.9 -> 5.4 us, at 16 nodes 17.0 -> 11.5; [32, 256]^T [32, 256] 9.1 -> 7.1)
+    if (p->batch * max_rows <= 128) e = launch_wgrad_f32<64, 64>(p, &tab, sms, xf, gf, pf, s);
+    else if (p->u <= 64) e = p->v <= 64 ? launch_wgrad_f32<64, 64>(p, &tab, sms, xf, gf, pf, s) : launch_wgrad_f32<64, 128>(p, &tab, sms, xf, gf, pf, s);
+    else                 e = p->v <= 64 ? launch_wgrad_f32<128, 64>(p, &tab, sms, xf, gf, pf, s) : launch_wgrad_f32<128, 128>(p, &tab, sms, xf, gf, pf, s);
   } else {
     const int tiles = ((p->u + BM - 1) / BM) * ((p->v + BN - 1) / BN);
     const long long rps = plan_splits(p, tiles, (long long)sms * 4, &tab);
@@ -854,7 +860,10 @@ int launch_wgrad(const fasteq_eqlinear_problem* p, const void* x, const void* go
     }
   }
   if (e == cudaSuccess) {
-    eqlinear_wgrad_reduce_kernel<T><<<(unsigned)((total + 31) / 32), dim3(32, 8), 0, s>>>(tab, partial, (T*)gw, p->num_paths, uv);
+    if (tab.split_first[p->num_paths] == p->num_paths)
+      eqlinear_wgrad_reduce_kernel<T, 1><<<(unsigned)((total + 255) / 256), dim3(256, 1), 0, s>>>(tab, partial, (T*)gw, p->num_paths, uv);
+    else
+      eqlinear_wgrad_reduce_kernel<T, 8><<<(unsigned)((total + 31) / 32), dim3(32, 8), 0, s>>>(tab, partial, (T*)gw, p->num_paths, uv);
     e = cudaGetLastError();
   }
   if (partial) cudaFreeAsync(partial, s);
