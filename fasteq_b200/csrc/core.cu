@@ -3,6 +3,7 @@
 // their own translation units of the same library.)
 #include <cstdio>
 #include <cstdint>
+#include <algorithm>
 #include <cuda_runtime.h>
 #include "fasteq_b200.h"
 #include "core_common.h"
@@ -53,6 +54,46 @@ extern "C" int fasteq_graph_check_sorted(const int32_t* dst, int64_t n, int32_t*
     check_sorted_kernel<<<(int)blocks, 256, 0, s>>>(dst, n, flag);
   }
   cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? FASTEQ_OK : cuda_fail(e);
+}
+
+// ---------------------------------------------------------------- order and degrees in one go
+// result[0] <- 1 if some edge comes before a smaller one, counts[r] <- edges of row r.  Equal indices of a warp are added as
+// one (runs of a sorted index; a receiver that has most edges).
+__global__ void __launch_bounds__(256) survey_kernel(const int* __restrict__ dst, long long n, long long n_rows, int* result, int* counts) {
+  const long long stride = (long long)gridDim.x * blockDim.x;
+  const int lane = threadIdx.x & 31;
+  int bad = 0;
+  for (long long i0 = (long long)blockIdx.x * blockDim.x + threadIdx.x - lane; i0 < n; i0 += stride) {
+    const long long i = i0 + lane;
+    const int v = i < n ? dst[i] : -1;
+    if (i + 1 < n) bad |= v > dst[i + 1];
+    const unsigned same = __match_any_sync(0xffffffffu, v);
+    if (v >= 0 && v < n_rows && lane == __ffs(same) - 1) atomicAdd(&counts[v], __popc(same));
+  }
+  if (bad) atomicExch(result, 1);
+}
+
+__global__ void __launch_bounds__(256) max_count_kernel(const int* __restrict__ counts, long long n_rows, int* result) {
+  int most = 0;
+  for (long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x; r < n_rows; r += (long long)gridDim.x * blockDim.x)
+    most = counts[r] > most ? counts[r] : most;
+  most = __reduce_max_sync(0xffffffffu, most);
+  if ((threadIdx.x & 31) == 0 && most > 0) atomicMax(result, most);
+}
+
+extern "C" int fasteq_graph_survey(const int32_t* dst, int64_t n_edges, int64_t n_rows, int32_t* result, fasteq_stream_t stream) {
+  if (!result || n_edges < 0 || n_rows < 0 || (n_edges > 0 && !dst)) return FASTEQ_INVALID;
+  if (n_edges > 0x7fffffffLL || n_rows >= 0x7fffffffLL) return FASTEQ_UNSUPPORTED;
+  cudaStream_t s = (cudaStream_t)stream;
+  cudaError_t e = cudaMemsetAsync(result, 0, (size_t)(2 + n_rows) * sizeof(int), s);
+  if (e != cudaSuccess) return cuda_fail(e);
+  if (n_edges > 0 && n_rows > 0) {
+    const long long wave = 148 * 8;                     // grid-stride loops: a wave of resident CTAs
+    survey_kernel<<<(unsigned)std::min<long long>((n_edges + 255) / 256, wave), 256, 0, s>>>(dst, n_edges, n_rows, result, result + 2);
+    max_count_kernel<<<(unsigned)std::min<long long>((n_rows + 255) / 256, wave), 256, 0, s>>>(result + 2, n_rows, result + 1);
+  }
+  e = cudaGetLastError();
   return e == cudaSuccess ? FASTEQ_OK : cuda_fail(e);
 }
 

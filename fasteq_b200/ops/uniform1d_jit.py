@@ -69,11 +69,11 @@ def get_module(spec: U1DSpec, direction: str, needs=(False, False, False), tunin
 # ----------------------------------------------------------------------------- graph plan
 
 class GraphPlan:
-    """Receiver-sorted CSR view of a scatter index: sortedness, permutation, segment offsets
+    """Receiver-sorted CSR view of a scatter index: sortedness, permutation, segment offsets, largest degree
     and per-grid partitions.  Built once per index tensor (one host sync) and cached.  Each build step
     leaves an event behind it; ``ready_on_current_stream`` makes a later user on another stream wait for them."""
 
-    def __init__(self, dst: torch.Tensor, n_rows: int, seg_ptr: Optional[torch.Tensor] = None):
+    def __init__(self, dst: torch.Tensor, n_rows: int, seg_ptr: Optional[torch.Tensor] = None, max_degree: Optional[int] = None):
         if dst.dim() != 1:
             raise ValueError("scatter index must be 1-D")
         core = _cabi.core()
@@ -90,14 +90,17 @@ class GraphPlan:
             if seg_ptr.numel() != self.n_rows + 1 or seg_ptr.dtype != torch.int32 or seg_ptr.device != dev:
                 raise ValueError("seg_ptr must be an int32 tensor of n_rows + 1 offsets on the index's device")
             self.sorted, self.perm, self.seg_ptr = True, None, seg_ptr.contiguous()
+            # where the caller does not know it: no receiver set has a smaller one, and to read it back would be the sync saved
+            self.max_degree = int(max_degree) if max_degree is not None else -(-self.n_edges // max(self.n_rows, 1))
             return
         stream = _cabi.stream(dev)
         dst32 = dst.to(torch.int32).contiguous()
-        flag = torch.empty(1, dtype=torch.int32, device=dev)
+        survey = torch.empty(2 + self.n_rows, dtype=torch.int32, device=dev)
         with _cabi.on_device(dev):
-            _cabi.check(core.fasteq_graph_check_sorted(dst32.data_ptr(), self.n_edges, flag.data_ptr(), stream), core,
-                        "fasteq_graph_check_sorted")
-            self.sorted = bool(flag.item())
+            _cabi.check(core.fasteq_graph_survey(dst32.data_ptr(), self.n_edges, self.n_rows, survey.data_ptr(), stream), core,
+                        "fasteq_graph_survey")
+            unsorted, self.max_degree = survey[:2].tolist()
+            self.sorted = not unsorted
             if self.sorted:
                 self.perm = None
                 sorted_dst = dst32
@@ -191,8 +194,9 @@ def graph_plan(dst: torch.Tensor, n_rows: int) -> GraphPlan:
     return plan
 
 
-def register_sorted_plan(dst: torch.Tensor, n_rows: int, seg_ptr: torch.Tensor, owner: Optional[str] = None) -> GraphPlan:
-    """Install the plan of a receiver-sorted index whose CSR offsets are already known.  ``owner``: a tag of
+def register_sorted_plan(dst: torch.Tensor, n_rows: int, seg_ptr: torch.Tensor, owner: Optional[str] = None,
+                         max_degree: Optional[int] = None) -> GraphPlan:
+    """Install the plan of a receiver-sorted index whose CSR offsets (and largest degree, if the caller has it) are known.  ``owner``: a tag of
     the caller that rebuilds its graph over and over (a neighbour-list builder): its previous plan is dropped
     instead of filling the cache with dead index tensors."""
     key = _plan_key(dst, n_rows)
@@ -202,7 +206,7 @@ def register_sorted_plan(dst: torch.Tensor, n_rows: int, seg_ptr: torch.Tensor, 
             _PLANS.pop(old, None)
         _OWNED[owner] = key
     _PLANS.pop(key, None)
-    plan = GraphPlan(dst, n_rows, seg_ptr)
+    plan = GraphPlan(dst, n_rows, seg_ptr, max_degree)
     plan._keepalive = dst.detach()
     _insert_plan(key, plan)
     return plan
@@ -336,7 +340,7 @@ class _Call:
             g.seg_ptr = self.plan.seg_ptr.data_ptr()
             g.perm = self.plan.perm.data_ptr() if self.plan.perm is not None else None
             pipelines = _sm_count(dev) * int(mod.desc.ctas_per_sm)
-            if 0 < self.n_edges and self.n_out_rows < SPLIT_ROWS_PER_PIPELINE * pipelines:
+            if split_receivers(mod.desc, self.n_out_rows, self.n_edges, self.plan.max_degree, pipelines):
                 g.n_parts = max(1, min(pipelines, max(self.n_out_rows, (self.n_edges + 3) // 4)))
                 part = self.plan.partition(g.n_parts, split=True)
                 part_edge = part[1].data_ptr()
@@ -351,10 +355,37 @@ class _Call:
         return g, part_edge
 
 
-# Below this many receivers per pipeline the shares are cut between edges: a share of whole receivers is up to one receiver
-# longer than the mean (the whole kernel, when there are fewer receivers than pipelines), while a split costs the forward one
-# output row per pipeline written, read and added.  Beyond it the two are within noise of each other.
+# Below this many receivers per pipeline shares may be cut between edges.
 SPLIT_ROWS_PER_PIPELINE = 32
+
+
+def split_receivers(desc: _cabi.U1DDesc, n_rows: int, n_edges: int, max_degree: int, pipelines: int) -> bool:
+    """Whether a launch's shares are cut between edges instead of between receivers.
+
+    The longest share of whole receivers is the longest receiver where each has a pipeline, and about one receiver longer than the
+    mean where pipelines take several.
+
+    The backward pays only for receivers that two pipelines begin, and takes the cut throughout: 0.02 to 1.02 of the time on whole
+    receivers over graphs of 1 to 15,000 receivers of 1 to 60 edges (once 1.08: 18.7 against 17.4 us, 512 equal rows of 33 channels).  The exception are FP64 rows in two thread groups, whose
+    beginning costs as much as several edges: where equal receivers fill whole shares almost evenly they keep them (2,000 receivers of
+    exactly 8 edges: 425 whole, 482 us cut; of 8 on average 516 and 489).
+
+    The forward also pays for the carry rows and their launch, 2 to 18 us: what 24 to 30 edges of one pipeline take in FP32, half as
+    many in the kernels with the slowest edges (rows that cannot travel as bulk copies; FP64 rows in two thread groups).  55 segments
+    of 128 channels: 512 receivers of 8 edges 16.8 whole, 24.4 us cut; of 30 edges on average 48.3 and 42.6; of exactly 30 edges 30.1
+    and 42.6; 4,000 receivers of 16 edges 97 and 102, of 30 edges 167 and 162; 55 segments of 64 channels, 2,000 of 30 edges 69.5
+    and 60.9.  With these limits no forward of the sweep (529 graphs over seven signatures) is slower than on whole receivers by
+    more than two runs of one differ."""
+    if n_edges == 0 or n_rows >= SPLIT_ROWS_PER_PIPELINE * pipelines:
+        return False
+    wide = desc.dtype == 1 and desc.out_segs > 64
+    if desc.direction == 1:
+        even = 4 * max_degree * n_rows <= 5 * n_edges and n_rows > pipelines
+        return not (wide and even and -(-n_rows // pipelines) * max_degree * pipelines - n_edges < 8 * pipelines)
+    slow = wide or desc.u * (8 if desc.dtype == 1 else 4) % 16 != 0
+    if n_rows <= pipelines:
+        return max_degree * pipelines - n_edges >= (16 if slow else 32) * pipelines
+    return max_degree >= (24 if slow else 40)
 
 
 _META_CACHE: Dict[Tuple, Tuple[torch.Tensor, np.ndarray]] = {}

@@ -200,7 +200,7 @@ def sweep(spec: U1DSpec, direction: str, needs=(True, True, True), n_boxes: int 
         gph.n_edges, gph.n_out_rows, gph.x_rows, gph.y_rows = E, N, N, E
         gph.x_index, gph.y_index, gph.seg_ptr, gph.perm = src.data_ptr(), None, plan.seg_ptr.data_ptr(), None
         pipelines = u1d._sm_count(dev) * int(mod.desc.ctas_per_sm)
-        split = N < u1d.SPLIT_ROWS_PER_PIPELINE * pipelines                 # shares as the operator cuts them
+        split = u1d.split_receivers(mod.desc, N, E, plan.max_degree, pipelines)     # shares as the operator cuts them
         n_parts = max(1, min(pipelines, N))
         part = plan.partition(n_parts, split)
         gph.part_ptr, gph.n_parts = part.data_ptr(), n_parts

@@ -190,6 +190,10 @@ int fasteq_core_abi_version(void);
 /* sorted_flag[0] (device int32) <- 1 if dst is non-decreasing else 0. */
 int fasteq_graph_check_sorted(const int32_t* dst, int64_t n_edges, int32_t* sorted_flag, fasteq_stream_t stream);
 
+/* The same and the edges of each row at once: result (device, 2 + n_rows int32) <- [1 if dst is NOT non-decreasing else 0,
+ * the largest count, the counts].  Indices outside [0, n_rows) are not counted. */
+int fasteq_graph_survey(const int32_t* dst, int64_t n_edges, int64_t n_rows, int32_t* result, fasteq_stream_t stream);
+
 /* CSR offsets of a non-decreasing receiver index: seg_ptr[r] = first position with dst >= r,
  * seg_ptr[n_rows] = n_edges.  Receiver indices outside [0, n_rows) are not reported: edges with a negative
  * index fall before row 0 and edges with an index >= n_rows after the last row, so no segment contains them
