@@ -69,6 +69,7 @@ def core():
         lib.fasteq_core_abi_version.restype = C.c_int
         lib.fasteq_graph_check_sorted.argtypes = [C.c_void_p, C.c_int64, C.c_void_p, C.c_void_p]
         lib.fasteq_graph_survey.argtypes = [C.c_void_p, C.c_int64, C.c_int64, C.c_void_p, C.c_void_p]
+        lib.fasteq_order_by_species.argtypes = [C.c_void_p, C.c_int64, C.c_void_p, C.c_void_p, C.c_void_p]
         lib.fasteq_graph_build_csr.argtypes = [C.c_void_p, C.c_int64, C.c_int64, C.c_void_p, C.c_void_p]
         lib.fasteq_graph_partition.argtypes = [C.c_void_p, C.c_int64, C.c_int64, C.c_int32, C.c_void_p, C.c_void_p]
         lib.fasteq_graph_partition_edges.argtypes = [C.c_void_p, C.c_int64, C.c_int64, C.c_int32, C.c_void_p, C.c_void_p, C.c_void_p]

@@ -359,32 +359,54 @@ __global__ void __launch_bounds__(NT) fasteq_stc_bwd_sum_kernel(const T* __restr
     L += [f"      ST(gxp + {a} * U, ga{a});" for a in range(spec.x1_segs)]
     L.append("    }\n  }\n}")
     L.append(r"""
-// gx0[s][d][u] = sum of the partial sums of species s: 32 channels by 8 interleaved shares of its CTAs, both in a fixed order
+// gx0[s][d][u] = sum of the partial sums of species s, for 32 channels and DS weights per CTA.  Bound by latency: the CTA looks the
+// species' nodes up together (256 positions at a time; two binary searches were twenty loads one after the other, 35 us of
+// a 67 us backward with 89 species), and few sums go one after the other in a thread per (channel, weight) while many go in eight
+// interleaved shares, with the same additions in the same order where both apply (the launch takes eight weights per CTA where a
+// species has about eight sums at most).
+template <int DS>
 __global__ void __launch_bounds__(256) fasteq_stc_sum_parts_kernel(const int* __restrict__ species, const T* __restrict__ partial,
     long long batch, int n_parts, T* __restrict__ gx0) {
   __shared__ T share[8][33];
-  const int s = blockIdx.x / D, d = blockIdx.x % D, u = blockIdx.y * 32 + threadIdx.x;
+  constexpr int GROUPS = (D + DS - 1) / DS;
+  const int s = blockIdx.x / GROUPS, d0 = blockIdx.x % GROUPS * DS, u = blockIdx.y * 32 + threadIdx.x;
+  const int tid = threadIdx.y * 32 + threadIdx.x;
   long long bound[2];                                  // first positions of species s and s + 1 in the order
   for (int e = 0; e < 2; ++e) {
-    long long a = e ? bound[0] : 0, b = batch;
-    while (a < b) {
-      const long long mid = (a + b) >> 1;
-      if (species[mid] < s + e) a = mid + 1; else b = mid;
+    long long a = e ? bound[0] : 0, n = batch - a;     // the answer is one of a .. a + n
+    while (n > 0) {
+      const long long step = (n + 255) / 256, at = tid * step;
+      const int below = __syncthreads_count(at < n && species[at < n ? a + at : a] < s + e);      // a prefix of the probes
+      if (below == 0) break;
+      const long long next = (long long)(below - 1) * step + 1, left = n - next;
+      a += next; n = left < step - 1 ? left : step - 1;
     }
     bound[e] = a;
   }
-  T sum = T(0);
-  if (bound[0] < bound[1] && u < U) {
-    // the CTA of position i is the largest c with floor(batch * c / n_parts) <= i
-    const long long first = ((bound[0] + 1) * n_parts - 1) / batch, last = (bound[1] * n_parts - 1) / batch;
-    for (long long c = first + threadIdx.y; c <= last; c += 8) sum += partial[((size_t)(c + s) * D + d) * U + u];
-  }
-  share[threadIdx.y][threadIdx.x] = sum;
-  __syncthreads();
-  if (threadIdx.y == 0 && u < U) {
-#pragma unroll
-    for (int k = 1; k < 8; ++k) sum += share[k][threadIdx.x];
+  const bool any = bound[0] < bound[1];
+  // the CTA of position i is the largest c with floor(batch * c / n_parts) <= i
+  const long long first = any ? ((bound[0] + 1) * n_parts - 1) / batch : 0, last = any ? (bound[1] * n_parts - 1) / batch : -1;
+  if (DS == 8 && last - first < 8) {
+    const int d = d0 + threadIdx.y;
+    if (d >= D || u >= U) return;
+    T sum = T(0);
+#pragma unroll 8
+    for (long long c = first; c <= last; ++c) sum += partial[((size_t)(c + s) * D + d) * U + u];
     gx0[((size_t)s * D + d) * U + u] = sum;
+    return;
+  }
+  for (int d = d0; d < D && d < d0 + DS; ++d) {
+    T sum = T(0);
+    if (u < U)
+      for (long long c = first + threadIdx.y; c <= last; c += 8) sum += partial[((size_t)(c + s) * D + d) * U + u];
+    share[threadIdx.y][threadIdx.x] = sum;
+    __syncthreads();
+    if (threadIdx.y == 0 && u < U) {
+#pragma unroll
+      for (int k = 1; k < 8; ++k) sum += share[k][threadIdx.x];
+      gx0[((size_t)s * D + d) * U + u] = sum;
+    }
+    if (DS > 1) __syncthreads();
   }
 }
 
@@ -428,8 +450,12 @@ extern "C" int fasteq_stc_backward_summed(const void* go, const void* x1, const 
   if (e != cudaSuccess) return cuda_fail(e);
   fasteq_stc_bwd_sum_kernel<<<(unsigned)n_parts, NT, 0, s>>>((const T*)go, (const T*)x1, (const T*)x0, (const long long*)order,
                                                              species_sorted, batch, n_species, (T*)gx1, (T*)partial, st);
-  fasteq_stc_sum_parts_kernel<<<dim3((unsigned)(n_species * D), (U + 31) / 32), dim3(32, 8), 0, s>>>(species_sorted, (const T*)partial,
-                                                                                                  batch, n_parts, (T*)gx0);
+  if (n_parts + n_species <= 8 * n_species)
+    fasteq_stc_sum_parts_kernel<8><<<dim3((unsigned)(n_species * ((D + 7) / 8)), (U + 31) / 32), dim3(32, 8), 0, s>>>(
+        species_sorted, (const T*)partial, batch, n_parts, (T*)gx0);
+  else
+    fasteq_stc_sum_parts_kernel<1><<<dim3((unsigned)(n_species * D), (U + 31) / 32), dim3(32, 8), 0, s>>>(
+        species_sorted, (const T*)partial, batch, n_parts, (T*)gx0);
   e = cudaGetLastError();
   return e == cudaSuccess ? FASTEQ_OK : cuda_fail(e);
 }

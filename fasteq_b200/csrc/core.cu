@@ -120,6 +120,46 @@ extern "C" int fasteq_graph_build_csr(const int32_t* dst, int64_t n_edges, int64
   return e == cudaSuccess ? FASTEQ_OK : cuda_fail(e);
 }
 
+// ---------------------------------------------------------------- nodes by species
+// A node's place in a stable order by species is the number of smaller species plus that of equal ones before it: one
+// comparison per pair of nodes, the species of all nodes in shared memory.  Bound by issue (n / 4 loads and 2 n instructions per
+// warp, a warp per scheduler).  torch's stable sort took 15 to 20 us of the summed backward of 200 to 3,000 nodes: 33 -> 14 us at 200,
+// 79 -> 72 at 3,000, 177 -> 167 at 8,000.
+constexpr int ORDER_MAX = 8192;
+
+__global__ void __launch_bounds__(128) species_order_kernel(const int* __restrict__ species, int n, long long* __restrict__ order,
+                                                            int* __restrict__ species_sorted) {
+  __shared__ __align__(16) int all[ORDER_MAX];
+  const int padded = (n + 31) & ~31;
+  for (int j = threadIdx.x; j < padded; j += 128) all[j] = j < n ? species[j] : 0x7fffffff;
+  __syncthreads();
+  const int i = blockIdx.x * 128 + threadIdx.x, warp_first = i & ~31;
+  if (warp_first >= n) return;
+  const int mine = all[i < padded ? i : 0];
+  int place = 0;
+#pragma unroll 4
+  for (int j = 0; j < warp_first; j += 4) {
+    const int4 v = *reinterpret_cast<const int4*>(all + j);
+    place += (v.x <= mine) + (v.y <= mine) + (v.z <= mine) + (v.w <= mine);
+  }
+  for (int j = warp_first; j < warp_first + 32; ++j) place += all[j] < mine || (all[j] == mine && j < i);
+#pragma unroll 4
+  for (int j = warp_first + 32; j < padded; j += 4) {
+    const int4 v = *reinterpret_cast<const int4*>(all + j);
+    place += (v.x < mine) + (v.y < mine) + (v.z < mine) + (v.w < mine);
+  }
+  if (i < n) { order[place] = i; species_sorted[place] = mine; }
+}
+
+extern "C" int fasteq_order_by_species(const int32_t* species, int64_t n, int64_t* order, int32_t* species_sorted, fasteq_stream_t stream) {
+  if (n < 0 || (n > 0 && (!species || !order || !species_sorted))) return FASTEQ_INVALID;
+  if (n > ORDER_MAX) return FASTEQ_UNSUPPORTED;
+  if (n == 0) return FASTEQ_OK;
+  species_order_kernel<<<(unsigned)((n + 127) / 128), 128, 0, (cudaStream_t)stream>>>(species, (int)n, (long long*)order, species_sorted);
+  cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? FASTEQ_OK : cuda_fail(e);
+}
+
 // ---------------------------------------------------------------- partition
 __global__ void partition_kernel(const int* __restrict__ seg_ptr, long long n_rows, long long n_edges, int n_parts,
                                  int* __restrict__ part_ptr) {

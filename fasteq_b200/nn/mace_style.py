@@ -127,7 +127,9 @@ class MACEStyleModel(torch.nn.Module):
         if self.fuse_geometry and not second_order and edge_geometry_usable(pos, self.num_basis):
             vec, radial = edge_geometry(pos, edge_src, edge_dst, edge_shift, self.r_max, self.num_basis, self.envelope_p)
         else:
-            # index_select: its gradient is one scatter launch, that of advanced indexing sorts the index first
+            # index_select: its gradient is one scatter launch, that of advanced indexing sorts the index first.  The scatter adds
+            # with atomics, so the last bits of the gradients of ``pos`` and ``embedding`` differ from run to run, as those
+            # of the sender features in the tensor products do; torch.use_deterministic_algorithms makes these two repeatable
             vec = pos.index_select(0, edge_src) + edge_shift - pos.index_select(0, edge_dst)
             r = vec.norm(dim=-1)
             radial = bessel_basis(r, self.r_max, self.num_basis) * polynomial_cutoff(r, self.r_max, self.envelope_p).unsqueeze(-1)

@@ -150,6 +150,23 @@ class FastSymmetricTensorContractionUniform1dFunction(torch.autograd.Function):
         return (gx1 if need_x1 else None), gx0, None, None, None, None, None, None
 
 
+# Up to here (32 KB of shared memory) one launch counts every node's place; its work grows with the square of the nodes, so that a
+# sort takes over beyond
+ORDER_BY_COUNTING = 8192
+
+
+def _by_species(species):
+    """``(species in ascending order, their nodes)``, nodes of equal species in their own order."""
+    n = species.numel()
+    if n > ORDER_BY_COUNTING:
+        return torch.sort(species, stable=True)
+    lib = _cabi.core()
+    ascending, order = torch.empty_like(species), torch.empty(n, dtype=torch.int64, device=species.device)
+    _cabi.check(lib.fasteq_order_by_species(species.data_ptr(), n, order.data_ptr(), ascending.data_ptr(), _cabi.stream(species.device)),
+                lib, "fasteq_order_by_species")
+    return ascending, order
+
+
 def _backward_summed(go, x1, x0, i32, spec):
     """``(grad_x1, grad_x0)`` with the weight gradient summed by species in the kernel (see ``_emit_summed_backward``)."""
     B, S = x1.shape[0], x0.shape[0]
@@ -158,7 +175,7 @@ def _backward_summed(go, x1, x0, i32, spec):
     with _cabi.on_device(x1.device):
         parts = C.c_int32(0)
         _cabi.check(lib.fasteq_stc_backward_summed_parts(B, C.byref(parts)), lib, "fasteq_stc_backward_summed_parts")
-        species, order = torch.sort(i32.view(-1), stable=True)
+        species, order = _by_species(i32.view(-1))
         partial = torch.empty((parts.value + S, spec.x0_segs, spec.u), dtype=x1.dtype, device=x1.device)
         _cabi.check(lib.fasteq_stc_backward_summed(go.data_ptr(), x1.data_ptr(), x0.data_ptr(), order.data_ptr(), species.data_ptr(),
                                                    B, S, parts.value, partial.data_ptr(), gx1.data_ptr(), gx0.data_ptr(),

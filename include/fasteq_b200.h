@@ -203,6 +203,10 @@ int fasteq_graph_survey(const int32_t* dst, int64_t n_edges, int64_t n_rows, int
 int fasteq_graph_build_csr(const int32_t* dst_sorted, int64_t n_edges, int64_t n_rows, int32_t* seg_ptr,
                            fasteq_stream_t stream);
 
+/* Stable order of n <= 8192 nodes by species (FASTEQ_UNSUPPORTED beyond): order [n] lists the nodes, species_sorted [n] their
+ * species in that order, as fasteq_stc_backward_summed takes them.  Any species values. */
+int fasteq_order_by_species(const int32_t* species, int64_t n, int64_t* order, int32_t* species_sorted, fasteq_stream_t stream);
+
 /* Split segments into n_parts contiguous ranges of about equal WORK, the work of a segment being its edge
  * count plus one (a receiver without edges still costs a row store): part_ptr[p] = first segment s with
  * seg_ptr[s] + s >= p * (n_edges + n_rows) / n_parts, part_ptr[n_parts] = n_rows. */

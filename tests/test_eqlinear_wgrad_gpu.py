@@ -22,10 +22,9 @@ def test_weight_gradient(dtype, tol, u, v, batch):
     wd = w.cuda().requires_grad_(True)
     (gw,) = torch.autograd.grad(fast_equi_linear(d, wd, x.cuda()), wd, go.cuda())
     xr, gr = x.double().reshape(batch, 12, u), go.double().reshape(batch, 9, v)
-    rows = [(0, 0, 1), (1, 1, 3), (4, 1, 3), (7, 4, 5)]
+    rows = [(0, 0, 1, 1), (1, 1, 3, 2), (4, 1, 3, 2), (7, 4, 5, 1)]      # first rows, rows, paths into the same output irrep
     got = gw.cpu().double().reshape(4, u, v)
-    for q, (i, o, n) in enumerate(rows):
-        want = torch.einsum("btu,btv->uv", xr[:, i:i + n], gr[:, o:o + n])
-        scale = (got[q] * want).sum() / (want * want).sum()            # the path's normalisation
-        err = (got[q] / scale - want).norm() / want.norm()
-        assert scale > 0 and err <= tol, (q, float(err))              # 2e-6: about 30 round-offs, blocked sums of 32 rows
+    for q, (i, o, n, into) in enumerate(rows):
+        want = torch.einsum("btu,btv->uv", xr[:, i:i + n], gr[:, o:o + n]) / (into * u) ** 0.5      # 1 / sqrt(fan-in)
+        err = (got[q] - want).norm() / want.norm()
+        assert err <= tol, (q, float(err))                            # 2e-6: about 30 round-offs, blocked sums of 32 rows
