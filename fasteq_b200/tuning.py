@@ -14,6 +14,8 @@ receiver's grad_out row (shared memory, L1, tensor memory) -- and the procedure 
   operator front-end asks ``lookup`` before it falls back to ``codegen.u1d.untuned`` (the heuristic default and one rule).
 
 ``python -m fasteq_b200.tuning`` sweeps the standard signatures and rewrites the file.
+The entries in the file were timed on shares of whole receivers, and without the configuration that ``codegen.u1d.untuned`` gives
+medium 64-channel rows; a sweep now cuts shares as the operator does and times that one too.
 """
 from __future__ import annotations
 
@@ -86,12 +88,12 @@ def smem_bytes(spec: U1DSpec, tun: _emit.Tuning, direction: str, need_gy: bool =
 
 
 def candidates(spec: U1DSpec, direction: str, needs=(True, True, True)) -> List[_emit.Tuning]:
-    """Launch configurations worth timing: the heuristic default and its neighbours in (two to six pipelines, thread
-    groups, ring depth, resident CTAs, passes; backward: the grad_out row staged in shared memory, read through L1 or
-    parked in tensor memory; L2 prefetch distance) that fit 227 KB of shared memory, 1024 threads per CTA and 512
-    columns of tensor memory."""
+    """Launch configurations worth timing: the heuristic default, what a signature without an entry runs with where that differs,
+    and the default's neighbours in (two to six pipelines, thread groups, ring depth, resident CTAs, passes; backward: the
+    grad_out row staged in shared memory, read through L1 or parked in tensor memory; L2 prefetch distance) that fit 227 KB of
+    shared memory, 1024 threads per CTA and 512 columns of tensor memory."""
     base = _emit.default_tuning(spec, direction)
-    out: List[_emit.Tuning] = [base]
+    out: List[_emit.Tuning] = list(dict.fromkeys([base, _emit.untuned(spec, direction)]))
     wpg = base.ct // (32 * base.vec)
     two_groups_ok = direction == "fwd" or not (spec.w_shared or spec.y_vec or spec.y_indexed or not spec.x_indexed)
 

@@ -120,3 +120,11 @@ def test_tensor_memory_columns_are_returned_on_every_consumer_exit():
     assert tail.index("bar.sync 1") < tail.index("scratch_tmem_free(")
     assert kernel.index("scratch_tmem_alloc(") < kernel.index("p.run(flush, begin);")
     assert consumer.count("if (!mbar_wait(") >= 1 and "break;" in consumer
+
+
+@pytest.mark.parametrize("in1,lmax", [("64x0e+64x1o", 3), ("128x0e+128x1o", 3)])
+@pytest.mark.parametrize("direction", ["fwd", "bwd"])
+def test_sweep_times_what_a_missing_entry_runs_with(in1, lmax, direction):
+    from fasteq_b200.prebuild import cwtp_spec
+    spec = cwtp_spec(in1, lmax, lmax, "f32")
+    assert gen.untuned(spec, direction) in tuning.candidates(spec, direction, (direction == "bwd",) * 3)
