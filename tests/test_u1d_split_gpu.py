@@ -52,3 +52,33 @@ def test_split_receivers_match_oracle(dtype, tol, kind, u, lmax, presorted):
     for name, got, want in zip(("out", "gw", "gx", "gy"), (out,) + grads, ref):
         err = np.abs(got.detach().cpu().double().numpy().reshape(want.shape) - want).max() / np.abs(want).max()
         assert err <= tol, (name, err)
+
+
+@pytest.mark.parametrize("presorted", [True, False])
+def test_operands_at_odd_addresses_of_a_tensor_memory_layout(presorted):
+    """55 segments of 64 channels park their gradient rows in tensor memory; at odd 4-byte addresses with one channel per thread."""
+    from fasteq_b200.codegen import u1d as gen
+    from fasteq_b200.ops import fast_uniform1d_jit
+    from fasteq_b200.ops import uniform1d_jit as u1d
+    sh = Irreps.spherical_harmonics(3)
+    io, ins = full_channelwise_instructions("64x0e+64x1o", sh, 3)
+    d = channelwise_tensor_product("64x0e+64x1o", sh, io, ins)
+    g = torch.Generator(device="cuda").manual_seed(9)
+    N, E = 37, 901
+    rand = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    operands = rand(E, d.w_seg_num * 64), rand(N, d.x_seg_num * 64), rand(E, d.y_seg_num), rand(N, d.out_seg_num * 64)
+    dst = torch.randint(0, N, (E,), device="cuda", generator=g, dtype=torch.int32)
+    dst = dst.sort().values if presorted else dst
+    src = torch.randint(0, N, (E,), device="cuda", generator=g, dtype=torch.int32)
+    odd = lambda t: torch.empty(t.numel() + 1, device="cuda")[1:].view(t.shape).copy_(t)
+
+    def run(w, x, y, r):
+        w, x, y = (t.requires_grad_(True) for t in (w, x, y))
+        out = fast_uniform1d_jit(w, x, y, {1: src}, {0: dst}, d.meta(torch.float32, "cuda"))
+        return (out.detach(),) + torch.autograd.grad(out, (w, x, y), r)
+
+    aligned = run(*(t.clone() for t in operands))
+    spec = next(s for s, direction, *_ in u1d._MODULES if direction == "bwd" and (s.u, s.out_segs) == (64, 55) and s.dtype == "f32")
+    assert gen.untuned(spec, "bwd").go_tmem
+    for a, b in zip(run(*(odd(t) for t in operands)), aligned):
+        assert (a - b).abs().max() <= 1e-5 * b.abs().max()           # two orders of the same FP32 sums
