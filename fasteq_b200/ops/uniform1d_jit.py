@@ -355,8 +355,9 @@ class _Call:
         return g, part_edge
 
 
-# Below this many receivers per pipeline shares may be cut between edges.
+# Below this many receivers per pipeline shares may be cut between edges, backward and forward.
 SPLIT_ROWS_PER_PIPELINE = 32
+SPLIT_ROWS_PER_PIPELINE_FORWARD = 14
 
 
 def split_receivers(desc: _cabi.U1DDesc, n_rows: int, n_edges: int, max_degree: int, pipelines: int) -> bool:
@@ -375,13 +376,17 @@ def split_receivers(desc: _cabi.U1DDesc, n_rows: int, n_edges: int, max_degree: 
     of 128 channels: 512 receivers of 8 edges 16.8 whole, 24.4 us cut; of 30 edges on average 48.3 and 42.6; of exactly 30 edges 30.1
     and 42.6; 4,000 receivers of 16 edges 97 and 102, of 30 edges 167 and 162; 55 segments of 64 channels, 2,000 of 30 edges 69.5
     and 60.9.  With these limits no forward of the sweep (529 graphs over seven signatures) is slower than on whole receivers by
-    more than two runs of one differ."""
+    more than two runs of one differ.  With many receivers per pipeline the cut gains nothing and the forward loses by it: 52 edges
+    on average, 55 segments of 128 channels, 4,000 receivers (7 per pipeline) 288 whole, 267 us cut; 6,000 (10) 411 and 393;
+    9,000 (15) 594 and 607; 12,288 (21) 803 and 862; FP64, 55 segments of 64 channels, 10 per pipeline 462 and 445, 15 675 and 721."""
     if n_edges == 0 or n_rows >= SPLIT_ROWS_PER_PIPELINE * pipelines:
         return False
     wide = desc.dtype == 1 and desc.out_segs > 64
     if desc.direction == 1:
         even = 4 * max_degree * n_rows <= 5 * n_edges and n_rows > pipelines
         return not (wide and even and -(-n_rows // pipelines) * max_degree * pipelines - n_edges < 8 * pipelines)
+    if n_rows >= SPLIT_ROWS_PER_PIPELINE_FORWARD * pipelines:
+        return False
     slow = wide or desc.u * (8 if desc.dtype == 1 else 4) % 16 != 0
     if n_rows <= pipelines:
         return max_degree * pipelines - n_edges >= (16 if slow else 32) * pipelines

@@ -18,11 +18,13 @@ def test_a_forward_is_cut_only_where_the_longest_receiver_outweighs_the_carries(
     assert not cut(192, 16, 25) and cut(192, 16, 25, u=33)                          # rows of 132 bytes: no bulk copies
     assert not cut(1024, 16, 29) and cut(1024, 16, 29, f64=True, out_segs=106)
     assert not cut(592 * u1d.SPLIT_ROWS_PER_PIPELINE, 50, 80) and not cut(5, 0, 0)
+    assert cut(6000, 52, 83) and not cut(9000, 52, 84) and not cut(12_288, 52, 83)  # many receivers per pipeline: nothing to gain
     # equal receivers that fill whole shares of the slowest rows
     even = lambda rows, degree, longest, **k: u1d.split_receivers(_desc(1, **k), rows, rows * degree, longest, 296)
     assert not even(2000, 8, 8, f64=True, out_segs=106) and not even(2000, 30, 30, f64=True, out_segs=106)
     assert even(2000, 8, 19, f64=True, out_segs=106) and even(1024, 30, 30, f64=True, out_segs=106) and even(2000, 8, 8)
     assert even(64, 8, 8, f64=True, out_segs=106)
+    assert u1d.split_receivers(_desc(1), 12_288, 12_288 * 52, 83, 592)
     # the backward carries nothing
     assert u1d.split_receivers(_desc(1), 512, 4096, 19, 592) and not u1d.split_receivers(_desc(1), 592 * 32, 592 * 32 * 50, 80, 592)
 
