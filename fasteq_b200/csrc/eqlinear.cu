@@ -18,6 +18,7 @@
 #include "core_common.h"
 #include "gemm_tf32x3.h"
 #include "fasteq_device.cuh"
+#include "wgrad_bf16x6.cuh"
 
 using namespace fasteq;
 
@@ -562,28 +563,24 @@ __device__ __forceinline__ int path_of_split(const WgradTable& tab, int num_path
   return q;
 }
 
-// FP32 weight gradient.  Bound: the FP32 pipe (a [64 .. 128] x 128 product per 512 .. 1024 bytes read), so the tile is 8 x 8
-// outputs per thread with packed two-column FMAs (32 issue slots per 64 multiply-adds leave room for the shared-memory
-// reads) and the rows come through a four-stage cp.async ring with one barrier per 16 rows.  The chunks that are summed on
-// their own are 32 rows.  TM x TN follows the extents (64 or 128 each): a 64-channel operand does not pay for a 128-wide tile.
+// FP32 weight gradient of a few rows (up to 128 a path; more go to the tensor cores): 64 x 64 tiles, 8 x 8 outputs per thread with packed
+// two-column FMAs (32 issue slots per 64 multiply-adds leave room for the shared-memory reads), rows through a four-stage
+// cp.async ring with one barrier per 16 rows.  Bound: latency, hence small tiles and many CTAs.  The chunks that are summed on
+// their own are 32 rows.
 // Rows of (batch, 2l + 1) blocks are addressed by one small multiplication per copy: `t / rows` is (t * inv) >> 16, exact for
 // t < 144 and rows <= 128 (the launcher sends longer blocks to the general kernel).
-// Measured with the reduction: [80000, 64]^T [80000, 1280] 1063 -> 324 us (40 TFLOP/s), [80000, 64]^T [80000, 64] 110 -> 35 us,
-// the 128-channel SO3Linear after the tensor product at 12,288 nodes 1425 -> 367 us; the error against FP64 fell by 10-40 %.
-constexpr int WG_BK = 16, WG_STAGES = 4, WG_MAX_ROWS = 128;
-__host__ __device__ constexpr int wg_threads(int tm, int tn) { return tm * tn / 64; }
-__host__ __device__ constexpr int wg_smem(int tm, int tn) { return WG_STAGES * WG_BK * (tm + tn) * (int)sizeof(float); }
+constexpr int WG_BK = 16, WG_STAGES = 4, WG_MAX_ROWS = 128, WG_TILE = 64, WG_THREADS = WG_TILE * WG_TILE / 64;
+constexpr int WG_SMEM = WG_STAGES * WG_BK * 2 * WG_TILE * (int)sizeof(float);
 
 __device__ __forceinline__ void cp_async16(void* dst, const void* src, bool valid) {
   const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(valid ? 16 : 0) : "memory");
 }
 
-template <int TM, int TN>
-__global__ void __launch_bounds__(wg_threads(TM, TN)) eqlinear_wgrad_f32_kernel(const __grid_constant__ WgradTable tab,
+__global__ void __launch_bounds__(WG_THREADS) eqlinear_wgrad_f32_kernel(const __grid_constant__ WgradTable tab,
     const float* __restrict__ X, const float* __restrict__ G, float* __restrict__ partial, long long batch, int in_rows,
     int out_rows, int u, int v, int num_paths, long long rows_per_split) {
-  constexpr int NTH = wg_threads(TM, TN), XP = WG_BK * TM / 4 / NTH, GP = WG_BK * TN / 4 / NTH;
+  constexpr int TM = WG_TILE, TN = WG_TILE, NTH = WG_THREADS, XP = WG_BK * TM / 4 / NTH, GP = WG_BK * TN / 4 / NTH;
   extern __shared__ __align__(16) float wg_ring[];
   float* sX = wg_ring;                                // [WG_STAGES][WG_BK][TM]
   float* sG = wg_ring + WG_STAGES * WG_BK * TM;       // [WG_STAGES][WG_BK][TN]
@@ -669,6 +666,213 @@ __global__ void __launch_bounds__(wg_threads(TM, TN)) eqlinear_wgrad_f32_kernel(
       const float2 s0 = vadd(acc[i][2 * h], part[i][2 * h]), s1 = vadd(acc[i][2 * h + 1], part[i][2 * h + 1]);
       *reinterpret_cast<float4*>(dst + (size_t)m * v + n) = make_float4(s0.x, s0.y, s1.x, s1.y);
     }
+  }
+}
+
+// The tensor-core kernel (see wgrad_bf16x6.cuh).  The M operand is the wider of X and G (`swap`: G), so that a 64-channel operand
+// sits on the N side.  A path's chunks are numbered irrep row by irrep row, `chunks_per_row` = ceil(batch / 32) to each.
+template <int TN>
+__global__ void __launch_bounds__(wg::THREADS, 1) eqlinear_wgrad_tc_kernel(const __grid_constant__ CUtensorMap tmM,
+    const __grid_constant__ CUtensorMap tmN, const __grid_constant__ WgradTable tab, const float* __restrict__ X,
+    const float* __restrict__ G, float* __restrict__ partial, long long batch, int in_rows, int out_rows, int u, int v, int num_paths,
+    int chunks_per_row, int chunks_per_split, int swap, int* status) {
+  using namespace fasteq::wg;
+  using namespace fasteq::tc;
+  constexpr int HALF = TN / 2, B_PART = b_part(TN), N_ROWS = ROWS * TN / 128, M_RAW = ROWS * TM, N_RAW = ROWS * TN;
+  extern __shared__ unsigned char wg_raw[];
+  unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(wg_raw) + 1023) & ~uintptr_t(1023));
+  float* raw_m = reinterpret_cast<float*>(smem + STAGES * 3 * B_PART);        // [RAW][ROWS][TM]
+  float* raw_n = raw_m + RAW * M_RAW;                                         // [RAW][ROWS][TN]
+  float* outer = raw_n + RAW * N_RAW;                                         // [HALF][256]: second-level sums of the drain threads
+  uint64_t* raw_full = reinterpret_cast<uint64_t*>(outer + TM * TN);          // [2][RAW] chunk of the M / N operand has landed
+  uint64_t* raw_empty = raw_full + 2 * RAW;                                   // [2][RAW] it has been read
+  uint64_t* full = raw_empty + 2 * RAW;                                       // [STAGES] both operands of a chunk split
+  uint64_t* empty = full + STAGES;                                            // [STAGES] its MMAs have read them
+  uint64_t* acc_full = empty + STAGES;                                        // [2]
+  uint64_t* acc_empty = acc_full + 2;                                         // [2]
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
+  int* redo = reinterpret_cast<int*>(tmem_slot + 1);                          // [2]: a sum is not finite; the largest |sum|'s bits
+
+  int split, tile;
+  decode_cta(tab, num_paths, &split, &tile);
+  const int q = path_of_split(tab, num_paths, split);
+  const int M = swap ? v : u, N = swap ? u : v;
+  const int n_tiles = (N + TN - 1) / TN, m0 = (tile / n_tiles) * TM, n0 = (tile % n_tiles) * TN;
+  const int first = (split - tab.split_first[q]) * chunks_per_split;
+  const int n_chunks = min(chunks_per_split, tab.rows[q] * chunks_per_row - first);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < 2 * RAW; ++s) { mbar_init(&raw_full[s], 1); mbar_init(&raw_empty[s], 4); }
+    for (int s = 0; s < STAGES; ++s) { mbar_init(&full[s], 8); mbar_init(&empty[s], 1); }
+    for (int b = 0; b < 2; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 8); }
+    mbar_fence_init();
+    redo[0] = 0; redo[1] = 0;
+  }
+  if (warp == 16) tmem_alloc(tmem_slot, 512);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_slot, tmem_a = tmem + 2 * TN;
+  float* dst = partial + (size_t)split * u * v;
+
+  if (warp < 8) {
+    const bool m_side = warp < 4;
+    uint64_t* landed = raw_full + (m_side ? 0 : RAW);
+    // TN = 64: two threads per channel of the N operand, 16 rows each
+    const int n = (threadIdx.x & 127) % TN, half_rows = ((threadIdx.x & 127) / TN) * N_ROWS;
+    const uint32_t lane_base = tmem_a + ((uint32_t)((warp & 3) * 32) << 16);
+    for (int i = 0; i < n_chunks; ++i) {
+      const int s = i % STAGES;
+      mbar_wait(&landed[i % RAW], (uint32_t)(i / RAW) & 1u, status);
+      mbar_wait(&empty[s], ((uint32_t)(i / STAGES) & 1u) ^ 1u, status);
+      if (m_side) {
+        tc_fence_after();
+        const float* c = raw_m + (i % RAW) * M_RAW + (threadIdx.x & 127);
+#pragma unroll
+        for (int ks = 0; ks < 2; ++ks) {
+          uint32_t p[3][8];
+#pragma unroll
+          for (int j = 0; j < 8; ++j)
+            split_pair(make_float2(c[(16 * ks + 2 * j) * TM], c[(16 * ks + 2 * j + 1) * TM]), p[0][j], p[1][j], p[2][j]);
+#pragma unroll
+          for (int e = 0; e < 3; ++e) tmem_st_8(lane_base + (uint32_t)(s * A_COLS + e * (ROWS / 2) + ks * 8), p[e]);
+        }
+        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+        tc_fence_before();
+      } else {
+        const float* c = raw_n + (i % RAW) * N_RAW + half_rows * TN + n;
+        unsigned char* st = smem + (size_t)s * 3 * B_PART + n * 64;
+#pragma unroll
+        for (int h = 0; h < N_ROWS / 8; ++h) {
+          uint32_t p[3][4];
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            split_pair(make_float2(c[(8 * h + 2 * j) * TN], c[(8 * h + 2 * j + 1) * TN]), p[0][j], p[1][j], p[2][j]);
+          const int chunk = ((half_rows / 8 + h) ^ ((n >> 1) & 3)) << 4;
+#pragma unroll
+          for (int e = 0; e < 3; ++e) *reinterpret_cast<uint4*>(st + e * B_PART + chunk) = make_uint4(p[e][0], p[e][1], p[e][2], p[e][3]);
+        }
+        fence_async_smem();
+      }
+      __syncwarp();
+      if (lane == 0) { mbar_arrive(&full[s]); mbar_arrive(&raw_empty[(m_side ? 0 : RAW) + i % RAW]); }
+    }
+  } else if (warp == 17) {
+    if (lane == 0) {
+      const int row_m = swap ? tab.out_row[q] : tab.in_row[q], row_n = swap ? tab.in_row[q] : tab.out_row[q];
+      int t = first / chunks_per_row, c = first - t * chunks_per_row;
+      for (int i = 0; i < n_chunks; ++i) {
+        const int s = i % RAW;
+        const uint32_t parity = ((uint32_t)(i / RAW) & 1u) ^ 1u;
+        mbar_wait(&raw_empty[s], parity, status);
+        mbar_arrive_expect_tx(&raw_full[s], (uint32_t)(M_RAW * 4));
+        tma_load_3d(raw_m + s * M_RAW, &tmM, m0, row_m + t, c * ROWS, &raw_full[s]);
+        mbar_wait(&raw_empty[RAW + s], parity, status);
+        mbar_arrive_expect_tx(&raw_full[RAW + s], (uint32_t)(N_RAW * 4));
+        tma_load_3d(raw_n + s * N_RAW, &tmN, n0, row_n + t, c * ROWS, &raw_full[RAW + s]);
+        if (++c == chunks_per_row) { c = 0; ++t; }
+      }
+    }
+  } else if (warp == 16) {
+    // an MMA holds up the thread that issues it until the ones before it are nearly done, hence a warp of its own
+    if (lane == 0) {
+      const uint32_t idesc = idesc_bf16_m128(TN);
+      for (int i = 0; i < n_chunks; ++i) {
+        const int s = i % STAGES, buf = i & 1;
+        mbar_wait(&acc_empty[buf], ((uint32_t)(i >> 1) & 1u) ^ 1u, status);
+        mbar_wait(&full[s], (uint32_t)(i / STAGES) & 1u, status);
+        tc_fence_after();
+        const uint32_t d = tmem + (uint32_t)(buf * TN), a = tmem_a + (uint32_t)(s * A_COLS), b = smem_u32(smem) + (uint32_t)(s * 3 * B_PART);
+        // smallest products first, so that the large sum is truncated in its own two steps only
+        constexpr int PA[6] = {2, 0, 1, 1, 0, 0}, PB[6] = {0, 2, 1, 0, 1, 0};
+#pragma unroll
+        for (int e = 0; e < 6; ++e)
+#pragma unroll
+          for (int ks = 0; ks < 2; ++ks)
+            mma_bf16_a_tmem(d, a + (uint32_t)(PA[e] * (ROWS / 2) + ks * 8), desc_sw64(b + (uint32_t)(PB[e] * B_PART + ks * 32)), idesc, (e | ks) ? 1u : 0u);
+        mma_commit(&empty[s]);
+        mma_commit(&acc_full[buf]);
+      }
+    }
+  } else {
+    const int quarter = warp & 3, half = (warp - 8) >> 2, t = threadIdx.x - 256;
+    const uint32_t cols = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(half * HALF);
+    float2 acc[HALF / 2];
+#pragma unroll
+    for (int j = 0; j < HALF / 2; ++j) acc[j] = make_float2(0.f, 0.f);
+    bool spilled = false;
+    for (int i = 0; i < n_chunks; ++i) {
+      const int buf = i & 1;
+      mbar_wait(&acc_full[buf], (uint32_t)(i >> 1) & 1u, status);
+      tc_fence_after();
+#pragma unroll
+      for (int c = 0; c < HALF / 16; ++c) {
+        uint32_t r[16];
+        tmem_ld_16(cols + (uint32_t)(buf * TN + c * 16), r);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc[c * 8 + j] = vadd(acc[c * 8 + j], make_float2(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1])));
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&acc_empty[buf]);
+      if ((i + 1) % OUTER == 0 || i + 1 == n_chunks) {
+#pragma unroll
+        for (int j = 0; j < HALF / 2; ++j) {
+          float* o = outer + 2 * j * 256 + t;
+          o[0] = spilled ? o[0] + acc[j].x : acc[j].x;
+          o[256] = spilled ? o[256] + acc[j].y : acc[j].y;
+          acc[j] = make_float2(0.f, 0.f);
+        }
+        spilled = true;
+      }
+    }
+    const int m = m0 + quarter * 32 + lane, nb = n0 + half * HALF;
+    const size_t sm = swap ? 1 : (size_t)v, sn = swap ? (size_t)v : 1;
+    float top = 0.f;
+    bool bad = false;
+    if (m < M) {
+#pragma unroll
+      for (int j = 0; j < HALF; j += 4) {
+        if (nb + j >= N) break;                  // extents are multiples of four
+        float o[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          o[k] = outer[(j + k) * 256 + t];
+          top = fmaxf(top, fabsf(o[k]));
+          bad = bad || !(fabsf(o[k]) <= 3.402823466e38f);
+        }
+        if (!swap) {
+          *reinterpret_cast<float4*>(dst + (size_t)m * v + nb + j) = make_float4(o[0], o[1], o[2], o[3]);
+        } else {
+#pragma unroll
+          for (int k = 0; k < 4; ++k) dst[(size_t)m * sm + (size_t)(nb + j + k) * sn] = o[k];
+        }
+      }
+    }
+    if (bad) atomicOr(&redo[0], 1);
+    atomicMax(&redo[1], __float_as_int(top));
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 16) { tc_fence_after(); tmem_dealloc(tmem, 512); }
+  const float largest = __int_as_float(redo[1]);
+  if (redo[0] == 0 && !(largest > 0.f && largest < 1e-20f)) return;
+  const float* Xq = X + (size_t)tab.in_row[q] * u;
+  const float* Gq = G + (size_t)tab.out_row[q] * v;
+  for (int e = threadIdx.x; e < TM * TN; e += THREADS) {
+    const int m = m0 + e % TM, n = n0 + e / TM;
+    if (m >= M || n >= N) continue;
+    const int iu = swap ? n : m, iv = swap ? m : n;
+    float sum = 0.f;
+    for (int c = first; c < first + n_chunks; ++c) {
+      const int t = c / chunks_per_row;
+      const long long b0 = (long long)(c - t * chunks_per_row) * ROWS, b1 = b0 + ROWS < batch ? b0 + ROWS : batch;
+      float part = 0.f;
+      for (long long b = b0; b < b1; ++b) part = fmaf(Xq[((size_t)b * in_rows + t) * u + iu], Gq[((size_t)b * out_rows + t) * v + iv], part);
+      sum += part;
+    }
+    dst[(size_t)iu * v + iv] = sum;
   }
 }
 
@@ -776,44 +980,64 @@ __global__ void __launch_bounds__(256) eqlinear_wgrad_reduce_kernel(const __grid
 // Shares the rows of all paths over whole waves of CTAs: for one to four waves the shortest equal share (a multiple of 32
 // rows, at least 128) that fits them, and of these the one that ends first, a CTA's fixed cost (fill, drain, its tile of
 // partial sums) counted as 64 rows.  Equal shares matter because paths have 1 to 2l + 1 rows per batch entry.
-long long plan_splits(const fasteq_eqlinear_problem* p, long long tiles, long long wave, WgradTable* tab) {
+long long plan_splits(const fasteq_eqlinear_problem* p, long long batch, long long tiles, long long wave, WgradTable* tab, long long fixed = 64) {
   auto count = [&](long long rps) {
     long long n = 0;
-    for (int q = 0; q < p->num_paths; ++q) n += (p->batch * p->rows[q] + rps - 1) / rps;
+    for (int q = 0; q < p->num_paths; ++q) n += (batch * p->rows[q] + rps - 1) / rps;
     return n * tiles;
   };
   long long longest = 128, best = 0, best_cost = 0;
-  for (int q = 0; q < p->num_paths; ++q) longest = std::max<long long>(longest, (p->batch * p->rows[q] + 31) / 32 * 32);
+  for (int q = 0; q < p->num_paths; ++q) longest = std::max<long long>(longest, (batch * p->rows[q] + 31) / 32 * 32);
   for (int k = 1; k <= 4; ++k) {
     long long lo = 4, hi = longest / 32;              // in units of 32 rows
     while (lo < hi) {
       const long long mid = (lo + hi) / 2;
       if (count(mid * 32) <= k * wave) hi = mid; else lo = mid + 1;
     }
-    const long long rps = lo * 32, waves = (count(rps) + wave - 1) / wave, cost = waves * (rps + 64);
+    const long long rps = lo * 32, waves = (count(rps) + wave - 1) / wave, cost = waves * (rps + fixed);
     if (!best || cost < best_cost) { best = rps; best_cost = cost; }
   }
   tab->split_first[0] = 0;
   for (int q = 0; q < p->num_paths; ++q)
-    tab->split_first[q + 1] = tab->split_first[q] + (int)((p->batch * p->rows[q] + best - 1) / best);
+    tab->split_first[q + 1] = tab->split_first[q] + (int)((batch * p->rows[q] + best - 1) / best);
   return best;
 }
 
-template <int TM, int TN>
 cudaError_t launch_wgrad_f32(const fasteq_eqlinear_problem* p, WgradTable* tab, int sms, const float* x, const float* go, float** partial,
                              cudaStream_t s) {
-  auto* kernel = eqlinear_wgrad_f32_kernel<TM, TN>;
   int per_sm = 0;
-  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, wg_smem(TM, TN));
-  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, wg_threads(TM, TN), wg_smem(TM, TN));
+  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, eqlinear_wgrad_f32_kernel, WG_THREADS, WG_SMEM);
   if (e != cudaSuccess) return e;
-  const int tiles = ((p->u + TM - 1) / TM) * ((p->v + TN - 1) / TN);
-  const long long rps = plan_splits(p, tiles, (long long)sms * std::max(per_sm, 1), tab);
+  const int tiles = ((p->u + WG_TILE - 1) / WG_TILE) * ((p->v + WG_TILE - 1) / WG_TILE);
+  const long long rps = plan_splits(p, p->batch, tiles, (long long)sms * std::max(per_sm, 1), tab);
   e = cudaMallocAsync((void**)partial, (size_t)tab->split_first[p->num_paths] * p->u * p->v * sizeof(float), s);
   if (e != cudaSuccess) return e;
-  kernel<<<(unsigned)tab->split_first[p->num_paths] * (unsigned)tiles, wg_threads(TM, TN), wg_smem(TM, TN), s>>>(
+  eqlinear_wgrad_f32_kernel<<<(unsigned)tab->split_first[p->num_paths] * (unsigned)tiles, WG_THREADS, WG_SMEM, s>>>(
       *tab, x, go, *partial, p->batch, p->in_rows, p->out_rows, p->u, p->v, p->num_paths, rps);
   return cudaGetLastError();
+}
+
+template <int TN>
+int launch_wgrad_tc(const fasteq_eqlinear_problem* p, WgradTable* tab, int sms, const float* x, const float* go, float** partial, cudaStream_t s) {
+  const bool swap = p->v > p->u;
+  const int M = swap ? p->v : p->u, N = swap ? p->u : p->v, tiles = ((M + wg::TM - 1) / wg::TM) * ((N + TN - 1) / TN);
+  const int m_rows = swap ? p->out_rows : p->in_rows, n_rows = swap ? p->in_rows : p->out_rows;
+  const long long chunks_per_row = (p->batch + wg::ROWS - 1) / wg::ROWS;
+  const long long rps = plan_splits(p, chunks_per_row * wg::ROWS, tiles, sms, tab, 256);
+  CUtensorMap mm, mn;
+  int rc = tc::make_map_rows(&mm, swap ? go : x, M, m_rows, p->batch, wg::TM, wg::ROWS);
+  if (rc == FASTEQ_OK) rc = tc::make_map_rows(&mn, swap ? x : go, N, n_rows, p->batch, TN, wg::ROWS);
+  if (rc != FASTEQ_OK) return rc;
+  int* status = nullptr;
+  cudaError_t e = tc::status_word(&status);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(eqlinear_wgrad_tc_kernel<TN>, cudaFuncAttributeMaxDynamicSharedMemorySize, wg::smem_bytes(TN));
+  if (e == cudaSuccess) e = cudaMallocAsync((void**)partial, (size_t)tab->split_first[p->num_paths] * p->u * p->v * sizeof(float), s);
+  if (e != cudaSuccess) return cuda_fail(e);
+  eqlinear_wgrad_tc_kernel<TN><<<(unsigned)tab->split_first[p->num_paths] * (unsigned)tiles, wg::THREADS, wg::smem_bytes(TN), s>>>(
+      mm, mn, *tab, x, go, *partial, p->batch, p->in_rows, p->out_rows, p->u, p->v, p->num_paths, (int)chunks_per_row, (int)(rps / wg::ROWS),
+      swap ? 1 : 0, status);
+  e = cudaGetLastError();
+  return e == cudaSuccess ? FASTEQ_OK : cuda_fail(e);
 }
 
 template <typename T>
@@ -840,18 +1064,21 @@ int launch_wgrad(const fasteq_eqlinear_problem* p, const void* x, const void* go
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (e != cudaSuccess) return cuda_fail(e);
   T* partial = nullptr;
-  if (sizeof(T) == 4 && p->u % 4 == 0 && p->v % 4 == 0 && max_rows <= WG_MAX_ROWS &&
-      ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(go)) & 15u) == 0) {   // 16-byte row pieces
-    const float *xf = (const float*)x, *gf = (const float*)go;
-    float** pf = (float**)&partial;
-    // up to 128 rows every path is one share, and what counts is how many CTAs start and how little each stores: 64 x 64 tiles
-    // whatever the extents (that SO3Linear 6.9 -> 5.4 us, at 16 nodes 17.0 -> 11.5; [32, 256]^T [32, 256] 9.1 -> 7.1)
-    if (p->batch * max_rows <= 128) e = launch_wgrad_f32<64, 64>(p, &tab, sms, xf, gf, pf, s);
-    else if (p->u <= 64) e = p->v <= 64 ? launch_wgrad_f32<64, 64>(p, &tab, sms, xf, gf, pf, s) : launch_wgrad_f32<64, 128>(p, &tab, sms, xf, gf, pf, s);
-    else                 e = p->v <= 64 ? launch_wgrad_f32<128, 64>(p, &tab, sms, xf, gf, pf, s) : launch_wgrad_f32<128, 128>(p, &tab, sms, xf, gf, pf, s);
+  const bool quads = sizeof(T) == 4 && p->u % 4 == 0 && p->v % 4 == 0 &&
+                     ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(go)) & 15u) == 0;   // 16-byte row pieces
+  const float *xf = (const float*)x, *gf = (const float*)go;
+  float** pf = (float**)&partial;
+  // The tensor cores from 129 rows on, in chunks of 32 batch entries of one irrep row (a batch below 16 would leave most of a chunk
+  // empty).  Up to 128 rows every path is one share, and what counts is how many CTAs start and how little each stores: the
+  // ten-path SO3Linear of 128 channels takes 9.7 us at 8 nodes and 18.5 on the tensor cores, at 33 nodes 22.9 and 18.9.
+  if (quads && p->batch >= 16 && p->batch * max_rows > 128 && p->batch <= 0x7fffffffLL && (p->batch / 32 + 1) * max_rows < (1LL << 30)) {
+    const int rc = std::min(p->u, p->v) <= 64 ? launch_wgrad_tc<64>(p, &tab, sms, xf, gf, pf, s) : launch_wgrad_tc<128>(p, &tab, sms, xf, gf, pf, s);
+    if (rc != FASTEQ_OK) return rc;
+  } else if (quads && max_rows <= WG_MAX_ROWS) {
+    e = launch_wgrad_f32(p, &tab, sms, xf, gf, pf, s);
   } else {
     const int tiles = ((p->u + BM - 1) / BM) * ((p->v + BN - 1) / BN);
-    const long long rps = plan_splits(p, tiles, (long long)sms * 4, &tab);
+    const long long rps = plan_splits(p, p->batch, tiles, (long long)sms * 4, &tab);
     e = cudaMallocAsync((void**)&partial, (size_t)tab.split_first[p->num_paths] * uv * sizeof(T), s);
     if (e == cudaSuccess) {
       eqlinear_wgrad_kernel<T><<<(unsigned)tab.split_first[p->num_paths] * (unsigned)tiles, NT, 0, s>>>(

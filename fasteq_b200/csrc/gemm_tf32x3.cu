@@ -720,23 +720,30 @@ static PFN_cuTensorMapEncodeTiled get_encode() {
   return fn;
 }
 
-// 3-D FP32 tensor [d2][d1][d0] (d0 contiguous), box [b2][b1][b0], 128-byte swizzle, zero fill outside
-int make_map(CUtensorMap* m, const float* base, uint64_t d0, uint64_t d1, uint64_t d2, uint64_t stride1_elems,
-                    uint64_t stride2_elems, uint32_t b0, uint32_t b1, uint32_t b2) {
+static int encode_map(CUtensorMap* m, const float* base, const cuuint64_t (&dims)[3], const cuuint64_t (&strides)[2], const cuuint32_t (&box)[3],
+                      CUtensorMapSwizzle swizzle) {
   PFN_cuTensorMapEncodeTiled enc = get_encode();
   if (!enc) return FASTEQ_INTERNAL;
-  cuuint64_t dims[3] = {d0, d1, d2};
-  cuuint64_t strides[2] = {stride1_elems * 4, stride2_elems * 4};
-  cuuint32_t box[3] = {b0, b1, b2};
-  cuuint32_t es[3] = {1, 1, 1};
+  const cuuint32_t es[3] = {1, 1, 1};
   CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float*>(base), dims, strides, box, es,
-                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                   CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) {
     snprintf(g_cuda_err, sizeof(g_cuda_err), "cuTensorMapEncodeTiled failed with CUresult %d", (int)r);
     return FASTEQ_CUDA_ERROR;
   }
   return FASTEQ_OK;
+}
+
+// 3-D FP32 tensor [d2][d1][d0] (d0 contiguous), box [b2][b1][b0], 128-byte swizzle, zero fill outside
+int make_map(CUtensorMap* m, const float* base, uint64_t d0, uint64_t d1, uint64_t d2, uint64_t stride1_elems,
+                    uint64_t stride2_elems, uint32_t b0, uint32_t b1, uint32_t b2) {
+  return encode_map(m, base, {d0, d1, d2}, {stride1_elems * 4, stride2_elems * 4}, {b0, b1, b2}, CU_TENSOR_MAP_SWIZZLE_128B);
+}
+
+int make_map_rows(CUtensorMap* m, const float* base, int width, int rows, long long batch, int box_width, int box_batch) {
+  return encode_map(m, base, {(cuuint64_t)width, (cuuint64_t)rows, (cuuint64_t)batch}, {(cuuint64_t)width * 4, (cuuint64_t)rows * width * 4},
+                    {(cuuint32_t)box_width, 1u, (cuuint32_t)box_batch}, CU_TENSOR_MAP_SWIZZLE_NONE);
 }
 
 bool supported(long long M, int a_rows, int K, int P, int N, int c_rows, const void* A, const void* Bt, const void* C) {
@@ -872,6 +879,8 @@ int dense(const float* A, const float* Bt, const float* split_in, float* C, long
   if (tmp) cudaFreeAsync(tmp, s);
   return rc;
 }
+
+cudaError_t status_word(int** word) { return cudaGetSymbolAddress((void**)word, g_tc_status); }
 
 int device_status(int* code) {
   int v = 0, zero = 0;

@@ -1,0 +1,74 @@
+"""FP32 weight gradient on the tensor cores (more than 128 rows): edges of its chunks of 32 batch entries, of its tiles and of its second-level
+sums, operands that bf16 parts cannot hold, and its error against the blocked FP32 sums it replaced."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _grad(g, x):
+    from fasteq_b200.ops.dense import _matmul_tn, tensorcore_device_status
+    out = _matmul_tn(g, x)
+    assert tensorcore_device_status() == 0
+    return out
+
+
+def _operands(m, n, k, scale=1.0):
+    gen = torch.Generator(device="cuda").manual_seed(m + n + k)
+    return [torch.randn(m, c, device="cuda", generator=gen) * scale for c in (n, k)]
+
+
+@pytest.mark.parametrize("m", [129, 160, 161, 512, 513, 5000, 100_003])
+@pytest.mark.parametrize("n,k", [(4, 4), (64, 64), (60, 128), (128, 68), (132, 128), (260, 132)])
+def test_against_float64(m, n, k):
+    g, x = _operands(m, n, k)
+    want = g.double().t() @ x.double()
+    # per chunk two truncated steps (2^-24 each) and one rounding, 16 chunks and up to 60 second-level sums in random walks: below
+    # 2^-24 * (2 + sqrt(8) + sqrt(30) / 4); the sums in chunks of 32 FP32 products reach 2.2e-7 at 100,000 rows
+    assert (_grad(g, x) - want).norm() <= 3e-7 * want.norm()
+
+
+@pytest.mark.parametrize("batch", [15, 16, 31, 33, 64, 100])
+def test_irrep_rows_of_short_batches(batch):
+    """Rows are 32 entries of one irrep row each: batches on both sides of a chunk, and of the limit of the tensor-core kernel."""
+    from fasteq_b200 import descriptors
+    from fasteq_b200.irreps import Irreps
+    from fasteq_b200.ops import fast_equi_linear
+    d = descriptors.linear(Irreps("64x0e+64x4e"), Irreps("132x4e+132x0e"))
+    gen = torch.Generator(device="cuda").manual_seed(batch)
+    x, go = (torch.randn(batch, 10 * c, device="cuda", generator=gen) for c in (64, 132))
+    w = torch.randn(d.num_weights, device="cuda", generator=gen).requires_grad_(True)
+    (gw,) = torch.autograd.grad(fast_equi_linear(d, w, x), w, go)
+    xr, gr = x.double().view(batch, 10, 64), go.double().view(batch, 10, 132)
+    got = gw.double().view(2, 64, 132)
+    for q, (i, o, n) in enumerate([(0, 9, 1), (1, 0, 9)]):
+        want = torch.einsum("btu,btv->uv", xr[:, i:i + n], gr[:, o:o + n]) / 8.0
+        assert (got[q] - want).norm() <= 3e-7 * want.norm()
+
+
+@pytest.mark.parametrize("value", [float("inf"), -float("inf"), float("nan"), 3.4e38])
+def test_values_beyond_bf16(value):
+    """Infinities and NaN reach exactly the sums they reach in FP32; a value bf16 would round to infinity stays finite."""
+    g, x = _operands(1000, 64, 132)
+    g[517, 3] = value
+    x[517] *= 1e-3
+    want = g.double().t() @ x.double()
+    got = _grad(g, x)
+    assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isposinf(), want.isposinf()) and torch.equal(got.isneginf(), want.isneginf())
+    fine = want.isfinite()
+    assert (got.double() - want)[fine].abs().max() <= 1e-6 * want[fine].abs().max()
+
+
+@pytest.mark.parametrize("scale", [1e-36, 1e-19, 1e18])
+def test_small_and_large_operands(scale):
+    g, x = _operands(700, 64, 64)
+    g, x = g * scale, (x if scale < 1e-30 else x * scale)
+    want = g.double().t() @ x.double()
+    # 1e-36: products near FP32's smallest normal number, rounded to multiples of 2^-149
+    assert (_grad(g, x).double() - want).norm() <= 3e-7 * want.norm() + (2.0 ** -149 * 700 * 64 if scale < 1e-18 else 0.0)
+
+
+def test_zero_and_repeat():
+    g, x = _operands(4000, 128, 128)
+    assert torch.equal(_grad(g, x), _grad(g, x))                     # fixed order of the sums
+    assert torch.count_nonzero(_grad(torch.zeros_like(g), x)) == 0
