@@ -88,6 +88,8 @@ class U1DModule:
         lib.fasteq_u1d_backward.argtypes = [C.POINTER(U1DGraph)] + [C.c_void_p] * 8
         lib.fasteq_u1d_forward_split.argtypes = [C.POINTER(U1DGraph)] + [C.c_void_p] * 7
         lib.fasteq_u1d_backward_split.argtypes = [C.POINTER(U1DGraph)] + [C.c_void_p] * 9
+        lib.fasteq_u1d_tangent_forward.argtypes = [C.POINTER(U1DGraph)] + [C.c_void_p] * 10
+        lib.fasteq_u1d_tangent_backward.argtypes = [C.POINTER(U1DGraph)] + [C.c_void_p] * 12
         lib.fasteq_u1d_device_status.argtypes = [C.POINTER(C.c_int32)]
         lib.fasteq_last_cuda_error.restype = C.c_char_p
         if hasattr(lib, "fasteq_u1d_forward_noalloc"):   # forward modules only
@@ -119,6 +121,14 @@ class U1DModule:
     def backward_split(self, graph: U1DGraph, part_edge: int, go: int, w: int, x: int, y: int, gw, gx, gy, stream: int) -> None:
         check(self.lib.fasteq_u1d_backward_split(C.byref(graph), part_edge, go, w, x, y, gw, gx, gy, stream), self.lib,
               "fasteq_u1d_backward_split")
+
+    def tangent_forward(self, graph: U1DGraph, part_edge, carry, *pointers) -> None:
+        """``pointers``: w, x, y, their tangents (None where the module has none), out, stream."""
+        check(self.lib.fasteq_u1d_tangent_forward(C.byref(graph), part_edge, carry, *pointers), self.lib, "fasteq_u1d_tangent_forward")
+
+    def tangent_backward(self, graph: U1DGraph, part_edge, *pointers) -> None:
+        """``pointers``: grad_out, w, x, y, their tangents, the three gradients, stream."""
+        check(self.lib.fasteq_u1d_tangent_backward(C.byref(graph), part_edge, *pointers), self.lib, "fasteq_u1d_tangent_backward")
 
     def device_status(self) -> int:
         v = C.c_int32(0)

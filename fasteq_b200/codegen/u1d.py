@@ -116,6 +116,10 @@ def untuned(spec: U1DSpec, direction: str) -> Tuning:
     columns at 55 segments) instead of two CTAs of four with 14 KB tiles each.  40 segments, 160,000 edges: 218 -> 208 us;
     55 segments, 80,533 edges: 146 -> 140 us.  Shorter rows have small tiles already, longer ones do not fit the columns."""
     base = default_tuning(spec, direction)
+    if direction == "bwd" and spec.dual and base.groups == 1 and spec.u % base.ct == 0 and tmem_columns(spec, base) <= 512:
+        # second order: two rows of every operand in a stage leave no room for the gradient tile beside a ring of any depth
+        fit = (_SMEM_BUDGET // base.pipes - 256) // _stage_bytes(spec, base.ct, base.ct // base.vec // 32 * spec.y_segs * spec.elem_bytes)
+        return replace(base, stages=max(2, min(4, fit)), min_blocks=1, go_smem=False, go_tmem=True)
     if direction != "bwd" or not (spec.scattered and base.vec == 2 and base.ct == 64 and 32 <= spec.out_segs <= 64):
         return base
     fit = (_SMEM_BUDGET // 8 - 256) // _stage_bytes(spec, 64, spec.y_segs * spec.elem_bytes)
@@ -133,11 +137,15 @@ def _stage_bytes(spec: U1DSpec, ct: int, extra: int) -> int:
     w = 0 if spec.w_shared else spec.w_segs * ct * e
     x = spec.x_segs * ct * e
     y = spec.y_segs * ct * e if spec.y_vec else (spec.y_segs * e + 15) // 16 * 16
+    if spec.dual:
+        w, x, y = w * (1 + spec.dual[0]), x * (1 + spec.dual[1]), y * (1 + spec.dual[2])
     return (w + x + y + 32 + extra + 127) // 128 * 128
 
 def _cfg(spec: U1DSpec, tun: Tuning, extra_bytes: int, ncons_warps: int, emit_empty: bool = True) -> str:
     b = lambda v: "true" if v else "false"
     vtype = "float2" if tun.vec == 2 else spec.ctype
+    dual = "" if not spec.dual else (f"#define FASTEQ_U1D_DUAL\nconstexpr bool DUAL_W = {b(spec.dual[0])}, DUAL_X = {b(spec.dual[1])}, "
+                                     f"DUAL_Y = {b(spec.dual[2])};\n")
     return f"""namespace cfg {{
 using T = {spec.ctype};
 using V = {vtype};   // what one thread carries per segment: one channel, or two packed FP32 channels
@@ -147,7 +155,7 @@ constexpr int PREFETCH = {tun.prefetch};
 constexpr bool EMIT_EMPTY_ROWS = {b(emit_empty)}, BEGIN_PER_SEGMENT = {b(not emit_empty)};
 constexpr bool Y_VEC = {b(spec.y_vec)}, W_SHARED = {b(spec.w_shared)}, X_INDEXED = {b(spec.x_indexed)}, Y_INDEXED = {b(spec.y_indexed)}, SCATTERED = {b(spec.scattered)};
 constexpr bool Y_SH = {b(bool(spec.y_sh))};   // the y operand holds edge vectors [rows, 3]; the producer evaluates their harmonics
-}}  // namespace cfg
+{dual}}}  // namespace cfg
 """ + (emit_sh_device(spec.y_sh[0], spec.dtype, spec.y_sh[1], spec.y_sh[2]) if spec.y_sh else SH_DEVICE_STUB)
 
 
@@ -368,15 +376,34 @@ def _vlit(c: float, dtype: str) -> str:
     return f"VS::bc({lit(c, dtype)})"
 
 
-def _sum_expr(items, dtype: str) -> List[str]:
+def _sum_expr(items, dtype: str, name: str = "t", p: str = "p") -> List[str]:
     """Statements computing ``t = sum c * p_j_k`` with fused multiply-adds."""
     out = []
     for n, (j, k, c) in enumerate(items):
         if n == 0:
-            out.append(f"V t = p_{j}_{k};" if c == 1.0 else f"V t = vmul({_vlit(c, dtype)}, p_{j}_{k});")
+            out.append(f"V {name} = {p}_{j}_{k};" if c == 1.0 else f"V {name} = vmul({_vlit(c, dtype)}, {p}_{j}_{k});")
         else:
-            out.append(f"t = vfma({_vlit(c, dtype)}, p_{j}_{k}, t);")
+            out.append(f"{name} = vfma({_vlit(c, dtype)}, {p}_{j}_{k}, {name});")
     return out
+
+
+def _tangent_pointers(spec: U1DSpec, ind: str) -> List[str]:
+    if not spec.dual:
+        return []
+    return [f"{ind}const T* sw2 = reinterpret_cast<const T*>(st + OFF_W2) + ch; (void)sw2;",
+            f"{ind}const T* sx2 = reinterpret_cast<const T*>(st + OFF_X2) + ch; (void)sx2;",
+            f"{ind}const T* sy2 = reinterpret_cast<const T*>(st + OFF_Y2); (void)sy2;",
+            "#define W2(i) VS::ld(sw2 + (i) * CT)"]
+
+
+def _tangent_products(spec: U1DSpec, products, ind: str) -> List[str]:
+    """``t_j_k``, the derivative of the product ``x[j] * y[k]`` along the tangents of x and y."""
+    _, dx, dy = spec.dual
+    L = []
+    for j, k in products:
+        e = [f"x2_{j}, y{k}"] * dx + [f"x{j}, y2_{k}"] * dy
+        L.append(f"{ind}const V t_{j}_{k} = " + (f"vmul({e[0]});" if len(e) == 1 else f"vfma({e[1]}, vmul({e[0]}));"))
+    return L
 
 
 def _load_xy(spec: U1DSpec, ind: str) -> List[str]:
@@ -385,6 +412,10 @@ def _load_xy(spec: U1DSpec, ind: str) -> List[str]:
         L += [f"{ind}const V y{k} = VS::ld(sy + {k} * CT);" for k in range(spec.y_segs)]
     else:
         L += [f"{ind}const V y{k} = VS::bc(sy[{k}]);" for k in range(spec.y_segs)]
+    if spec.dual and spec.dual[1]:
+        L += [f"{ind}const V x2_{j} = VS::ld(sx2 + {j} * CT);" for j in range(spec.x_segs)]
+    if spec.dual and spec.dual[2]:
+        L += [f"{ind}const V y2_{k} = VS::bc(sy2[{k}]);" for k in range(spec.y_segs)]
     return L
 
 
@@ -422,6 +453,8 @@ def _emit_block_fwd(spec: U1DSpec, b: Block, owned: set, slot_of: Dict[int, int]
     terms = [t for t in b.terms if t.v in owned]
     if not terms:
         return []
+    if spec.dual:
+        return _emit_block_fwd_dual(spec, terms, slot_of, ind)
     if _is_diagonal(terms):
         L = [ind + "{"]
         for kind, i, sh, c, ov in _diagonal_runs(terms):
@@ -443,8 +476,98 @@ def _emit_block_fwd(spec: U1DSpec, b: Block, owned: set, slot_of: Dict[int, int]
     return L
 
 
+def _sum_of(pairs) -> str:
+    """``a * b + c * d + ...`` of operand-name pairs."""
+    e = f"vmul({pairs[0][0]}, {pairs[0][1]})"
+    for a, b in pairs[1:]:
+        e = f"vfma({a}, {b}, {e})"
+    return e
+
+
+def _emit_block_fwd_dual(spec: U1DSpec, terms, slot_of: Dict[int, int], ind: str) -> List[str]:
+    """The derivative of a block's outputs along the tangents: ``w . t' + w' . t`` with ``t' = sum c p'`` of the product's derivatives."""
+    dw, dx, dy = spec.dual
+    L = [ind + "{"]
+    if _is_diagonal(terms):
+        for kind, i, sh, c, ov in _diagonal_runs(terms):
+            (S, O), (ds, do) = (("x", "y"), (dx, dy)) if kind == "x" else (("y", "x"), (dy, dx))
+            scaled = lambda e: e if c == 1.0 else f"vmul({_vlit(c, spec.dtype)}, {e})"
+            L.append(f"{ind}  {{")
+            along = [(f"W2({i})", f"{S}{sh}")] * dw + [(f"W({i})", f"{S}2_{sh}")] * ds       # d(w S)
+            if along:
+                L.append(f"{ind}    const V a = {scaled(_sum_of(along))};")
+            if do:
+                L.append(f"{ind}    const V b = {scaled(_sum_of([(f'W({i})', f'{S}{sh}')]))};")
+            for o, v in ov:
+                if along:
+                    L.append(f"{ind}    acc{slot_of[v]} = vfma(a, {O}{o}, acc{slot_of[v]});")
+                if do:
+                    L.append(f"{ind}    acc{slot_of[v]} = vfma(b, {O}2_{o}, acc{slot_of[v]});")
+            L.append(f"{ind}  }}")
+        return L + [ind + "}"]
+    used = sorted({(j, k) for t in terms for j, k, _ in t.items})
+    if dw:
+        L += [f"{ind}  const V p_{j}_{k} = vmul(x{j}, y{k});" for (j, k) in used]
+    if dx or dy:
+        L += _tangent_products(spec, used, ind + "  ")
+    for t in terms:
+        acc = f"acc{slot_of[t.v]}"
+        if dw:
+            L.append(f"{ind}  {{ " + " ".join(_sum_expr(t.items, spec.dtype)) + f" {acc} = vfma(W2({t.i}), t, {acc}); }}")
+        if dx or dy:
+            L.append(f"{ind}  {{ " + " ".join(_sum_expr(t.items, spec.dtype, "t", "t")) + f" {acc} = vfma(W({t.i}), t, {acc}); }}")
+    return L + [ind + "}"]
+
+
+def _dual_host(spec: U1DSpec):
+    """Parameters, null check, alignment and arguments of a second-order module's tangents, as text for its launcher."""
+    if not spec.dual:
+        return "", "", "", ""
+    names = [n for n, on in zip(("w2", "x2", "y2"), spec.dual) if on]
+    return ("const void* w2, const void* x2, const void* y2, ", "".join(f" || !{n}" for n in names),
+            "".join(f" && aligned16({n})" for n in names), ", (const T*)w2, (const T*)x2, (const T*)y2")
+
+
+# What a second-order module exports beside the description and the status word; the first-order entry points refuse.
+_DUAL_REFUSED = r"""
+extern "C" int fasteq_u1d_forward(const fasteq_u1d_graph*, const void*, const void*, const void*, void*, fasteq_stream_t) { return FASTEQ_UNSUPPORTED; }
+extern "C" int fasteq_u1d_forward_split(const fasteq_u1d_graph*, const int32_t*, void*, const void*, const void*, const void*, void*,
+                                        fasteq_stream_t) { return FASTEQ_UNSUPPORTED; }
+extern "C" int fasteq_u1d_backward(const fasteq_u1d_graph*, const void*, const void*, const void*, const void*, void*, void*, void*,
+                                   fasteq_stream_t) { return FASTEQ_UNSUPPORTED; }
+extern "C" int fasteq_u1d_backward_split(const fasteq_u1d_graph*, const int32_t*, const void*, const void*, const void*, const void*, void*,
+                                         void*, void*, fasteq_stream_t) { return FASTEQ_UNSUPPORTED; }
+"""
+_NO_TANGENT_FORWARD = r"""
+extern "C" int fasteq_u1d_tangent_forward(const fasteq_u1d_graph*, const int32_t*, void*, const void*, const void*, const void*, const void*,
+                                          const void*, const void*, void*, fasteq_stream_t) { return FASTEQ_UNSUPPORTED; }
+"""
+_NO_TANGENT_BACKWARD = r"""
+extern "C" int fasteq_u1d_tangent_backward(const fasteq_u1d_graph*, const int32_t*, const void*, const void*, const void*, const void*, const void*,
+                                           const void*, const void*, void*, void*, void*, fasteq_stream_t) { return FASTEQ_UNSUPPORTED; }
+"""
+_DUAL_FORWARD = r"""
+extern "C" int fasteq_u1d_tangent_forward(const fasteq_u1d_graph* gh, const int32_t* part_edge, void* carry, const void* w, const void* x,
+                                          const void* y, const void* w2, const void* x2, const void* y2, void* out, fasteq_stream_t stream) {
+  if (!gh || (part_edge && (!gh->part_ptr || gh->n_parts < 1 || !carry || gh->n_parts > gh->n_edges + gh->n_out_rows))) return FASTEQ_INVALID;
+  return run_forward(gh, part_edge, carry, w, x, y, w2, x2, y2, out, stream);
+}
+""" + _NO_TANGENT_BACKWARD + _DUAL_REFUSED
+_DUAL_BACKWARD = r"""
+extern "C" int fasteq_u1d_tangent_backward(const fasteq_u1d_graph* gh, const int32_t* part_edge, const void* go, const void* w, const void* x,
+                                           const void* y, const void* w2, const void* x2, const void* y2, void* gw, void* gx, void* gy,
+                                           fasteq_stream_t stream) {
+  if (!gh || (part_edge && (!gh->part_ptr || gh->n_parts < 1))) return FASTEQ_INVALID;
+  return run_backward(gh, part_edge, go, w, x, y, w2, x2, y2, gw, gx, gy, stream);
+}
+""" + _NO_TANGENT_FORWARD + _DUAL_REFUSED
+
+
 def emit_forward(spec: U1DSpec, tun: Tuning) -> str:
     _check_tuning(spec, tun)
+    host_params, host_null, host_aligned, host_args = _dual_host(spec)
+    dual_params = "" if not spec.dual else ", const T* __restrict__ w2, const T* __restrict__ x2, const T* __restrict__ y2"
+    set_tangents = "" if not spec.dual else " p.w2 = w2; p.x2 = x2; p.y2 = y2;"
     blocks = build_blocks(spec)
     G = tun.groups
     owners = split_out_segments(blocks, spec.out_segs, G)
@@ -463,7 +586,7 @@ constexpr int SMEM_BYTES = cfg::PIPES * PIPE_BYTES;
 
 __global__ void __launch_bounds__(NTHREADS, {tun.min_blocks})
 fasteq_u1d_fwd_kernel(const Graph g, const T* __restrict__ w, const T* __restrict__ x, const T* __restrict__ y,
-                      T* __restrict__ out, T* __restrict__ carry) {{
+                      T* __restrict__ out, T* __restrict__ carry{dual_params}) {{
   extern __shared__ __align__(128) unsigned char smem_all[];
   if (threadIdx.x == 0) {{
     for (int p = 0; p < cfg::PIPES; ++p) {{
@@ -484,7 +607,7 @@ fasteq_u1d_fwd_kernel(const Graph g, const T* __restrict__ w, const T* __restric
   unsigned char* stages = smem + BAR_BYTES;
   if (is_producer) {{
     Producer p{{g, w, x, y, stages, full, empty, lane, 0u, (int)blockIdx.x * cfg::PIPES + pipe}};
-    p.run([](unsigned char*) {{}}, [](int, int, int) {{}});
+{set_tangents and "   "}{set_tangents and set_tangents + chr(10)}    p.run([](unsigned char*) {{}}, [](int, int, int) {{}});
     return;
   }}
   const int ptid = threadIdx.x - pipe * cfg::NCONS_WARPS * 32;   // thread index inside the pipeline
@@ -506,7 +629,7 @@ fasteq_u1d_fwd_kernel(const Graph g, const T* __restrict__ w, const T* __restric
       const T* sy = reinterpret_cast<const T*>(st + OFF_Y){' + ch' if spec.y_vec else ''};
 {wdef}
 """)
-    body = _load_xy(spec, "      ")
+    body = _tangent_pointers(spec, "      ") + _load_xy(spec, "      ")
     for gi in range(G):
         owned = set(owners[gi])
         slot_of = {v: s for s, v in enumerate(owners[gi])}
@@ -571,19 +694,19 @@ __global__ void __launch_bounds__(256) fasteq_u1d_carry_kernel(const int* __rest
 }}
 
 static int run_forward(const fasteq_u1d_graph* gh, const int32_t* part_edge, void* carry, const void* w, const void* x, const void* y,
-                       void* out, fasteq_stream_t stream) {{
+                       {host_params}void* out, fasteq_stream_t stream) {{
   Graph g; int grid = 1;
   int rc = fill_graph(gh, &g, &grid, {tun.min_blocks});
   if (rc != FASTEQ_OK) return rc;
   if (gh->n_out_rows == 0 && gh->n_edges == 0) return FASTEQ_OK;
-  if (!out || (gh->n_edges > 0 && (!w || !x || !y))) return FASTEQ_INVALID;
+  if (!out || (gh->n_edges > 0 && (!w || !x || !y{host_null}))) return FASTEQ_INVALID;
   g.part_edge = part_edge;
-  g.bulk_ok = aligned16(w) && aligned16(x) && aligned16(y) && ((U * sizeof(T)) % 16 == 0) && ((CT * sizeof(T)) % 16 == 0);
+  g.bulk_ok = aligned16(w) && aligned16(x) && aligned16(y){host_aligned} && ((U * sizeof(T)) % 16 == 0) && ((CT * sizeof(T)) % 16 == 0);
   if (VEC == 2 && ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(carry)) & 7u)) return FASTEQ_INVALID;
   cudaError_t e = cudaFuncSetAttribute(fasteq_u1d_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
   if (e != cudaSuccess) return cuda_fail(e);
   fasteq_u1d_fwd_kernel<<<grid, NTHREADS, SMEM_BYTES, (cudaStream_t)stream>>>(
-      g, (const T*)w, (const T*)x, (const T*)y, (T*)out, (T*)carry);
+      g, (const T*)w, (const T*)x, (const T*)y, (T*)out, (T*)carry{host_args});
   if (part_edge)
     fasteq_u1d_carry_kernel<<<(unsigned)gh->n_parts, 256, 0, (cudaStream_t)stream>>>(
         gh->seg_ptr, gh->part_ptr, part_edge, gh->n_parts, (int)gh->n_out_rows, (const T*)carry, (T*)out);
@@ -592,6 +715,11 @@ static int run_forward(const fasteq_u1d_graph* gh, const int32_t* part_edge, voi
   return FASTEQ_OK;
 }}
 
+""")
+    if spec.dual:
+        src.append(_DUAL_FORWARD)
+        return "\n".join(src)
+    src.append(f"""
 extern "C" int fasteq_u1d_forward(const fasteq_u1d_graph* gh, const void* w, const void* x, const void* y, void* out,
                                   fasteq_stream_t stream) {{
   return run_forward(gh, nullptr, nullptr, w, x, y, out, stream);
@@ -615,6 +743,7 @@ extern "C" int fasteq_u1d_backward_split(const fasteq_u1d_graph*, const int32_t*
 }}
 """)
     src.append(_NOALLOC_FORWARD.replace("@MINB@", str(tun.min_blocks)))
+    src.append(_NO_TANGENT_FORWARD + _NO_TANGENT_BACKWARD)
     return "\n".join(src)
 
 
@@ -664,6 +793,10 @@ def emit_backward(spec: U1DSpec, tun: Tuning, need_gw: bool, need_gx: bool, need
     with warp shuffles, then across warps by the producer warp when the stage is recycled.
     """
     _check_tuning(spec, tun)
+    host_params, host_null, host_aligned, host_args = _dual_host(spec)
+    dual_params = "" if not spec.dual else ", const T* __restrict__ w2, const T* __restrict__ x2, const T* __restrict__ y2"
+    set_tangents = "" if not spec.dual else "    p.w2 = w2; p.x2 = x2; p.y2 = y2;\n"
+    dw, dx, dy = spec.dual or (False, False, False)
     G = tun.groups
     if G not in (1, 2):
         raise ValueError("the backward kernel takes one or two thread groups")
@@ -695,7 +828,7 @@ constexpr bool GY_ATOMIC = cfg::Y_INDEXED || (!cfg::Y_VEC && NCT > 1);
 
 __global__ void __launch_bounds__(NTHREADS, {tun.min_blocks})
 fasteq_u1d_bwd_kernel(const Graph g, const T* __restrict__ go, const T* __restrict__ w, const T* __restrict__ x,
-                      const T* __restrict__ y, T* __restrict__ gw, T* __restrict__ gx, T* __restrict__ gy) {{
+                      const T* __restrict__ y, T* __restrict__ gw, T* __restrict__ gx, T* __restrict__ gy{dual_params}) {{
   extern __shared__ __align__(128) unsigned char smem_all[];
   if (threadIdx.x == 0) {{
     for (int p = 0; p < cfg::PIPES; ++p) {{
@@ -730,7 +863,7 @@ fasteq_u1d_bwd_kernel(const Graph g, const T* __restrict__ go, const T* __restri
   unsigned char* gobuf = stages + STAGES * STAGE_BYTES;
   if (is_producer) {{
     Producer p{{g, w, x, y, stages, full, empty, lane, 0u, (int)blockIdx.x * cfg::PIPES + pipe}};
-    uint32_t nseg = 0;
+{set_tangents}    uint32_t nseg = 0;
     auto begin = [&](int row, int ct, int ln) {{
       if (NGO == 0) return;
       // stage the receiver's grad_out tile once per segment
@@ -842,7 +975,7 @@ fasteq_u1d_bwd_kernel(const Graph g, const T* __restrict__ go, const T* __restri
         L.append("#define GO(v) go_##v")       # loaded from tensor memory at the head of each block
     else:
         L.append("#define GO(v) VS::ld(sgo + (v) * CT)" if tun.go_smem else "#define GO(v) VS::ldg(sgo + (size_t)(v) * U)")
-    L += _load_xy(spec, "      ")
+    L += _tangent_pointers(spec, "      ") + _load_xy(spec, "      ")
     if need_gx:
         L += [f"      V gx{j} = VS::zero();" for j in range(spec.x_segs)]
     if need_gy and spec.y_vec:
@@ -909,6 +1042,64 @@ fasteq_u1d_bwd_kernel(const Graph g, const T* __restrict__ go, const T* __restri
             out.append(f"{ind}}}")
         return out
 
+    def dual_diag(b: Block, ind: str) -> List[str]:
+        # the gradients of (w S)' . d + w S . d' with d = sum_v go[v] O[v], the primes along the tangents
+        out = []
+        for kind, i, sh, c, ov in _diagonal_runs(b.terms):
+            (S, O), (ds, do) = (("x", "y"), (dx, dy)) if kind == "x" else (("y", "x"), (dy, dx))
+            need_gs, need_go = (need_gx, need_gy) if kind == "x" else (need_gy, need_gx)
+            scaled = lambda e: e if c == 1.0 else f"vmul({_vlit(c, dt)}, {e})"
+            out.append(f"{ind}{{")
+            if (need_gw and ds) or (need_gs and dw):
+                out.append(f"{ind}  const V d = {scaled(_sum_of([(f'GO({v})', f'{O}{o}') for o, v in ov]))};")
+            if (need_gw or need_gs) and do:
+                out.append(f"{ind}  const V e = {scaled(_sum_of([(f'GO({v})', f'{O}2_{o}') for o, v in ov]))};")
+            if need_gw:
+                for a, on, d in ((f"{S}2_{sh}", ds, "d"), (f"{S}{sh}", do, "e")):
+                    if on:
+                        out.append(f"{ind}  gw{i} = vfma({a}, {d}, gw{i});")
+            if need_gs:
+                g_ = f"g{S}{sh}"
+                for a, on, d in ((f"W2({i})", dw, "d"), (f"W({i})", do, "e")):
+                    if on:
+                        out.append(f"{ind}  {g_} = vfma({a}, {d}, {g_});")
+            along = [(f"W2({i})", f"{S}{sh}")] * dw + [(f"W({i})", f"{S}2_{sh}")] * ds
+            if need_go and along:
+                out.append(f"{ind}  const V s = {scaled(_sum_of(along))};")
+                for o, v in ov:
+                    out.append(f"{ind}  g{O}{o} = vfma(s, GO({v}), g{O}{o});")
+            out.append(f"{ind}}}")
+        return out
+
+    def dual_part(b: Block, ind: str) -> List[str]:
+        # S = sum_v go[v] (w t' + w' t):  gw += go t';  with q = sum c w go and q' = sum c w' go:  gx += q y' + q' y, gy += q x' + q' x
+        need_q, need_q2 = (need_gx and dy) or (need_gy and dx), (need_gx or need_gy) and dw
+        out = _tangent_products(spec, b.products, ind) if need_gw and (dx or dy) else []
+        for name, on in (("q", need_q), ("r", need_q2)):
+            if on:
+                out += [f"{ind}V {name}_{j}_{k};" for (j, k) in b.products]
+        seen = set()
+        for t in b.terms:
+            out.append(f"{ind}{{ const V gv = GO({t.v});")
+            if need_gw and (dx or dy):
+                out.append(f"{ind}  " + " ".join(_sum_expr(t.items, dt, "t", "t")) + f" gw{t.i} = vfma(gv, t, gw{t.i});")
+            for name, wt, on in (("q", f"W({t.i})", need_q), ("r", f"W2({t.i})", need_q2)):
+                if not on:
+                    continue
+                out.append(f"{ind}  const V g{name} = vmul({wt}, gv);")
+                for j, k, c in t.items:
+                    out.append(f"{ind}  {name}_{j}_{k} = " + (f"vfma({_vlit(c, dt)}, g{name}, {name}_{j}_{k});" if (j, k) in seen
+                                                             else f"vmul({_vlit(c, dt)}, g{name});"))
+            seen |= {(j, k) for j, k, _ in t.items}
+            out.append(f"{ind}}}")
+        for (j, k) in b.products:
+            for need, g_, own, on in ((need_gx, f"gx{j}", f"y{{}}{k}", dy), (need_gy, f"gy{k}", f"x{{}}{j}", dx)):
+                if need and on:
+                    out.append(f"{ind}{g_} = vfma(q_{j}_{k}, {own.format('2_')}, {g_});")
+                if need and dw:
+                    out.append(f"{ind}{g_} = vfma(r_{j}_{k}, {own.format('')}, {g_});")
+        return out
+
     for gi in range(G):
         gblocks = blocks if G == 1 else restrict_blocks(blocks, owners[gi])
         last_block_of_i: Dict[int, int] = {}
@@ -926,7 +1117,9 @@ fasteq_u1d_bwd_kernel(const Graph g, const T* __restrict__ go, const T* __restri
                 L += [f"      scratch_tmem_ld(tmem_go + {v}u * GO_COLS, go_{v});" for v in vs]
                 L.append(f"      scratch_tmem_wait_ld(go_{vs[0]});")
                 L += [f"      scratch_tmem_pin(go_{v});" for v in vs[1:]]
-            if _is_diagonal(b.terms):
+            if spec.dual:
+                L.append("      {"); L += (dual_diag if _is_diagonal(b.terms) else dual_part)(b, "        "); L.append("      }")
+            elif _is_diagonal(b.terms):
                 L.append("      {"); L += diag_part(b, "        "); L.append("      }")
             elif tun.two_pass or not (need_gw and need_q):
                 if need_gw:
@@ -1020,16 +1213,8 @@ fasteq_u1d_bwd_kernel(const Graph g, const T* __restrict__ go, const T* __restri
         elif not spec.y_vec:
             zero.append(f"if (gy && GY_ATOMIC) {{ e = cudaMemsetAsync(gy, 0, (size_t)gh->n_edges * {ycols} * sizeof(T), s); if (e != cudaSuccess) return cuda_fail(e); }}")
     src.append(f"""
-extern "C" int fasteq_u1d_forward(const fasteq_u1d_graph*, const void*, const void*, const void*, void*, fasteq_stream_t) {{
-  return FASTEQ_UNSUPPORTED;  // this module holds the backward kernel only
-}}
-extern "C" int fasteq_u1d_forward_split(const fasteq_u1d_graph*, const int32_t*, void*, const void*, const void*, const void*, void*,
-                                        fasteq_stream_t) {{
-  return FASTEQ_UNSUPPORTED;
-}}
-
 static int run_backward(const fasteq_u1d_graph* gh, const int32_t* part_edge, const void* go, const void* w, const void* x,
-                        const void* y, void* gw, void* gx, void* gy, fasteq_stream_t stream) {{
+                        const void* y, {host_params}void* gw, void* gx, void* gy, fasteq_stream_t stream) {{
   Graph g; int grid = 1;
   int rc = fill_graph(gh, &g, &grid, {tun.min_blocks});
   if (rc != FASTEQ_OK) return rc;
@@ -1038,19 +1223,32 @@ static int run_backward(const fasteq_u1d_graph* gh, const int32_t* part_edge, co
   {' '.join(zero)}
   if (gh->n_edges == 0) return FASTEQ_OK;          // per-edge buffers are empty (and may be null); the rest is zeroed
   if ((NEED_GW && !gw) || (NEED_GX && !gx) || (NEED_GY && !gy)) return FASTEQ_INVALID;
-  if (!go || !w || !x || !y) return FASTEQ_INVALID;
+  if (!go || !w || !x || !y{host_null}) return FASTEQ_INVALID;
   g.part_edge = part_edge;
-  g.bulk_ok = aligned16(w) && aligned16(x) && aligned16(y) && aligned16(go) && ((U * sizeof(T)) % 16 == 0) &&
+  g.bulk_ok = aligned16(w) && aligned16(x) && aligned16(y) && aligned16(go){host_aligned} && ((U * sizeof(T)) % 16 == 0) &&
               ((CT * sizeof(T)) % 16 == 0);
   if (VEC == 2 && ((reinterpret_cast<uintptr_t>(gw) | reinterpret_cast<uintptr_t>(gx) | reinterpret_cast<uintptr_t>(gy)) & 7u))
     return FASTEQ_INVALID;
   e = cudaFuncSetAttribute(fasteq_u1d_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
   if (e != cudaSuccess) return cuda_fail(e);
   fasteq_u1d_bwd_kernel<<<grid, NTHREADS, SMEM_BYTES, s>>>(g, (const T*)go, (const T*)w, (const T*)x, (const T*)y,
-                                                          (T*)gw, (T*)gx, (T*)gy);
+                                                          (T*)gw, (T*)gx, (T*)gy{host_args});
   e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e);
   return FASTEQ_OK;
+}}
+
+""")
+    if spec.dual:
+        src.append(_DUAL_BACKWARD)
+        return "\n".join(src)
+    src.append(f"""
+extern "C" int fasteq_u1d_forward(const fasteq_u1d_graph*, const void*, const void*, const void*, void*, fasteq_stream_t) {{
+  return FASTEQ_UNSUPPORTED;  // this module holds the backward kernel only
+}}
+extern "C" int fasteq_u1d_forward_split(const fasteq_u1d_graph*, const int32_t*, void*, const void*, const void*, const void*, void*,
+                                        fasteq_stream_t) {{
+  return FASTEQ_UNSUPPORTED;
 }}
 
 extern "C" int fasteq_u1d_backward(const fasteq_u1d_graph* gh, const void* go, const void* w, const void* x,
@@ -1065,6 +1263,7 @@ extern "C" int fasteq_u1d_backward_split(const fasteq_u1d_graph* gh, const int32
   return run_backward(gh, part_edge, go, w, x, y, gw, gx, gy, stream);
 }}
 """)
+    src.append(_NO_TANGENT_FORWARD + _NO_TANGENT_BACKWARD)
     return "\n".join(src)
 
 

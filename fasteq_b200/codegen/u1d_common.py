@@ -39,6 +39,7 @@ class U1DSpec:
     scattered: bool = True      # output rows summed over the edges of a receiver segment
     y_sh: tuple = ()            # (degrees, normalize, normalization): y rows are edge vectors [rows, 3] and the
                                 # kernel evaluates their spherical harmonics itself (scalar-y mode only)
+    dual: tuple = ()            # (w, x, y): second-order module, with a tangent row beside each operand marked True
 
     def __hash__(self) -> int:
         # specs key the module and tuning caches on every operator call; the path table has hundreds of entries, so its
@@ -46,7 +47,7 @@ class U1DSpec:
         h = self.__dict__.get("_hash")
         if h is None:
             h = hash((self.paths, self.w_segs, self.x_segs, self.y_segs, self.out_segs, self.u, self.dtype, self.y_vec,
-                      self.w_shared, self.x_indexed, self.y_indexed, self.scattered, self.y_sh))
+                      self.w_shared, self.x_indexed, self.y_indexed, self.scattered, self.y_sh, self.dual))
             object.__setattr__(self, "_hash", h)
         return h
 
@@ -62,6 +63,8 @@ class U1DSpec:
         h = hashlib.sha256()
         h.update(repr((self.paths, self.w_segs, self.x_segs, self.y_segs, self.out_segs, self.u, self.dtype,
                        self.y_vec, self.w_shared, self.x_indexed, self.y_indexed, self.scattered, self.y_sh, extra)).encode())
+        if self.dual:
+            h.update(repr(self.dual).encode())
         return h.hexdigest()[:16]
 
 

@@ -34,7 +34,16 @@ constexpr int Y_TILE_BYTES = cfg::Y_VEC ? YSEG * CT * (int)sizeof(T) : round_up(
 constexpr int OFF_W = 0;
 constexpr int OFF_X = OFF_W + W_TILE_BYTES;
 constexpr int OFF_Y = OFF_X + X_TILE_BYTES;
-constexpr int OFF_META = OFF_Y + Y_TILE_BYTES;
+// second-order modules (per-edge weights, gathered x, scalar y): the tangents' rows of the same edge, where there are any
+#ifdef FASTEQ_U1D_DUAL
+constexpr bool W2 = cfg::DUAL_W, X2 = cfg::DUAL_X, Y2 = cfg::DUAL_Y;
+#else
+constexpr bool W2 = false, X2 = false, Y2 = false;
+#endif
+constexpr int OFF_W2 = OFF_Y + Y_TILE_BYTES;
+constexpr int OFF_X2 = OFF_W2 + (W2 ? W_TILE_BYTES : 0);
+constexpr int OFF_Y2 = OFF_X2 + (X2 ? X_TILE_BYTES : 0);
+constexpr int OFF_META = OFF_Y2 + (Y2 ? Y_TILE_BYTES : 0);
 constexpr int OFF_EXTRA = OFF_META + 32;          // per-stage scratch the backward uses (gy partials)
 constexpr int STAGE_BYTES = round_up(OFF_EXTRA + cfg::STAGE_EXTRA_BYTES, 128);
 constexpr int BAR_BYTES = 256;                    // full[STAGES], empty[STAGES], aux barriers
@@ -83,10 +92,11 @@ struct Producer {
   // this pipeline's carry row instead of the output), else 0
   int carry = 0;
   bool failed = false;   // a wait of this lane gave up: the warp stops issuing copies and reductions (see dead())
+  const T* w2 = nullptr; const T* x2 = nullptr; const T* y2 = nullptr;   // tangents (second-order modules)
 
   static __device__ __forceinline__ int valid_of(int ct) { return (U - ct * CT) < CT ? (U - ct * CT) : CT; }
   static __device__ __forceinline__ uint32_t tx_bytes(int valid) {
-    return (uint32_t)((cfg::W_SHARED ? 0 : WSEG) + XSEG + (cfg::Y_VEC ? YSEG : 0)) * (uint32_t)(valid * sizeof(T));
+    return (uint32_t)((cfg::W_SHARED ? 0 : WSEG) + XSEG + (cfg::Y_VEC ? YSEG : 0) + (W2 ? WSEG : 0) + (X2 ? XSEG : 0)) * (uint32_t)(valid * sizeof(T));
   }
   __device__ __forceinline__ int checked(int r, long long n) {
     if (r < 0 || (long long)r >= n) { atomicExch(g.status, (int)kDevBadIndex); return 0; }
@@ -122,6 +132,21 @@ struct Producer {
         const T* src = x + (size_t)xr * XSEG * U;
         if (FULL_ROW) bulk_g2s(st + OFF_X, src, (uint32_t)(XSEG * U * sizeof(T)), &full[stage]);
         else for (int s = 0; s < XSEG; ++s) bulk_g2s(st + OFF_X + (size_t)s * CT * sizeof(T), src + (size_t)s * U + ct * CT, piece, &full[stage]);
+      }
+      if (W2) {
+        const T* src = w2 + (size_t)e * WSEG * U;
+        if (FULL_ROW) bulk_g2s(st + OFF_W2, src, (uint32_t)(WSEG * U * sizeof(T)), &full[stage]);
+        else for (int s = 0; s < WSEG; ++s) bulk_g2s(st + OFF_W2 + (size_t)s * CT * sizeof(T), src + (size_t)s * U + ct * CT, piece, &full[stage]);
+      }
+      if (X2) {
+        const T* src = x2 + (size_t)xr * XSEG * U;
+        if (FULL_ROW) bulk_g2s(st + OFF_X2, src, (uint32_t)(XSEG * U * sizeof(T)), &full[stage]);
+        else for (int s = 0; s < XSEG; ++s) bulk_g2s(st + OFF_X2 + (size_t)s * CT * sizeof(T), src + (size_t)s * U + ct * CT, piece, &full[stage]);
+      }
+      if (Y2) {
+        const T* src = y2 + (size_t)yr * YSEG;
+#pragma unroll
+        for (int k = 0; k < YSEG; ++k) cp_async_elem(st + OFF_Y2 + k * sizeof(T), src + k);
       }
       if (cfg::Y_VEC) {
         const T* src = y + (size_t)yr * YSEG * U;
@@ -197,6 +222,9 @@ struct Producer {
       const int valid = valid_of(ct);
       if (!cfg::W_SHARED) copy_tile(st + OFF_W, w + (size_t)e * WSEG * U, WSEG, ct, valid, false, &full[stage], lane);
       copy_tile(st + OFF_X, x + (size_t)xr * XSEG * U, XSEG, ct, valid, false, &full[stage], lane);
+      if (W2) copy_tile(st + OFF_W2, w2 + (size_t)e * WSEG * U, WSEG, ct, valid, false, &full[stage], lane);
+      if (X2) copy_tile(st + OFF_X2, x2 + (size_t)xr * XSEG * U, XSEG, ct, valid, false, &full[stage], lane);
+      if (Y2) for (int k = lane; k < YSEG; k += 32) cp_async_elem(st + OFF_Y2 + k * sizeof(T), y2 + (size_t)yr * YSEG + k);
       if (cfg::Y_VEC) copy_tile(st + OFF_Y, y + (size_t)yr * YSEG * U, YSEG, ct, valid, false, &full[stage], lane);
       else if (!cfg::Y_SH) for (int k = lane; k < YSEG; k += 32) cp_async_elem(st + OFF_Y + k * sizeof(T), y + (size_t)yr * YSEG + k);
     }

@@ -14,8 +14,14 @@ def wanted(ctx, i: int) -> bool:
     is not the one running under functional transforms) the gradient counts as wanted."""
     if not ctx.needs_input_grad[i]:
         return False
-    if not torch.is_grad_enabled():
-        return True
+    return True if not torch.is_grad_enabled() else asked(ctx, i)
+
+
+def asked(ctx, i: int) -> bool:
+    """``wanted`` in every pass: the loss of a training step is differentiated with respect to the weights, and nobody asks for the
+    gradients of the edge harmonics there."""
+    if not ctx.needs_input_grad[i]:
+        return False
     try:
         return bool(torch._C._will_engine_execute_node(ctx.next_functions[i][0]))
     except (RuntimeError, AttributeError, IndexError, TypeError):

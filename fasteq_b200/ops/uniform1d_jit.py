@@ -16,6 +16,7 @@ built once per index tensor and cached.
 from __future__ import annotations
 
 import ctypes
+import dataclasses
 import threading
 from collections import OrderedDict
 from contextlib import contextmanager
@@ -28,8 +29,9 @@ from .. import _build, _cabi
 from .. import tuning as _tuning
 from ..codegen import u1d as _emit
 from ..codegen.u1d_common import U1DSpec, make_spec
+from ._needs import asked
 
-_EMITTER_VERSION = "u1d-v6"
+_EMITTER_VERSION = "u1d-v7"
 _MODULES: Dict[Tuple, _cabi.U1DModule] = {}
 _TUNING_OVERRIDE: Dict[str, _emit.Tuning] = {}
 _lock = threading.Lock()
@@ -421,7 +423,6 @@ def _tuning_for(spec: U1DSpec, direction: str, tensors, needs=(False, False, Fal
     offset (a contiguous view into a larger buffer) get the one-channel-per-thread module instead."""
     tun = _TUNING_OVERRIDE.get(direction) or _tuning.lookup(spec, direction, needs) or _emit.untuned(spec, direction)
     if tun.vec == 2 and any(t is not None and t.data_ptr() % 8 for t in tensors):
-        import dataclasses
         return dataclasses.replace(tun, vec=1, pipes=1, groups=max(tun.groups, 1), min_blocks=min(tun.min_blocks + 1, 3))
     return tun
 
@@ -459,17 +460,77 @@ def _run_bwd(call: _Call, grad_out, w, x, y, needs):
     return gw, gx, gy
 
 
+_DUAL_SPECS: Dict[Tuple[U1DSpec, Tuple[bool, bool, bool]], U1DSpec] = {}
+
+
+def _dual_spec(spec: U1DSpec, has: Tuple[bool, bool, bool]) -> Optional[U1DSpec]:
+    """The second-order signature with tangents where ``has`` says so; ``None`` for the operand forms without such modules."""
+    if not (spec.scattered and spec.x_indexed) or spec.w_shared or spec.y_vec or spec.y_indexed or spec.y_sh:
+        return None
+    hit = _DUAL_SPECS.get((spec, has))
+    if hit is None:
+        if len(_DUAL_SPECS) > 256:
+            _DUAL_SPECS.clear()
+        hit = _DUAL_SPECS[(spec, has)] = dataclasses.replace(spec, dual=has)
+    return hit
+
+
+def _second_order(call: _Call, go, w, x, y, tangents, wants):
+    """``(d_go, d_w, d_x, d_y)`` of ``<go, F(w', x, y) + F(w, x', y) + F(w, x, y')>``, ``tangents = (w', x', y')`` with ``None`` for those that
+    are zero: one pass over the edges for the first and one for the others."""
+    has = tuple(t is not None for t in tangents)
+    spec = _dual_spec(call.spec, has)
+    if spec is None:
+        return _second_order_composed(call, go, w, x, y, tangents, wants)
+    dev, ptr = x.device, lambda t: t.data_ptr() if t is not None else None
+    operands = tuple(ptr(t) for t in (w, x, y) + tangents)
+    out = [None] * 4
+    with _cabi.on_device(dev):
+        stream = _cabi.stream(dev)
+        if wants[0]:
+            out[0] = torch.empty((call.n_out_rows, call.out_segs * call.u), dtype=x.dtype, device=dev)
+            mod = get_module(spec, "fwd", tuning=_tuning_for(spec, "fwd", (w, x, y, out[0]) + tangents))
+            g, part_edge = call.graph(mod, dev)
+            carry = torch.empty((g.n_parts, call.out_segs * call.u), dtype=x.dtype, device=dev) if part_edge is not None else None
+            mod.tangent_forward(g, part_edge, ptr(carry), *operands, out[0].data_ptr(), stream)
+        # a gradient needs a tangent on another operand
+        needs = tuple(wants[1 + i] and any(has[j] for j in range(3) if j != i) for i in range(3))
+        if any(needs):
+            out[1:] = [torch.empty_like(t) if n else None for t, n in zip((w, x, y), needs)]
+            mod = get_module(spec, "bwd", needs, tuning=_tuning_for(spec, "bwd", (go, w, x, y, *out[1:]) + tangents, needs))
+            g, part_edge = call.graph(mod, dev)
+            mod.tangent_backward(g, part_edge, go.data_ptr(), *operands, *(ptr(t) for t in out[1:]), stream)
+    return tuple(out)
+
+
+def _second_order_composed(call: _Call, go, w, x, y, tangents, wants):
+    """The same from first-order launches.  The operator is trilinear in (w, x, y), so every term is a forward or a one-gradient backward of
+    the same signature with an operand swapped for its tangent:
+
+        d_go = F(w', x, y) + F(w, x', y) + F(w, x, y')
+        d_w  = Bw(go; x', y) + Bw(go; x, y')      (Bw = gradient with respect to the weight slot)
+        d_x  = Bx(go; w', y) + Bx(go; w, y')
+        d_y  = By(go; w', x) + By(go; w, x')
+    """
+    operands = (w, x, y)
+    out = [None] * 4
+
+    def swapped(i):
+        return tuple(tangents[i] if k == i else t for k, t in enumerate(operands))
+
+    for i, t in enumerate(tangents):
+        if t is None:
+            continue
+        terms = [(0, _run_fwd(call, *swapped(i)))] if wants[0] else []
+        terms += [(1 + k, _run_bwd(call, go, *swapped(i), tuple(n == k for n in range(3)))[k]) for k in range(3) if k != i and wants[1 + k]]
+        for k, v in terms:
+            out[k] = v if out[k] is None else out[k] + v
+    return tuple(out)
+
+
 class FastUniform1dBackwardFunction(torch.autograd.Function):
     """First backward as a differentiable function (reference: fasteq/ops/uniform1d_jit.py:3098-3188),
-    so that force losses can be trained.  The operator is trilinear in (w, x, y), hence every term of
-    the second backward is again a forward or a one-gradient backward of the same signature with two
-    operands swapped for incoming second-order gradients; no separate double-backward kernels exist:
-
-        d_go = F(ggw, x, y) + F(w, ggx, y) + F(w, x, ggy)
-        d_w  = Bw(go; ggx, y) + Bw(go; x, ggy)      (Bw = gradient with respect to the weight slot)
-        d_x  = Bx(go; ggw, y) + Bx(go; w, ggy)
-        d_y  = By(go; ggw, x) + By(go; w, ggx)
-    """
+    so that force losses can be trained; its own backward is ``_second_order``."""
 
     @staticmethod
     def forward(ctx, grad_out, w, x, y, call, needs):
@@ -481,41 +542,13 @@ class FastUniform1dBackwardFunction(torch.autograd.Function):
         return outs
 
     @staticmethod
-    def backward(ctx, ggw, ggx, ggy):
+    def backward(ctx, *tangents):
         go, w, x, y = ctx.saved_tensors
-        call, needs = ctx.call, ctx.needs
-        ggw = ggw.contiguous() if (ggw is not None and needs[0]) else None
-        ggx = ggx.contiguous() if (ggx is not None and needs[1]) else None
-        ggy = ggy.contiguous() if (ggy is not None and needs[2]) else None
-        want_go, want_w, want_x, want_y = ctx.needs_input_grad[:4]
-
-        def add(a, b):
-            return b if a is None else (a if b is None else a + b)
-
-        d_go = d_w = d_x = d_y = None
-        if want_go:
-            if ggw is not None:
-                d_go = add(d_go, _run_fwd(call, ggw, x, y))
-            if ggx is not None:
-                d_go = add(d_go, _run_fwd(call, w, ggx, y))
-            if ggy is not None:
-                d_go = add(d_go, _run_fwd(call, w, x, ggy))
-        if want_w:
-            if ggx is not None:
-                d_w = add(d_w, _run_bwd(call, go, w, ggx, y, (True, False, False))[0])
-            if ggy is not None:
-                d_w = add(d_w, _run_bwd(call, go, w, x, ggy, (True, False, False))[0])
-        if want_x:
-            if ggw is not None:
-                d_x = add(d_x, _run_bwd(call, go, ggw, x, y, (False, True, False))[1])
-            if ggy is not None:
-                d_x = add(d_x, _run_bwd(call, go, w, x, ggy, (False, True, False))[1])
-        if want_y:
-            if ggw is not None:
-                d_y = add(d_y, _run_bwd(call, go, ggw, x, y, (False, False, True))[2])
-            if ggx is not None:
-                d_y = add(d_y, _run_bwd(call, go, w, ggx, y, (False, False, True))[2])
-        return d_go, d_w, d_x, d_y, None, None
+        tangents = tuple(t.contiguous() if (t is not None and n) else None for t, n in zip(tangents, ctx.needs))
+        if all(t is None for t in tangents):
+            return (None,) * 6
+        wants = tuple(asked(ctx, i) for i in range(4))
+        return _second_order(ctx.call, go, w, x, y, tangents, wants) + (None, None)
 
 
 class FastUniform1dJITFunction(torch.autograd.Function):
@@ -533,7 +566,7 @@ class FastUniform1dJITFunction(torch.autograd.Function):
     @staticmethod
     def backward(ctx, grad_out):
         w, x, y = ctx.saved_tensors
-        needs = tuple(bool(n) for n in ctx.needs_input_grad[:3])
+        needs = tuple(asked(ctx, i) for i in range(3))
         if not any(needs):
             return None, None, None, None, None, None
         if ctx.call.y_sh:

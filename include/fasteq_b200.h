@@ -120,6 +120,16 @@ int fasteq_u1d_backward(const fasteq_u1d_graph* g /* host */, const void* grad_o
 int fasteq_u1d_backward_split(const fasteq_u1d_graph* g /* host */, const int32_t* part_edge, const void* grad_out, const void* w,
                               const void* x, const void* y, void* grad_w, void* grad_x, void* grad_y, fasteq_stream_t stream);
 
+/* Second order.  Modules of this kind hold a tangent row (w2, x2, y2, shaped like w, x, y; NULL where the module has none) beside
+ * operands: per-edge weights, gathered x, scalar y, scattered output.  `part_edge` may be NULL (whole receivers; `carry` is not read then).
+ *   tangent_forward :  out = F(w2, x, y) + F(w, x2, y) + F(w, x, y2)
+ *   tangent_backward:  the gradients of <grad_out, that sum> with respect to w, x and y */
+int fasteq_u1d_tangent_forward(const fasteq_u1d_graph* g /* host */, const int32_t* part_edge, void* carry, const void* w, const void* x,
+                               const void* y, const void* w2, const void* x2, const void* y2, void* out, fasteq_stream_t stream);
+int fasteq_u1d_tangent_backward(const fasteq_u1d_graph* g /* host */, const int32_t* part_edge, const void* grad_out, const void* w,
+                                const void* x, const void* y, const void* w2, const void* x2, const void* y2, void* grad_w, void* grad_x,
+                                void* grad_y, fasteq_stream_t stream);
+
 /* Reads and clears the device-side status word of this module (synchronises the device).
  * 0 = no fault; otherwise the code of the first fault (1 wait timeout, 2 index out of range). */
 int fasteq_u1d_device_status(int32_t* code /* host */);
