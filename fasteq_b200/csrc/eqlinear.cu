@@ -368,6 +368,7 @@ struct GapTable {
 template <typename T>
 __global__ void __launch_bounds__(256) zero_gaps_kernel(T* __restrict__ C, long long batch, int c_rows_per_b, int N,
                                                         const __grid_constant__ GapTable gaps) {
+  let_next_kernel_begin();
   for (long long b = blockIdx.x; b < batch; b += gridDim.x)
     for (int g = 0; g < gaps.n; ++g) {
       T* p = C + ((size_t)b * c_rows_per_b + gaps.start[g]) * (size_t)N;
@@ -958,6 +959,7 @@ __global__ void __launch_bounds__(NT) eqlinear_wgrad_kernel(const __grid_constan
 template <typename T, int Y>
 __global__ void __launch_bounds__(256) eqlinear_wgrad_reduce_kernel(const __grid_constant__ WgradTable tab, const T* __restrict__ partial,
                                                                     T* __restrict__ gw, int num_paths, long long uv) {
+  let_next_kernel_begin();
   constexpr int X = 256 / Y;
   __shared__ T share[Y][X + 1];
   const long long i = (long long)blockIdx.x * X + threadIdx.x, total = (long long)num_paths * uv;
@@ -1003,35 +1005,62 @@ long long plan_splits(const fasteq_eqlinear_problem* p, long long batch, long lo
   return best;
 }
 
-cudaError_t launch_wgrad_f32(const fasteq_eqlinear_problem* p, WgradTable* tab, int sms, const float* x, const float* go, float** partial,
-                             cudaStream_t s) {
+// Where the partial sums live: the caller's buffer, or a stream-ordered temporary.  The temporary's pool gives its memory back at
+// every synchronisation, and the next call then waits for the driver (1 to 6 ms for 10 to 40 MB), so the front-end brings a buffer.
+// With `need` set nothing is launched: it receives the bytes a call would take.
+struct WgradScratch {
+  void* given = nullptr;
+  long long given_bytes = 0;
+  long long* need = nullptr;
+  void* own = nullptr;
+  // FASTEQ_OK with `*p` set; or the status to return (FASTEQ_OK with `*p` null: `need` is answered)
+  int get(void** p, long long bytes, cudaStream_t s) {
+    *p = nullptr;
+    if (need) { *need = bytes; return FASTEQ_OK; }
+    if (given) {
+      if (given_bytes < bytes) return FASTEQ_INVALID;
+      *p = given;
+      return FASTEQ_OK;
+    }
+    cudaError_t e = cudaMallocAsync(&own, (size_t)bytes, s);
+    if (e != cudaSuccess) return cuda_fail(e);
+    *p = own;
+    return FASTEQ_OK;
+  }
+};
+
+int launch_wgrad_f32(const fasteq_eqlinear_problem* p, WgradTable* tab, int sms, const float* x, const float* go, float** partial,
+                     WgradScratch& scratch, cudaStream_t s) {
   int per_sm = 0;
   cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, eqlinear_wgrad_f32_kernel, WG_THREADS, WG_SMEM);
-  if (e != cudaSuccess) return e;
+  if (e != cudaSuccess) return cuda_fail(e);
   const int tiles = ((p->u + WG_TILE - 1) / WG_TILE) * ((p->v + WG_TILE - 1) / WG_TILE);
   const long long rps = plan_splits(p, p->batch, tiles, (long long)sms * std::max(per_sm, 1), tab);
-  e = cudaMallocAsync((void**)partial, (size_t)tab->split_first[p->num_paths] * p->u * p->v * sizeof(float), s);
-  if (e != cudaSuccess) return e;
+  const int rc = scratch.get((void**)partial, (long long)tab->split_first[p->num_paths] * p->u * p->v * (long long)sizeof(float), s);
+  if (!*partial) return rc;
   eqlinear_wgrad_f32_kernel<<<(unsigned)tab->split_first[p->num_paths] * (unsigned)tiles, WG_THREADS, WG_SMEM, s>>>(
       *tab, x, go, *partial, p->batch, p->in_rows, p->out_rows, p->u, p->v, p->num_paths, rps);
-  return cudaGetLastError();
+  e = cudaGetLastError();
+  return e == cudaSuccess ? FASTEQ_OK : cuda_fail(e);
 }
 
 template <int TN>
-int launch_wgrad_tc(const fasteq_eqlinear_problem* p, WgradTable* tab, int sms, const float* x, const float* go, float** partial, cudaStream_t s) {
+int launch_wgrad_tc(const fasteq_eqlinear_problem* p, WgradTable* tab, int sms, const float* x, const float* go, float** partial,
+                    WgradScratch& scratch, cudaStream_t s) {
   const bool swap = p->v > p->u;
   const int M = swap ? p->v : p->u, N = swap ? p->u : p->v, tiles = ((M + wg::TM - 1) / wg::TM) * ((N + TN - 1) / TN);
   const int m_rows = swap ? p->out_rows : p->in_rows, n_rows = swap ? p->in_rows : p->out_rows;
   const long long chunks_per_row = (p->batch + wg::ROWS - 1) / wg::ROWS;
   const long long rps = plan_splits(p, chunks_per_row * wg::ROWS, tiles, sms, tab, 256);
+  int rc = scratch.get((void**)partial, (long long)tab->split_first[p->num_paths] * p->u * p->v * (long long)sizeof(float), s);
+  if (!*partial) return rc;
   CUtensorMap mm, mn;
-  int rc = tc::make_map_rows(&mm, swap ? go : x, M, m_rows, p->batch, wg::TM, wg::ROWS);
+  rc = tc::make_map_rows(&mm, swap ? go : x, M, m_rows, p->batch, wg::TM, wg::ROWS);
   if (rc == FASTEQ_OK) rc = tc::make_map_rows(&mn, swap ? x : go, N, n_rows, p->batch, TN, wg::ROWS);
   if (rc != FASTEQ_OK) return rc;
   int* status = nullptr;
   cudaError_t e = tc::status_word(&status);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(eqlinear_wgrad_tc_kernel<TN>, cudaFuncAttributeMaxDynamicSharedMemorySize, wg::smem_bytes(TN));
-  if (e == cudaSuccess) e = cudaMallocAsync((void**)partial, (size_t)tab->split_first[p->num_paths] * p->u * p->v * sizeof(float), s);
   if (e != cudaSuccess) return cuda_fail(e);
   eqlinear_wgrad_tc_kernel<TN><<<(unsigned)tab->split_first[p->num_paths] * (unsigned)tiles, wg::THREADS, wg::smem_bytes(TN), s>>>(
       mm, mn, *tab, x, go, *partial, p->batch, p->in_rows, p->out_rows, p->u, p->v, p->num_paths, (int)chunks_per_row, (int)(rps / wg::ROWS),
@@ -1041,9 +1070,9 @@ int launch_wgrad_tc(const fasteq_eqlinear_problem* p, WgradTable* tab, int sms, 
 }
 
 template <typename T>
-int launch_wgrad(const fasteq_eqlinear_problem* p, const void* x, const void* go, void* gw, cudaStream_t s) {
+int launch_wgrad(const fasteq_eqlinear_problem* p, const void* x, const void* go, void* gw, WgradScratch scratch, cudaStream_t s) {
   if (!p || p->num_paths < 1 || p->num_paths > kMaxPaths || p->u < 1 || p->v < 1 || p->batch < 0) return FASTEQ_INVALID;
-  if (!p->in_row || !p->out_row || !p->rows || !p->coeff || !gw) return FASTEQ_INVALID;
+  if (!p->in_row || !p->out_row || !p->rows || !p->coeff || (!gw && !scratch.need)) return FASTEQ_INVALID;
   WgradTable tab;
   int max_rows = 1;
   for (int q = 0; q < p->num_paths; ++q) {
@@ -1054,6 +1083,7 @@ int launch_wgrad(const fasteq_eqlinear_problem* p, const void* x, const void* go
     max_rows = std::max(max_rows, p->rows[q]);
   }
   const long long uv = (long long)p->u * p->v, total = uv * p->num_paths;
+  if (p->batch == 0 && scratch.need) { *scratch.need = 0; return FASTEQ_OK; }
   if (p->batch == 0) {
     cudaError_t e = cudaMemsetAsync(gw, 0, (size_t)total * sizeof(T), s);
     return e == cudaSuccess ? FASTEQ_OK : cuda_fail(e);
@@ -1064,6 +1094,7 @@ int launch_wgrad(const fasteq_eqlinear_problem* p, const void* x, const void* go
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (e != cudaSuccess) return cuda_fail(e);
   T* partial = nullptr;
+  int rc = FASTEQ_OK;
   const bool quads = sizeof(T) == 4 && p->u % 4 == 0 && p->v % 4 == 0 &&
                      ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(go)) & 15u) == 0;   // 16-byte row pieces
   const float *xf = (const float*)x, *gf = (const float*)go;
@@ -1072,29 +1103,31 @@ int launch_wgrad(const fasteq_eqlinear_problem* p, const void* x, const void* go
   // empty).  Up to 128 rows every path is one share, and what counts is how many CTAs start and how little each stores: the
   // ten-path SO3Linear of 128 channels takes 9.7 us at 8 nodes and 18.5 on the tensor cores, at 33 nodes 22.9 and 18.9.
   if (quads && p->batch >= 16 && p->batch * max_rows > 128 && p->batch <= 0x7fffffffLL && (p->batch / 32 + 1) * max_rows < (1LL << 30)) {
-    const int rc = std::min(p->u, p->v) <= 64 ? launch_wgrad_tc<64>(p, &tab, sms, xf, gf, pf, s) : launch_wgrad_tc<128>(p, &tab, sms, xf, gf, pf, s);
-    if (rc != FASTEQ_OK) return rc;
+    rc = std::min(p->u, p->v) <= 64 ? launch_wgrad_tc<64>(p, &tab, sms, xf, gf, pf, scratch, s)
+                                    : launch_wgrad_tc<128>(p, &tab, sms, xf, gf, pf, scratch, s);
   } else if (quads && max_rows <= WG_MAX_ROWS) {
-    e = launch_wgrad_f32(p, &tab, sms, xf, gf, pf, s);
+    rc = launch_wgrad_f32(p, &tab, sms, xf, gf, pf, scratch, s);
   } else {
     const int tiles = ((p->u + BM - 1) / BM) * ((p->v + BN - 1) / BN);
     const long long rps = plan_splits(p, p->batch, tiles, (long long)sms * 4, &tab);
-    e = cudaMallocAsync((void**)&partial, (size_t)tab.split_first[p->num_paths] * uv * sizeof(T), s);
-    if (e == cudaSuccess) {
+    rc = scratch.get((void**)&partial, (long long)tab.split_first[p->num_paths] * uv * (long long)sizeof(T), s);
+    if (partial) {
       eqlinear_wgrad_kernel<T><<<(unsigned)tab.split_first[p->num_paths] * (unsigned)tiles, NT, 0, s>>>(
           tab, (const T*)x, (const T*)go, partial, p->batch, p->in_rows, p->out_rows, p->u, p->v, p->num_paths, rps);
       e = cudaGetLastError();
+      if (e != cudaSuccess) rc = cuda_fail(e);
     }
   }
-  if (e == cudaSuccess) {
+  if (rc == FASTEQ_OK && partial) {
     if (tab.split_first[p->num_paths] == p->num_paths)
       eqlinear_wgrad_reduce_kernel<T, 1><<<(unsigned)((total + 255) / 256), dim3(256, 1), 0, s>>>(tab, partial, (T*)gw, p->num_paths, uv);
     else
       eqlinear_wgrad_reduce_kernel<T, 8><<<(unsigned)((total + 31) / 32), dim3(32, 8), 0, s>>>(tab, partial, (T*)gw, p->num_paths, uv);
     e = cudaGetLastError();
+    if (e != cudaSuccess) rc = cuda_fail(e);
   }
-  if (partial) cudaFreeAsync(partial, s);
-  return e == cudaSuccess ? FASTEQ_OK : cuda_fail(e);
+  if (scratch.own) cudaFreeAsync(scratch.own, s);
+  return rc;
 }
 
 int dispatch(const fasteq_eqlinear_problem* p, bool dgrad, const void* w, const void* a, void* c, fasteq_stream_t stream) {
@@ -1124,13 +1157,37 @@ extern "C" int fasteq_eqlinear_dgrad(const fasteq_eqlinear_problem* p, const voi
   return dispatch(p, true, w, grad_out, grad_x, stream);
 }
 
+namespace {
+int wgrad(const fasteq_eqlinear_problem* p, const void* x, const void* grad_out, void* grad_w, WgradScratch scratch, fasteq_stream_t stream) {
+  if (!p) return FASTEQ_INVALID;
+  if (p->precision == FASTEQ_EQLIN_FP64) return launch_wgrad<double>(p, x, grad_out, grad_w, scratch, (cudaStream_t)stream);
+  if (p->precision == FASTEQ_EQLIN_TF32X3 || p->precision == FASTEQ_EQLIN_FP32)
+    return launch_wgrad<float>(p, x, grad_out, grad_w, scratch, (cudaStream_t)stream);
+  return FASTEQ_INVALID;
+}
+}  // namespace
+
 extern "C" int fasteq_eqlinear_wgrad(const fasteq_eqlinear_problem* p, const void* x, const void* grad_out, void* grad_w,
                                      fasteq_stream_t stream) {
-  if (!p) return FASTEQ_INVALID;
-  if (p->precision == FASTEQ_EQLIN_FP64) return launch_wgrad<double>(p, x, grad_out, grad_w, (cudaStream_t)stream);
-  if (p->precision == FASTEQ_EQLIN_TF32X3 || p->precision == FASTEQ_EQLIN_FP32)
-    return launch_wgrad<float>(p, x, grad_out, grad_w, (cudaStream_t)stream);
-  return FASTEQ_INVALID;
+  return wgrad(p, x, grad_out, grad_w, WgradScratch{}, stream);
+}
+
+extern "C" int fasteq_eqlinear_wgrad_scratch(const fasteq_eqlinear_problem* p, const void* x, const void* grad_out, int64_t* bytes) {
+  if (!bytes) return FASTEQ_INVALID;
+  long long need = 0;
+  WgradScratch scratch;
+  scratch.need = &need;
+  const int rc = wgrad(p, x, grad_out, nullptr, scratch, nullptr);
+  *bytes = need;
+  return rc;
+}
+
+extern "C" int fasteq_eqlinear_wgrad_with(const fasteq_eqlinear_problem* p, const void* x, const void* grad_out, void* grad_w, void* scratch,
+                                          int64_t scratch_bytes, fasteq_stream_t stream) {
+  if (!scratch) return FASTEQ_INVALID;
+  WgradScratch given;
+  given.given = scratch; given.given_bytes = scratch_bytes;
+  return wgrad(p, x, grad_out, grad_w, given, stream);
 }
 
 extern "C" int fasteq_eqlinear_pack(const fasteq_eqlinear_problem* p, int32_t dgrad, const void* w, void* packed,

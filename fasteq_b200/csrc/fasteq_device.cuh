@@ -102,6 +102,16 @@ __device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.w
 template <int N>
 __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group %0;" ::"n"(N) : "memory"); }
 
+// Programmatic dependent launch.  A kernel started by launch_dependent (launch.cuh) may begin while the one before it in the stream is
+// still running: it sets up its barriers and tensor memory, then every thread waits here for the end of that kernel, before it touches
+// global memory.  Every thread of such a kernel has to pass here, so that its end means the end of all earlier ones too.
+__device__ __forceinline__ void wait_for_previous_kernel() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+// in a kernel started the ordinary way: the next one may come once every CTA has begun
+__device__ __forceinline__ void let_next_kernel_begin() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // generic-proxy writes to shared memory -> visible to the async proxy (bulk stores)
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 

@@ -84,7 +84,8 @@ def _fma_wgrad(x: torch.Tensor, g: torch.Tensor) -> torch.Tensor:
     out = torch.empty((x.shape[1], g.shape[1]), dtype=x.dtype, device=x.device)
     if x.shape[0] == 0:
         return out.zero_()
-    _fma_call("fasteq_eqlinear_wgrad", _fma_problem(x.shape[0], x.shape[1], g.shape[1], x.dtype), x, g, out)
+    from .eqlinear import wgrad_into
+    wgrad_into(_fma_problem(x.shape[0], x.shape[1], g.shape[1], x.dtype), x, g, out)
     return out
 
 
@@ -112,19 +113,16 @@ def _gemm(a: torch.Tensor, bt: torch.Tensor, weight: torch.Tensor = None, transp
     lib = _lib()
     with _cabi.on_device(a.device):
         stream = _cabi.stream(a.device)
-        split = None
-        if weight is not None:
-            def build():
-                b = bt.contiguous()
-                sp = torch.empty(2 * b.numel(), dtype=torch.float32, device=b.device)
-                _cabi.check(lib.fasteq_gemm_tf32x3_split(b.data_ptr(), b.numel(), sp.data_ptr(), stream), lib, "fasteq_gemm_tf32x3_split")
-                return sp
-            split = _prepared.get((weight,), ("dense", transposed), build)
-        if split is not None:
-            rc = lib.fasteq_gemm_tf32x3_presplit(a.data_ptr(), split.data_ptr(), out.data_ptr(), M, N, K, stream)
-        else:
-            bt = bt.contiguous()
-            rc = lib.fasteq_gemm_tf32x3(a.data_ptr(), bt.data_ptr(), out.data_ptr(), M, N, K, stream)
+
+        def build():
+            b = bt.contiguous()
+            sp = torch.empty(2 * b.numel(), dtype=torch.float32, device=b.device)
+            _cabi.check(lib.fasteq_gemm_tf32x3_split(b.data_ptr(), b.numel(), sp.data_ptr(), stream), lib, "fasteq_gemm_tf32x3_split")
+            return sp
+        split = _prepared.get((weight,), ("dense", transposed), build) if weight is not None else None
+        if split is None:
+            split = build()
+        rc = lib.fasteq_gemm_tf32x3_presplit(a.data_ptr(), split.data_ptr(), out.data_ptr(), M, N, K, stream)
     if rc == 1:   # FASTEQ_UNSUPPORTED (operand alignment): the FP32 FMA tile kernel takes any shape and alignment
         return _fma_gemm(a, bt.t())
     _cabi.check(rc, lib, "fasteq_gemm_tf32x3")

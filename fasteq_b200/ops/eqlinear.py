@@ -130,6 +130,8 @@ def _core():
         lib.fasteq_eqlinear_forward.argtypes = [C.POINTER(_Problem), C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]
         lib.fasteq_eqlinear_dgrad.argtypes = [C.POINTER(_Problem), C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]
         lib.fasteq_eqlinear_wgrad.argtypes = [C.POINTER(_Problem), C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]
+        lib.fasteq_eqlinear_wgrad_scratch.argtypes = [C.POINTER(_Problem), C.c_void_p, C.c_void_p, C.POINTER(C.c_int64)]
+        lib.fasteq_eqlinear_wgrad_with.argtypes = [C.POINTER(_Problem), C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64, C.c_void_p]
         lib.fasteq_eqlinear_pack.argtypes = [C.POINTER(_Problem), C.c_int32, C.c_void_p, C.c_void_p, C.c_void_p]
         lib.fasteq_eqlinear_forward_packed.argtypes = [C.POINTER(_Problem), C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]
         lib.fasteq_eqlinear_dgrad_packed.argtypes = [C.POINTER(_Problem), C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]
@@ -162,8 +164,9 @@ def _order_weights(w3d, mapping):
     return w3d[torch.tensor(wps, device=w3d.device)].contiguous()
 
 
-def _packed_weights(w, w3, geom_key, prob, dgrad: bool, lib, stream):
-    """Pre-scaled, K-major, TF32-split weight blocks of this problem and direction (cached per weight version)."""
+def _packed_weights(w, w3, geom_key, prob, dgrad: bool, lib, stream, keep: bool):
+    """Pre-scaled, K-major, TF32-split weight blocks of this problem and direction.  Cached per weight version with ``keep``; built for
+    this call alone where a cotangent stands in the weights' place and where the cache must not be used."""
     def build():
         packed = torch.empty(2 * w3.numel(), dtype=torch.float32, device=w3.device)
         rc = lib.fasteq_eqlinear_pack(C.byref(prob), 1 if dgrad else 0, w3.data_ptr(), packed.data_ptr(), stream)
@@ -171,13 +174,14 @@ def _packed_weights(w, w3, geom_key, prob, dgrad: bool, lib, stream):
             return None
         _cabi.check(rc, lib, "fasteq_eqlinear_pack")
         return packed
-    return _prepared.get((w,), ("eqlinear", geom_key, dgrad), build)
+    packed = _prepared.get((w,), ("eqlinear", geom_key, dgrad), build) if keep else None
+    return build() if packed is None else packed
 
 
-def _run(lib, prob, w, w3, a, c, geom_key, precision, dgrad: bool, stream):
+def _run(lib, prob, w, w3, a, c, geom_key, precision, dgrad: bool, stream, keep: bool = True):
     """One forward / grad_x launch: through prepared weights when the tensor-core path takes the problem."""
     if precision == _TF32:
-        packed = _packed_weights(w, w3, geom_key, prob, dgrad, lib, stream)
+        packed = _packed_weights(w, w3, geom_key, prob, dgrad, lib, stream, keep)
         if packed is not None:
             fn = lib.fasteq_eqlinear_dgrad_packed if dgrad else lib.fasteq_eqlinear_forward_packed
             rc = fn(C.byref(prob), packed.data_ptr(), a.data_ptr(), c.data_ptr(), stream)
@@ -187,6 +191,18 @@ def _run(lib, prob, w, w3, a, c, geom_key, precision, dgrad: bool, stream):
     fn = lib.fasteq_eqlinear_dgrad if dgrad else lib.fasteq_eqlinear_forward
     _cabi.check(fn(C.byref(prob), w3.data_ptr(), a.data_ptr(), c.data_ptr(), stream), lib,
                 "fasteq_eqlinear_dgrad" if dgrad else "fasteq_eqlinear_forward")
+
+
+def wgrad_into(prob, x, g, dw) -> None:
+    """The weight gradient of a problem, its partial sums in memory of torch's allocator."""
+    lib, need = _core(), C.c_int64(0)
+    with _cabi.on_device(dw.device):
+        stream = _cabi.stream(dw.device)
+        _cabi.check(lib.fasteq_eqlinear_wgrad_scratch(C.byref(prob), x.data_ptr(), g.data_ptr(), C.byref(need)), lib,
+                    "fasteq_eqlinear_wgrad_scratch")
+        scratch = torch.empty(max(need.value, 16), dtype=torch.uint8, device=dw.device)
+        _cabi.check(lib.fasteq_eqlinear_wgrad_with(C.byref(prob), x.data_ptr(), g.data_ptr(), dw.data_ptr(), scratch.data_ptr(),
+                                                   scratch.numel(), stream), lib, "fasteq_eqlinear_wgrad_with")
 
 
 class _Plan:
@@ -207,22 +223,22 @@ class _Plan:
         mapping, _, u, v, _, _ = self.geom
         return _order_weights(w.reshape(len(mapping), u, v).contiguous(), mapping)
 
-    def forward(self, w, x):
+    def forward(self, w, x, keep: bool = True):
         mapping, coeff, u, v, I, J = self.geom
         x3 = x.reshape(self.batch, I, u).contiguous()
         out = torch.empty((self.batch, J, v), dtype=x.dtype, device=x.device)
         with _cabi.on_device(x.device):
             _run(_core(), self._problem(), w, self._w3(w), x3, out, self.key, self.precision, False,
-                 _cabi.stream(x.device))
+                 _cabi.stream(x.device), keep)
         return out.reshape(self.batch, J * v)
 
-    def dgrad(self, w, g):
+    def dgrad(self, w, g, keep: bool = True):
         mapping, coeff, u, v, I, J = self.geom
         g3 = g.reshape(self.batch, J, v).contiguous()
         dx = torch.empty((self.batch, I, u), dtype=g3.dtype, device=g3.device)
         with _cabi.on_device(g3.device):
             _run(_core(), self._problem(), w, self._w3(w), g3, dx, self.key, self.precision, True,
-                 _cabi.stream(g3.device))
+                 _cabi.stream(g3.device), keep)
         return dx.reshape(self.batch, I * u)
 
     def wgrad(self, x, g):
@@ -230,10 +246,7 @@ class _Plan:
         x3 = x.reshape(self.batch, I, u).contiguous()
         g3 = g.reshape(self.batch, J, v).contiguous()
         dw = torch.empty((len(mapping), u, v), dtype=g3.dtype, device=g3.device)
-        lib = _core()
-        with _cabi.on_device(g3.device):
-            _cabi.check(lib.fasteq_eqlinear_wgrad(C.byref(self._problem()), x3.data_ptr(), g3.data_ptr(), dw.data_ptr(),
-                                                  _cabi.stream(g3.device)), lib, "fasteq_eqlinear_wgrad")
+        wgrad_into(self._problem(), x3, g3, dw)
         wps = [m[2] for m in mapping]
         if wps != list(range(len(wps))):      # block q of the table is block wps[q] of the caller's tensor
             full = torch.empty_like(dw)
@@ -290,14 +303,14 @@ class _EqLinearBackwardFn(torch.autograd.Function):
             if ggx is not None:
                 d_go = plan.forward(w, ggx)
             if ggw is not None:
-                t = plan.forward(ggw, x)
+                t = plan.forward(ggw, x, keep=False)
                 d_go = t if d_go is None else d_go + t
             if d_go is not None:
                 d_go = d_go.reshape(go.shape)
         if want_w and ggx is not None:
             d_w = plan.wgrad(ggx, go)
         if want_x and ggw is not None:
-            d_x = plan.dgrad(ggw, go).reshape(x.shape)
+            d_x = plan.dgrad(ggw, go, keep=False).reshape(x.shape)
         return d_go, d_w, d_x, None, None, None
 
 

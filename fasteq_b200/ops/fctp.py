@@ -20,7 +20,7 @@ from typing import Dict, List, Tuple
 import torch
 
 from .. import _cabi
-from .eqlinear import _core, _make_problem
+from .eqlinear import _core, _make_problem, wgrad_into
 
 __all__ = ["fast_fctp", "fctp_species_groups"]
 
@@ -160,8 +160,7 @@ class FastFullyConnectedTensorProductPathFused(torch.autograd.Function):
                                                           gxs[start:start + n].data_ptr(), stream), lib, "fasteq_eqlinear_dgrad")
                 if need_w:
                     gws = torch.empty((len(mapping), U, W), dtype=gs.dtype, device=gs.device)
-                    _cabi.check(lib.fasteq_eqlinear_wgrad(C.byref(prob), xs[start:start + n].data_ptr(), gs[start:start + n].data_ptr(),
-                                                          gws.data_ptr(), stream), lib, "fasteq_eqlinear_wgrad")
+                    wgrad_into(prob, xs[start:start + n], gs[start:start + n], gws)
                     gw4[:, :, s, :].index_add_(0, pidx, gws)                     # several runs may share a weight path
                 start += n
                 wi += 1

@@ -309,10 +309,14 @@ int fasteq_eqlinear_dgrad_packed(const fasteq_eqlinear_problem* p /* host */, co
  * Needed to train the mixing weights.  The reference's public operator returns no weight gradient
  * (eqlinear_runtime.py:104); its FP32 back-end keeps a reduction kernel for one
  * (fasteq/cuda/src/eqlinear/backends/fp32/reduce_dw.cu:12).  FP32 (also for FASTEQ_EQLIN_TF32X3) or FP64
- * FMA arithmetic, two deterministic stages: per-chunk partial sums in a stream-ordered temporary, then
- * their reduction.  grad_w [num_paths, u, v] is fully overwritten. */
+ * accuracy, two deterministic stages: partial sums, then their reduction.  grad_w [num_paths, u, v] is fully overwritten.
+ * `_wgrad` keeps the partial sums in a stream-ordered temporary; `_wgrad_with` in the caller's scratch (16-byte aligned device memory
+ * of at least the bytes `_wgrad_scratch` names for the same problem and operands, not in use by other work on the device meanwhile). */
 int fasteq_eqlinear_wgrad(const fasteq_eqlinear_problem* p /* host */, const void* x, const void* grad_out,
                           void* grad_w, fasteq_stream_t stream);
+int fasteq_eqlinear_wgrad_scratch(const fasteq_eqlinear_problem* p /* host */, const void* x, const void* grad_out, int64_t* bytes /* host */);
+int fasteq_eqlinear_wgrad_with(const fasteq_eqlinear_problem* p /* host */, const void* x, const void* grad_out, void* grad_w, void* scratch,
+                               int64_t scratch_bytes, fasteq_stream_t stream);
 
 /* The same operator in the shape of the reference's backend interface: a table of function pointers per precision,
  * field for field the EqLinearBackendApi / EqLinearProblemC / EqLinearPathC / EqLinearPlanInfo of
