@@ -482,8 +482,7 @@ constexpr int VEC = 1;
 template <typename... P> static bool misaligned(P...) { return false; }
 """
 
-_PACKED = """#include "fasteq_device.cuh"
-typedef float2 V;        // what a thread carries per segment: two channels
+_PACKED = """typedef float2 V;        // what a thread carries per segment: two channels
 constexpr int VEC = 2;
 #define LD(p) (*reinterpret_cast<const float2*>(p))
 #define ST(p, v) (*reinterpret_cast<float2*>(p) = (v))
@@ -516,6 +515,7 @@ def emit_stc(spec: STCSpec, direction: str, need_gx0: bool = False, packed: bool
 #include <cstdint>
 #include <cuda_runtime.h>
 #include "fasteq_b200.h"
+#include "fasteq_device.cuh"
 typedef {spec.ctype} T;
 constexpr int U = {spec.u}, A = {spec.x1_segs}, D = {spec.x0_segs}, OSEG = {spec.out_segs}, NT = {threads};
 {_PACKED if packed else _SCALAR}{_COMMON}
@@ -531,6 +531,7 @@ extern "C" int fasteq_stc_describe(fasteq_stc_desc* d) {{
         body.append(f"""
 __global__ void __launch_bounds__(NT) fasteq_stc_fwd_kernel(const T* __restrict__ x1, const T* __restrict__ x0,
     const int* __restrict__ i0, long long batch, long long n_species, T* __restrict__ out, int* status) {{
+  fasteq::let_next_kernel_begin();
   for (long long b = blockIdx.x; b < batch; b += gridDim.x) {{
     int sp = i0[b];
     if (sp < 0 || sp >= n_species) {{ atomicExch(status, 2); sp = 0; }}
@@ -575,6 +576,7 @@ constexpr bool NEED_GX0 = {str(need_gx0).lower()};
 __global__ void __launch_bounds__(NT) fasteq_stc_bwd_kernel(const T* __restrict__ go, const T* __restrict__ x1,
     const T* __restrict__ x0, const int* __restrict__ i0, long long batch, long long n_species, T* __restrict__ gx1,
     T* __restrict__ gx0n, int* status) {{
+  fasteq::let_next_kernel_begin();
   for (long long b = blockIdx.x; b < batch; b += gridDim.x) {{
     int sp = i0[b];
     if (sp < 0 || sp >= n_species) {{ atomicExch(status, 2); sp = 0; }}

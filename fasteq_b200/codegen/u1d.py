@@ -325,7 +325,7 @@ def _prelude(spec: U1DSpec, tun: Tuning, extra_bytes: int, ncons_warps: int, emi
     return ("// Generated by fasteq_b200.codegen.u1d -- do not edit.\n"
             "#include <atomic>\n#include <cstdio>\n#include <cstdint>\n#include <cuda_runtime.h>\n"
             '#include "fasteq_b200.h"\n' + _cfg(spec, tun, extra_bytes, ncons_warps, emit_empty) +
-            '#include "u1d_pipeline.cuh"\nusing namespace fasteq;\nusing namespace fasteq::u1d;\n'
+            '#include "u1d_pipeline.cuh"\n#include "launch.cuh"\nusing namespace fasteq;\nusing namespace fasteq::u1d;\n'
             "using V = cfg::V;\nusing VS = VT<V>;\nconstexpr int VEC = VS::N;\nconstexpr int TPG = CT / VEC;  // threads per group\n")
 
 
@@ -596,6 +596,7 @@ fasteq_u1d_fwd_kernel(const Graph g, const T* __restrict__ w, const T* __restric
     mbar_fence_init();
   }}
   __syncthreads();
+  wait_for_previous_kernel();
   // warps [0, PIPES * NCONS_WARPS) consume, the last PIPES warps produce; pipeline p owns consumer
   // warps [p * NCONS_WARPS, (p + 1) * NCONS_WARPS) and producer warp PIPES * NCONS_WARPS + p
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -665,6 +666,7 @@ fasteq_u1d_fwd_kernel(const Graph g, const T* __restrict__ w, const T* __restric
 // Bound by latency (two dependent index loads, then the rows): the indices a CTA may need come in one go.
 __global__ void __launch_bounds__(256) fasteq_u1d_carry_kernel(const int* __restrict__ seg_ptr, const int* __restrict__ part_ptr,
     const int* __restrict__ part_edge, int n_parts, int n_out_rows, const T* __restrict__ carry, T* __restrict__ out) {{
+  let_next_kernel_begin();
   const int p = blockIdx.x, before = p > 0 ? p - 1 : 0;
   const int row = part_ptr[p], row_before = part_ptr[before], row_after = part_ptr[p + 1];
   const int edge = part_edge[p], edge_before = part_edge[before];
@@ -705,8 +707,9 @@ static int run_forward(const fasteq_u1d_graph* gh, const int32_t* part_edge, voi
   if (VEC == 2 && ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(carry)) & 7u)) return FASTEQ_INVALID;
   cudaError_t e = cudaFuncSetAttribute(fasteq_u1d_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
   if (e != cudaSuccess) return cuda_fail(e);
-  fasteq_u1d_fwd_kernel<<<grid, NTHREADS, SMEM_BYTES, (cudaStream_t)stream>>>(
+  e = launch_dependent(fasteq_u1d_fwd_kernel, (unsigned)grid, NTHREADS, SMEM_BYTES, (cudaStream_t)stream,
       g, (const T*)w, (const T*)x, (const T*)y, (T*)out, (T*)carry{host_args});
+  if (e != cudaSuccess) return cuda_fail(e);
   if (part_edge)
     fasteq_u1d_carry_kernel<<<(unsigned)gh->n_parts, 256, 0, (cudaStream_t)stream>>>(
         gh->seg_ptr, gh->part_ptr, part_edge, gh->n_parts, (int)gh->n_out_rows, (const T*)carry, (T*)out);
@@ -840,6 +843,7 @@ fasteq_u1d_bwd_kernel(const Graph g, const T* __restrict__ go, const T* __restri
     mbar_fence_init();
   }}
   __syncthreads();
+  wait_for_previous_kernel();
   const int warp_all = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // tensor-memory gradient rows: warp 0 allocates, everyone reads the base address from the last word of the first
   // barrier block (free when no gradient tile lives in shared memory)
@@ -1231,9 +1235,8 @@ static int run_backward(const fasteq_u1d_graph* gh, const int32_t* part_edge, co
     return FASTEQ_INVALID;
   e = cudaFuncSetAttribute(fasteq_u1d_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
   if (e != cudaSuccess) return cuda_fail(e);
-  fasteq_u1d_bwd_kernel<<<grid, NTHREADS, SMEM_BYTES, s>>>(g, (const T*)go, (const T*)w, (const T*)x, (const T*)y,
-                                                          (T*)gw, (T*)gx, (T*)gy{host_args});
-  e = cudaGetLastError();
+  e = launch_dependent(fasteq_u1d_bwd_kernel, (unsigned)grid, NTHREADS, SMEM_BYTES, s, g, (const T*)go, (const T*)w, (const T*)x, (const T*)y,
+                       (T*)gw, (T*)gx, (T*)gy{host_args});
   if (e != cudaSuccess) return cuda_fail(e);
   return FASTEQ_OK;
 }}

@@ -55,6 +55,7 @@ __global__ void __launch_bounds__(256) edge_geometry_fwd_kernel(const T* __restr
                                                                 const int* __restrict__ dst, const T* __restrict__ shift,
                                                                 long long n_edges, long long n_nodes, T r_max, int n_basis, int p,
                                                                 T* __restrict__ vec, T* __restrict__ basis, int* status) {
+  let_next_kernel_begin();
   const T pi = T(3.14159265358979323846);
   for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < n_edges; e += (long long)gridDim.x * blockDim.x) {
     const long long s = src[e], d = dst[e];

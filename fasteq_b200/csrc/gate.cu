@@ -11,6 +11,7 @@
 #include <cuda_runtime.h>
 #include "fasteq_b200.h"
 #include "core_common.h"
+#include "fasteq_device.cuh"
 
 using namespace fasteq;
 
@@ -57,6 +58,7 @@ template <typename T, int V> __device__ __forceinline__ void st_pack(T* p, const
 template <typename T, int V>
 __global__ void __launch_bounds__(256) gate_fwd_kernel(const T* __restrict__ x, T* __restrict__ out, long long batch, int u,
                                                        const __grid_constant__ GateTable t) {
+  let_next_kernel_begin();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const int per_row = u / V;
   if (i >= batch * per_row) return;
@@ -89,6 +91,7 @@ __global__ void __launch_bounds__(256) gate_fwd_kernel(const T* __restrict__ x, 
 template <typename T, int V>
 __global__ void __launch_bounds__(256) gate_bwd_kernel(const T* __restrict__ x, const T* __restrict__ go, T* __restrict__ gx,
                                                        long long batch, int u, const __grid_constant__ GateTable t) {
+  let_next_kernel_begin();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const int per_row = u / V;
   if (i >= batch * per_row) return;

@@ -24,6 +24,7 @@
 //                  staging slabs and TMA stores
 // Every mbarrier wait is bounded (about two seconds), after which a status word is set and the
 // waiter falls through; TMEM is always released before the CTA ends.  Single-CTA copies only, no clusters.
+#include <algorithm>
 #include <cstdio>
 #include <cstdint>
 #include <cuda.h>
@@ -34,6 +35,7 @@
 #include "fasteq_device.cuh"
 #include "gemm_tf32x3.h"
 #include "tcgen05_util.cuh"
+#include "launch.cuh"
 
 namespace fasteq {
 namespace tc {
@@ -135,6 +137,7 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  wait_for_previous_kernel();
   const uint32_t tmem_base = *tmem_slot;
   const uint32_t tmem_a = tmem_base + (uint32_t)(4 * BN);     // A_TMEM: [STAGES][hi 32 columns | lo 32 columns]
 
@@ -513,7 +516,7 @@ struct AspCfg {
 __global__ void __launch_bounds__(NT_ASP, 1)
 gemm_tf32x3_asp_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmBhi,
                        const __grid_constant__ CUtensorMap tmBlo, const __grid_constant__ CUtensorMap tmC, long long M, int N, int K,
-                       int m_blocks, int* status) {
+                       int m_blocks, int col_shares, int* status) {
   using C_ = AspCfg;
   constexpr int RING = C_::RING;
   extern __shared__ unsigned char smem_raw[];
@@ -533,9 +536,16 @@ gemm_tf32x3_asp_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int n_tiles = (N + AS_BN - 1) / AS_BN;
+  // an item is a row block, or where there are few of those a share of its weight tiles
+  const int all_tiles = (N + AS_BN - 1) / AS_BN, n_items = m_blocks * col_shares;
   const int n_kb = (K + BK - 1) / BK;            // <= KB
   const int first = (int)blockIdx.x, stride = (int)gridDim.x;
+  struct Item { int blk, nt0, n_tiles; };
+  auto item_of = [&](int item) {
+    if (col_shares == 1) return Item{item, 0, all_tiles};
+    const int blk = item / col_shares, share = item - blk * col_shares, nt0 = all_tiles * share / col_shares;
+    return Item{blk, nt0, all_tiles * (share + 1) / col_shares - nt0};
+  };
 
   if (threadIdx.x == 0) {
     for (int b = 0; b < 2; ++b) {
@@ -549,6 +559,7 @@ gemm_tf32x3_asp_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  wait_for_previous_kernel();
   const uint32_t tmem_base = *tmem_slot;
 
   if (warp == 0) {
@@ -560,16 +571,17 @@ gemm_tf32x3_asp_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
         mbar_arrive_expect_tx(&a_full[buf], (uint32_t)(n_kb * C_::A_BYTES));
         for (int kb = 0; kb < n_kb; ++kb) tma_load_3d(dst + (size_t)kb * C_::A_BYTES, &tmA, kb * BK, 0, blk * BM, &a_full[buf]);
       };
-      if (first < m_blocks) load_a(0, first);
+      if (first < n_items) load_a(0, item_of(first).blk);
       int it = 0;
-      for (int j = 0, blk = first; blk < m_blocks; ++j, blk += stride) {
-        bool next_pending = blk + stride < m_blocks;
+      for (int j = 0, item = first; item < n_items; ++j, item += stride) {
+        const Item im = item_of(item);
+        bool next_pending = item + stride < n_items;
         int local = 0;
-        for (int nti = 0; nti < n_tiles; ++nti) {
-          const int nt = (nti + blk) % n_tiles;     // staggered walk over the weight tiles (see the epilogue)
+        for (int nti = 0; nti < im.n_tiles; ++nti) {
+          const int nt = im.nt0 + (nti + im.blk) % im.n_tiles;     // staggered walk over the weight tiles (see the epilogue)
           for (int kb = 0; kb < n_kb; ++kb, ++it, ++local) {
             // the next A block is requested once this block's first weight tiles are on their way
-            if (next_pending && local == 2) { load_a(j + 1, blk + stride); next_pending = false; }
+            if (next_pending && local == 2) { load_a(j + 1, item_of(item + stride).blk); next_pending = false; }
             const int s = it % RING;
             mbar_wait(&b_empty[s], ((it / RING) & 1u) ^ 1u, status);
             unsigned char* st = b_base + (size_t)s * 2 * C_::B_BYTES;
@@ -578,7 +590,7 @@ gemm_tf32x3_asp_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
             tma_load_3d(st + C_::B_BYTES, &tmBlo, kb * BK, nt * AS_BN, 0, &b_full[s]);
           }
         }
-        if (next_pending) load_a(j + 1, blk + stride);
+        if (next_pending) load_a(j + 1, item_of(item + stride).blk);
       }
     }
   } else if (warp == 1) {
@@ -586,8 +598,8 @@ gemm_tf32x3_asp_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
       const uint32_t idesc = idesc_tf32_m128(AS_BN);
       int it = 0;
       uint32_t t = 0;
-      for (int j = 0, blk = first; blk < m_blocks; ++j, blk += stride) {
-        const int abuf = j & 1;
+      for (int j = 0, item = first; item < n_items; ++j, item += stride) {
+        const int abuf = j & 1, n_tiles = item_of(item).n_tiles;
         mbar_wait(&a_split[abuf], ((uint32_t)j >> 1) & 1u, status);
         tc_fence_after();
         const uint32_t a_hi0 = tmem_base + C_::TMEM_A0 + (uint32_t)abuf * C_::TMEM_A_STRIDE, a_lo0 = a_hi0 + C_::TMEM_A_LO;
@@ -619,7 +631,7 @@ gemm_tf32x3_asp_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
     // thread = row of the block = its TMEM lane; 16-byte chunk q of row r sits at chunk position q ^ (r & 7)
     const int quarter = warp & 3;
     const int row = quarter * 32 + lane;
-    for (int j = 0, blk = first; blk < m_blocks; ++j, blk += stride) {
+    for (int j = 0, item = first; item < n_items; ++j, item += stride) {
       const int abuf = j & 1;
       mbar_wait(&a_full[abuf], ((uint32_t)j >> 1) & 1u, status);
       mbar_wait(&a_tmem_empty[abuf], (((uint32_t)j >> 1) & 1u) ^ 1u, status);
@@ -650,12 +662,13 @@ gemm_tf32x3_asp_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
     unsigned char* slab = store_base + (size_t)quarter * 2 * 4096;
     int chunk_no = 0;
     uint32_t t = 0;
-    for (int j = 0, blk = first; blk < m_blocks; ++j, blk += stride) {
-      const long long row0 = (long long)blk * BM + quarter * 32;
-      for (int nti = 0; nti < n_tiles; ++nti, ++t) {
+    for (int item = first; item < n_items; item += stride) {
+      const Item im = item_of(item);
+      const long long row0 = (long long)im.blk * BM + quarter * 32;
+      for (int nti = 0; nti < im.n_tiles; ++nti, ++t) {
         // row block b starts at weight tile b mod n_tiles: the CTAs do not all fetch the same weight lines from L2
         // at the same moment
-        const int nt = (nti + blk) % n_tiles;
+        const int nt = im.nt0 + (nti + im.blk) % im.n_tiles;
         const uint32_t buf = t & 1u;
         mbar_wait(&acc_full[buf], (t >> 1) & 1u, status);
         tc_fence_after();
@@ -776,8 +789,7 @@ static int launch_bn(const TcTable& tab, const CUtensorMap& ma, const CUtensorMa
   const int sms = sm_count();
   if (sms < 1) return FASTEQ_CUDA_ERROR;
   const unsigned grid = (unsigned)(total < sms ? total : sms);     // one persistent CTA per SM
-  gemm_tf32x3_kernel<BN, A_TMEM><<<grid, NT_P, Cfg<BN>::SMEM_BYTES, s>>>(ma, mbh, mbl, mc, tab, M, N, K, total, (int)m_tiles, n_tiles, st);
-  e = cudaGetLastError();
+  e = launch_dependent(gemm_tf32x3_kernel<BN, A_TMEM>, grid, NT_P, Cfg<BN>::SMEM_BYTES, s, ma, mbh, mbl, mc, tab, M, N, K, total, (int)m_tiles, n_tiles, st);
   return e == cudaSuccess ? FASTEQ_OK : cuda_fail(e);
 }
 
@@ -829,9 +841,16 @@ static int launch_as_persistent(const CUtensorMap& ma, const CUtensorMap& mbh, c
   const long long m_blocks = (M + BM - 1) / BM;
   const int sms = sm_count();
   if (sms < 1) return FASTEQ_CUDA_ERROR;
-  const unsigned grid = (unsigned)(m_blocks < sms ? m_blocks : sms);     // one persistent CTA per SM
-  gemm_tf32x3_asp_kernel<<<grid, NT_ASP, AspCfg::SMEM_BYTES, s>>>(ma, mbh, mbl, mc, M, N, K, (int)m_blocks, st);
-  e = cudaGetLastError();
+  // Few row blocks leave SMs idle, or one more block to some of them: then a block's weight tiles are shared out, as far as the longest
+  // CTA (tiles, and about one for each share's block of A) gets shorter.  [10,000, 64] to 1280 columns, 79 blocks: 21.7 -> 15.1 us; 100 rows 18.7 -> 5.3,
+  // 4,000 20.9 -> 9.0, 20,000 39.9 -> 29.9, 40,000 56.1 -> 46.4, 80,000 unchanged.
+  const int n_tiles = (N + AS_BN - 1) / AS_BN;
+  int col_shares = 1;
+  auto longest = [&](long long shares) { return ((m_blocks * shares + sms - 1) / sms) * ((n_tiles + shares - 1) / shares + 1); };
+  for (int c = 2; m_blocks <= 4LL * sms && c <= n_tiles; ++c) if (longest(c) < longest(col_shares)) col_shares = c;
+  const long long items = m_blocks * col_shares;
+  const unsigned grid = (unsigned)(items < sms ? items : sms);     // one persistent CTA per SM
+  e = launch_dependent(gemm_tf32x3_asp_kernel, grid, NT_ASP, AspCfg::SMEM_BYTES, s, ma, mbh, mbl, mc, M, N, K, (int)m_blocks, col_shares, st);
   return e == cudaSuccess ? FASTEQ_OK : cuda_fail(e);
 }
 

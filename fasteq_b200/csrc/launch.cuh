@@ -1,0 +1,21 @@
+// Launch of a kernel that calls wait_for_previous_kernel(): it may begin before the kernel ahead of it in the stream has ended, so that its
+// launch and set-up (barriers, tensor memory, descriptors: 1 to 2 us) lie beside the other's tail.  Only for kernels that read and write
+// global memory after that wait alone, and through addresses no compiler can load from ahead of it (bulk and tensor copies, loads that
+// depend on them).  Captured into CUDA graphs as programmatic edges.
+#pragma once
+#include <cuda_runtime.h>
+
+namespace fasteq {
+
+template <typename... Params, typename... Args>
+cudaError_t launch_dependent(void (*kernel)(Params...), unsigned grid, unsigned threads, size_t smem, cudaStream_t stream, Args&&... args) {
+  cudaLaunchAttribute attr = {};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid); cfg.blockDim = dim3(threads); cfg.dynamicSmemBytes = smem; cfg.stream = stream;
+  cfg.attrs = &attr; cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+}
+
+}  // namespace fasteq

@@ -32,6 +32,7 @@
 #include "fasteq_device.cuh"
 #include "gemm_tf32x3.h"
 #include "tcgen05_util.cuh"
+#include "launch.cuh"
 
 namespace fasteq {
 namespace chain {
@@ -110,10 +111,6 @@ radial_chain_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
   const long long n_tiles = (a.M + BM - 1) / BM;
   const int n_tc = a.n_tc;
 
-  for (int i = threadIdx.x; i < H * NB; i += NT) {
-    const int j = i / NB, k = i % NB;
-    w1s[i] = k < a.nb ? a.w1[j * a.nb + k] : 0.f;
-  }
   if (threadIdx.x == 0) {
     mbar_init(w_full, 1);
     for (int t = 0; t < 2; ++t) { mbar_init(&a_ready[t], N_WORKERS); mbar_init(&z_full[t], 1); }
@@ -121,6 +118,11 @@ radial_chain_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
     mbar_fence_init();
   }
   if (warp == 1) tmem_alloc(tmem_slot, 2 * H);
+  wait_for_previous_kernel();
+  for (int i = threadIdx.x; i < H * NB; i += NT) {
+    const int j = i / NB, k = i % NB;
+    w1s[i] = k < a.nb ? *reinterpret_cast<const volatile float*>(a.w1 + j * a.nb + k) : 0.f;
+  }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -407,8 +409,7 @@ static int launch_nb(const CUtensorMap& tmw, const CUtensorMap& io0, const CUten
   if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return cuda_fail(e);
   const long long n_tiles = (a.M + BM - 1) / BM;
   const unsigned grid = (unsigned)(n_tiles < sms ? n_tiles : sms);
-  radial_chain_kernel<NB, BWD><<<grid, NT, SMEM_BYTES, s>>>(tmw, io0, io1, a, st);
-  e = cudaGetLastError();
+  e = launch_dependent(radial_chain_kernel<NB, BWD>, grid, NT, SMEM_BYTES, s, tmw, io0, io1, a, st);
   return e == cudaSuccess ? FASTEQ_OK : cuda_fail(e);
 }
 

@@ -6,6 +6,7 @@
 #include <cuda_runtime.h>
 #include "fasteq_b200.h"
 #include "core_common.h"
+#include "fasteq_device.cuh"
 
 using namespace fasteq;
 
@@ -14,6 +15,7 @@ namespace {
 template <typename T>
 __global__ void __launch_bounds__(256) readout_fwd_kernel(const T* __restrict__ h, const T* __restrict__ w, const T* __restrict__ e_in,
                                                           T* __restrict__ e, long long n, int c_count, long long d) {
+  let_next_kernel_begin();
   const long long node = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (node >= n) return;
@@ -29,6 +31,7 @@ __global__ void __launch_bounds__(256) readout_fwd_kernel(const T* __restrict__ 
 template <typename T>
 __global__ void __launch_bounds__(256) readout_bwd_kernel(const T* __restrict__ g, const T* __restrict__ w, T* __restrict__ gh, long long n,
                                                           int c_count, long long d) {
+  let_next_kernel_begin();
   const long long node = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
   if (node >= n) return;
   const T gv = g[node];

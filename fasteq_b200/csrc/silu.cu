@@ -11,6 +11,7 @@
 #include <cuda_runtime.h>
 #include "fasteq_b200.h"
 #include "core_common.h"
+#include "fasteq_device.cuh"
 
 using namespace fasteq;
 
@@ -24,6 +25,7 @@ template <typename T> __device__ __forceinline__ T times_slope(T g, T z, T s) { 
 template <typename T, int ORDER, int V>
 __global__ void __launch_bounds__(256) silu_kernel(const T* __restrict__ z, const T* __restrict__ g, const T* __restrict__ h,
                                                    T* __restrict__ out0, T* __restrict__ out1, long long n) {
+  let_next_kernel_begin();
   struct alignas(sizeof(T) * V) Pack { T v[V]; };
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n / V) {
