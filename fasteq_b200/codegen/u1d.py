@@ -707,9 +707,14 @@ static int run_forward(const fasteq_u1d_graph* gh, const int32_t* part_edge, voi
   if (VEC == 2 && ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(carry)) & 7u)) return FASTEQ_INVALID;
   cudaError_t e = cudaFuncSetAttribute(fasteq_u1d_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
   if (e != cudaSuccess) return cuda_fail(e);
-  e = launch_dependent(fasteq_u1d_fwd_kernel, (unsigned)grid, NTHREADS, SMEM_BYTES, (cudaStream_t)stream,
-      g, (const T*)w, (const T*)x, (const T*)y, (T*)out, (T*)carry{host_args});
-  if (e != cudaSuccess) return cuda_fail(e);
+  if (cfg::SCATTERED) {{             // every operand address comes from an index loaded after the kernel's wait: see launch.cuh
+    e = launch_dependent(fasteq_u1d_fwd_kernel, (unsigned)grid, NTHREADS, SMEM_BYTES, (cudaStream_t)stream,
+        g, (const T*)w, (const T*)x, (const T*)y, (T*)out, (T*)carry{host_args});
+    if (e != cudaSuccess) return cuda_fail(e);
+  }} else {{
+    fasteq_u1d_fwd_kernel<<<grid, NTHREADS, SMEM_BYTES, (cudaStream_t)stream>>>(
+        g, (const T*)w, (const T*)x, (const T*)y, (T*)out, (T*)carry{host_args});
+  }}
   if (part_edge)
     fasteq_u1d_carry_kernel<<<(unsigned)gh->n_parts, 256, 0, (cudaStream_t)stream>>>(
         gh->seg_ptr, gh->part_ptr, part_edge, gh->n_parts, (int)gh->n_out_rows, (const T*)carry, (T*)out);
@@ -1235,8 +1240,14 @@ static int run_backward(const fasteq_u1d_graph* gh, const int32_t* part_edge, co
     return FASTEQ_INVALID;
   e = cudaFuncSetAttribute(fasteq_u1d_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
   if (e != cudaSuccess) return cuda_fail(e);
-  e = launch_dependent(fasteq_u1d_bwd_kernel, (unsigned)grid, NTHREADS, SMEM_BYTES, s, g, (const T*)go, (const T*)w, (const T*)x, (const T*)y,
-                       (T*)gw, (T*)gx, (T*)gy{host_args});
+  if (cfg::SCATTERED) {{
+    e = launch_dependent(fasteq_u1d_bwd_kernel, (unsigned)grid, NTHREADS, SMEM_BYTES, s, g, (const T*)go, (const T*)w, (const T*)x, (const T*)y,
+                         (T*)gw, (T*)gx, (T*)gy{host_args});
+  }} else {{
+    fasteq_u1d_bwd_kernel<<<grid, NTHREADS, SMEM_BYTES, s>>>(g, (const T*)go, (const T*)w, (const T*)x, (const T*)y,
+                                                            (T*)gw, (T*)gx, (T*)gy{host_args});
+    e = cudaGetLastError();
+  }}
   if (e != cudaSuccess) return cuda_fail(e);
   return FASTEQ_OK;
 }}
