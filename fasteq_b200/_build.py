@@ -74,6 +74,49 @@ def build_core(force: bool = False) -> str:
     return CORE_SO
 
 
+FRONT = os.path.join(CSRC, "front")
+FRONT_SO = os.path.join(LIB, "fasteq_front.so")
+FRONT_SOURCES = ["module.cpp", "prepared.cpp", "layers.cpp", "edges.cpp", "u1d.cpp"]
+_front_lock = threading.Lock()
+
+
+def build_front(force: bool = False) -> str:
+    """The native host path: host code only, compiled with g++ against torch's headers."""
+    import sysconfig
+    import tempfile
+    from concurrent.futures import ThreadPoolExecutor
+    srcs = [os.path.join(FRONT, s) for s in FRONT_SOURCES]
+    deps = srcs + [os.path.join(FRONT, "front.h"), os.path.join(INCLUDE, "fasteq_b200.h")]
+    with _front_lock:
+        if not force and _newer(FRONT_SO, deps):
+            return FRONT_SO
+        import torch
+        base = os.path.dirname(torch.__file__)
+        cuda = os.path.dirname(os.path.dirname(nvcc_path()))
+        cxx = os.environ.get("CXX") or shutil.which("g++")
+        if not cxx:
+            raise BuildError("g++ not found: fasteq_b200 compiles its host path with it and has no fallback path")
+        flags = ["-O2", "-std=c++17", "-fPIC", "-DTORCH_EXTENSION_NAME=fasteq_front", "-DTORCH_API_INCLUDE_EXTENSION_H",
+                 f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
+        flags += [f"-I{p}" for p in (os.path.join(base, "include"), os.path.join(base, "include", "torch", "csrc", "api", "include"),
+                                     sysconfig.get_paths()["include"], os.path.join(cuda, "include"), INCLUDE)]
+        os.makedirs(LIB, exist_ok=True)
+        with tempfile.TemporaryDirectory(dir=LIB) as tmp:
+            def run(cmd):
+                r = subprocess.run(cmd, capture_output=True, text=True)
+                if r.returncode != 0:
+                    raise BuildError(f"{cmd[0]} failed ({' '.join(cmd)}):\n{r.stdout}\n{r.stderr}")
+            objs = [os.path.join(tmp, s[:-4] + ".o") for s in FRONT_SOURCES]
+            with ThreadPoolExecutor(len(srcs)) as ex:
+                list(ex.map(lambda so: run([cxx] + flags + ["-c", so[0], "-o", so[1]]), zip(srcs, objs)))
+            out = os.path.join(tmp, "fasteq_front.so")
+            libs = os.path.join(base, "lib")
+            run([cxx, "-shared", "-o", out] + objs + [f"-L{libs}", f"-Wl,-rpath,{libs}", f"-L{cuda}/lib64", "-ltorch", "-ltorch_cpu", "-ltorch_cuda",
+                                                       "-ltorch_python", "-lc10", "-lc10_cuda", "-lcudart"])
+            os.replace(out, FRONT_SO)
+    return FRONT_SO
+
+
 def build_generated(name: str, source: str, extra: Optional[List[str]] = None, force: bool = False) -> str:
     """Compile generated CUDA text into ``lib/jit/<name>.so`` unless an up-to-date build exists."""
     so = os.path.join(JIT, name + ".so")

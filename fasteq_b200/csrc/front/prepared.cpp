@@ -1,0 +1,102 @@
+// Cache of prepared (split / packed) weight forms for the tensor-core kernels, shared by the SO3Linear, dense and radial-chain
+// operators.  Keyed on the weight tensors' storage address and version, so an in-place update or a new tensor invalidates the entry; an
+// entry keeps the weights' storages alive (through detached aliases: a parameter object can be given another storage,
+// `module.double()` or `p.data = ...`) so the address cannot be reused while it exists.  An entry remembers the stream it was built
+// on and an event recorded behind the build: a later call on another stream waits for that event (and tells the allocator about the
+// new reader) before it uses the entry.  Plays the part of the reference's plan LRU
+// (fasteq/ops/auto_schedule/eqlinear_plan.py:38-41, :81-100, :167-187).
+//
+// Inside CUDA-graph capture a prepared form would be baked into the graph and go stale when the weights change, so the cache is bypassed
+// there unless the caller declares the weights frozen.
+#include "front.h"
+
+namespace front {
+namespace {
+
+struct Entry {
+  std::string key;
+  std::vector<Tensor> weights;
+  Tensor value;
+  at::cuda::CUDAEvent built;
+  std::set<cudaStream_t> ordered;      // streams already behind the build
+};
+
+constexpr int64_t kDefaultBudget = 256LL << 20;
+std::mutex lock;
+std::list<Entry> entries;              // most recently used first
+std::unordered_map<std::string, std::list<Entry>::iterator> index_of;
+int64_t bytes = 0, budget = kDefaultBudget;
+int frozen = 0;
+
+void drop_last() {
+  bytes -= entries.back().value.nbytes();
+  index_of.erase(entries.back().key);
+  entries.pop_back();
+}
+
+void append(std::string& key, int64_t v) { key.append(reinterpret_cast<const char*>(&v), sizeof v); }
+
+}  // namespace
+
+std::optional<Tensor> prepared(const std::vector<Tensor>& weights, const std::string& tag, const std::function<Tensor()>& build) {
+  std::string key = tag;
+  append(key, weights[0].device().index());
+  for (const Tensor& w : weights) {
+    append(key, (int64_t)w.const_data_ptr()); append(key, w._version()); append(key, w.numel());
+  }
+  const bool in_capture = capturing();
+  {
+    std::lock_guard<std::mutex> g(lock);
+    if (budget <= 0 || (in_capture && !frozen)) return std::nullopt;
+    auto hit = index_of.find(key);
+    if (hit != index_of.end()) {
+      entries.splice(entries.begin(), entries, hit->second);
+      Entry& e = entries.front();
+      if (!in_capture) {
+        auto cur = c10::cuda::getCurrentCUDAStream(e.value.device().index());
+        if (e.ordered.insert(cur.stream()).second) {
+          e.built.block(cur);
+          c10::cuda::CUDACachingAllocator::recordStream(e.value.storage().data_ptr(), cur);
+        }
+      }
+      return e.value;
+    }
+    if (in_capture) return std::nullopt;             // nothing persistent may be allocated inside a capture
+  }
+  Tensor value = build();
+  if (!value.defined()) return std::nullopt;
+  auto cur = c10::cuda::getCurrentCUDAStream(value.device().index());
+  Entry e;
+  e.key = key; e.value = value; e.ordered.insert(cur.stream());
+  for (const Tensor& w : weights) e.weights.push_back(w.detach());
+  e.built.record(cur);
+  std::lock_guard<std::mutex> g(lock);
+  auto hit = index_of.find(key);                      // another thread may have built it meanwhile
+  if (hit != index_of.end()) { bytes -= hit->second->value.nbytes(); entries.erase(hit->second); index_of.erase(hit); }
+  while (!entries.empty() && bytes + (int64_t)value.nbytes() > budget) drop_last();
+  entries.push_front(std::move(e));
+  index_of[key] = entries.begin();
+  bytes += value.nbytes();
+  return value;
+}
+
+void bind_prepared(py::module_& m) {
+  auto clear = [] {
+    std::lock_guard<std::mutex> g(lock);
+    entries.clear(); index_of.clear(); bytes = 0;
+  };
+  m.def("prepared_clear", clear);
+  m.def("prepared_set_budget", [clear](std::optional<int64_t> most) {
+    { std::lock_guard<std::mutex> g(lock); budget = most.value_or(kDefaultBudget); }
+    if (most && *most <= 0) clear();
+  });
+  m.def("prepared_freeze", [](int by) { std::lock_guard<std::mutex> g(lock); frozen += by; });
+  m.def("prepared_snapshot", [] {
+    std::vector<Tensor> out;
+    std::lock_guard<std::mutex> g(lock);
+    for (const Entry& e : entries) out.push_back(e.value);
+    return out;
+  });
+}
+
+}  // namespace front

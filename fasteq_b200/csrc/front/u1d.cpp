@@ -1,0 +1,252 @@
+// The tensor-product operator in its usual form: per-edge weights, sender gather, scalar y (or edge vectors), receiver scatter.
+#include "front.h"
+
+namespace front {
+namespace {
+
+using Flags = std::array<bool, 3>;
+
+struct U1DModule : torch::CustomClassHolder {
+  decltype(&fasteq_u1d_forward) forward; decltype(&fasteq_u1d_forward_split) forward_split;
+  decltype(&fasteq_u1d_backward) backward; decltype(&fasteq_u1d_backward_split) backward_split;
+  decltype(&fasteq_u1d_tangent_forward) tangent_forward; decltype(&fasteq_u1d_tangent_backward) tangent_backward;
+  decltype(&fasteq_last_cuda_error) error;
+  PyKeep object;
+};
+using Module = c10::intrusive_ptr<U1DModule>;
+
+// One operator signature: extents and the modules loaded for it so far.
+struct Signature : torch::CustomClassHolder {
+  int64_t u, w_segs, x_segs, y_segs, out_segs;
+  bool y_sh;
+  PyKeep load;                 // (direction, needs, tangents or None, odd address) -> (module, {name: address})
+  std::mutex lock;
+  std::unordered_map<int, Module> modules;
+  Signature(int64_t u_, int64_t w, int64_t x, int64_t y, int64_t o, bool sh, py::object l)
+      : u(u_), w_segs(w), x_segs(x), y_segs(y), out_segs(o), y_sh(sh), load(std::move(l)) {}
+  int64_t y_cols() const { return y_sh ? 3 : y_segs; }
+  Module module(bool backward, Flags needs, const Flags* tangents, bool odd) {
+    int key = backward | odd << 1;
+    for (int i = 0; i < 3; ++i) key |= needs[i] << (2 + i) | (tangents && (*tangents)[i]) << (5 + i);
+    if (tangents) key |= 1 << 8;
+    {
+      std::lock_guard<std::mutex> g(lock);
+      auto hit = modules.find(key);
+      if (hit != modules.end()) return hit->second;
+    }
+    auto m = c10::make_intrusive<U1DModule>();
+    {
+      py::gil_scoped_acquire gil;
+      py::tuple got = load.get()(backward ? "bwd" : "fwd", needs, tangents ? py::cast(*tangents) : py::none(), odd);
+      auto d = got[1].cast<std::unordered_map<std::string, uint64_t>>();
+#define F(name) m->name = reinterpret_cast<decltype(m->name)>(d.at("fasteq_u1d_" #name));
+      F(forward) F(forward_split) F(backward) F(backward_split) F(tangent_forward) F(tangent_backward)
+#undef F
+      m->error = reinterpret_cast<decltype(m->error)>(d.at("fasteq_last_cuda_error"));
+      m->object.p = py::object(got[0]).release().ptr();
+    }
+    std::lock_guard<std::mutex> g(lock);
+    return modules.emplace(key, m).first->second;
+  }
+};
+using Sig = c10::intrusive_ptr<Signature>;
+
+// A graph plan as the launches need it.  Shares are asked of the Python plan once per module; `ordered`: streams behind the plan's kernels.
+struct Plan : torch::CustomClassHolder {
+  struct Shares { Tensor part; int32_t n = 0; bool split = false; };
+  Tensor seg_ptr, perm;
+  int64_t n_rows, n_edges;
+  PyKeep share;                // module -> (partition tensor, n_parts, split)
+  PyKeep ready;                // orders the current stream behind the plan's kernels
+  PyKeep record;               // enters the plan into the lists of record_plans
+  std::mutex lock;
+  std::unordered_map<U1DModule*, std::pair<Module, Shares>> shares;
+  std::set<cudaStream_t> ordered;
+  Plan(Tensor s, std::optional<Tensor> p, int64_t rows, int64_t edges, py::object sh, py::object rd, py::object rc)
+      : seg_ptr(std::move(s)), n_rows(rows), n_edges(edges), share(std::move(sh)), ready(std::move(rd)), record(std::move(rc)) {
+    if (p) perm = *p;
+  }
+  Shares shares_of(const Module& m) {
+    {
+      std::lock_guard<std::mutex> g(lock);
+      auto hit = shares.find(m.get());
+      if (hit != shares.end()) return hit->second.second;
+    }
+    Shares s;
+    {
+      py::gil_scoped_acquire gil;
+      py::tuple got = share.get()(m->object.get());
+      s.part = got[0].cast<Tensor>(); s.n = got[1].cast<int32_t>(); s.split = got[2].cast<bool>();
+    }
+    std::lock_guard<std::mutex> g(lock);
+    shares.emplace(m.get(), std::make_pair(m, s));
+    return s;
+  }
+  void order(cudaStream_t s, bool recording) {
+    bool first;
+    { std::lock_guard<std::mutex> g(lock); first = !ordered.count(s); }
+    if (!first && !recording) return;
+    py::gil_scoped_acquire gil;
+    if (first) {
+      ready.get()();
+      if (!capturing()) { std::lock_guard<std::mutex> g(lock); ordered.insert(s); }
+    }
+    if (recording) record.get()();
+  }
+};
+using PlanPtr = c10::intrusive_ptr<Plan>;
+std::atomic<int> recording{0};
+
+struct Call : torch::CustomClassHolder {
+  Sig sig;
+  PlanPtr plan;
+  Tensor src;
+  int64_t x_rows;
+  PyKeep graph;                // the Python plan, which the native one knows only weakly
+};
+using CallPtr = c10::intrusive_ptr<Call>;
+
+// the launch's graph record; returns the address of the shares' first edges when they cut receivers
+const int32_t* graph_of(const Call& c, const Module& m, const Tensor& any, fasteq_u1d_graph* g, Plan::Shares* s) {
+  *s = c.plan->shares_of(m);
+  c.plan->order(stream_of(any), recording.load() > 0);
+  *g = {};
+  g->n_edges = c.plan->n_edges; g->n_out_rows = c.plan->n_rows; g->x_rows = c.x_rows; g->y_rows = c.plan->n_edges;
+  g->x_index = c.src.const_data_ptr<int32_t>();
+  g->seg_ptr = c.plan->seg_ptr.const_data_ptr<int32_t>();
+  g->perm = c.plan->perm.defined() ? c.plan->perm.const_data_ptr<int32_t>() : nullptr;
+  g->n_parts = s->n;
+  g->part_ptr = s->part.const_data_ptr<int32_t>();
+  return s->split ? g->part_ptr + s->n + 1 : nullptr;
+}
+
+bool odd(std::initializer_list<Tensor> ts) {
+  for (const Tensor& t : ts) if (t.defined() && reinterpret_cast<uintptr_t>(t.const_data_ptr()) % 8) return true;
+  return false;
+}
+
+Tensor forward_launch(const Call& c, const Tensor& w, const Tensor& x, const Tensor& y, const Tensor* t, const Flags* has) {
+  c10::cuda::CUDAGuard guard(x.device());
+  const int64_t cols = c.sig->out_segs * c.sig->u;
+  Tensor out = at::empty({c.plan->n_rows, cols}, x.options());
+  const Module m = c.sig->module(false, {false, false, false}, has, odd({w, x, y, out}) || (t && odd({t[0], t[1], t[2]})));
+  fasteq_u1d_graph g;
+  Plan::Shares s;
+  const int32_t* edge = graph_of(c, m, x, &g, &s);
+  Tensor carry;
+  if (edge) carry = at::empty({s.n, cols}, x.options());
+  cudaStream_t st = stream_of(x);
+  if (t) check(m->tangent_forward(&g, edge, mptr(carry), ptr(w), ptr(x), ptr(y), ptr(t[0]), ptr(t[1]), ptr(t[2]), mptr(out), st), "fasteq_u1d_tangent_forward", m->error);
+  else if (edge) check(m->forward_split(&g, edge, mptr(carry), ptr(w), ptr(x), ptr(y), mptr(out), st), "fasteq_u1d_forward_split", m->error);
+  else check(m->forward(&g, ptr(w), ptr(x), ptr(y), mptr(out), st), "fasteq_u1d_forward", m->error);
+  return out;
+}
+
+variable_list backward_launch(const Call& c, const Tensor& go, const Tensor& w, const Tensor& x, const Tensor& y, Flags needs, const Tensor* t, const Flags* has) {
+  c10::cuda::CUDAGuard guard(x.device());
+  variable_list d = {needs[0] ? at::empty_like(w) : Tensor(), needs[1] ? at::empty_like(x) : Tensor(), needs[2] ? at::empty_like(y) : Tensor()};
+  const Module m = c.sig->module(true, needs, has, odd({go, w, x, y, d[0], d[1], d[2]}) || (t && odd({t[0], t[1], t[2]})));
+  fasteq_u1d_graph g;
+  Plan::Shares s;
+  const int32_t* edge = graph_of(c, m, x, &g, &s);
+  cudaStream_t st = stream_of(x);
+  if (t) check(m->tangent_backward(&g, edge, ptr(go), ptr(w), ptr(x), ptr(y), ptr(t[0]), ptr(t[1]), ptr(t[2]), mptr(d[0]), mptr(d[1]), mptr(d[2]), st),
+               "fasteq_u1d_tangent_backward", m->error);
+  else if (edge) check(m->backward_split(&g, edge, ptr(go), ptr(w), ptr(x), ptr(y), mptr(d[0]), mptr(d[1]), mptr(d[2]), st), "fasteq_u1d_backward_split", m->error);
+  else check(m->backward(&g, ptr(go), ptr(w), ptr(x), ptr(y), mptr(d[0]), mptr(d[1]), mptr(d[2]), st), "fasteq_u1d_backward", m->error);
+  return d;
+}
+
+struct TensorProductBackward : torch::autograd::Function<TensorProductBackward> {
+  static variable_list forward(AutogradContext* ctx, const Tensor& go, const Tensor& w, const Tensor& x, const Tensor& y, const CallPtr& c, Flags needs) {
+    auto d = backward_launch(*c, go, w, x, y, needs, nullptr, nullptr);
+    ctx->save_for_backward({go, w, x, y});
+    ctx->saved_data["c"] = capsule(c);
+    ctx->saved_data["n"] = (int64_t)(needs[0] | needs[1] << 1 | needs[2] << 2);
+    ctx->set_materialize_grads(false);
+    for (int i = 0; i < 3; ++i) if (!needs[i]) d[i] = at::empty({0}, x.options());
+    return d;
+  }
+  // of <go, F(w', x, y) + F(w, x', y) + F(w, x, y')>: one pass over the edges for grad_out's gradient, one for the operands'
+  static variable_list backward(AutogradContext* ctx, variable_list gg) {
+    const auto saved = ctx->get_saved_variables();
+    const CallPtr c = uncapsule<Call>(ctx->saved_data["c"]);
+    const int64_t needed = ctx->saved_data["n"].toInt();
+    Tensor t[3];
+    Flags has{};
+    for (int i = 0; i < 3; ++i) {
+      if ((needed >> i & 1) && gg[i].defined()) t[i] = gg[i].contiguous();
+      has[i] = t[i].defined();
+    }
+    variable_list out(6);
+    if (!has[0] && !has[1] && !has[2]) return out;
+    const Tensor &go = saved[0], &w = saved[1], &x = saved[2], &y = saved[3];
+    if (ctx->needs_input_grad(0)) out[0] = forward_launch(*c, w, x, y, t, &has);
+    // a gradient needs a tangent on another operand
+    const Flags needs = {ctx->needs_input_grad(1) && (has[1] || has[2]), ctx->needs_input_grad(2) && (has[0] || has[2]),
+                         ctx->needs_input_grad(3) && (has[0] || has[1])};
+    if (needs[0] || needs[1] || needs[2]) {
+      auto d = backward_launch(*c, go, w, x, y, needs, t, &has);
+      for (int i = 0; i < 3; ++i) out[1 + i] = d[i];
+    }
+    return out;
+  }
+};
+
+struct TensorProduct : torch::autograd::Function<TensorProduct> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& w, const Tensor& x, const Tensor& y, const CallPtr& c) {
+    ctx->save_for_backward({w, x, y});
+    ctx->saved_data["c"] = capsule(c);
+    return forward_launch(*c, w, x, y, nullptr, nullptr);
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list gout) {
+    const auto saved = ctx->get_saved_variables();
+    const Tensor &w = saved[0], &x = saved[1], &y = saved[2];
+    const CallPtr c = uncapsule<Call>(ctx->saved_data["c"]);
+    const Flags needs = {ctx->needs_input_grad(0), ctx->needs_input_grad(1), ctx->needs_input_grad(2)};
+    if (!needs[0] && !needs[1] && !needs[2]) return variable_list(4);
+    const Tensor go = gout[0].contiguous();
+    variable_list d;
+    if (c->sig->y_sh) {
+      // not trilinear in the edge vector: the second-order kernels do not apply
+      if (at::GradMode::is_enabled() && (go.requires_grad() || w.requires_grad() || x.requires_grad() || y.requires_grad()))
+        throw std::runtime_error("fast_uniform1d_jit: no second-order gradient with in-kernel spherical harmonics; pass the harmonics as the y operand instead");
+      d = backward_launch(*c, go, w, x, y, needs, nullptr, nullptr);
+    } else {
+      d = TensorProductBackward::apply(go, w, x, y, c, needs);
+    }
+    for (int i = 0; i < 3; ++i) if (!needs[i]) d[i] = Tensor();
+    d.resize(4);
+    return d;
+  }
+};
+
+}  // namespace
+
+void bind_u1d(py::module_& m) {
+  py::class_<Signature, Sig>(m, "Signature").def(py::init([](int64_t u, int64_t w, int64_t x, int64_t y, int64_t o, bool sh, py::object load) {
+    return c10::make_intrusive<Signature>(u, w, x, y, o, sh, std::move(load));
+  }));
+  py::class_<Plan, PlanPtr>(m, "Plan")
+      .def(py::init([](Tensor seg, std::optional<Tensor> perm, int64_t rows, int64_t edges, py::object share, py::object ready, py::object record) {
+        return c10::make_intrusive<Plan>(std::move(seg), std::move(perm), rows, edges, std::move(share), std::move(ready), std::move(record));
+      }))
+      .def("reordered", [](Plan& p) { std::lock_guard<std::mutex> g(p.lock); p.ordered.clear(); });
+  m.def("u1d_recording", [](int by) { recording += by; });
+  // None: an operand this form does not take (the general path says what is wrong with it, or takes it)
+  m.def("u1d", [](const Tensor& w, const Tensor& x, const Tensor& y, const Tensor& src, const Sig& sig, const PlanPtr& plan, py::object graph) -> std::optional<Tensor> {
+    const int64_t E = plan->n_edges, u = sig->u;
+    for (const Tensor* t : {&w, &x, &y})
+      if (!t->is_cuda() || !t->is_contiguous() || t->dim() < 2 || t->scalar_type() != x.scalar_type() || t->device() != x.device()) return std::nullopt;
+    if (E == 0 || plan->n_rows == 0 || w.numel() != E * sig->w_segs * u || x.numel() != plan->n_rows * sig->x_segs * u || y.numel() != E * sig->y_cols() ||
+        (sig->y_sh && y.size(-1) != 3) || !src.is_cuda() || src.numel() != E)
+      return std::nullopt;
+    auto c = c10::make_intrusive<Call>();
+    c->sig = sig; c->plan = plan; c->x_rows = plan->n_rows;
+    c->graph.p = graph.release().ptr();
+    c->src = (src.scalar_type() == at::kInt ? src : src.to(at::kInt)).contiguous();
+    return TensorProduct::apply(w, x, y, c);
+  });
+}
+
+}  // namespace front

@@ -181,6 +181,9 @@ class LinearDescriptor:
                          tuple((int(i), self.v) for i in out_dims)]
         self.operands_and_subscripts = tuple(zip(self.operands, ("uv", "iu", "iv")))
 
+    def __getstate__(self):
+        return {k: v for k, v in self.__dict__.items() if k != "_native"}       # the operator's handle belongs to this process
+
     def get_dims(self, name: str):
         return {"u": [self.u], "v": [self.v]}[name]
 

@@ -15,9 +15,7 @@ import ctypes as C
 
 import torch
 
-from .. import _cabi
-from . import _prepared
-from ._needs import wanted
+from .. import _cabi, _front
 
 _ready = False
 
@@ -26,10 +24,7 @@ def _lib():
     global _ready
     lib = _cabi.core()
     if not _ready:
-        lib.fasteq_gemm_tf32x3.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64, C.c_int32, C.c_int32, C.c_void_p]
         lib.fasteq_tensorcore_device_status.argtypes = [C.POINTER(C.c_int32)]
-        lib.fasteq_gemm_tf32x3_split.argtypes = [C.c_void_p, C.c_int64, C.c_void_p, C.c_void_p]
-        lib.fasteq_gemm_tf32x3_presplit.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64, C.c_int32, C.c_int32, C.c_void_p]
         _ready = True
     return lib
 
@@ -103,87 +98,12 @@ def _matmul_tn(g: torch.Tensor, x: torch.Tensor) -> torch.Tensor:
     return g.t() @ x
 
 
-def _gemm(a: torch.Tensor, bt: torch.Tensor, weight: torch.Tensor = None, transposed: bool = False) -> torch.Tensor:
-    """a [M, K] @ bt[N, K]^T -> [M, N].  ``weight`` (optional) is the parameter ``bt`` derives from: its TF32 parts
-    are then prepared once per weight version instead of once per call."""
-    a = a.contiguous()
-    M, K = a.shape
-    N = bt.shape[0]
-    out = torch.empty((M, N), dtype=a.dtype, device=a.device)
-    lib = _lib()
-    with _cabi.on_device(a.device):
-        stream = _cabi.stream(a.device)
-
-        def build():
-            b = bt.contiguous()
-            sp = torch.empty(2 * b.numel(), dtype=torch.float32, device=b.device)
-            _cabi.check(lib.fasteq_gemm_tf32x3_split(b.data_ptr(), b.numel(), sp.data_ptr(), stream), lib, "fasteq_gemm_tf32x3_split")
-            return sp
-        split = _prepared.get((weight,), ("dense", transposed), build) if weight is not None else None
-        if split is None:
-            split = build()
-        rc = lib.fasteq_gemm_tf32x3_presplit(a.data_ptr(), split.data_ptr(), out.data_ptr(), M, N, K, stream)
-    if rc == 1:   # FASTEQ_UNSUPPORTED (operand alignment): the FP32 FMA tile kernel takes any shape and alignment
-        return _fma_gemm(a, bt.t())
-    _cabi.check(rc, lib, "fasteq_gemm_tf32x3")
-    return out
-
-
-class _Dense(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, x, weight):
-        ctx.save_for_backward(x, weight)
-        return _gemm(x, weight, weight, False)
-
-    @staticmethod
-    def backward(ctx, grad_out):
-        x, weight = ctx.saved_tensors
-        need_x, need_w = ctx.needs_input_grad[0], wanted(ctx, 1)
-        if not (need_x or need_w):
-            return None, None
-        gx, gw = _DenseBackward.apply(grad_out.contiguous(), x, weight, need_x, need_w)
-        return (gx if need_x else None), (gw if need_w else None)
-
-
-class _DenseBackward(torch.autograd.Function):
-    """First backward as a differentiable function (``y = x W^T`` is bilinear):
-    ``d_g = ggx W^T + x ggW^T``, ``d_x = g ggW``, ``d_W = g^T ggx``."""
-
-    @staticmethod
-    def forward(ctx, g, x, weight, need_x, need_w):
-        ctx.need = (need_x, need_w)
-        ctx.save_for_backward(g, x, weight)
-        ctx.set_materialize_grads(False)
-        gx = _gemm(g, weight.t(), weight, True) if need_x else x.new_empty((0,))     # [M, N] @ [N, K], Bt = weight^T [K, N]
-        gw = _matmul_tn(g, x) if need_w else weight.new_empty((0,))                  # reduction over the rows, fixed order
-        return gx, gw
-
-    @staticmethod
-    def backward(ctx, ggx, ggw):
-        g, x, weight = ctx.saved_tensors
-        ggx = ggx.contiguous() if (ggx is not None and ctx.need[0]) else None
-        ggw = ggw.contiguous() if (ggw is not None and ctx.need[1]) else None
-        want_g, want_x, want_w = ctx.needs_input_grad[:3]
-        d_g = d_x = d_w = None
-        if want_g:
-            if ggx is not None:
-                d_g = _gemm(ggx, weight, weight, False)
-            if ggw is not None:
-                t = _gemm(x, ggw)
-                d_g = t if d_g is None else d_g + t
-        if want_x and ggw is not None:
-            d_x = _gemm(g, ggw.t())
-        if want_w and ggx is not None:
-            d_w = _matmul_tn(g, ggx)
-        return d_g, d_x, d_w, None, None
-
-
 def dense(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
     """``x [..., K] @ weight[N, K]^T``."""
     lead = x.shape[:-1]
     x2 = x.reshape(-1, x.shape[-1])
     if _usable(x2, weight.shape[0], weight.shape[1]) and weight.dtype == torch.float32:
-        return _Dense.apply(x2, weight).reshape(*lead, weight.shape[0])
+        return _front.lib().dense(x2, weight).reshape(*lead, weight.shape[0])
     if x2.is_cuda and x2.dtype in (torch.float32, torch.float64) and weight.dtype == x2.dtype:
         return _DenseFMA.apply(x2, weight).reshape(*lead, weight.shape[0])
     return x @ weight.t()

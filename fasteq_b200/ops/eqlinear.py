@@ -17,9 +17,9 @@ from typing import Dict, List, Tuple
 
 import torch
 
-from .. import _cabi
+from .. import _cabi, _front
+from ..descriptors import LinearDescriptor
 from . import _prepared
-from ._needs import wanted
 
 __all__ = ["fast_equi_linear", "eqlinear_clear_plan_cache", "eqlinear_set_plan_cache", "eqlinear_debug_info"]
 
@@ -132,9 +132,6 @@ def _core():
         lib.fasteq_eqlinear_wgrad.argtypes = [C.POINTER(_Problem), C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]
         lib.fasteq_eqlinear_wgrad_scratch.argtypes = [C.POINTER(_Problem), C.c_void_p, C.c_void_p, C.POINTER(C.c_int64)]
         lib.fasteq_eqlinear_wgrad_with.argtypes = [C.POINTER(_Problem), C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64, C.c_void_p]
-        lib.fasteq_eqlinear_pack.argtypes = [C.POINTER(_Problem), C.c_int32, C.c_void_p, C.c_void_p, C.c_void_p]
-        lib.fasteq_eqlinear_forward_packed.argtypes = [C.POINTER(_Problem), C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]
-        lib.fasteq_eqlinear_dgrad_packed.argtypes = [C.POINTER(_Problem), C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]
         _core_ready = True
     return lib
 
@@ -145,52 +142,6 @@ def _make_problem(mapping, coeff, u, v, I, J, batch, precision):
     prob = _Problem(precision, u, v, I, J, P, batch, arr([m[0] for m in mapping]), arr([m[1] for m in mapping]),
                     arr([m[3] for m in mapping]), (C.c_double * P)(*coeff))
     return prob
-
-
-def _check_inputs(w, x, u, v, I, P):
-    if not (x.is_cuda and w.is_cuda):
-        raise RuntimeError("eqlinear: x and w must be CUDA tensors: fasteq_b200 has no CPU path")
-    if x.shape[-1] != I * u and x.numel() % (I * u) != 0:
-        raise ValueError(f"eqlinear: x has {x.numel()} elements, not a multiple of I*U = {I * u}")
-    if w.numel() != P * u * v:
-        raise ValueError(f"eqlinear: w has {w.numel()} elements, expected P*U*V = {P * u * v}")
-
-
-def _order_weights(w3d, mapping):
-    """Weight block of path q must sit at index q: reorder only if the descriptor says otherwise."""
-    wps = [m[2] for m in mapping]
-    if wps == list(range(len(wps))):
-        return w3d
-    return w3d[torch.tensor(wps, device=w3d.device)].contiguous()
-
-
-def _packed_weights(w, w3, geom_key, prob, dgrad: bool, lib, stream, keep: bool):
-    """Pre-scaled, K-major, TF32-split weight blocks of this problem and direction.  Cached per weight version with ``keep``; built for
-    this call alone where a cotangent stands in the weights' place and where the cache must not be used."""
-    def build():
-        packed = torch.empty(2 * w3.numel(), dtype=torch.float32, device=w3.device)
-        rc = lib.fasteq_eqlinear_pack(C.byref(prob), 1 if dgrad else 0, w3.data_ptr(), packed.data_ptr(), stream)
-        if rc == 1:      # FASTEQ_UNSUPPORTED
-            return None
-        _cabi.check(rc, lib, "fasteq_eqlinear_pack")
-        return packed
-    packed = _prepared.get((w,), ("eqlinear", geom_key, dgrad), build) if keep else None
-    return build() if packed is None else packed
-
-
-def _run(lib, prob, w, w3, a, c, geom_key, precision, dgrad: bool, stream, keep: bool = True):
-    """One forward / grad_x launch: through prepared weights when the tensor-core path takes the problem."""
-    if precision == _TF32:
-        packed = _packed_weights(w, w3, geom_key, prob, dgrad, lib, stream, keep)
-        if packed is not None:
-            fn = lib.fasteq_eqlinear_dgrad_packed if dgrad else lib.fasteq_eqlinear_forward_packed
-            rc = fn(C.byref(prob), packed.data_ptr(), a.data_ptr(), c.data_ptr(), stream)
-            if rc != 1:
-                _cabi.check(rc, lib, "fasteq_eqlinear_dgrad_packed" if dgrad else "fasteq_eqlinear_forward_packed")
-                return
-    fn = lib.fasteq_eqlinear_dgrad if dgrad else lib.fasteq_eqlinear_forward
-    _cabi.check(fn(C.byref(prob), w3.data_ptr(), a.data_ptr(), c.data_ptr(), stream), lib,
-                "fasteq_eqlinear_dgrad" if dgrad else "fasteq_eqlinear_forward")
 
 
 def wgrad_into(prob, x, g, dw) -> None:
@@ -211,42 +162,20 @@ class _Plan:
 
     def __init__(self, geom, precision, batch, w_shape):
         self.geom, self.precision, self.batch, self.w_shape = geom, precision, batch, tuple(w_shape)
-        mapping, coeff, u, v, I, J = geom
-        self.key = (tuple(mapping), tuple(coeff), u, v, I, J)
-        self.table = [(m[0], m[1], q, m[3]) for q, m in enumerate(mapping)]
 
-    def _problem(self):
-        mapping, coeff, u, v, I, J = self.geom
-        return _make_problem(self.table, coeff, u, v, I, J, self.batch, self.precision)
+    def forward(self, w, x):
+        return _front.lib().eqlinear_launch(_native(self.geom), w, x, self.precision, False)
 
-    def _w3(self, w):
-        mapping, _, u, v, _, _ = self.geom
-        return _order_weights(w.reshape(len(mapping), u, v).contiguous(), mapping)
-
-    def forward(self, w, x, keep: bool = True):
-        mapping, coeff, u, v, I, J = self.geom
-        x3 = x.reshape(self.batch, I, u).contiguous()
-        out = torch.empty((self.batch, J, v), dtype=x.dtype, device=x.device)
-        with _cabi.on_device(x.device):
-            _run(_core(), self._problem(), w, self._w3(w), x3, out, self.key, self.precision, False,
-                 _cabi.stream(x.device), keep)
-        return out.reshape(self.batch, J * v)
-
-    def dgrad(self, w, g, keep: bool = True):
-        mapping, coeff, u, v, I, J = self.geom
-        g3 = g.reshape(self.batch, J, v).contiguous()
-        dx = torch.empty((self.batch, I, u), dtype=g3.dtype, device=g3.device)
-        with _cabi.on_device(g3.device):
-            _run(_core(), self._problem(), w, self._w3(w), g3, dx, self.key, self.precision, True,
-                 _cabi.stream(g3.device), keep)
-        return dx.reshape(self.batch, I * u)
+    def dgrad(self, w, g):
+        return _front.lib().eqlinear_launch(_native(self.geom), w, g, self.precision, True)
 
     def wgrad(self, x, g):
         mapping, coeff, u, v, I, J = self.geom
         x3 = x.reshape(self.batch, I, u).contiguous()
         g3 = g.reshape(self.batch, J, v).contiguous()
         dw = torch.empty((len(mapping), u, v), dtype=g3.dtype, device=g3.device)
-        wgrad_into(self._problem(), x3, g3, dw)
+        table = [(m[0], m[1], q, m[3]) for q, m in enumerate(mapping)]
+        wgrad_into(_make_problem(table, coeff, u, v, I, J, self.batch, self.precision), x3, g3, dw)
         wps = [m[2] for m in mapping]
         if wps != list(range(len(wps))):      # block q of the table is block wps[q] of the caller's tensor
             full = torch.empty_like(dw)
@@ -255,70 +184,29 @@ class _Plan:
         return dw.reshape(self.w_shape)
 
 
-class _EqLinearFn(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, w, x, geom, precision):
-        mapping, coeff, u, v, I, J = geom
-        _check_inputs(w, x, u, v, I, len(mapping))
-        plan = _Plan(geom, precision, x.numel() // (I * u), w.shape)
-        ctx.plan = plan
-        ctx.save_for_backward(w, x)
-        return plan.forward(w, x)
-
-    @staticmethod
-    def backward(ctx, grad_out):
-        w, x = ctx.saved_tensors
-        need_w, need_x = wanted(ctx, 0), ctx.needs_input_grad[1]
-        if not (need_w or need_x):
-            return None, None, None, None
-        dw, dx = _EqLinearBackwardFn.apply(grad_out.contiguous(), w, x, ctx.plan, need_w, need_x)
-        return (dw if need_w else None), (dx.reshape(x.shape) if need_x else None), None, None
+def _native(geom):
+    """The native form of a geometry (``csrc/front/layers.cpp``): the operator, its gradient and its second order."""
+    mapping, coeff, u, v, I, J = geom
+    return _front.lib().Geometry([list(m) for m in mapping], list(coeff), u, v, I, J,
+                                 lambda x, g, precision, batch, w_shape: _Plan(geom, precision, batch, w_shape).wgrad(x, g))
 
 
-class _EqLinearBackwardFn(torch.autograd.Function):
-    """First backward as a differentiable function.  The operator is bilinear in (w, x), so each term of the
-    second backward is one of the three launches again, with a second-order cotangent in place of an operand:
-
-        d_go = F(w, ggx) + F(ggw, x)        d_w = Wg(ggx, go)        d_x = Dg(ggw, go)
-    """
-
-    @staticmethod
-    def forward(ctx, go, w, x, plan, need_w, need_x):
-        ctx.plan, ctx.need = plan, (need_w, need_x)
-        ctx.save_for_backward(go, w, x)
-        ctx.set_materialize_grads(False)
-        dw = plan.wgrad(x, go) if need_w else w.new_empty((0,))
-        dx = plan.dgrad(w, go) if need_x else x.new_empty((0,))
-        return dw, dx
-
-    @staticmethod
-    def backward(ctx, ggw, ggx):
-        go, w, x = ctx.saved_tensors
-        plan = ctx.plan
-        ggw = ggw.contiguous() if (ggw is not None and ctx.need[0]) else None
-        ggx = ggx.contiguous() if (ggx is not None and ctx.need[1]) else None
-        want_go, want_w, want_x = ctx.needs_input_grad[:3]
-        d_go = d_w = d_x = None
-        if want_go:
-            if ggx is not None:
-                d_go = plan.forward(w, ggx)
-            if ggw is not None:
-                t = plan.forward(ggw, x, keep=False)
-                d_go = t if d_go is None else d_go + t
-            if d_go is not None:
-                d_go = d_go.reshape(go.shape)
-        if want_w and ggx is not None:
-            d_w = plan.wgrad(ggx, go)
-        if want_x and ggw is not None:
-            d_x = plan.dgrad(ggw, go, keep=False).reshape(x.shape)
-        return d_go, d_w, d_x, None, None, None
+def _geometry(descriptor):
+    """Native geometry of a descriptor.  One of this package keeps its own, with the tables it was made from: they can be changed."""
+    if type(descriptor) is not LinearDescriptor:
+        return _native(_descriptor_problem(descriptor))
+    tables = (tuple(descriptor.paths), tuple(descriptor.operands), descriptor.operands_and_subscripts, descriptor.u, descriptor.v,
+              descriptor.coefficient_subscripts)
+    kept = descriptor.__dict__.get("_native")
+    if kept is None or kept[0] != tables:
+        kept = descriptor._native = (tables, _native(_descriptor_problem(descriptor)))
+    return kept[1]
 
 
 def fast_equi_linear(descriptor, w, x, *, compute_precision=None):
     """Forward, grad_x and grad_w for the uniform uv/iu/iv eqlinear operator."""
     precision = _resolve_precision(x, w, compute_precision)
-    geom = _descriptor_problem(descriptor)
-    return _EqLinearFn.apply(w, x, geom, precision)
+    return _front.lib().eqlinear(_geometry(descriptor), w, x, precision)
 
 
 def eqlinear_clear_plan_cache() -> None:

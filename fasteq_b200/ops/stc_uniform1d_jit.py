@@ -16,9 +16,8 @@ from typing import Dict, Optional, Tuple
 import numpy as np
 import torch
 
-from .. import _build, _cabi
+from .. import _build, _cabi, _front
 from ..codegen import stc as _emit
-from ._needs import wanted
 
 STC_PAD_VALUE = -1
 _EMITTER_VERSION = "stc-v5"
@@ -75,7 +74,7 @@ def get_module(spec: _emit.STCSpec, direction: str, need_gx0: bool = False, oper
     return mod
 
 
-def _spec_for(x1, coeffs_tensor, paths_tensor, x0_segs: int, num_out_segments: int, pad_value: int) -> _emit.STCSpec:
+def _spec_for(x1, coeffs_tensor, paths_tensor, x0_segs: int, num_out_segments: int, pad_value: int) -> Tuple:
     key = (id(paths_tensor), paths_tensor._version, id(coeffs_tensor), coeffs_tensor._version, x1.shape[1], x1.shape[2],
            x0_segs, num_out_segments, x1.dtype, pad_value)
     hit = _SPECS.get(key)
@@ -93,9 +92,9 @@ def _spec_for(x1, coeffs_tensor, paths_tensor, x0_segs: int, num_out_segments: i
                                    dtype="f32" if x1.dtype == torch.float32 else "f64", pad_value=pad_value)
         if len(_SPECS) > 64:
             _SPECS.clear()
-        hit = (spec, paths_tensor, coeffs_tensor)   # keep the tables alive: their ids are the key
+        hit = (spec, paths_tensor, coeffs_tensor, _native(spec))   # keep the tables alive: their ids are the key
         _SPECS[key] = hit
-    return hit[0]
+    return hit
 
 
 def _validate(x1, x0, i0):
@@ -112,42 +111,34 @@ def _validate(x1, x0, i0):
         raise ValueError("i0 must have one entry per row of x1")
 
 
-class FastSymmetricTensorContractionUniform1dFunction(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, x1, x0, i0, coeffs_tensor, paths_tensor, idx_lists_tensor, num_out_segments, pad_value):
-        _validate(x1, x0, i0)
-        if paths_tensor is None:
-            paths_tensor = idx_lists_tensor
-        spec = _spec_for(x1, coeffs_tensor, paths_tensor, x0.shape[1], num_out_segments, pad_value)
-        x1c, x0c = x1.contiguous(), x0.contiguous()
-        i32 = i0.to(torch.int32).contiguous()
-        B = x1c.shape[0]
-        out = torch.empty((B, spec.out_segs, spec.u), dtype=x1.dtype, device=x1.device)
-        mod = get_module(spec, "fwd", operands=(x1c, x0c))
-        with _cabi.on_device(x1.device):
-            _cabi.check(mod.lib.fasteq_stc_forward(x1c.data_ptr(), x0c.data_ptr(), i32.data_ptr(), B, x0c.shape[0], out.data_ptr(),
-                                                   _cabi.stream(x1.device)), mod.lib, "fasteq_stc_forward")
-        ctx.save_for_backward(x1, x0, i32)      # the inputs themselves, so that a second backward reaches them
-        ctx.spec = spec
-        return out.view(B, spec.out_segs * spec.u)
+class _OddAddress:
+    """Stands for an operand at an odd 4-byte offset."""
 
     @staticmethod
-    def backward(ctx, grad_out):
-        x1, x0, i32 = ctx.saved_tensors
-        spec = ctx.spec
-        need_x1, need_x0 = ctx.needs_input_grad[0], wanted(ctx, 1)
-        if not (need_x1 or need_x0):
-            return (None,) * 8
+    def data_ptr() -> int:
+        return 4
+
+
+_ODD = _OddAddress()
+
+
+def _native(spec: _emit.STCSpec):
+    """The operator on a signature (``csrc/front/edges.cpp``).  Its node launches the forward and the gradient of the features; gradients
+    of the weights and differentiable backwards come from here."""
+
+    def load(direction, odd):
+        lib = get_module(spec, direction, operands=(_ODD,) if odd else ()).lib
+        return _front.addresses(lib, ("fasteq_stc_forward", "fasteq_stc_backward", "fasteq_last_cuda_error"))
+
+    def general(go, x1, x0, i32, need_x1, need_x0):
         if need_x0 and not torch.is_grad_enabled():
             # a first-order backward: nothing differentiates the per-node weight gradients, so they never exist
-            gx1, gx0 = _backward_summed(grad_out.contiguous(), x1.contiguous(), x0.contiguous(), i32, spec)
-            return (gx1 if need_x1 else None), gx0, None, None, None, None, None, None
-        gx1, gx0n = FastSTCBackwardFunction.apply(grad_out.contiguous(), x1.contiguous(), x0.contiguous(), i32, spec, bool(need_x0))
-        gx0 = None
-        if need_x0:
-            # summed over nodes of equal species here (differentiable torch op; the kernel writes per-node rows)
-            gx0 = torch.zeros_like(x0).index_add(0, i32.long(), gx0n)
-        return (gx1 if need_x1 else None), gx0, None, None, None, None, None, None
+            return _backward_summed(go, x1, x0, i32, spec)
+        gx1, gx0n = FastSTCBackwardFunction.apply(go, x1, x0, i32, spec, need_x0)
+        # summed over nodes of equal species here (differentiable torch op; the kernel writes per-node rows)
+        return gx1, torch.zeros_like(x0).index_add(0, i32.long(), gx0n) if need_x0 else None
+
+    return _front.lib().Contraction(spec.u, spec.x1_segs, spec.x0_segs, spec.out_segs, load, general)
 
 
 # Up to here (32 KB of shared memory) one launch counts every node's place; its work grows with the square of the nodes, so that a
@@ -229,5 +220,8 @@ class FastSTCBackwardFunction(torch.autograd.Function):
 def fast_stc_uniform1d_jit(x1, x0, i0, coeffs_tensor, paths_tensor, idx_lists_tensor, num_out_segments: int, *,
                            pad_value: int = STC_PAD_VALUE, use_multiwarp_candidates: bool = False):
     """See module docstring.  ``use_multiwarp_candidates`` is accepted and ignored, as in the reference."""
-    return FastSymmetricTensorContractionUniform1dFunction.apply(x1, x0, i0, coeffs_tensor, paths_tensor, idx_lists_tensor,
-                                                                 int(num_out_segments), int(pad_value))
+    _validate(x1, x0, i0)
+    if paths_tensor is None:
+        paths_tensor = idx_lists_tensor
+    native = _spec_for(x1, coeffs_tensor, paths_tensor, x0.shape[1], int(num_out_segments), int(pad_value))[-1]
+    return _front.lib().symmetric_contraction(x1, x0, i0, native)

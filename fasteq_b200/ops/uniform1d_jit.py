@@ -15,9 +15,9 @@ built once per index tensor and cached.
 """
 from __future__ import annotations
 
-import ctypes
 import dataclasses
 import threading
+import weakref
 from collections import OrderedDict
 from contextlib import contextmanager
 from typing import Dict, List, Optional, Set, Tuple
@@ -25,7 +25,7 @@ from typing import Dict, List, Optional, Set, Tuple
 import numpy as np
 import torch
 
-from .. import _build, _cabi
+from .. import _build, _cabi, _front
 from .. import tuning as _tuning
 from ..codegen import u1d as _emit
 from ..codegen.u1d_common import U1DSpec, make_spec
@@ -85,6 +85,7 @@ class GraphPlan:
         self._parts: Dict[Tuple[int, bool], torch.Tensor] = {}
         self._ready: List[Tuple[int, torch.cuda.Event]] = []
         self._waited: Set[int] = set()          # streams already ordered behind every event in _ready
+        self._handle = None                     # the plan as the native host path keeps it
         self.device = dev
         if seg_ptr is not None:
             # the caller vouches for a receiver-sorted index and brings its CSR offsets (the GPU
@@ -123,6 +124,8 @@ class GraphPlan:
         ev.record(cur)
         self._ready = [(sid, e) for sid, e in self._ready if sid != cur.cuda_stream] + [(cur.cuda_stream, ev)]
         self._waited = set()
+        if self._handle is not None:
+            self._handle.reordered()
 
     def ready_on_current_stream(self) -> None:
         """Order the current stream behind the kernels that built this plan on other streams."""
@@ -143,6 +146,27 @@ class GraphPlan:
                 if t is not None:
                     t.record_stream(cur)
         self._waited.add(cur.cuda_stream)
+
+    def shares(self, desc: _cabi.U1DDesc) -> Tuple[torch.Tensor, int, bool]:
+        """``(partition, its pipelines, whether it cuts receivers)`` for a module's launches."""
+        pipelines = _sm_count(self.device) * int(desc.ctas_per_sm)
+        split = split_receivers(desc, self.n_rows, self.n_edges, self.max_degree, pipelines)
+        n = max(1, min(pipelines, max(self.n_rows, (self.n_edges + 3) // 4) if split else self.n_rows))
+        return self.partition(n, split), n, split
+
+    def record(self) -> None:
+        """Enter the plan into the lists of ``record_plans``."""
+        for rec in _RECORDERS:
+            if not any(p is self for p in rec):
+                rec.append(self)
+
+    def native(self):
+        """The plan for the native host path, which knows this object only weakly (its calls hold it)."""
+        if self._handle is None:
+            me = weakref.ref(self)
+            self._handle = _front.lib().Plan(self.seg_ptr, self.perm, self.n_rows, self.n_edges, lambda mod: me().shares(mod.desc),
+                                             lambda: me().ready_on_current_stream(), lambda: me().record())
+        return self._handle
 
     def partition(self, n_parts: int, split: bool = False) -> torch.Tensor:
         """First row of each share (``[1, n_parts + 1]``); with ``split`` shares are cut between edges and a second row holds
@@ -230,9 +254,11 @@ def record_plans():
     plans for as long as the graph is replayed (the cache alone may evict them)."""
     got: list = []
     _RECORDERS.append(got)
+    _front.lib().u1d_recording(1)
     try:
         yield got
     finally:
+        _front.lib().u1d_recording(-1)
         _RECORDERS.remove(got)
 
 
@@ -341,19 +367,10 @@ class _Call:
         if self.plan is not None:
             g.seg_ptr = self.plan.seg_ptr.data_ptr()
             g.perm = self.plan.perm.data_ptr() if self.plan.perm is not None else None
-            pipelines = _sm_count(dev) * int(mod.desc.ctas_per_sm)
-            if split_receivers(mod.desc, self.n_out_rows, self.n_edges, self.plan.max_degree, pipelines):
-                g.n_parts = max(1, min(pipelines, max(self.n_out_rows, (self.n_edges + 3) // 4)))
-                part = self.plan.partition(g.n_parts, split=True)
-                part_edge = part[1].data_ptr()
-            else:
-                g.n_parts = max(1, min(pipelines, self.n_out_rows))
-                part = self.plan.partition(g.n_parts)
-            g.part_ptr = part.data_ptr()
+            part, g.n_parts, split = self.plan.shares(mod.desc)
+            g.part_ptr, part_edge = part.data_ptr(), part[1].data_ptr() if split else None
             self.plan.ready_on_current_stream()
-            for rec in _RECORDERS:
-                if not any(p is self.plan for p in rec):
-                    rec.append(self.plan)
+            self.plan.record()
         return g, part_edge
 
 
@@ -421,8 +438,12 @@ def _tuning_for(spec: U1DSpec, direction: str, tensors, needs=(False, False, Fal
     """The launch configuration of this call: the measured winner of the signature when the tuning database has one,
     else the heuristic default.  Packed two-channel modules read and write 8-byte pairs; operands at an odd 4-byte
     offset (a contiguous view into a larger buffer) get the one-channel-per-thread module instead."""
+    return _tuning_at(spec, direction, any(t is not None and t.data_ptr() % 8 for t in tensors), needs)
+
+
+def _tuning_at(spec: U1DSpec, direction: str, odd: bool, needs) -> Optional[_emit.Tuning]:
     tun = _TUNING_OVERRIDE.get(direction) or _tuning.lookup(spec, direction, needs) or _emit.untuned(spec, direction)
-    if tun.vec == 2 and any(t is not None and t.data_ptr() % 8 for t in tensors):
+    if odd and tun.vec == 2:
         return dataclasses.replace(tun, vec=1, pipes=1, groups=max(tun.groups, 1), min_blocks=min(tun.min_blocks + 1, 3))
     return tun
 
@@ -580,6 +601,61 @@ class FastUniform1dJITFunction(torch.autograd.Function):
         return (gw if needs[0] else None), (gx if needs[1] else None), (gy if needs[2] else None), None, None, None
 
 
+_SIGNATURES: Dict[Tuple, Tuple] = {}
+_TABLES = ("i_list", "j_list", "k_list", "v_list", "coeff_list")
+_EXPORTS = tuple(f"fasteq_u1d_{n}" for n in ("forward", "forward_split", "backward", "backward_split", "tangent_forward", "tangent_backward")) + (
+    "fasteq_last_cuda_error",)
+
+
+def _signature(meta, dtype):
+    """``(native signature, columns of x)`` of the usual operand form (per-edge weights, sender gather, receiver scatter, one y value per
+    segment); ``None`` for the others."""
+    y_sh = meta.get("y_sh")
+    key = tuple((id(meta[k]), getattr(meta[k], "_version", 0)) for k in _TABLES) + (
+        meta["w_seg_num"], meta["x_seg_num"], meta["y_seg_num"], meta["out_seg_num"], meta["u_dim"], meta["size_list"][2], dtype,
+        tuple(y_sh) if y_sh else ())
+    hit = _SIGNATURES.get(key)
+    if hit is not None:
+        return hit[0]
+    made = None
+    segs = [int(meta[k]) for k in ("w_seg_num", "x_seg_num", "y_seg_num", "out_seg_num")]
+    u = int(meta["u_dim"])
+    if dtype in (torch.float32, torch.float64) and int(meta["size_list"][2]) // segs[2] == 1:
+        spec = make_spec(_np(meta["i_list"]), _np(meta["j_list"]), _np(meta["k_list"]), _np(meta["v_list"]), _np(meta["coeff_list"], True),
+                         w_segs=segs[0], x_segs=segs[1], y_segs=segs[2], out_segs=segs[3], u=u, dtype="f32" if dtype == torch.float32 else "f64",
+                         y_sh=tuple(y_sh) if y_sh else ())
+
+        def load(direction, needs, tangents, odd):
+            sp = spec if tangents is None else _dual_spec(spec, tuple(tangents))
+            mod = get_module(sp, direction, tuple(needs), tuning=_tuning_at(sp, direction, odd, tuple(needs)))
+            return mod, _front.addresses(mod.lib, _EXPORTS)
+        made = (_front.lib().Signature(u, *segs, bool(y_sh), load), segs[1] * u)
+    if len(_SIGNATURES) > 256:
+        _SIGNATURES.clear()
+    # the entry holds the table objects so their ids stay unique while it exists
+    _SIGNATURES[key] = (made, [meta[k] for k in _TABLES])
+    return made
+
+
+def _native_call(w, x, y, input_indices, output_indices, meta) -> Optional[torch.Tensor]:
+    """The call through the native host path, or ``None`` where its form is not the usual one (or something is wrong with it)."""
+    if _TUNING_OVERRIDE or not input_indices or not output_indices or len(input_indices) != 1:
+        return None
+    src, dst = input_indices.get(1), output_indices.get(0)
+    for t in (w, x, y, src, dst):
+        if not isinstance(t, torch.Tensor) or not t.is_cuda:
+            return None
+    try:
+        sig = _signature(meta, x.dtype)
+    except TypeError:                    # a table key that cannot be hashed
+        return None
+    if sig is None or x.numel() % sig[1]:
+        return None
+    plan = graph_plan(dst, x.numel() // sig[1])
+    return _front.lib().u1d(w, x, y, src, sig[0], plan.native(), plan)
+
+
 def fast_uniform1d_jit(w, x, y, input_indices, output_indices, meta, use_multiwarp_candidates: Optional[bool] = None):
     """See module docstring.  ``use_multiwarp_candidates`` is accepted and ignored, as in the reference."""
-    return FastUniform1dJITFunction.apply(w, x, y, input_indices, output_indices, meta)
+    out = _native_call(w, x, y, input_indices, output_indices, meta)
+    return FastUniform1dJITFunction.apply(w, x, y, input_indices, output_indices, meta) if out is None else out
