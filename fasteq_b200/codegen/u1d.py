@@ -162,6 +162,11 @@ constexpr bool Y_SH = {b(bool(spec.y_sh))};   // the y operand holds edge vector
 _HOST_COMMON = r"""
 __device__ int g_status_word;
 
+// Whether a launch may begin beside the kernel before it (launch.cuh).  Scattered forms only: there every operand address comes from an
+// index loaded after the kernel's wait.  And one CTA to an SM: where several fit, SMs that the kernel before leaves early take more than
+// their share of the persistent CTAs (33 channels, 663,522 edges, forward and backward 2.32 ms ordinary, 2.41 dependent).
+constexpr bool DEPENDENT = cfg::SCATTERED && 2 * SMEM_BYTES > 227 * 1024;
+
 static int* status_ptr() {
   int* p = nullptr;
   cudaGetSymbolAddress((void**)&p, g_status_word);
@@ -707,7 +712,7 @@ static int run_forward(const fasteq_u1d_graph* gh, const int32_t* part_edge, voi
   if (VEC == 2 && ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(carry)) & 7u)) return FASTEQ_INVALID;
   cudaError_t e = cudaFuncSetAttribute(fasteq_u1d_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
   if (e != cudaSuccess) return cuda_fail(e);
-  if (cfg::SCATTERED) {{             // every operand address comes from an index loaded after the kernel's wait: see launch.cuh
+  if (DEPENDENT) {{
     e = launch_dependent(fasteq_u1d_fwd_kernel, (unsigned)grid, NTHREADS, SMEM_BYTES, (cudaStream_t)stream,
         g, (const T*)w, (const T*)x, (const T*)y, (T*)out, (T*)carry{host_args});
     if (e != cudaSuccess) return cuda_fail(e);
@@ -1240,7 +1245,7 @@ static int run_backward(const fasteq_u1d_graph* gh, const int32_t* part_edge, co
     return FASTEQ_INVALID;
   e = cudaFuncSetAttribute(fasteq_u1d_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
   if (e != cudaSuccess) return cuda_fail(e);
-  if (cfg::SCATTERED) {{
+  if (DEPENDENT) {{
     e = launch_dependent(fasteq_u1d_bwd_kernel, (unsigned)grid, NTHREADS, SMEM_BYTES, s, g, (const T*)go, (const T*)w, (const T*)x, (const T*)y,
                          (T*)gw, (T*)gx, (T*)gy{host_args});
   }} else {{
