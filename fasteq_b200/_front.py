@@ -12,7 +12,7 @@ from . import _build, _cabi
 _CORE = ("eqlinear_pack", "eqlinear_forward", "eqlinear_dgrad", "eqlinear_forward_packed", "eqlinear_dgrad_packed", "eqlinear_wgrad_scratch",
          "eqlinear_wgrad_with", "gemm_tf32x3_split", "gemm_tf32x3_presplit", "radial_chain_prepare", "radial_chain_forward",
          "radial_chain_backward", "edge_geometry_forward", "edge_geometry_backward", "silu", "neighbors_work_bytes", "neighbors_count",
-         "neighbors_fill", "last_cuda_error")
+         "neighbors_fill", "graph_partition", "graph_partition_edges", "last_cuda_error")
 _lib = None
 _lock = threading.Lock()
 

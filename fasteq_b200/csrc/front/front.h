@@ -35,7 +35,7 @@ struct Core {
   F(eqlinear_pack) F(eqlinear_forward) F(eqlinear_dgrad) F(eqlinear_forward_packed) F(eqlinear_dgrad_packed)
   F(eqlinear_wgrad_scratch) F(eqlinear_wgrad_with) F(gemm_tf32x3_split) F(gemm_tf32x3_presplit)
   F(radial_chain_prepare) F(radial_chain_forward) F(radial_chain_backward) F(edge_geometry_forward) F(edge_geometry_backward)
-  F(silu) F(neighbors_work_bytes) F(neighbors_count) F(neighbors_fill) F(last_cuda_error)
+  F(silu) F(neighbors_work_bytes) F(neighbors_count) F(neighbors_fill) F(graph_partition) F(graph_partition_edges) F(last_cuda_error)
 #undef F
 };
 extern Core core;

@@ -1,5 +1,8 @@
 // The tensor-product operator in its usual form: per-edge weights, sender gather, scalar y (or edge vectors), receiver scatter.
 #include "front.h"
+#include <algorithm>
+#include <atomic>
+#include <map>
 
 namespace front {
 namespace {
@@ -51,20 +54,71 @@ struct Signature : torch::CustomClassHolder {
 };
 using Sig = c10::intrusive_ptr<Signature>;
 
-// A graph plan as the launches need it.  Shares are asked of the Python plan once per module; `ordered`: streams behind the plan's kernels.
+// Receiver-sorted view of a scatter index with the partitions its launches use.  Every kernel that builds a part of it leaves an event
+// behind; a launch on another stream waits for those first.
 struct Plan : torch::CustomClassHolder {
   struct Shares { Tensor part; int32_t n = 0; bool split = false; };
   Tensor seg_ptr, perm;
   int64_t n_rows, n_edges;
-  PyKeep share;                // module -> (partition tensor, n_parts, split)
-  PyKeep ready;                // orders the current stream behind the plan's kernels
-  PyKeep record;               // enters the plan into the lists of record_plans
+  PyKeep rule;                 // module -> (pipelines, whether their shares cut receivers)
   std::mutex lock;
+  std::map<std::pair<int64_t, bool>, Tensor> parts;
   std::unordered_map<U1DModule*, std::pair<Module, Shares>> shares;
-  std::set<cudaStream_t> ordered;
-  Plan(Tensor s, std::optional<Tensor> p, int64_t rows, int64_t edges, py::object sh, py::object rd, py::object rc)
-      : seg_ptr(std::move(s)), n_rows(rows), n_edges(edges), share(std::move(sh)), ready(std::move(rd)), record(std::move(rc)) {
+  std::vector<std::pair<cudaStream_t, std::shared_ptr<at::cuda::CUDAEvent>>> built;
+  std::set<cudaStream_t> ordered;      // streams already behind every event in `built`
+
+  Plan(Tensor s, std::optional<Tensor> p, int64_t rows, int64_t edges, py::object r)
+      : seg_ptr(std::move(s)), n_rows(rows), n_edges(edges), rule(std::move(r)) {
     if (p) perm = *p;
+  }
+  void mark_built() {
+    if (capturing()) return;
+    const auto cur = c10::cuda::getCurrentCUDAStream(seg_ptr.device().index());
+    auto e = std::make_shared<at::cuda::CUDAEvent>();
+    e->record(cur);
+    std::lock_guard<std::mutex> g(lock);
+    built.erase(std::remove_if(built.begin(), built.end(), [&](const auto& b) { return b.first == cur.stream(); }), built.end());
+    built.emplace_back(cur.stream(), std::move(e));
+    ordered.clear();
+  }
+  void order_current_stream() {
+    const auto cur = c10::cuda::getCurrentCUDAStream(seg_ptr.device().index());
+    std::vector<std::shared_ptr<at::cuda::CUDAEvent>> wait;
+    std::vector<Tensor> read;
+    {
+      std::lock_guard<std::mutex> g(lock);
+      if (built.empty() || ordered.count(cur.stream())) return;
+      if (capturing()) return;
+      for (const auto& b : built) if (b.first != cur.stream()) wait.push_back(b.second);
+      if (!wait.empty()) {
+        // a reader on a stream other than the building one: tell the allocator, so that an evicted plan's buffers are not handed out again
+        // while this stream still reads them
+        read.push_back(seg_ptr);
+        if (perm.defined()) read.push_back(perm);
+        for (const auto& p : parts) read.push_back(p.second);
+      }
+      ordered.insert(cur.stream());
+    }
+    for (const auto& e : wait) e->block(cur);
+    for (const Tensor& t : read) c10::cuda::CUDACachingAllocator::recordStream(t.storage().data_ptr(), cur);
+  }
+  // first row of each share [1, n + 1]; with `split` shares are cut between edges and a second row holds their first edges
+  Tensor partition(int64_t n, bool split) {
+    {
+      std::lock_guard<std::mutex> g(lock);
+      auto hit = parts.find({n, split});
+      if (hit != parts.end()) return hit->second;
+    }
+    c10::cuda::CUDAGuard guard(seg_ptr.device());
+    order_current_stream();
+    Tensor p = at::empty({split ? 2 : 1, n + 1}, seg_ptr.options());
+    int32_t* d = p.data_ptr<int32_t>();
+    cudaStream_t s = stream_of(p);
+    if (split) check(core.graph_partition_edges(seg_ptr.const_data_ptr<int32_t>(), n_rows, n_edges, (int32_t)n, d, d + n + 1, s), "fasteq_graph_partition_edges", core.last_cuda_error);
+    else check(core.graph_partition(seg_ptr.const_data_ptr<int32_t>(), n_rows, n_edges, (int32_t)n, d, s), "fasteq_graph_partition", core.last_cuda_error);
+    { std::lock_guard<std::mutex> g(lock); parts.emplace(std::make_pair(n, split), p); }
+    mark_built();
+    return p;
   }
   Shares shares_of(const Module& m) {
     {
@@ -75,41 +129,37 @@ struct Plan : torch::CustomClassHolder {
     Shares s;
     {
       py::gil_scoped_acquire gil;
-      py::tuple got = share.get()(m->object.get());
-      s.part = got[0].cast<Tensor>(); s.n = got[1].cast<int32_t>(); s.split = got[2].cast<bool>();
+      py::tuple got = rule.get()(m->object.get());
+      s.n = got[0].cast<int32_t>(); s.split = got[1].cast<bool>();
     }
+    s.part = partition(s.n, s.split);
     std::lock_guard<std::mutex> g(lock);
     shares.emplace(m.get(), std::make_pair(m, s));
     return s;
   }
-  void order(cudaStream_t s, bool recording) {
-    bool first;
-    { std::lock_guard<std::mutex> g(lock); first = !ordered.count(s); }
-    if (!first && !recording) return;
-    py::gil_scoped_acquire gil;
-    if (first) {
-      ready.get()();
-      if (!capturing()) { std::lock_guard<std::mutex> g(lock); ordered.insert(s); }
-    }
-    if (recording) record.get()();
-  }
 };
 using PlanPtr = c10::intrusive_ptr<Plan>;
 std::atomic<int> recording{0};
+PyObject* record_plan = nullptr;     // enters a Python plan into the lists of record_plans
 
 struct Call : torch::CustomClassHolder {
   Sig sig;
   PlanPtr plan;
   Tensor src;
   int64_t x_rows;
-  PyKeep graph;                // the Python plan, which the native one knows only weakly
+  PyKeep graph;                // the Python plan
 };
 using CallPtr = c10::intrusive_ptr<Call>;
 
 // the launch's graph record; returns the address of the shares' first edges when they cut receivers
-const int32_t* graph_of(const Call& c, const Module& m, const Tensor& any, fasteq_u1d_graph* g, Plan::Shares* s) {
+const int32_t* graph_of(const Call& c, const Module& m, fasteq_u1d_graph* g, Plan::Shares* s) {
   *s = c.plan->shares_of(m);
-  c.plan->order(stream_of(any), recording.load() > 0);
+  c.plan->order_current_stream();
+  if (recording.load() > 0) {
+    py::gil_scoped_acquire gil;
+    const py::handle record = record_plan;
+    record(c.graph.get());
+  }
   *g = {};
   g->n_edges = c.plan->n_edges; g->n_out_rows = c.plan->n_rows; g->x_rows = c.x_rows; g->y_rows = c.plan->n_edges;
   g->x_index = c.src.const_data_ptr<int32_t>();
@@ -132,7 +182,7 @@ Tensor forward_launch(const Call& c, const Tensor& w, const Tensor& x, const Ten
   const Module m = c.sig->module(false, {false, false, false}, has, odd({w, x, y, out}) || (t && odd({t[0], t[1], t[2]})));
   fasteq_u1d_graph g;
   Plan::Shares s;
-  const int32_t* edge = graph_of(c, m, x, &g, &s);
+  const int32_t* edge = graph_of(c, m, &g, &s);
   Tensor carry;
   if (edge) carry = at::empty({s.n, cols}, x.options());
   cudaStream_t st = stream_of(x);
@@ -148,7 +198,7 @@ variable_list backward_launch(const Call& c, const Tensor& go, const Tensor& w, 
   const Module m = c.sig->module(true, needs, has, odd({go, w, x, y, d[0], d[1], d[2]}) || (t && odd({t[0], t[1], t[2]})));
   fasteq_u1d_graph g;
   Plan::Shares s;
-  const int32_t* edge = graph_of(c, m, x, &g, &s);
+  const int32_t* edge = graph_of(c, m, &g, &s);
   cudaStream_t st = stream_of(x);
   if (t) check(m->tangent_backward(&g, edge, ptr(go), ptr(w), ptr(x), ptr(y), ptr(t[0]), ptr(t[1]), ptr(t[2]), mptr(d[0]), mptr(d[1]), mptr(d[2]), st),
                "fasteq_u1d_tangent_backward", m->error);
@@ -228,10 +278,17 @@ void bind_u1d(py::module_& m) {
     return c10::make_intrusive<Signature>(u, w, x, y, o, sh, std::move(load));
   }));
   py::class_<Plan, PlanPtr>(m, "Plan")
-      .def(py::init([](Tensor seg, std::optional<Tensor> perm, int64_t rows, int64_t edges, py::object share, py::object ready, py::object record) {
-        return c10::make_intrusive<Plan>(std::move(seg), std::move(perm), rows, edges, std::move(share), std::move(ready), std::move(record));
+      .def(py::init([](Tensor seg, std::optional<Tensor> perm, int64_t rows, int64_t edges, py::object rule) {
+        return c10::make_intrusive<Plan>(std::move(seg), std::move(perm), rows, edges, std::move(rule));
       }))
-      .def("reordered", [](Plan& p) { std::lock_guard<std::mutex> g(p.lock); p.ordered.clear(); });
+      .def("mark_built", &Plan::mark_built)
+      .def("order_current_stream", &Plan::order_current_stream)
+      .def("partition", &Plan::partition)
+      .def("parts", [](Plan& p) {
+        std::lock_guard<std::mutex> g(p.lock);
+        return p.parts;
+      });
+  m.def("u1d_on_record", [](py::object f) { Py_XDECREF(record_plan); record_plan = f.release().ptr(); });
   m.def("u1d_recording", [](int by) { recording += by; });
   // None: an operand this form does not take (the general path says what is wrong with it, or takes it)
   m.def("u1d", [](const Tensor& w, const Tensor& x, const Tensor& y, const Tensor& src, const Sig& sig, const PlanPtr& plan, py::object graph) -> std::optional<Tensor> {

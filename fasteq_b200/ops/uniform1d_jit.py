@@ -17,10 +17,9 @@ from __future__ import annotations
 
 import dataclasses
 import threading
-import weakref
 from collections import OrderedDict
 from contextlib import contextmanager
-from typing import Dict, List, Optional, Set, Tuple
+from typing import Dict, List, Optional, Tuple
 
 import numpy as np
 import torch
@@ -82,10 +81,6 @@ class GraphPlan:
         self.n_rows = int(n_rows)
         self.n_edges = int(dst.numel())
         dev = dst.device
-        self._parts: Dict[Tuple[int, bool], torch.Tensor] = {}
-        self._ready: List[Tuple[int, torch.cuda.Event]] = []
-        self._waited: Set[int] = set()          # streams already ordered behind every event in _ready
-        self._handle = None                     # the plan as the native host path keeps it
         self.device = dev
         if seg_ptr is not None:
             # the caller vouches for a receiver-sorted index and brings its CSR offsets (the GPU
@@ -95,6 +90,7 @@ class GraphPlan:
             self.sorted, self.perm, self.seg_ptr = True, None, seg_ptr.contiguous()
             # where the caller does not know it: no receiver set has a smaller one, and to read it back would be the sync saved
             self.max_degree = int(max_degree) if max_degree is not None else -(-self.n_edges // max(self.n_rows, 1))
+            self.native = self._native()
             return
         stream = _cabi.stream(dev)
         dst32 = dst.to(torch.int32).contiguous()
@@ -114,44 +110,25 @@ class GraphPlan:
             self.seg_ptr = torch.empty(self.n_rows + 1, dtype=torch.int32, device=dev)
             _cabi.check(core.fasteq_graph_build_csr(sorted_dst.data_ptr(), self.n_edges, self.n_rows,
                                                     self.seg_ptr.data_ptr(), stream), core, "fasteq_graph_build_csr")
-        self._mark_built()
+        self.native = self._native()
+        self.native.mark_built()
 
-    def _mark_built(self) -> None:
-        cur = torch.cuda.current_stream(self.device)
-        if torch.cuda.is_current_stream_capturing():
-            return
-        ev = torch.cuda.Event()
-        ev.record(cur)
-        self._ready = [(sid, e) for sid, e in self._ready if sid != cur.cuda_stream] + [(cur.cuda_stream, ev)]
-        self._waited = set()
-        if self._handle is not None:
-            self._handle.reordered()
+    def _native(self):
+        """The offsets, partitions and events (``csrc/front/u1d.cpp``), which operator calls use without this object."""
+        n_rows, n_edges, max_degree, device = self.n_rows, self.n_edges, self.max_degree, self.device
+        return _front.lib().Plan(self.seg_ptr, self.perm, n_rows, n_edges, lambda mod: _shares(mod.desc, n_rows, n_edges, max_degree, device))
+
+    @property
+    def _parts(self) -> Dict[Tuple[int, bool], torch.Tensor]:
+        return self.native.parts()
 
     def ready_on_current_stream(self) -> None:
         """Order the current stream behind the kernels that built this plan on other streams."""
-        if not self._ready or torch.cuda.is_current_stream_capturing():
-            return
-        if _cabi.stream(self.device) in self._waited:
-            return
-        cur = torch.cuda.current_stream(self.device)
-        foreign = False
-        for sid, ev in self._ready:
-            if sid != cur.cuda_stream:
-                cur.wait_event(ev)
-                foreign = True
-        if foreign:
-            # a reader on a stream other than the building one: tell the allocator, so that an evicted
-            # plan's buffers are not handed out again while this stream still reads them
-            for t in (self.seg_ptr, self.perm, *self._parts.values()):
-                if t is not None:
-                    t.record_stream(cur)
-        self._waited.add(cur.cuda_stream)
+        self.native.order_current_stream()
 
     def shares(self, desc: _cabi.U1DDesc) -> Tuple[torch.Tensor, int, bool]:
         """``(partition, its pipelines, whether it cuts receivers)`` for a module's launches."""
-        pipelines = _sm_count(self.device) * int(desc.ctas_per_sm)
-        split = split_receivers(desc, self.n_rows, self.n_edges, self.max_degree, pipelines)
-        n = max(1, min(pipelines, max(self.n_rows, (self.n_edges + 3) // 4) if split else self.n_rows))
+        n, split = _shares(desc, self.n_rows, self.n_edges, self.max_degree, self.device)
         return self.partition(n, split), n, split
 
     def record(self) -> None:
@@ -160,32 +137,17 @@ class GraphPlan:
             if not any(p is self for p in rec):
                 rec.append(self)
 
-    def native(self):
-        """The plan for the native host path, which knows this object only weakly (its calls hold it)."""
-        if self._handle is None:
-            me = weakref.ref(self)
-            self._handle = _front.lib().Plan(self.seg_ptr, self.perm, self.n_rows, self.n_edges, lambda mod: me().shares(mod.desc),
-                                             lambda: me().ready_on_current_stream(), lambda: me().record())
-        return self._handle
-
     def partition(self, n_parts: int, split: bool = False) -> torch.Tensor:
         """First row of each share (``[1, n_parts + 1]``); with ``split`` shares are cut between edges and a second row holds
         their first edges."""
-        p = self._parts.get((n_parts, split))
-        if p is None:
-            core = _cabi.core()
-            p = torch.empty((2 if split else 1, n_parts + 1), dtype=torch.int32, device=self.device)
-            with _cabi.on_device(self.device):
-                stream = _cabi.stream(self.device)
-                if split:
-                    _cabi.check(core.fasteq_graph_partition_edges(self.seg_ptr.data_ptr(), self.n_rows, self.n_edges, n_parts, p[0].data_ptr(),
-                                                                  p[1].data_ptr(), stream), core, "fasteq_graph_partition_edges")
-                else:
-                    _cabi.check(core.fasteq_graph_partition(self.seg_ptr.data_ptr(), self.n_rows, self.n_edges, n_parts,
-                                                            p.data_ptr(), stream), core, "fasteq_graph_partition")
-            self._parts[(n_parts, split)] = p
-            self._mark_built()
-        return p
+        return self.native.partition(n_parts, split)
+
+
+def _shares(desc: _cabi.U1DDesc, n_rows: int, n_edges: int, max_degree: int, device) -> Tuple[int, bool]:
+    """``(pipelines with a share, whether shares cut receivers)`` for a module's launches over a graph."""
+    pipelines = _sm_count(device) * int(desc.ctas_per_sm)
+    split = split_receivers(desc, n_rows, n_edges, max_degree, pipelines)
+    return max(1, min(pipelines, max(n_rows, (n_edges + 3) // 4) if split else n_rows)), split
 
 
 _PLANS: "OrderedDict[Tuple, GraphPlan]" = OrderedDict()   # least recently used first
@@ -254,6 +216,7 @@ def record_plans():
     plans for as long as the graph is replayed (the cache alone may evict them)."""
     got: list = []
     _RECORDERS.append(got)
+    _front.lib().u1d_on_record(GraphPlan.record)
     _front.lib().u1d_recording(1)
     try:
         yield got
@@ -652,7 +615,7 @@ def _native_call(w, x, y, input_indices, output_indices, meta) -> Optional[torch
     if sig is None or x.numel() % sig[1]:
         return None
     plan = graph_plan(dst, x.numel() // sig[1])
-    return _front.lib().u1d(w, x, y, src, sig[0], plan.native(), plan)
+    return _front.lib().u1d(w, x, y, src, sig[0], plan.native, plan)
 
 
 def fast_uniform1d_jit(w, x, y, input_indices, output_indices, meta, use_multiwarp_candidates: Optional[bool] = None):
