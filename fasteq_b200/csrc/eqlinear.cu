@@ -776,25 +776,25 @@ __global__ void __launch_bounds__(wg::THREADS, 1) eqlinear_wgrad_tc_kernel(const
       }
     }
   } else if (warp == 16) {
-    // an MMA holds up the thread that issues it until the ones before it are nearly done, hence a warp of its own
-    if (lane == 0) {
-      const uint32_t idesc = idesc_bf16_m128(TN);
-      for (int i = 0; i < n_chunks; ++i) {
-        const int s = i % STAGES, buf = i & 1;
-        mbar_wait(&acc_empty[buf], ((uint32_t)(i >> 1) & 1u) ^ 1u, status);
-        mbar_wait(&full[s], (uint32_t)(i / STAGES) & 1u, status);
-        tc_fence_after();
-        const uint32_t d = tmem + (uint32_t)(buf * TN), a = tmem_a + (uint32_t)(s * A_COLS), b = smem_u32(smem) + (uint32_t)(s * 3 * B_PART);
-        // smallest products first, so that the large sum is truncated in its own two steps only
-        constexpr int PA[6] = {2, 0, 1, 1, 0, 0}, PB[6] = {0, 2, 1, 0, 1, 0};
+    const uint32_t idesc = idesc_bf16_m128(TN), tm = uniform(tmem);
+    const uint64_t desc0 = desc_sw64(uniform(smem_u32(smem)));
+    for (int i = 0; i < n_chunks; ++i) {
+      const int s = i % STAGES, buf = i & 1;
+      mbar_wait(&acc_empty[buf], ((uint32_t)(i >> 1) & 1u) ^ 1u, status);
+      mbar_wait(&full[s], (uint32_t)(i / STAGES) & 1u, status);
+      __syncwarp();
+      tc_fence_after();
+      const uint32_t d = tm + (uint32_t)(buf * TN), a = tm + (uint32_t)(2 * TN + s * A_COLS);
+      const uint64_t b = desc_at(desc0, (uint32_t)(s * 3 * B_PART));
+      // smallest products first, so that the large sum is truncated in its own two steps only
+      constexpr int PA[6] = {2, 0, 1, 1, 0, 0}, PB[6] = {0, 2, 1, 0, 1, 0};
 #pragma unroll
-        for (int e = 0; e < 6; ++e)
+      for (int e = 0; e < 6; ++e)
 #pragma unroll
-          for (int ks = 0; ks < 2; ++ks)
-            mma_bf16_a_tmem(d, a + (uint32_t)(PA[e] * (ROWS / 2) + ks * 8), desc_sw64(b + (uint32_t)(PB[e] * B_PART + ks * 32)), idesc, (e | ks) ? 1u : 0u);
-        mma_commit(&empty[s]);
-        mma_commit(&acc_full[buf]);
-      }
+        for (int ks = 0; ks < 2; ++ks)
+          warp_mma_bf16_a_tmem(d, a + (uint32_t)(PA[e] * (ROWS / 2) + ks * 8), desc_at(b, (uint32_t)(PB[e] * B_PART + ks * 32)), idesc, (e | ks) ? 1u : 0u);
+      warp_mma_commit(&empty[s]);
+      warp_mma_commit(&acc_full[buf]);
     }
   } else {
     const int quarter = warp & 3, half = (warp - 8) >> 2, t = threadIdx.x - 256;

@@ -165,44 +165,44 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
       }
     }
   } else if (warp == 1) {
-    // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      // instruction descriptors: D = F32, A = B = TF32, both K-major, M = 128; N = 2 BN for the product of
-      // A_hi with the stacked [B_hi; B_lo] tile, N = BN for A_lo x B_hi
-      const uint32_t idesc2 = idesc_tf32_m128(2 * BN), idesc1 = idesc_tf32_m128(BN);
-      int it = 0;
-      uint32_t lt = 0;
-      for (long long tile = blockIdx.x; tile < n_tiles_total; tile += gridDim.x, ++lt) {
-        const Tile tl = decode_tile(tab, item_g, tile, m_tiles, n_tiles, kb_per_seg, BN);
-        const uint32_t buf = lt & 1u;
-        mbar_wait(&acc_empty[buf], ((lt >> 1) & 1u) ^ 1u, status);
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        // columns [0, BN): hi x hi;  [BN, 2 BN): hi x lo + lo x hi (small terms, kept apart so that their
-        // sum is not absorbed one rounding at a time into the large accumulator)
-        const uint32_t tmem_d = tmem_base + buf * (uint32_t)(2 * BN);
-        for (int kb = 0; kb < tl.n_kb; ++kb, ++it) {
-          const int s = it % STAGES;
-          mbar_wait(&full_split[s], (it / STAGES) & 1u, status);
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          const uint32_t a_hi = smem_u32(stage_base + (size_t)s * C_::STAGE_BYTES);
-          const uint32_t a_lo = a_hi + C_::A_BYTES;
-          const uint32_t b_hi = a_hi + 2 * C_::A_BYTES;    // B_hi tile, B_lo tile right behind it
+    // ------------------------------------------------------------------ MMA issuer (whole warp, one elected lane)
+    // instruction descriptors: D = F32, A = B = TF32, both K-major, M = 128; N = 2 BN for the product of
+    // A_hi with the stacked [B_hi; B_lo] tile, N = BN for A_lo x B_hi
+    const uint32_t idesc2 = idesc_tf32_m128(2 * BN), idesc1 = idesc_tf32_m128(BN);
+    const uint32_t tm = uniform(tmem_base), ring = uniform(smem_u32(stage_base));
+    const uint64_t desc0 = make_desc(ring);
+    int it = 0;
+    uint32_t lt = 0;
+    for (long long tile = blockIdx.x; tile < n_tiles_total; tile += gridDim.x, ++lt) {
+      const int n_kb = (int)uniform((uint32_t)decode_tile(tab, item_g, tile, m_tiles, n_tiles, kb_per_seg, BN).n_kb);
+      const uint32_t buf = lt & 1u;
+      mbar_wait(&acc_empty[buf], ((lt >> 1) & 1u) ^ 1u, status);
+      tc_fence_after();
+      // columns [0, BN): hi x hi;  [BN, 2 BN): hi x lo + lo x hi (small terms, kept apart so that their
+      // sum is not absorbed one rounding at a time into the large accumulator)
+      const uint32_t tmem_d = tm + buf * (uint32_t)(2 * BN);
+      for (int kb = 0; kb < n_kb; ++kb, ++it) {
+        const int s = it % STAGES;
+        mbar_wait(&full_split[s], (it / STAGES) & 1u, status);
+        __syncwarp();
+        tc_fence_after();
+        const uint64_t a_hi = desc_at(desc0, (uint32_t)(s * C_::STAGE_BYTES));
+        const uint64_t a_lo = desc_at(a_hi, C_::A_BYTES), b_hi = desc_at(a_hi, 2 * C_::A_BYTES);    // B_hi tile, B_lo tile right behind it
+        const uint32_t ta = tm + (uint32_t)(4 * BN) + (uint32_t)(s * 2 * BK);
 #pragma unroll
-          for (int kk = 0; kk < BK / 8; ++kk) {
-            const uint32_t off = kk * 32;   // 8 TF32 values = 32 bytes along K inside the 128-byte swizzle row
-            if (A_TMEM) {
-              const uint32_t ta = tmem_a + (uint32_t)(s * 2 * BK + kk * 8);
-              mma_tf32_a_tmem(tmem_d, ta, make_desc(b_hi + off), idesc2, (kb | kk) ? 1u : 0u);
-              mma_tf32_a_tmem(tmem_d + (uint32_t)BN, ta + (uint32_t)BK, make_desc(b_hi + off), idesc1, 1u);
-            } else {
-              mma_tf32(tmem_d, make_desc(a_hi + off), make_desc(b_hi + off), idesc2, (kb | kk) ? 1u : 0u);
-              mma_tf32(tmem_d + (uint32_t)BN, make_desc(a_lo + off), make_desc(b_hi + off), idesc1, 1u);
-            }
+        for (int kk = 0; kk < BK / 8; ++kk) {
+          const uint32_t off = kk * 32;   // 8 TF32 values = 32 bytes along K inside the 128-byte swizzle row
+          if (A_TMEM) {
+            warp_mma_tf32_a_tmem(tmem_d, ta + kk * 8, desc_at(b_hi, off), idesc2, (kb | kk) ? 1u : 0u);
+            warp_mma_tf32_a_tmem(tmem_d + (uint32_t)BN, ta + (uint32_t)(BK + kk * 8), desc_at(b_hi, off), idesc1, 1u);
+          } else {
+            warp_mma_tf32(tmem_d, desc_at(a_hi, off), desc_at(b_hi, off), idesc2, (kb | kk) ? 1u : 0u);
+            warp_mma_tf32(tmem_d + (uint32_t)BN, desc_at(a_lo, off), desc_at(b_hi, off), idesc1, 1u);
           }
-          mma_commit(&empty[s]);            // the stage may be refilled once these MMAs have read it
         }
-        mma_commit(&acc_full[buf]);
+        warp_mma_commit(&empty[s]);            // the stage may be refilled once these MMAs have read it
       }
+      warp_mma_commit(&acc_full[buf]);
     }
   } else if (warp < 6) {
     // ------------------------------------------------------------------ split raw tiles into hi / lo
@@ -307,6 +307,185 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
 }
 
 // ------------------------------------------------------------------------------------------------
+// Long, narrow plain product (N <= 64: the gradient of the wide radial layer's input, [E, weight_numel] to 64): two 128-row tiles of A to a
+// CTA.  With one tile the four stages of the grouped kernel cover 64 KB of A while a load takes 1.7 us to arrive, and as many bytes of
+// weights (hi and lo, 16 KB per k-block) as of A come through L2.  Two tiles share a weight k-block and have 128 KB of A in flight.
+// Tensor memory: tile t accumulates in columns 128 t (hi x hi) and 128 t + 64 (cross terms), single-buffered; the split A in two slots of
+// [tile][hi 32 | lo 32] from column 256.
+//   warp 0: TMA producer   warp 1: MMA issue   warps 2-5, 6-9: split of tile 0, 1   warps 10-13: accumulator read-back and TMA stores
+// Items are pairs of tiles as long as there are whole rounds of them for all SMs, then single tiles.  The sums are those of the grouped
+// kernel.  Measured at 64 columns, grouped kernel -> this one: [320,000, 1280] 408 -> 320 us (5.1 TB/s), [320,000, 1920] 566 -> 477,
+// [534,914, 512] 267 -> 223, [40,000, 256] 32.7 -> 15.2.
+constexpr int LK_BN = 64, LK_STAGES = 4, LK_SLOTS = 2, NT_LK = 448;
+struct LkCfg {
+  static constexpr int A_BYTES = BM * BK * 4, B_BYTES = LK_BN * BK * 4;
+  static constexpr int STAGE_BYTES = 2 * A_BYTES + 2 * B_BYTES;      // A tiles 0 and 1, B hi and lo
+  static constexpr int STORE_BYTES = 4 * 2 * 4096;
+  static constexpr int SMEM_BYTES = LK_STAGES * STAGE_BYTES + STORE_BYTES + 1024 + 1024;
+  static constexpr uint32_t TMEM_A = 256, SLOT_COLS = 128;
+};
+
+__global__ void __launch_bounds__(NT_LK, 1)
+gemm_tf32x3_longk_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmBhi,
+                         const __grid_constant__ CUtensorMap tmBlo, const __grid_constant__ CUtensorMap tmC, long long M, int N, int n_kb,
+                         int n_pairs, int n_items, int* status) {
+  using C_ = LkCfg;
+  extern __shared__ unsigned char smem_raw[];
+  unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  unsigned char* store_base = smem + LK_STAGES * C_::STAGE_BYTES;
+  uint64_t* full_raw = reinterpret_cast<uint64_t*>(store_base + C_::STORE_BYTES);   // [STAGES] TMA landed
+  uint64_t* empty = full_raw + LK_STAGES;        // [STAGES] the MMAs have read B (and the split warps A before them)
+  uint64_t* full_split = empty + LK_STAGES;      // [SLOTS] both tiles' parts are in tensor memory
+  uint64_t* slot_empty = full_split + LK_SLOTS;  // [SLOTS] the MMAs have read them
+  uint64_t* acc_full = slot_empty + LK_SLOTS;    // 1
+  uint64_t* acc_empty = acc_full + 1;            // [2 tiles]
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < LK_STAGES; ++s) { mbar_init(&full_raw[s], 1); mbar_init(&empty[s], 1); }
+    for (int s = 0; s < LK_SLOTS; ++s) { mbar_init(&full_split[s], 8); mbar_init(&slot_empty[s], 1); }
+    mbar_init(acc_full, 1);
+    for (int t = 0; t < 2; ++t) mbar_init(&acc_empty[t], 4);
+    mbar_fence_init();
+  }
+  if (warp == 1) tmem_alloc(tmem_slot, 512);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  wait_for_previous_kernel();
+  const uint32_t tmem = *tmem_slot;
+  // item -> first tile and number of tiles
+  auto first_tile = [&](int item) { return item < n_pairs ? 2 * item : n_pairs + item; };
+  auto tiles_of = [&](int item) { return item < n_pairs ? 2 : 1; };
+
+  if (warp == 0) {
+    if (lane == 0) {
+      int it = 0;
+      for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
+        const int tile = first_tile(item), nt = tiles_of(item), start = tile % n_kb;    // staggered: not all CTAs ask for the same weights at once
+        for (int kbi = 0; kbi < n_kb; ++kbi, ++it) {
+          const int kb = kbi + start < n_kb ? kbi + start : kbi + start - n_kb, s = it % LK_STAGES;
+          mbar_wait(&empty[s], ((it / LK_STAGES) & 1u) ^ 1u, status);
+          unsigned char* st = smem + (size_t)s * C_::STAGE_BYTES;
+          mbar_arrive_expect_tx(&full_raw[s], (uint32_t)(nt * C_::A_BYTES + 2 * C_::B_BYTES));
+          for (int t = 0; t < nt; ++t) tma_load_3d(st + t * C_::A_BYTES, &tmA, kb * BK, 0, (tile + t) * BM, &full_raw[s]);
+          tma_load_3d(st + 2 * C_::A_BYTES, &tmBhi, kb * BK, 0, 0, &full_raw[s]);
+          tma_load_3d(st + 2 * C_::A_BYTES + C_::B_BYTES, &tmBlo, kb * BK, 0, 0, &full_raw[s]);
+        }
+      }
+    }
+  } else if (warp == 1) {
+    const uint32_t idesc2 = idesc_tf32_m128(2 * LK_BN), idesc1 = idesc_tf32_m128(LK_BN), tm = uniform(tmem);
+    const uint64_t desc0 = make_desc(uniform(smem_u32(smem)) + 2 * C_::A_BYTES);
+    int it = 0;
+    uint32_t n = 0;                              // items done
+    for (int item = blockIdx.x; item < n_items; item += gridDim.x, ++n) {
+      const bool two = tiles_of(item) == 2;
+      mbar_wait(&acc_empty[0], (n & 1u) ^ 1u, status);      // the accumulators have been read back
+      mbar_wait(&acc_empty[1], (n & 1u) ^ 1u, status);
+      for (int kb = 0; kb < n_kb; ++kb, ++it) {
+        const int s = it % LK_STAGES, slot = it % LK_SLOTS;
+        mbar_wait(&full_split[slot], (it / LK_SLOTS) & 1u, status);
+        __syncwarp();
+        tc_fence_after();
+        const uint64_t b = desc_at(desc0, (uint32_t)(s * C_::STAGE_BYTES));
+        const uint32_t ta = tm + C_::TMEM_A + (uint32_t)(slot * C_::SLOT_COLS);
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
+          if (t == 1 && !two) break;
+#pragma unroll
+          for (int kk = 0; kk < BK / 8; ++kk) {
+            warp_mma_tf32_a_tmem(tm + t * 2 * LK_BN, ta + (uint32_t)(t * 2 * BK + kk * 8), desc_at(b, kk * 32), idesc2, (kb | kk) ? 1u : 0u);
+            warp_mma_tf32_a_tmem(tm + t * 2 * LK_BN + LK_BN, ta + (uint32_t)(t * 2 * BK + BK + kk * 8), desc_at(b, kk * 32), idesc1, 1u);
+          }
+        }
+        warp_mma_commit(&empty[s]);
+        warp_mma_commit(&slot_empty[slot]);
+      }
+      warp_mma_commit(acc_full);
+    }
+  } else if (warp < 10) {
+    // thread = row of the tile = its TMEM lane; 16-byte chunk j of row r sits at chunk position j ^ (r & 7)
+    const int t = (warp - 2) >> 2, quarter = warp & 3, row = quarter * 32 + lane;
+    int it = 0;
+    for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
+      const bool live = t < tiles_of(item);
+      for (int kb = 0; kb < n_kb; ++kb, ++it) {
+        const int s = it % LK_STAGES, slot = it % LK_SLOTS;
+        mbar_wait(&slot_empty[slot], ((it / LK_SLOTS) & 1u) ^ 1u, status);
+        if (live) {
+          mbar_wait(&full_raw[s], (it / LK_STAGES) & 1u, status);
+          tc_fence_after();
+          const unsigned char* a = smem + (size_t)s * C_::STAGE_BYTES + t * C_::A_BYTES + row * 128;
+          uint32_t hi_bits[32], lo_bits[32];
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            const float4 v = *reinterpret_cast<const float4*>(a + ((j ^ (row & 7)) << 4));
+            float4 h, l;
+            split_tf32(v.x, h.x, l.x); split_tf32(v.y, h.y, l.y); split_tf32(v.z, h.z, l.z); split_tf32(v.w, h.w, l.w);
+            hi_bits[4 * j] = __float_as_uint(h.x); hi_bits[4 * j + 1] = __float_as_uint(h.y);
+            hi_bits[4 * j + 2] = __float_as_uint(h.z); hi_bits[4 * j + 3] = __float_as_uint(h.w);
+            lo_bits[4 * j] = __float_as_uint(l.x); lo_bits[4 * j + 1] = __float_as_uint(l.y);
+            lo_bits[4 * j + 2] = __float_as_uint(l.z); lo_bits[4 * j + 3] = __float_as_uint(l.w);
+          }
+          const uint32_t ta = tmem + ((uint32_t)(quarter * 32) << 16) + C_::TMEM_A + (uint32_t)(slot * C_::SLOT_COLS + t * 2 * BK);
+          tmem_st_32(ta, hi_bits);
+          tmem_st_32(ta + (uint32_t)BK, lo_bits);
+          tc_fence_before();
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&full_split[slot]);
+      }
+    }
+  } else {
+    const int quarter = warp & 3;
+    unsigned char* slab = store_base + (size_t)quarter * 2 * 4096;
+    uint32_t n = 0;
+    int chunk_no = 0;
+    for (int item = blockIdx.x; item < n_items; item += gridDim.x, ++n) {
+      mbar_wait(acc_full, n & 1u, status);
+      tc_fence_after();
+      for (int t = 0; t < 2; ++t) {
+        if (t < tiles_of(item)) {
+          const long long row0 = (long long)(first_tile(item) + t) * BM + quarter * 32;
+#pragma unroll 1
+          for (int c = 0; c < LK_BN / 32; ++c, ++chunk_no) {
+            uint32_t r[32], q[32];
+            const uint32_t taddr = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(t * 2 * LK_BN + c * 32);
+            tmem_ld_32(taddr, r);                      // hi x hi
+            tmem_ld_32(taddr + (uint32_t)LK_BN, q);    // hi x lo + lo x hi
+#pragma unroll
+            for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) + __uint_as_float(q[j]));
+            unsigned char* sl = slab + (size_t)(chunk_no & 1) * 4096;
+            if (lane == 0) bulk_wait_read<1>();        // the slab used two chunks ago has been read by its store
+            __syncwarp();
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+              *reinterpret_cast<float4*>(sl + lane * 128 + ((j ^ (lane & 7)) << 4)) =
+                  make_float4(__uint_as_float(r[4 * j]), __uint_as_float(r[4 * j + 1]), __uint_as_float(r[4 * j + 2]), __uint_as_float(r[4 * j + 3]));
+            fence_async_smem();
+            __syncwarp();
+            if (lane == 0) {
+              if (c * 32 < N && row0 < M)
+                asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%1, %2, %3}], [%4];"
+                             ::"l"(&tmC), "r"(c * 32), "r"(0), "r"((int)row0), "r"(smem_u32(sl)) : "memory");
+              bulk_commit();
+            }
+          }
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&acc_empty[t]);     // (a tile the item does not have counts as read)
+      }
+    }
+    if (lane == 0) bulk_wait_read<0>();
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) { tc_fence_after(); tmem_dealloc(tmem, 512); }
+}
+
+// ------------------------------------------------------------------------------------------------
 // "A-stationary" variant for a shallow, wide layer (K <= 128, many N tiles: the last layer of the radial
 // MLP, 64 -> weight_numel).  One CTA owns a 128-row block of A, loads and splits it once, then walks
 // all N tiles: pre-split weight tiles (hi / lo arrays prepared once per call) stream through a ring,
@@ -380,33 +559,33 @@ gemm_tf32x3_as_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      const uint32_t idesc = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(AS_BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
-      mbar_wait(a_split, 0u, status);
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      int it = 0;
-      for (int nt = 0; nt < n_tiles; ++nt) {
-        const int buf = nt & 1;
-        mbar_wait(&acc_empty[buf], (((uint32_t)nt >> 1) & 1u) ^ 1u, status);
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t tmem_d = tmem_base + (uint32_t)(buf * AS_BN);
-        for (int kb = 0; kb < n_kb; ++kb, ++it) {
-          const int s = it % RING;
-          mbar_wait(&b_full[s], (it / RING) & 1u, status);
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          const uint32_t a_hi = smem_u32(a_base + (size_t)kb * 2 * C_::A_BYTES), a_lo = a_hi + C_::A_BYTES;
-          const uint32_t b_hi = smem_u32(b_base + (size_t)s * 2 * C_::B_BYTES), b_lo = b_hi + C_::B_BYTES;
+    const uint32_t idesc = idesc_tf32_m128(AS_BN), tm = uniform(tmem_base);
+    const uint64_t a0 = make_desc(uniform(smem_u32(a_base))), b0 = make_desc(uniform(smem_u32(b_base)));
+    mbar_wait(a_split, 0u, status);
+    tc_fence_after();
+    int it = 0;
+    for (int nt = 0; nt < n_tiles; ++nt) {
+      const int buf = nt & 1;
+      mbar_wait(&acc_empty[buf], (((uint32_t)nt >> 1) & 1u) ^ 1u, status);
+      tc_fence_after();
+      const uint32_t tmem_d = tm + (uint32_t)(buf * AS_BN);
+      for (int kb = 0; kb < n_kb; ++kb, ++it) {
+        const int s = it % RING;
+        mbar_wait(&b_full[s], (it / RING) & 1u, status);
+        __syncwarp();
+        tc_fence_after();
+        const uint64_t a_hi = desc_at(a0, (uint32_t)(kb * 2 * C_::A_BYTES)), a_lo = desc_at(a_hi, C_::A_BYTES);
+        const uint64_t b_hi = desc_at(b0, (uint32_t)(s * 2 * C_::B_BYTES)), b_lo = desc_at(b_hi, C_::B_BYTES);
 #pragma unroll
-          for (int kk = 0; kk < BK / 8; ++kk) {
-            const uint32_t off = kk * 32;
-            mma_tf32(tmem_d, make_desc(a_lo + off), make_desc(b_hi + off), idesc, (kb | kk) ? 1u : 0u);
-            mma_tf32(tmem_d, make_desc(a_hi + off), make_desc(b_lo + off), idesc, 1u);
-            mma_tf32(tmem_d, make_desc(a_hi + off), make_desc(b_hi + off), idesc, 1u);
-          }
-          mma_commit(&b_empty[s]);
+        for (int kk = 0; kk < BK / 8; ++kk) {
+          const uint32_t off = kk * 32;
+          warp_mma_tf32(tmem_d, desc_at(a_lo, off), desc_at(b_hi, off), idesc, (kb | kk) ? 1u : 0u);
+          warp_mma_tf32(tmem_d, desc_at(a_hi, off), desc_at(b_lo, off), idesc, 1u);
+          warp_mma_tf32(tmem_d, desc_at(a_hi, off), desc_at(b_hi, off), idesc, 1u);
         }
-        mma_commit(&acc_full[buf]);
+        warp_mma_commit(&b_empty[s]);
       }
+      warp_mma_commit(&acc_full[buf]);
     }
   } else {
     const int tid = threadIdx.x - 64;
@@ -594,38 +773,38 @@ gemm_tf32x3_asp_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      const uint32_t idesc = idesc_tf32_m128(AS_BN);
-      int it = 0;
-      uint32_t t = 0;
-      for (int j = 0, item = first; item < n_items; ++j, item += stride) {
-        const int abuf = j & 1, n_tiles = item_of(item).n_tiles;
-        mbar_wait(&a_split[abuf], ((uint32_t)j >> 1) & 1u, status);
+    const uint32_t idesc = idesc_tf32_m128(AS_BN), tm = uniform(tmem_base);
+    const uint64_t desc0 = make_desc(uniform(smem_u32(b_base)));
+    int it = 0;
+    uint32_t t = 0;
+    for (int j = 0, item = first; item < n_items; ++j, item += stride) {
+      const int abuf = j & 1, n_tiles = item_of(item).n_tiles;
+      mbar_wait(&a_split[abuf], ((uint32_t)j >> 1) & 1u, status);
+      tc_fence_after();
+      const uint32_t a_hi0 = tm + C_::TMEM_A0 + (uint32_t)abuf * C_::TMEM_A_STRIDE, a_lo0 = a_hi0 + C_::TMEM_A_LO;
+      for (int nt = 0; nt < n_tiles; ++nt, ++t) {
+        const uint32_t buf = t & 1u;
+        mbar_wait(&acc_empty[buf], ((t >> 1) & 1u) ^ 1u, status);
         tc_fence_after();
-        const uint32_t a_hi0 = tmem_base + C_::TMEM_A0 + (uint32_t)abuf * C_::TMEM_A_STRIDE, a_lo0 = a_hi0 + C_::TMEM_A_LO;
-        for (int nt = 0; nt < n_tiles; ++nt, ++t) {
-          const uint32_t buf = t & 1u;
-          mbar_wait(&acc_empty[buf], ((t >> 1) & 1u) ^ 1u, status);
+        const uint32_t tmem_d = tm + buf * AS_BN;
+        for (int kb = 0; kb < n_kb; ++kb, ++it) {
+          const int s = it % RING;
+          mbar_wait(&b_full[s], (it / RING) & 1u, status);
+          __syncwarp();
           tc_fence_after();
-          const uint32_t tmem_d = tmem_base + buf * AS_BN;
-          for (int kb = 0; kb < n_kb; ++kb, ++it) {
-            const int s = it % RING;
-            mbar_wait(&b_full[s], (it / RING) & 1u, status);
-            tc_fence_after();
-            const uint32_t b_hi = smem_u32(b_base + (size_t)s * 2 * C_::B_BYTES), b_lo = b_hi + C_::B_BYTES;
+          const uint64_t b_hi = desc_at(desc0, (uint32_t)(s * 2 * C_::B_BYTES)), b_lo = desc_at(b_hi, C_::B_BYTES);
 #pragma unroll
-            for (int kk = 0; kk < BK / 8; ++kk) {
-              const uint32_t off = kk * 32, col = (uint32_t)(kb * BK + kk * 8);
-              mma_tf32_a_tmem(tmem_d, a_lo0 + col, make_desc(b_hi + off), idesc, (kb | kk) ? 1u : 0u);
-              mma_tf32_a_tmem(tmem_d, a_hi0 + col, make_desc(b_lo + off), idesc, 1u);
-              mma_tf32_a_tmem(tmem_d, a_hi0 + col, make_desc(b_hi + off), idesc, 1u);
-            }
-            mma_commit(&b_empty[s]);
+          for (int kk = 0; kk < BK / 8; ++kk) {
+            const uint32_t off = kk * 32, col = (uint32_t)(kb * BK + kk * 8);
+            warp_mma_tf32_a_tmem(tmem_d, a_lo0 + col, desc_at(b_hi, off), idesc, (kb | kk) ? 1u : 0u);
+            warp_mma_tf32_a_tmem(tmem_d, a_hi0 + col, desc_at(b_lo, off), idesc, 1u);
+            warp_mma_tf32_a_tmem(tmem_d, a_hi0 + col, desc_at(b_hi, off), idesc, 1u);
           }
-          mma_commit(&acc_full[buf]);
+          warp_mma_commit(&b_empty[s]);
         }
-        mma_commit(&a_tmem_empty[abuf]);
+        warp_mma_commit(&acc_full[buf]);
       }
+      warp_mma_commit(&a_tmem_empty[abuf]);
     }
   } else if (warp < 6) {
     // thread = row of the block = its TMEM lane; 16-byte chunk q of row r sits at chunk position q ^ (r & 7)
@@ -793,6 +972,23 @@ static int launch_bn(const TcTable& tab, const CUtensorMap& ma, const CUtensorMa
   return e == cudaSuccess ? FASTEQ_OK : cuda_fail(e);
 }
 
+// From here on two row tiles share the weights' k-blocks (see gemm_tf32x3_longk_kernel), and from 2 tiles to an SM on:
+// fewer would leave SMs idle in pairs.  Measured from 256 columns up; below, an SM's tiles are mostly fill and drain either way.
+constexpr int LONG_K = 256;
+
+static int launch_long_k(const CUtensorMap& ma, const CUtensorMap& mbh, const CUtensorMap& mbl, const CUtensorMap& mc, long long M, int N, int K,
+                         int sms, cudaStream_t s) {
+  int* st = nullptr;
+  cudaError_t e = cudaGetSymbolAddress((void**)&st, g_tc_status);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_tf32x3_longk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, LkCfg::SMEM_BYTES);
+  if (e != cudaSuccess) return cuda_fail(e);
+  const long long tiles = (M + BM - 1) / BM;
+  const int n_pairs = (int)(tiles / (2 * sms) * sms), n_items = (int)(tiles - n_pairs);
+  e = launch_dependent(gemm_tf32x3_longk_kernel, (unsigned)(n_items < sms ? n_items : sms), NT_LK, LkCfg::SMEM_BYTES, s, ma, mbh, mbl, mc, M, N,
+                       (K + BK - 1) / BK, n_pairs, n_items, st);
+  return e == cudaSuccess ? FASTEQ_OK : cuda_fail(e);
+}
+
 // Bt_hi / Bt_lo: the [P, N, K] weight blocks already split into their TF32 parts (split_weights / the
 // SO3Linear packing kernel do it once per call; the blocks are tiny next to A)
 int launch(const TcTable& tab, const float* A, long long M, int a_rows, int K, const float* Bt_hi, const float* Bt_lo, int P, int N,
@@ -808,6 +1004,9 @@ int launch(const TcTable& tab, const float* A, long long M, int a_rows, int K, c
   if (rc != FASTEQ_OK) return rc;
   rc = make_map(&mc, C, (uint64_t)N, (uint64_t)c_rows, (uint64_t)M, (uint64_t)N, (uint64_t)c_rows * N, 32, 1, 32);
   if (rc != FASTEQ_OK) return rc;
+  const int sms = sm_count();
+  if (sms < 1) return FASTEQ_CUDA_ERROR;
+  if (BN == 64 && a_rows == 1 && c_rows == 1 && P == 1 && K >= LONG_K && M >= 2LL * sms * BM) return launch_long_k(ma, mbh, mbl, mc, M, N, K, sms, s);
   return BN == 64 ? launch_bn<64>(tab, ma, mbh, mbl, mc, M, N, K, s) : launch_bn<128>(tab, ma, mbh, mbl, mc, M, N, K, s);
 }
 

@@ -137,8 +137,9 @@ radial_chain_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
             tma_load_3d(w_base + l * W_LAYER_BYTES + kb * (2 * H * BK * 4) + hl * (H * BK * 4), &tmW, kb * BK, 0, l * 2 + hl, w_full);
     }
   } else if (warp == 1) {
-    if (lane == 0 && n_tc > 0) {
-      const uint32_t idesc = idesc_tf32_m128(H);
+    if (n_tc > 0) {
+      const uint32_t idesc = idesc_tf32_m128(H), tm = uniform(tmem_base);
+      const uint64_t a0 = make_desc(uniform(smem_u32(a_base))), w0 = make_desc(uniform(smem_u32(w_base)));
       mbar_wait(w_full, 0u, status);
       tc_fence_after();
       uint32_t cnt[2] = {0u, 0u};
@@ -154,21 +155,22 @@ radial_chain_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
             if (slot == 1 && !has1) continue;
             mbar_wait(&a_ready[slot], cnt[slot] & 1u, status);
             ++cnt[slot];
+            __syncwarp();
             tc_fence_after();
-            const uint32_t tmem_d = tmem_base + (uint32_t)(slot * H);
+            const uint32_t tmem_d = tm + (uint32_t)(slot * H);
 #pragma unroll
             for (int kb = 0; kb < 2; ++kb) {
-              const uint32_t a_hi = smem_u32(a_base + kb * (2 * BM * BK * 4)), a_lo = a_hi + BM * BK * 4;
-              const uint32_t b_hi = smem_u32(w_base + s * W_LAYER_BYTES + kb * (2 * H * BK * 4)), b_lo = b_hi + H * BK * 4;
+              const uint64_t a_hi = desc_at(a0, kb * (2 * BM * BK * 4)), a_lo = desc_at(a_hi, BM * BK * 4);
+              const uint64_t b_hi = desc_at(w0, (uint32_t)(s * W_LAYER_BYTES + kb * (2 * H * BK * 4))), b_lo = desc_at(b_hi, H * BK * 4);
 #pragma unroll
               for (int kk = 0; kk < BK / 8; ++kk) {
                 const uint32_t off = kk * 32;
-                mma_tf32(tmem_d, make_desc(a_lo + off), make_desc(b_hi + off), idesc, (kb | kk) ? 1u : 0u);
-                mma_tf32(tmem_d, make_desc(a_hi + off), make_desc(b_lo + off), idesc, 1u);
-                mma_tf32(tmem_d, make_desc(a_hi + off), make_desc(b_hi + off), idesc, 1u);
+                warp_mma_tf32(tmem_d, desc_at(a_lo, off), desc_at(b_hi, off), idesc, (kb | kk) ? 1u : 0u);
+                warp_mma_tf32(tmem_d, desc_at(a_hi, off), desc_at(b_lo, off), idesc, 1u);
+                warp_mma_tf32(tmem_d, desc_at(a_hi, off), desc_at(b_hi, off), idesc, 1u);
               }
             }
-            mma_commit(&z_full[slot]);
+            warp_mma_commit(&z_full[slot]);
           }
         }
       }

@@ -32,26 +32,39 @@ __device__ __forceinline__ uint32_t idesc_tf32_m128(int n) {
   return (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
 }
 
-__device__ __forceinline__ void mma_tf32(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+// MMA and commit, issued by one elected lane of a converged warp.  The loop around them then runs warp-uniform and keeps addresses and descriptors
+// in uniform registers; a loop under `if (lane == 0)` moves each operand there for every MMA, which takes longer than the MMA itself:
+// 45 against 32.6 clocks at N = 64, about 100 with descriptors built in the loop, 64.6 at N = 128 either way.
+__device__ __forceinline__ void warp_mma_tf32(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}"
+      "{\n\t.reg .pred p, one;\n\tsetp.ne.b32 p, %4, 0;\n\telect.sync _|one, 0xffffffff;\n\t"
+      "@one tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}"
       ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-
 // A operand read from tensor memory (lane = row, one 32-bit column per K element) instead of shared memory
-__device__ __forceinline__ void mma_tf32_a_tmem(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+__device__ __forceinline__ void warp_mma_tf32_a_tmem(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, p;\n\t}"
+      "{\n\t.reg .pred p, one;\n\tsetp.ne.b32 p, %4, 0;\n\telect.sync _|one, 0xffffffff;\n\t"
+      "@one tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, p;\n\t}"
       ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-
-__device__ __forceinline__ void mma_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+__device__ __forceinline__ void warp_mma_bf16_a_tmem(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p, one;\n\tsetp.ne.b32 p, %4, 0;\n\telect.sync _|one, 0xffffffff;\n\t"
+      "@one tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+      ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
 }
+__device__ __forceinline__ void warp_mma_commit(uint64_t* bar) {
+  asm volatile("{\n\t.reg .pred one;\n\telect.sync _|one, 0xffffffff;\n\t"
+               "@one tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(smem_u32(bar)) : "memory");
+}
+// a value every lane holds, in a form the compiler knows to be warp-uniform
+__device__ __forceinline__ uint32_t uniform(uint32_t v) { return __shfl_sync(0xffffffffu, v, 0); }
+// shared-memory descriptor `bytes` further on
+__device__ __forceinline__ uint64_t desc_at(uint64_t desc, uint32_t bytes) { return desc + (uint64_t)(bytes >> 4); }
 
 // whole-warp calls
 __device__ __forceinline__ void tmem_alloc(uint32_t* slot_in_smem, uint32_t columns) {

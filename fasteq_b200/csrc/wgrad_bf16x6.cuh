@@ -11,7 +11,7 @@
 //   warp 17     TMA loads of both operands' chunks, [32][channels], up to three ahead; entries and channels beyond the ends come as zeros
 //   warps 0-3   M operand, thread = channel = TMEM lane: split, packed in pairs of rows, tcgen05.st
 //   warps 4-7   N operand, thread = channel: the same into K-major bf16 tiles (64-byte swizzle), 16 bytes at a time
-//   warp 16     issues the twelve 128 x TN x 16 MMAs of a chunk from one lane
+//   warp 16     issues the twelve 128 x TN x 16 MMAs of a chunk
 //   warps 8-15  add finished chunks (two accumulators alternate) to their registers and store the tile
 // so no operand needs a transpose pass: the contraction index is the row, which is the K axis of both register packings.
 // Bound: the MMAs (92 clocks each at TN = 128, twelve per 32 rows) next to the splitting (about 20 issue slots per row and SM).  Measured
@@ -45,13 +45,6 @@ __device__ __forceinline__ uint64_t desc_sw64(uint32_t smem_addr) {
 // D = F32, A = B = BF16, both K-major, M = 128
 __device__ __forceinline__ uint32_t idesc_bf16_m128(int n) {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
-}
-__device__ __forceinline__ void mma_bf16_a_tmem(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
 }
 __device__ __forceinline__ void tmem_st_8(uint32_t taddr, const uint32_t (&r)[8]) {
   asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
