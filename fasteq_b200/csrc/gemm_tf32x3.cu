@@ -47,8 +47,11 @@ constexpr int NT_P = 320;   // persistent grouped kernel: 10 warps
 template <int BN> struct Cfg {
   static constexpr int A_BYTES = BM * BK * 4;          // 16 KB
   static constexpr int B_BYTES = BN * BK * 4;
-  static constexpr int STAGE_BYTES = 2 * A_BYTES + 2 * B_BYTES;
-  static constexpr int STAGES = (BN <= 64) ? 4 : 3;     // ring depth that fits the 227 KB of one CTA
+  // BN = 128: raw A, split in place, and A_lo; BN = 64 splits into tensor memory.  B hi and lo behind
+  static constexpr int B_OFF = BN <= 64 ? A_BYTES : 2 * A_BYTES;
+  static constexpr int STAGE_BYTES = B_OFF + 2 * B_BYTES;
+  static constexpr int STAGES = (BN <= 64) ? 6 : 3;     // ring depth that fits the 227 KB of one CTA
+  static constexpr int SLOTS = (BN <= 64) ? 4 : STAGES; // split A: 4 x 64 tensor-memory columns, or the stage's own
   static constexpr int STORE_BYTES = 4 * 2 * 4096;     // per epilogue warp: two 32 x 32 FP32 slabs for the TMA stores
   static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + STORE_BYTES + 1024 /* barriers */ + 1024 /* alignment slack */;
 };
@@ -100,16 +103,18 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   using C_ = Cfg<BN>;
-  constexpr int STAGES = C_::STAGES;
+  constexpr int STAGES = C_::STAGES, SLOTS = C_::SLOTS;
   constexpr uint32_t TMEM_COLS = A_TMEM ? 512u : (uint32_t)(4 * BN);
-  static_assert(!A_TMEM || 4 * BN + STAGES * 2 * BK <= 512, "tensor memory: accumulators + A ring");
+  static_assert(A_TMEM == (BN <= 64), "the stage layout");
+  static_assert(!A_TMEM || 4 * BN + SLOTS * 2 * BK <= 512, "tensor memory: accumulators + A ring");
   unsigned char* stage_base = smem;
   unsigned char* store_base = smem + STAGES * C_::STAGE_BYTES;     // [4 warps][2 slabs][32 rows x 128 B]
   uint64_t* bars = reinterpret_cast<uint64_t*>(store_base + C_::STORE_BYTES);
   uint64_t* full_raw = bars;                 // [STAGES] TMA landed
-  uint64_t* full_split = bars + STAGES;      // [STAGES] hi / lo tiles ready
-  uint64_t* empty = bars + 2 * STAGES;       // [STAGES] MMAs have consumed the stage
-  uint64_t* acc_full = bars + 3 * STAGES;    // [2] accumulator complete
+  uint64_t* empty = bars + STAGES;           // [STAGES] MMAs have consumed the stage
+  uint64_t* full_split = empty + STAGES;     // [SLOTS] hi / lo tiles ready
+  uint64_t* slot_empty = full_split + SLOTS; // [SLOTS] (A_TMEM) MMAs have consumed the split A
+  uint64_t* acc_full = slot_empty + SLOTS;   // [2] accumulator complete
   uint64_t* acc_empty = acc_full + 2;        // [2] accumulator read back by the four epilogue warps
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
 
@@ -126,7 +131,8 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
   const int kb_per_seg = (K + BK - 1) / BK;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < STAGES; ++s) { mbar_init(&full_raw[s], 1); mbar_init(&full_split[s], 4); mbar_init(&empty[s], 1); }
+    for (int s = 0; s < STAGES; ++s) { mbar_init(&full_raw[s], 1); mbar_init(&empty[s], 1); }
+    for (int s = 0; s < SLOTS; ++s) { mbar_init(&full_split[s], 4); mbar_init(&slot_empty[s], 1); }
     for (int b = 0; b < 2; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 4); }
     mbar_fence_init();
   }
@@ -139,7 +145,7 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   wait_for_previous_kernel();
   const uint32_t tmem_base = *tmem_slot;
-  const uint32_t tmem_a = tmem_base + (uint32_t)(4 * BN);     // A_TMEM: [STAGES][hi 32 columns | lo 32 columns]
+  const uint32_t tmem_a = tmem_base + (uint32_t)(4 * BN);     // A_TMEM: [SLOTS][hi 32 columns | lo 32 columns]
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
@@ -159,8 +165,8 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
           const int k0 = (kb % kb_per_seg) * BK;
           mbar_arrive_expect_tx(&full_raw[s], (uint32_t)(C_::A_BYTES + 2 * C_::B_BYTES));
           tma_load_3d(st, &tmA, k0, tab.path_a_row[seg] + tl.t, (int)tl.m0, &full_raw[s]);
-          tma_load_3d(st + 2 * C_::A_BYTES, &tmBhi, k0, tl.n0, tab.path_w[seg], &full_raw[s]);
-          tma_load_3d(st + 2 * C_::A_BYTES + C_::B_BYTES, &tmBlo, k0, tl.n0, tab.path_w[seg], &full_raw[s]);
+          tma_load_3d(st + C_::B_OFF, &tmBhi, k0, tl.n0, tab.path_w[seg], &full_raw[s]);
+          tma_load_3d(st + C_::B_OFF + C_::B_BYTES, &tmBlo, k0, tl.n0, tab.path_w[seg], &full_raw[s]);
         }
       }
     }
@@ -182,13 +188,13 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
       // sum is not absorbed one rounding at a time into the large accumulator)
       const uint32_t tmem_d = tm + buf * (uint32_t)(2 * BN);
       for (int kb = 0; kb < n_kb; ++kb, ++it) {
-        const int s = it % STAGES;
-        mbar_wait(&full_split[s], (it / STAGES) & 1u, status);
+        const int s = it % STAGES, slot = it % SLOTS;
+        mbar_wait(&full_split[slot], (it / SLOTS) & 1u, status);
         __syncwarp();
         tc_fence_after();
         const uint64_t a_hi = desc_at(desc0, (uint32_t)(s * C_::STAGE_BYTES));
-        const uint64_t a_lo = desc_at(a_hi, C_::A_BYTES), b_hi = desc_at(a_hi, 2 * C_::A_BYTES);    // B_hi tile, B_lo tile right behind it
-        const uint32_t ta = tm + (uint32_t)(4 * BN) + (uint32_t)(s * 2 * BK);
+        const uint64_t a_lo = desc_at(a_hi, C_::A_BYTES), b_hi = desc_at(a_hi, C_::B_OFF);    // B_hi tile, B_lo tile right behind it
+        const uint32_t ta = tm + (uint32_t)(4 * BN) + (uint32_t)(slot * 2 * BK);
 #pragma unroll
         for (int kk = 0; kk < BK / 8; ++kk) {
           const uint32_t off = kk * 32;   // 8 TF32 values = 32 bytes along K inside the 128-byte swizzle row
@@ -201,6 +207,7 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
           }
         }
         warp_mma_commit(&empty[s]);            // the stage may be refilled once these MMAs have read it
+        if (A_TMEM) warp_mma_commit(&slot_empty[slot]);
       }
       warp_mma_commit(&acc_full[buf]);
     }
@@ -211,7 +218,8 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
     for (long long tile = blockIdx.x; tile < n_tiles_total; tile += gridDim.x) {
       const Tile tl = decode_tile(tab, item_g, tile, m_tiles, n_tiles, kb_per_seg, BN);
       for (int kb = 0; kb < tl.n_kb; ++kb, ++it) {
-        const int s = it % STAGES;
+        const int s = it % STAGES, slot = it % SLOTS;
+        if (A_TMEM) mbar_wait(&slot_empty[slot], ((it / SLOTS) & 1u) ^ 1u, status);
         mbar_wait(&full_raw[s], (it / STAGES) & 1u, status);
         unsigned char* st = stage_base + (size_t)s * C_::STAGE_BYTES;
         float4* a_hi = reinterpret_cast<float4*>(st);
@@ -234,7 +242,8 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
             lo_bits[4 * j] = __float_as_uint(lo.x); lo_bits[4 * j + 1] = __float_as_uint(lo.y);
             lo_bits[4 * j + 2] = __float_as_uint(lo.z); lo_bits[4 * j + 3] = __float_as_uint(lo.w);
           }
-          const uint32_t ta = tmem_a + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(s * 2 * BK);
+          const uint32_t ta = tmem_a + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(slot * 2 * BK);
+          tc_fence_after();
           tmem_st_32(ta, hi_bits);
           tmem_st_32(ta + (uint32_t)BK, lo_bits);
           tc_fence_before();
@@ -247,7 +256,7 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
           fence_async_smem();               // generic-proxy writes -> visible to the tensor core's async proxy
         }
         __syncwarp();
-        if (lane == 0) mbar_arrive(&full_split[s]);
+        if (lane == 0) mbar_arrive(&full_split[slot]);
       }
     }
   } else {
