@@ -668,15 +668,15 @@ fasteq_u1d_fwd_kernel(const Graph g, const T* __restrict__ w, const T* __restric
     src.append(f"""
 // Receivers whose edges several pipelines shared: the pipeline that began one stored its sum, every later one left its own in
 // its carry row; they are added in pipeline order.  One CTA per pipeline, working where the first carry of a receiver sits.
-// Bound by latency (two dependent index loads, then the rows): the indices a CTA may need come in one go.
+// Bound by latency (two dependent index loads, then the rows): the indices a CTA may need come in one go, while the forward still runs.
 __global__ void __launch_bounds__(256) fasteq_u1d_carry_kernel(const int* __restrict__ seg_ptr, const int* __restrict__ part_ptr,
-    const int* __restrict__ part_edge, int n_parts, int n_out_rows, const T* __restrict__ carry, T* __restrict__ out) {{
-  let_next_kernel_begin();
+    const int* __restrict__ part_edge, int n_parts, int n_out_rows, const T* carry, T* out) {{
   const int p = blockIdx.x, before = p > 0 ? p - 1 : 0;
   const int row = part_ptr[p], row_before = part_ptr[before], row_after = part_ptr[p + 1];
   const int edge = part_edge[p], edge_before = part_edge[before];
+  const int first = seg_ptr[row < n_out_rows ? row : 0];
+  wait_for_previous_kernel();                       // the plan was there before the forward began; its sums are not
   if (row >= n_out_rows) return;
-  const int first = seg_ptr[row];
   if (edge <= first) return;                                                     // starts at a receiver's first edge
   if (p > 0 && row_before == row && edge_before > first) return;                 // an earlier pipeline holds the first carry
   T* o = out + (size_t)row * OSEG * U;
@@ -720,10 +720,10 @@ static int run_forward(const fasteq_u1d_graph* gh, const int32_t* part_edge, voi
     fasteq_u1d_fwd_kernel<<<grid, NTHREADS, SMEM_BYTES, (cudaStream_t)stream>>>(
         g, (const T*)w, (const T*)x, (const T*)y, (T*)out, (T*)carry{host_args});
   }}
-  if (part_edge)
-    fasteq_u1d_carry_kernel<<<(unsigned)gh->n_parts, 256, 0, (cudaStream_t)stream>>>(
-        gh->seg_ptr, gh->part_ptr, part_edge, gh->n_parts, (int)gh->n_out_rows, (const T*)carry, (T*)out);
   e = cudaGetLastError();
+  if (part_edge && e == cudaSuccess)
+    e = launch_dependent(fasteq_u1d_carry_kernel, (unsigned)gh->n_parts, 256u, 0, (cudaStream_t)stream, gh->seg_ptr, gh->part_ptr, part_edge,
+                         (int)gh->n_parts, (int)gh->n_out_rows, (const T*)carry, (T*)out);
   if (e != cudaSuccess) return cuda_fail(e);
   return FASTEQ_OK;
 }}

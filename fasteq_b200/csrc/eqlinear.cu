@@ -19,6 +19,7 @@
 #include "gemm_tf32x3.h"
 #include "fasteq_device.cuh"
 #include "wgrad_bf16x6.cuh"
+#include "launch.cuh"
 
 using namespace fasteq;
 
@@ -714,6 +715,7 @@ __global__ void __launch_bounds__(wg::THREADS, 1) eqlinear_wgrad_tc_kernel(const
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  wait_for_previous_kernel();
   const uint32_t tmem = *tmem_slot, tmem_a = tmem + 2 * TN;
   float* dst = partial + (size_t)split * u * v;
 
@@ -957,9 +959,9 @@ __global__ void __launch_bounds__(NT) eqlinear_wgrad_kernel(const __grid_constan
 // Y = 8; a few rows make one split per path, and seven of eight threads would have none of it (ten-path SO3Linear of 128
 // channels, one node: 10.2 us with Y = 8, 6.9 with 1; general kernel in FP64 12.3 and 8.9).
 template <typename T, int Y>
-__global__ void __launch_bounds__(256) eqlinear_wgrad_reduce_kernel(const __grid_constant__ WgradTable tab, const T* __restrict__ partial,
-                                                                    T* __restrict__ gw, int num_paths, long long uv) {
-  let_next_kernel_begin();
+__global__ void __launch_bounds__(256) eqlinear_wgrad_reduce_kernel(const __grid_constant__ WgradTable tab, const T* partial, T* gw,
+                                                                    int num_paths, long long uv) {
+  wait_for_previous_kernel();
   constexpr int X = 256 / Y;
   __shared__ T share[Y][X + 1];
   const long long i = (long long)blockIdx.x * X + threadIdx.x, total = (long long)num_paths * uv;
@@ -1062,10 +1064,9 @@ int launch_wgrad_tc(const fasteq_eqlinear_problem* p, WgradTable* tab, int sms, 
   cudaError_t e = tc::status_word(&status);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(eqlinear_wgrad_tc_kernel<TN>, cudaFuncAttributeMaxDynamicSharedMemorySize, wg::smem_bytes(TN));
   if (e != cudaSuccess) return cuda_fail(e);
-  eqlinear_wgrad_tc_kernel<TN><<<(unsigned)tab->split_first[p->num_paths] * (unsigned)tiles, wg::THREADS, wg::smem_bytes(TN), s>>>(
-      mm, mn, *tab, x, go, *partial, p->batch, p->in_rows, p->out_rows, p->u, p->v, p->num_paths, (int)chunks_per_row, (int)(rps / wg::ROWS),
-      swap ? 1 : 0, status);
-  e = cudaGetLastError();
+  e = launch_dependent(eqlinear_wgrad_tc_kernel<TN>, (unsigned)tab->split_first[p->num_paths] * (unsigned)tiles, wg::THREADS, wg::smem_bytes(TN), s,
+                       mm, mn, *tab, x, go, *partial, p->batch, p->in_rows, p->out_rows, p->u, p->v, p->num_paths, (int)chunks_per_row,
+                       (int)(rps / wg::ROWS), swap ? 1 : 0, status);
   return e == cudaSuccess ? FASTEQ_OK : cuda_fail(e);
 }
 
@@ -1120,10 +1121,9 @@ int launch_wgrad(const fasteq_eqlinear_problem* p, const void* x, const void* go
   }
   if (rc == FASTEQ_OK && partial) {
     if (tab.split_first[p->num_paths] == p->num_paths)
-      eqlinear_wgrad_reduce_kernel<T, 1><<<(unsigned)((total + 255) / 256), dim3(256, 1), 0, s>>>(tab, partial, (T*)gw, p->num_paths, uv);
+      e = launch_dependent(eqlinear_wgrad_reduce_kernel<T, 1>, (unsigned)((total + 255) / 256), dim3(256, 1), 0, s, tab, partial, (T*)gw, p->num_paths, uv);
     else
-      eqlinear_wgrad_reduce_kernel<T, 8><<<(unsigned)((total + 31) / 32), dim3(32, 8), 0, s>>>(tab, partial, (T*)gw, p->num_paths, uv);
-    e = cudaGetLastError();
+      e = launch_dependent(eqlinear_wgrad_reduce_kernel<T, 8>, (unsigned)((total + 31) / 32), dim3(32, 8), 0, s, tab, partial, (T*)gw, p->num_paths, uv);
     if (e != cudaSuccess) rc = cuda_fail(e);
   }
   if (scratch.own) cudaFreeAsync(scratch.own, s);

@@ -1003,7 +1003,13 @@ static int launch_long_k(const CUtensorMap& ma, const CUtensorMap& mbh, const CU
 int launch(const TcTable& tab, const float* A, long long M, int a_rows, int K, const float* Bt_hi, const float* Bt_lo, int P, int N,
            float* C, int c_rows, cudaStream_t s) {
   if (tab.n_items < 1 || tab.n_items > 65535) return FASTEQ_UNSUPPORTED;
-  const int BN = N <= 64 ? 64 : 128;
+  const int sms = sm_count();
+  if (sms < 1) return FASTEQ_CUDA_ERROR;
+  // 64-column tiles where they fit one wave: a tile's time is that of its k-blocks one after the other, and half a tile's are shorter
+  // (half the weights, half the MMAs): the eleven launches of a one-cell MACE step at 192 nodes, with the carries beside the forward,
+  // 362 -> 344 us for the step.
+  const long long tiles64 = ((M + BM - 1) / BM) * ((N + 63) / 64) * tab.n_items;
+  const int BN = N <= 64 || tiles64 <= sms ? 64 : 128;
   alignas(64) CUtensorMap ma, mbh, mbl, mc;
   int rc = make_map(&ma, A, (uint64_t)K, (uint64_t)a_rows, (uint64_t)M, (uint64_t)K, (uint64_t)a_rows * K, BK, 1, BM);
   if (rc != FASTEQ_OK) return rc;
@@ -1013,9 +1019,7 @@ int launch(const TcTable& tab, const float* A, long long M, int a_rows, int K, c
   if (rc != FASTEQ_OK) return rc;
   rc = make_map(&mc, C, (uint64_t)N, (uint64_t)c_rows, (uint64_t)M, (uint64_t)N, (uint64_t)c_rows * N, 32, 1, 32);
   if (rc != FASTEQ_OK) return rc;
-  const int sms = sm_count();
-  if (sms < 1) return FASTEQ_CUDA_ERROR;
-  if (BN == 64 && a_rows == 1 && c_rows == 1 && P == 1 && K >= LONG_K && M >= 2LL * sms * BM) return launch_long_k(ma, mbh, mbl, mc, M, N, K, sms, s);
+  if (N <= 64 && a_rows == 1 && c_rows == 1 && P == 1 && K >= LONG_K && M >= 2LL * sms * BM) return launch_long_k(ma, mbh, mbl, mc, M, N, K, sms, s);
   return BN == 64 ? launch_bn<64>(tab, ma, mbh, mbl, mc, M, N, K, s) : launch_bn<128>(tab, ma, mbh, mbl, mc, M, N, K, s);
 }
 
