@@ -11,17 +11,20 @@
 // 64 x 64 layers run as 3xTF32 tensor-core products (same split as gemm_tf32x3.cu) chained through
 // shared memory and TMEM.
 //
-// One persistent CTA per SM walks tiles of 128 edges, two at a time ("slots"): while the tensor core works on one
-// slot's layer the workers compute the other slot's activation, so neither the MMA round trip nor the
-// activation arithmetic sits idle; both slots share the one operand region (it is only busy during an MMA) and
-// have their own TMEM accumulator:
-//   warp 0    : loads the pre-split hidden weights once (TMA, SWIZZLE_128B), they stay resident
-//   warp 1    : issues the tcgen05.mma of a layer when the eight worker warps have written its operand
-//   warps 2-9 : workers; a thread owns half a row of the tile (TMEM lane = row, 32 of the 64 columns):
-//               it writes its part of the A operand (hi / lo, swizzled K-major) itself, reads the
-//               accumulator back with tcgen05.ld and applies SiLU / the stored derivative.  Rows of
-//               [E, 64] tensors enter and leave through per-warp 32 x 32 swizzled slabs and tiled TMA
-//               loads / stores, so that global traffic is made of full 128-byte lines.
+// One persistent CTA per SM holds two groups of eight worker warps; each walks its own tiles of 128 edges, so that one group's
+// activation arithmetic runs while the tensor core works on the other's layer, without an order between them.  The A operand
+// never touches shared memory: a worker splits its values and writes them to tensor memory (lane = row, one column per
+// K element), where the MMA reads them; through shared memory a layer cost 64 KB of writes and 96 KB of operand reads per tile.
+//   warps 0-1   : issue the tcgen05.mma of a group's layer when its eight workers have written the operand; warp 0 first
+//                 loads the pre-split hidden weights (TMA, SWIZZLE_128B), which stay resident
+//   warps 2-17  : workers; a thread owns half a row of its group's tile (TMEM lane = row, 32 of the 64 columns).  Rows of
+//                 [E, 64] tensors enter and leave through per-warp 32 x 32 swizzled slabs and tiled TMA
+//                 loads / stores, so that global traffic is made of full 128-byte lines.
+// What bounds it: neither memory (DRAM at 34 / 42 % forward / backward) nor issue (half the slots) but the chain of a tile - operand, MMA
+// (24 x 33 clocks and the round trip), activation, twice - of which two are in flight; a third does not fit tensor memory
+// (192 columns each).  Three layers of 64 behind 8 basis functions, forward / backward: 640,000 edges 211 / 245 -> 173 / 169 us (eight
+// workers alternating between two tiles, operand in shared memory, dE/db zero-filled and added to -> this), 9,984 edges 11.3 / 13.9 -> 8.9 / 8.1 us.
+// The next tile's first layer beside the last MMA was slower (180 / 200 us: spills at the 96 registers of 18 warps).
 // Every mbarrier wait is bounded; a timeout sets a status word and the kernel drains.
 #include <cstdio>
 #include <cstdint>
@@ -41,22 +44,26 @@ using namespace fasteq::tc;
 
 constexpr int H = 64;                 // hidden width
 constexpr int BM = 128, BK = 32;
-constexpr int NT = 320;
-constexpr int N_WORKERS = 8;          // worker warps
+constexpr int GROUPS = 2;             // tiles in flight per CTA
+constexpr int N_WORKERS = 8;          // worker warps of a group
+constexpr int NT = 32 * GROUPS * (1 + N_WORKERS);
+constexpr int GROUP_COLUMNS = 3 * H;  // tensor memory of a group: accumulator, operand hi, operand lo
+constexpr int TMEM_COLUMNS = 512;     // power of two above GROUPS * GROUP_COLUMNS
 constexpr int MAX_TC = 2;             // tensor-core layers (hidden layers after the first)
 constexpr int W_LAYER_BYTES = 2 * 2 * H * BK * 4;    // [kb][hi | lo] of a 64 x 64 matrix: 32 KB
-constexpr int A_BYTES = 2 * 2 * BM * BK * 4;         // [kb][hi | lo] of a 128 x 64 tile: 64 KB
 constexpr int SLAB_BYTES = 32 * 128;                 // 32 rows x 32 FP32 columns
 constexpr int MAX_NB = 16;
-constexpr int SMEM_BYTES = MAX_TC * W_LAYER_BYTES + A_BYTES + N_WORKERS * 2 * SLAB_BYTES + H * MAX_NB * 4 + 1024 /* barriers */ +
-                           1024 /* alignment */;
+constexpr int EXCHANGE_BYTES = GROUPS * 4 * 32 * MAX_NB * 4;   // backward: dE/db of the right half-rows on its way to the left ones
+constexpr int SMEM_BYTES = MAX_TC * W_LAYER_BYTES + GROUPS * N_WORKERS * 2 * SLAB_BYTES + H * MAX_NB * 4 + EXCHANGE_BYTES +
+                           1024 /* barriers */ + 1024 /* alignment */;
 
 struct Args {
   const float* basis;      // [M, nb]
   const float* w1;         // [H, nb]
-  float* grad_basis;       // backward: dE/db [M, nb], zero-filled by the caller, accumulated with red.add
+  float* grad_basis;       // backward: dE/db [M, nb]
   long long M;
   int nb, n_tc;
+  bool rows_in_vectors;    // nb fills the padded row and basis / grad_basis start on 16 bytes: float4 accesses
 };
 
 __device__ __forceinline__ void silu_and_derivative(float z, float& h, float& d) {
@@ -68,19 +75,6 @@ __device__ __forceinline__ void silu_and_derivative(float z, float& h, float& d)
 // 16-byte chunk c of row r of a 128-byte-row tile sits at chunk position c ^ (r & 7) (SWIZZLE_128B)
 __device__ __forceinline__ float4* swz(unsigned char* tile, int r, int c) {
   return reinterpret_cast<float4*>(tile + r * 128 + ((c ^ (r & 7)) << 4));
-}
-
-// this thread's 32 values (columns 32 * half ..) -> row `row` of k-block `half` of the A operand
-__device__ __forceinline__ void write_operand(unsigned char* A, int half, int row, const float (&v)[32]) {
-  unsigned char* hi_tile = A + half * (2 * BM * BK * 4);
-#pragma unroll
-  for (int c = 0; c < 8; ++c) {
-    float4 hi, lo;
-    split_tf32(v[4 * c + 0], hi.x, lo.x); split_tf32(v[4 * c + 1], hi.y, lo.y);
-    split_tf32(v[4 * c + 2], hi.z, lo.z); split_tf32(v[4 * c + 3], hi.w, lo.w);
-    *swz(hi_tile, row, c) = hi;
-    *swz(hi_tile + BM * BK * 4, row, c) = lo;
-  }
 }
 
 __device__ __forceinline__ void tma_store_block(const CUtensorMap* map, int col0, long long row0, int z, const void* slab) {
@@ -97,27 +91,28 @@ radial_chain_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   unsigned char* w_base = smem;                                   // [MAX_TC][kb][hi 8 KB | lo 8 KB]
-  unsigned char* a_base = smem + MAX_TC * W_LAYER_BYTES;          // [kb][hi 16 KB | lo 16 KB]
-  unsigned char* slab_base = a_base + A_BYTES;                    // [8 warps][2][4 KB]
-  float* w1s = reinterpret_cast<float*>(slab_base + N_WORKERS * 2 * SLAB_BYTES);   // [H][NB], zero padded
-  uint64_t* bars = reinterpret_cast<uint64_t*>(reinterpret_cast<unsigned char*>(w1s) + H * MAX_NB * 4);
-  uint64_t* w_full = bars;            // 1
-  uint64_t* a_ready = bars + 1;       // [2 slots] the eight worker warps have written the slot's operand
-  uint64_t* z_full = bars + 3;        // [2 slots] the slot's accumulator is complete
-  uint64_t* slab_full = bars + 5;     // [8 warps][2] backward: a TMA load has landed in the slab
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 5 + 2 * N_WORKERS);
+  unsigned char* slab_base = smem + MAX_TC * W_LAYER_BYTES;       // [16 warps][2][4 KB]
+  float* w1s = reinterpret_cast<float*>(slab_base + GROUPS * N_WORKERS * 2 * SLAB_BYTES);   // [H][NB], zero padded
+  float4* exchange = reinterpret_cast<float4*>(w1s + H * MAX_NB);  // [group][quarter][NB / 4][lane]
+  uint64_t* bars = reinterpret_cast<uint64_t*>(reinterpret_cast<unsigned char*>(exchange) + EXCHANGE_BYTES);
+  uint64_t* w_full = bars;                      // 1
+  uint64_t* a_ready = bars + 1;                 // [groups] the eight worker warps have written the group's operand
+  uint64_t* z_full = bars + 1 + GROUPS;         // [groups] the group's accumulator is complete
+  uint64_t* slab_full = bars + 1 + 2 * GROUPS;  // [16 warps][2] backward: a TMA load has landed in the slab
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(slab_full + 2 * GROUPS * N_WORKERS);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const long long n_tiles = (a.M + BM - 1) / BM;
+  const int n_rows = (int)a.M, n_tiles = (int)((a.M + BM - 1) / BM);   // row numbers up to n_rows + BM fit (checked by the caller)
+  const int step = GROUPS * (int)gridDim.x;     // a group's tiles: blockIdx.x + group * gridDim.x, + step, ...
   const int n_tc = a.n_tc;
 
   if (threadIdx.x == 0) {
     mbar_init(w_full, 1);
-    for (int t = 0; t < 2; ++t) { mbar_init(&a_ready[t], N_WORKERS); mbar_init(&z_full[t], 1); }
-    for (int i = 0; i < 2 * N_WORKERS; ++i) mbar_init(&slab_full[i], 1);
+    for (int g = 0; g < GROUPS; ++g) { mbar_init(&a_ready[g], N_WORKERS); mbar_init(&z_full[g], 1); }
+    for (int i = 0; i < 2 * GROUPS * N_WORKERS; ++i) mbar_init(&slab_full[i], 1);
     mbar_fence_init();
   }
-  if (warp == 1) tmem_alloc(tmem_slot, 2 * H);
+  if (warp == 1) tmem_alloc(tmem_slot, TMEM_COLUMNS);
   wait_for_previous_kernel();
   for (int i = threadIdx.x; i < H * NB; i += NT) {
     const int j = i / NB, k = i % NB;
@@ -128,100 +123,81 @@ radial_chain_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
-  if (warp == 0) {
-    if (lane == 0 && n_tc > 0) {
-      mbar_arrive_expect_tx(w_full, (uint32_t)(n_tc * W_LAYER_BYTES));
-      for (int l = 0; l < n_tc; ++l)
-        for (int kb = 0; kb < 2; ++kb)
-          for (int hl = 0; hl < 2; ++hl)
-            tma_load_3d(w_base + l * W_LAYER_BYTES + kb * (2 * H * BK * 4) + hl * (H * BK * 4), &tmW, kb * BK, 0, l * 2 + hl, w_full);
-    }
-  } else if (warp == 1) {
+  if (warp < GROUPS) {
+    // ------------------------------------------------------------------ MMA issue, one warp per group
     if (n_tc > 0) {
-      const uint32_t idesc = idesc_tf32_m128(H), tm = uniform(tmem_base);
-      const uint64_t a0 = make_desc(uniform(smem_u32(a_base))), w0 = make_desc(uniform(smem_u32(w_base)));
+      if (warp == 0 && lane == 0) {
+        mbar_arrive_expect_tx(w_full, (uint32_t)(n_tc * W_LAYER_BYTES));
+        for (int l = 0; l < n_tc; ++l)
+          for (int kb = 0; kb < 2; ++kb)
+            for (int hl = 0; hl < 2; ++hl)
+              tma_load_3d(w_base + l * W_LAYER_BYTES + kb * (2 * H * BK * 4) + hl * (H * BK * 4), &tmW, kb * BK, 0, l * 2 + hl, w_full);
+      }
+      __syncwarp();
+      const int group = (int)uniform((uint32_t)warp);
+      const uint32_t idesc = idesc_tf32_m128(H), tmem_d = uniform(tmem_base) + (uint32_t)(group * GROUP_COLUMNS);
+      const uint32_t a_hi = tmem_d + H, a_lo = tmem_d + 2 * H;
+      const uint64_t w0 = make_desc(uniform(smem_u32(w_base)));
       mbar_wait(w_full, 0u, status);
       tc_fence_after();
-      uint32_t cnt[2] = {0u, 0u};
-      // two tiles ("slots") are in flight per CTA; the workers hand over operands in the fixed order
-      // (slot 0, step s), (slot 1, step s), (slot 0, step s + 1), ... and both slots share the one operand region
-      for (long long pair = 0;; ++pair) {
-        const long long t0 = blockIdx.x + 2 * pair * gridDim.x;
-        if (t0 >= n_tiles) break;
-        const bool has1 = t0 + gridDim.x < n_tiles;
+      uint32_t cnt = 0u;
+      for (int t = (int)blockIdx.x + group * (int)gridDim.x; t < n_tiles; t += step) {
         for (int s = 0; s < n_tc; ++s) {
+          mbar_wait(&a_ready[group], cnt & 1u, status);
+          ++cnt;
+          __syncwarp();
+          tc_fence_after();
 #pragma unroll
-          for (int slot = 0; slot < 2; ++slot) {
-            if (slot == 1 && !has1) continue;
-            mbar_wait(&a_ready[slot], cnt[slot] & 1u, status);
-            ++cnt[slot];
-            __syncwarp();
-            tc_fence_after();
-            const uint32_t tmem_d = tm + (uint32_t)(slot * H);
+          for (int kb = 0; kb < 2; ++kb) {
+            const uint64_t b_hi = desc_at(w0, (uint32_t)(s * W_LAYER_BYTES + kb * (2 * H * BK * 4))), b_lo = desc_at(b_hi, H * BK * 4);
 #pragma unroll
-            for (int kb = 0; kb < 2; ++kb) {
-              const uint64_t a_hi = desc_at(a0, kb * (2 * BM * BK * 4)), a_lo = desc_at(a_hi, BM * BK * 4);
-              const uint64_t b_hi = desc_at(w0, (uint32_t)(s * W_LAYER_BYTES + kb * (2 * H * BK * 4))), b_lo = desc_at(b_hi, H * BK * 4);
-#pragma unroll
-              for (int kk = 0; kk < BK / 8; ++kk) {
-                const uint32_t off = kk * 32;
-                warp_mma_tf32(tmem_d, desc_at(a_lo, off), desc_at(b_hi, off), idesc, (kb | kk) ? 1u : 0u);
-                warp_mma_tf32(tmem_d, desc_at(a_hi, off), desc_at(b_lo, off), idesc, 1u);
-                warp_mma_tf32(tmem_d, desc_at(a_hi, off), desc_at(b_hi, off), idesc, 1u);
-              }
+            for (int kk = 0; kk < BK / 8; ++kk) {
+              const uint32_t off = kk * 32, col = (uint32_t)(kb * BK + kk * 8);
+              warp_mma_tf32_a_tmem(tmem_d, a_lo + col, desc_at(b_hi, off), idesc, (kb | kk) ? 1u : 0u);
+              warp_mma_tf32_a_tmem(tmem_d, a_hi + col, desc_at(b_lo, off), idesc, 1u);
+              warp_mma_tf32_a_tmem(tmem_d, a_hi + col, desc_at(b_hi, off), idesc, 1u);
             }
-            warp_mma_commit(&z_full[slot]);
           }
+          warp_mma_commit(&z_full[group]);
         }
       }
     }
   } else {
     // ------------------------------------------------------------------ workers
-    const int wk = warp - 2;                          // 0..7
+    const int group = (warp - GROUPS) / N_WORKERS;
+    const int wk = (warp - GROUPS) % N_WORKERS;       // 0..7 within the group
     const int half = wk >> 2;                         // which 32 of the 64 columns
     const int quarter = warp & 3;                     // the TMEM lanes this warp may read
-    const int trow = quarter * 32 + lane;             // row of the tile = TMEM lane
-    const uint32_t tmem_lane = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(half * 32);
-    unsigned char* slab[2] = {slab_base + wk * 2 * SLAB_BYTES, slab_base + wk * 2 * SLAB_BYTES + SLAB_BYTES};
-    uint64_t* full[2] = {&slab_full[2 * wk], &slab_full[2 * wk + 1]};
-    uint32_t n_full[2] = {0u, 0u}, n_z[2] = {0u, 0u}, n_store = 0;
+    const uint32_t tmem_lane = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(group * GROUP_COLUMNS + half * 32);
+    unsigned char* slab0 = slab_base + (warp - GROUPS) * 2 * SLAB_BYTES;
+    uint64_t* full = &slab_full[2 * (warp - GROUPS)];
+    uint32_t n_full[2] = {0u, 0u}, n_z = 0u, n_store = 0u;
     const int col0 = half * 32;
 
-    // ---- backward: tiled TMA loads of [32 rows x 32 columns] blocks into this warp's two slabs.  Every block is
-    // requested one phase before it is read: the blocks of a slot's start (dE/dh_L -> slab 0, top derivative ->
-    // slab 1) while the other slot starts, the lower derivative of slot t (-> slab t) after both slots have started.
-    auto request = [&](int which, const CUtensorMap* map, int z, long long row0) {
+    // ---- backward: tiled TMA loads of [32 rows x 32 columns] blocks into this warp's two slabs: dE/dh_L in slab 0, the top and then
+    // the lower derivative in slab 1.  Every block is requested as soon as its slab has been read, one phase before it is needed.
+    auto request = [&](int which, const CUtensorMap* map, int z, int row0) {
       fence_async_smem();                 // earlier generic reads of the slab precede the async write
       __syncwarp();
       if (lane == 0) {
-        mbar_arrive_expect_tx(full[which], SLAB_BYTES);
-        tma_load_3d(slab[which], map, col0, (int)row0, z, full[which]);
+        mbar_arrive_expect_tx(&full[which], SLAB_BYTES);
+        tma_load_3d(slab0 + which * SLAB_BYTES, map, col0, row0, z, &full[which]);
       }
     };
-    auto landed = [&](int which) { mbar_wait(full[which], n_full[which] & 1u, status); ++n_full[which]; };
-    auto request_start = [&](long long row0) {          // the two blocks a slot's start reads
-      request(0, &tmIO0, 0, row0);
-      if (n_tc > 0) request(1, &tmIO1, n_tc - 1, row0);
-    };
-    // ---- forward: one 32 x 32 block leaves through the slabs (alternating) as a tiled TMA store
-    auto store_block = [&](const float (&val)[32], const CUtensorMap* map, int z, long long row0) {
-      unsigned char* sl = slab[n_store & 1u];
-      if (lane == 0) bulk_wait_read<1>();     // the slab used two stores ago has been read
-      __syncwarp();
-#pragma unroll
-      for (int c = 0; c < 8; ++c) *swz(sl, lane, c) = make_float4(val[4 * c], val[4 * c + 1], val[4 * c + 2], val[4 * c + 3]);
-      fence_async_smem();
-      __syncwarp();
-      if (lane == 0) {
-        if (row0 < a.M) tma_store_block(map, col0, row0, z, sl);
-        bulk_commit();
-      }
-      ++n_store;
-    };
-    auto load_basis = [&](float (&bb)[NB], long long row0, bool exists) {
+    auto landed = [&](int which) { mbar_wait(&full[which], n_full[which] & 1u, status); ++n_full[which]; };
+    auto load_basis = [&](float (&bb)[NB], int row0, bool exists) {
       const long long r = row0 + lane;
+      const bool mine = exists && r < n_rows;
+      if (a.rows_in_vectors) {
 #pragma unroll
-      for (int k = 0; k < NB; ++k) bb[k] = (exists && r < a.M && k < a.nb) ? __ldg(a.basis + r * a.nb + k) : 0.f;
+        for (int k = 0; k < NB; k += 4) {
+          const float4 q = mine ? __ldg(reinterpret_cast<const float4*>(a.basis + r * NB + k)) : make_float4(0.f, 0.f, 0.f, 0.f);
+          bb[k] = q.x; bb[k + 1] = q.y; bb[k + 2] = q.z; bb[k + 3] = q.w;
+        }
+      } else {
+#pragma unroll
+        for (int k = 0; k < NB; ++k) bb[k] = (mine && k < a.nb) ? __ldg(a.basis + r * a.nb + k) : 0.f;
+      }
     };
     auto first_layer = [&](const float (&bb)[NB], int j, float& h, float& d) {
       float z = 0.f;
@@ -229,137 +205,156 @@ radial_chain_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
       for (int k = 0; k < NB; ++k) z = fmaf(w1s[(col0 + j) * NB + k], bb[k], z);
       silu_and_derivative(z, h, d);
     };
-    auto hand_over = [&](int slot, const float (&val)[32]) {     // operand of the slot's next layer -> MMA warp
-      write_operand(a_base, half, trow, val);
-      fence_async_smem();              // generic-proxy writes -> visible to the tensor core's async proxy
-      tc_fence_before();               // this thread's earlier accumulator reads precede the next MMA
+    // ---- forward: one 32 x 32 block leaves through the slabs (alternating) as a tiled TMA store
+    auto begin_store = [&]() {
+      if (lane == 0) bulk_wait_read<1>();     // the slab used two stores ago has been read
       __syncwarp();
-      if (lane == 0) mbar_arrive(&a_ready[slot]);
+      return slab0 + (n_store & 1u) * SLAB_BYTES;
     };
-    auto accumulator = [&](int slot, uint32_t (&r)[32]) {        // waits for the slot's MMA, then reads its 32 columns
-      mbar_wait(&z_full[slot], n_z[slot] & 1u, status);
-      ++n_z[slot];
-      tc_fence_after();
-      tmem_ld_32(tmem_lane + (uint32_t)(slot * H), r);
+    auto end_store = [&](const unsigned char* sl, const CUtensorMap* map, int z, int row0) {
+      fence_async_smem();
+      __syncwarp();
+      if (lane == 0) {
+        if (row0 < n_rows) tma_store_block(map, col0, row0, z, sl);
+        bulk_commit();
+      }
+      ++n_store;
     };
 
-    const long long stride = (long long)gridDim.x * BM;
-    long long row0_of[2];
-    float b[2][NB], v[32];
-    if (BWD && (long long)blockIdx.x < n_tiles) request_start((long long)blockIdx.x * BM + quarter * 32);
-    for (long long pair = 0;; ++pair) {
-      const long long t0 = blockIdx.x + 2 * pair * gridDim.x;
-      if (t0 >= n_tiles) break;
-      const bool has1 = t0 + gridDim.x < n_tiles;
-      const bool has_next = t0 + 2 * gridDim.x < n_tiles;
-      row0_of[0] = t0 * BM + quarter * 32;
-      row0_of[1] = row0_of[0] + stride;
-      load_basis(b[0], row0_of[0], true);
-      load_basis(b[1], row0_of[1], has1);
+    float b[NB], v[32];
+    int t = (int)blockIdx.x + group * (int)gridDim.x;
+    if (t < n_tiles) {
+      const int row0 = t * BM + quarter * 32;
+      if (!BWD) {
+        load_basis(b, row0, true);
+      } else {
+        request(0, &tmIO0, 0, row0);
+        if (n_tc > 0) request(1, &tmIO1, n_tc - 1, row0);
+      }
+    }
+    for (; t < n_tiles; t += step) {
+      const int row0 = t * BM + quarter * 32;
+      const bool has_next = t + step < n_tiles;
+      const int next_row0 = has_next ? row0 + step * BM : row0;
 
-      // start of a slot: the operand of the first tensor-core layer (or, without one, the final vector)
-      auto start = [&](int slot) {
-        if (!BWD) {
+      // the operand of the first tensor-core layer (or, without one, the final vector)
+      if (!BWD) {
 #pragma unroll
-          for (int j = 0; j < 32; ++j) { float d; first_layer(b[slot], j, v[j], d); }
-        } else {
-          landed(0);
-          if (n_tc > 0) landed(1);
+        for (int j = 0; j < 32; ++j) { float d; first_layer(b, j, v[j], d); }
+        load_basis(b, next_row0, has_next);
+      } else {
+        load_basis(b, row0, true);
+        landed(0);
+        if (n_tc > 0) landed(1);
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+          float4 gv = *swz(slab0, lane, c);
+          if (n_tc > 0) {
+            const float4 dv = *swz(slab0 + SLAB_BYTES, lane, c);
+            gv.x *= dv.x; gv.y *= dv.y; gv.z *= dv.z; gv.w *= dv.w;
+          }
+          v[4 * c] = gv.x; v[4 * c + 1] = gv.y; v[4 * c + 2] = gv.z; v[4 * c + 3] = gv.w;
+        }
+        if (n_tc > 1) request(1, &tmIO1, n_tc - 2, row0);
+        else if (n_tc > 0 && has_next) request(1, &tmIO1, n_tc - 1, next_row0);
+        if (has_next) request(0, &tmIO0, 0, next_row0);
+      }
+
+      for (int s = 0; s < n_tc; ++s) {
+        // operand of layer s -> tensor memory; the accumulator of the layer before has been read by this thread
+        {
+          uint32_t part[32];
+#pragma unroll
+          for (int j = 0; j < 32; ++j) {
+            float hi, lo;
+            split_tf32(v[j], hi, lo);
+            part[j] = __float_as_uint(hi);
+            v[j] = lo;
+          }
+          tmem_st_32_begin(tmem_lane + H, part);
+#pragma unroll
+          for (int j = 0; j < 32; ++j) part[j] = __float_as_uint(v[j]);
+          tmem_st_32(tmem_lane + 2 * H, part);
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&a_ready[group]);
+        uint32_t r[32];
+        mbar_wait(&z_full[group], n_z & 1u, status);
+        ++n_z;
+        tc_fence_after();
+        tmem_ld_32(tmem_lane, r);
+        if (!BWD) {
+          unsigned char* sl = begin_store();
 #pragma unroll
           for (int c = 0; c < 8; ++c) {
-            float4 gv = *swz(slab[0], lane, c);
-            if (n_tc > 0) {
-              const float4 dv = *swz(slab[1], lane, c);
-              gv.x *= dv.x; gv.y *= dv.y; gv.z *= dv.z; gv.w *= dv.w;
-            }
-            v[4 * c] = gv.x; v[4 * c + 1] = gv.y; v[4 * c + 2] = gv.z; v[4 * c + 3] = gv.w;
+            float4 d;
+            silu_and_derivative(__uint_as_float(r[4 * c]), v[4 * c], d.x);
+            silu_and_derivative(__uint_as_float(r[4 * c + 1]), v[4 * c + 1], d.y);
+            silu_and_derivative(__uint_as_float(r[4 * c + 2]), v[4 * c + 2], d.z);
+            silu_and_derivative(__uint_as_float(r[4 * c + 3]), v[4 * c + 3], d.w);
+            *swz(sl, lane, c) = d;
           }
-          // both slabs are free: what is read next?
-          if (slot == 0 && has1) request_start(row0_of[1]);
-          else {
-            // both slots have started (or there is only one): the lower derivatives, else the next pair's start
-            if (n_tc > 1) {
-              request(0, &tmIO1, n_tc - 2, row0_of[0]);
-              if (has1) request(1, &tmIO1, n_tc - 2, row0_of[1]);
-            } else if (has_next) {
-              request_start(row0_of[0] + 2 * stride);
-            }
-          }
-        }
-      };
-      // after tensor-core layer s of a slot: the operand of layer s + 1, or the final vector
-      auto after_layer = [&](int slot, int s, const uint32_t (&r)[32]) {
-        if (!BWD) {
-          float d[32];
-#pragma unroll
-          for (int j = 0; j < 32; ++j) silu_and_derivative(__uint_as_float(r[j]), v[j], d[j]);
-          store_block(d, &tmIO1, s, row0_of[slot]);
+          end_store(sl, &tmIO1, s, row0);
         } else {
           const bool more = s + 1 < n_tc;      // multiply by the derivative of the layer below (n_tc <= 2: s == 0)
-          if (more) landed(slot);
+          if (more) landed(1);
 #pragma unroll
           for (int c = 0; c < 8; ++c) {
             float4 dv = make_float4(1.f, 1.f, 1.f, 1.f);
-            if (more) dv = *swz(slab[slot], lane, c);
+            if (more) dv = *swz(slab0 + SLAB_BYTES, lane, c);
             v[4 * c] = __uint_as_float(r[4 * c]) * dv.x; v[4 * c + 1] = __uint_as_float(r[4 * c + 1]) * dv.y;
             v[4 * c + 2] = __uint_as_float(r[4 * c + 2]) * dv.z; v[4 * c + 3] = __uint_as_float(r[4 * c + 3]) * dv.w;
           }
-          // slab `slot` is free again: the next pair's start blocks go there (dE/dh_L into slab 0, derivative into slab 1)
-          if (more && has_next) {
-            if (slot == 0) request(0, &tmIO0, 0, row0_of[0] + 2 * stride);
-            else request(1, &tmIO1, n_tc - 1, row0_of[0] + 2 * stride);
-          }
+          if (more && has_next) request(1, &tmIO1, n_tc - 1, next_row0);
         }
-      };
-      auto finish = [&](int slot) {
-        if (!BWD) {
-          store_block(v, &tmIO0, 0, row0_of[slot]);
-        } else {
-          float gb[NB];
-#pragma unroll
-          for (int k = 0; k < NB; ++k) gb[k] = 0.f;
-#pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            float h, d;
-            first_layer(b[slot], j, h, d);
-            const float gz = v[j] * d;
-#pragma unroll
-            for (int k = 0; k < NB; ++k) gb[k] = fmaf(gz, w1s[(col0 + j) * NB + k], gb[k]);
-          }
-          const long long row = row0_of[slot] + lane;
-          if (row < a.M) {
-            // the two half-row owners of an edge add into a zero-filled row: two addends, order-independent
-#pragma unroll
-            for (int k = 0; k < NB; ++k)
-              if (k < a.nb) red_add(a.grad_basis + row * a.nb + k, gb[k]);
-          }
-        }
-      };
-
-      if (n_tc == 0) {
-        start(0); finish(0);
-        if (has1) { start(1); finish(1); }
-        continue;
       }
-      // slot 0's first operand goes to the tensor core; slot 1's is computed while that MMA runs
-      start(0);
-      hand_over(0, v);
-      if (has1) start(1);
-      for (int s = 0; s < n_tc; ++s) {
-        uint32_t r[32];
-        // here: MMA (slot 0, layer s) is in flight, v holds slot 1's operand for layer s
-        accumulator(0, r);                       // the operand region is free again
-        if (has1) hand_over(1, v);               // MMA (slot 1, layer s) starts
-        after_layer(0, s, r);                    // ... and runs while slot 0's activation is computed
-        if (s + 1 == n_tc) finish(0);
-        if (has1) {
-          accumulator(1, r);                     // the operand region is free again
-          if (s + 1 < n_tc) hand_over(0, v);     // MMA (slot 0, layer s + 1) starts
-          after_layer(1, s, r);
-          if (s + 1 == n_tc) finish(1);
-        } else if (s + 1 < n_tc) {
-          hand_over(0, v);
+
+      if (!BWD) {
+        unsigned char* sl = begin_store();
+#pragma unroll
+        for (int c = 0; c < 8; ++c) *swz(sl, lane, c) = make_float4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
+        end_store(sl, &tmIO0, 0, row0);
+      } else {
+        float gb[NB];
+#pragma unroll
+        for (int k = 0; k < NB; ++k) gb[k] = 0.f;
+#pragma unroll
+        for (int j = 0; j < 32; ++j) {
+          float h, d;
+          first_layer(b, j, h, d);
+          const float gz = v[j] * d;
+#pragma unroll
+          for (int k = 0; k < NB; ++k) gb[k] = fmaf(gz, w1s[(col0 + j) * NB + k], gb[k]);
         }
+        // the two half-rows of an edge meet: the right one's sums go through shared memory to the left one's thread
+        float4* ex = exchange + (group * 4 + quarter) * (MAX_NB / 4) * 32 + lane;
+        const int pair_barrier = 1 + group * 4 + quarter;
+        if (half == 1) {
+#pragma unroll
+          for (int k = 0; k < NB; k += 4) ex[(k / 4) * 32] = make_float4(gb[k], gb[k + 1], gb[k + 2], gb[k + 3]);
+        }
+        named_barrier_sync(pair_barrier, 64);      // written
+        const long long row = row0 + lane;
+        if (half == 0) {
+#pragma unroll
+          for (int k = 0; k < NB; k += 4) {
+            const float4 q = ex[(k / 4) * 32];
+            const float4 sum = make_float4(gb[k] + q.x, gb[k + 1] + q.y, gb[k + 2] + q.z, gb[k + 3] + q.w);
+            if (row < n_rows) {
+              float* out = a.grad_basis + row * a.nb + k;
+              if (a.rows_in_vectors) {
+                *reinterpret_cast<float4*>(out) = sum;
+              } else {
+                if (k < a.nb) out[0] = sum.x;
+                if (k + 1 < a.nb) out[1] = sum.y;
+                if (k + 2 < a.nb) out[2] = sum.z;
+                if (k + 3 < a.nb) out[3] = sum.w;
+              }
+            }
+          }
+        }
+        named_barrier_sync(pair_barrier, 64);      // read: the next tile may write
       }
     }
     if (!BWD && lane == 0) bulk_wait_read<0>();   // the slabs must outlive their stores
@@ -368,7 +363,7 @@ radial_chain_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
   __syncthreads();
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, 2 * H);
+    tmem_dealloc(tmem_base, TMEM_COLUMNS);
   }
 }
 
@@ -438,11 +433,9 @@ static int run(Args a, const float* const* w_hidden, const float* prepared_in, c
   if (!a.basis || !a.w1 || !io0 || (a.n_tc > 0 && ((!w_hidden && !prepared_in) || !io1)) || (BWD && !a.grad_basis)) return FASTEQ_INVALID;
   if ((reinterpret_cast<uintptr_t>(io0) | reinterpret_cast<uintptr_t>(io1) | reinterpret_cast<uintptr_t>(prepared_in)) & 15u)
     return FASTEQ_UNSUPPORTED;
+  a.rows_in_vectors = (a.nb == 8 || a.nb == MAX_NB) &&
+                      !((reinterpret_cast<uintptr_t>(a.basis) | reinterpret_cast<uintptr_t>(a.grad_basis)) & 15u);
   cudaError_t e;
-  if (BWD) {
-    e = cudaMemsetAsync(a.grad_basis, 0, (size_t)a.M * a.nb * sizeof(float), s);
-    if (e != cudaSuccess) return cuda_fail(e);
-  }
   float* tmp = nullptr;
   alignas(64) CUtensorMap tmw, tm0, tm1;
   const int n_alloc = a.n_tc > 0 ? a.n_tc : 1;
