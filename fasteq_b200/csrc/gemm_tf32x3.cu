@@ -17,9 +17,8 @@
 //   warp 0       : TMA producer -- 3-D tiled loads (SWIZZLE_128B) of the raw A and Bt k-blocks
 //   warp 1       : allocates TMEM, issues tcgen05.mma (kind::tf32, M = 128, N = BN, K = 8) from one lane,
 //                  releases ring stages and signals the epilogue with tcgen05.commit
-//   warps 2..5   : split each raw k-block into hi / lo tiles: in place in shared memory at BN = 128 (the
-//                  swizzle is position preserving), into tensor memory at BN = 64 (thread = row = TMEM
-//                  lane, tcgen05.st; the MMAs then take their A operand from tensor memory)
+//   warps 2..5   : split each raw A k-block into hi / lo parts in tensor memory (thread = row = TMEM
+//                  lane, tcgen05.st), from where the MMAs take their A operand
 //   warps 6..9   : read a finished accumulator with tcgen05.ld and store the tile through swizzled
 //                  staging slabs and TMA stores
 // Every mbarrier wait is bounded (about two seconds), after which a status word is set and the
@@ -47,11 +46,11 @@ constexpr int NT_P = 320;   // persistent grouped kernel: 10 warps
 template <int BN> struct Cfg {
   static constexpr int A_BYTES = BM * BK * 4;          // 16 KB
   static constexpr int B_BYTES = BN * BK * 4;
-  // BN = 128: raw A, split in place, and A_lo; BN = 64 splits into tensor memory.  B hi and lo behind
-  static constexpr int B_OFF = BN <= 64 ? A_BYTES : 2 * A_BYTES;
+  static constexpr int B_OFF = A_BYTES;                // raw A, then B hi and lo
   static constexpr int STAGE_BYTES = B_OFF + 2 * B_BYTES;
-  static constexpr int STAGES = (BN <= 64) ? 6 : 3;     // ring depth that fits the 227 KB of one CTA
-  static constexpr int SLOTS = (BN <= 64) ? 4 : STAGES; // split A: 4 x 64 tensor-memory columns, or the stage's own
+  static constexpr int STAGES = (BN <= 64) ? 6 : 4;     // ring depth that fits the 227 KB of one CTA
+  static constexpr int SLOTS = 4;                       // split A: 4 x 64 tensor-memory columns
+  static constexpr int ACCUMULATORS = 256 / (2 * BN);   // in the other 256: two tiles of 64 columns, one of 128
   static constexpr int STORE_BYTES = 4 * 2 * 4096;     // per epilogue warp: two 32 x 32 FP32 slabs for the TMA stores
   static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + STORE_BYTES + 1024 /* barriers */ + 1024 /* alignment slack */;
 };
@@ -90,11 +89,13 @@ __device__ __forceinline__ Tile decode_tile(const TcTable& tab, const unsigned c
   return r;
 }
 
-// A_TMEM (BN = 64, where tensor memory has room: accumulators 256 columns, A ring 4 x 64): the split warps write
-// the hi / lo parts of a k-block to tensor memory (thread = row = TMEM lane, tcgen05.st) and the MMAs take A from
-// there, which removes 32 KB of shared-memory writes and 32 KB of reads per k-block from the pipe that bounds the
-// long-K case.
-template <int BN, bool A_TMEM>
+// Shared memory bounds a k-block: TMA fills, the split's reads and the MMAs' operand reads share its 128 bytes per clock.  With the
+// split A in tensor memory (thread = row = TMEM lane, tcgen05.st) that is 112 KB at 128 columns, 875 clocks beside 773 of MMAs; split in
+// place in shared memory it was 176 KB.  SO3Linear after the tensor product (40 rows of 128 channels to 16): 12,288 nodes 112.7 -> 95.5 us a
+// direction (3.7 TB/s of features, 744 MB through L2 with the weights), 1,536 nodes 21.0 -> 17.9.
+// The price at 128 columns is a single accumulator (256 columns with its cross terms): the epilogue takes it to registers whole and
+// hands it back before it stores.
+template <int BN>
 __global__ void __launch_bounds__(NT_P, 1)
 gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmBhi,
                    const __grid_constant__ CUtensorMap tmBlo, const __grid_constant__ CUtensorMap tmC,
@@ -103,20 +104,19 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   using C_ = Cfg<BN>;
-  constexpr int STAGES = C_::STAGES, SLOTS = C_::SLOTS;
-  constexpr uint32_t TMEM_COLS = A_TMEM ? 512u : (uint32_t)(4 * BN);
-  static_assert(A_TMEM == (BN <= 64), "the stage layout");
-  static_assert(!A_TMEM || 4 * BN + SLOTS * 2 * BK <= 512, "tensor memory: accumulators + A ring");
+  constexpr int STAGES = C_::STAGES, SLOTS = C_::SLOTS, ACC = C_::ACCUMULATORS;
+  constexpr uint32_t TMEM_COLS = 512, TMEM_A = 256;
+  static_assert(ACC * 2 * BN == (int)TMEM_A && SLOTS * 2 * BK <= 256, "tensor memory: accumulators + A ring");
   unsigned char* stage_base = smem;
   unsigned char* store_base = smem + STAGES * C_::STAGE_BYTES;     // [4 warps][2 slabs][32 rows x 128 B]
   uint64_t* bars = reinterpret_cast<uint64_t*>(store_base + C_::STORE_BYTES);
   uint64_t* full_raw = bars;                 // [STAGES] TMA landed
   uint64_t* empty = bars + STAGES;           // [STAGES] MMAs have consumed the stage
-  uint64_t* full_split = empty + STAGES;     // [SLOTS] hi / lo tiles ready
-  uint64_t* slot_empty = full_split + SLOTS; // [SLOTS] (A_TMEM) MMAs have consumed the split A
-  uint64_t* acc_full = slot_empty + SLOTS;   // [2] accumulator complete
-  uint64_t* acc_empty = acc_full + 2;        // [2] accumulator read back by the four epilogue warps
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
+  uint64_t* full_split = empty + STAGES;     // [SLOTS] hi / lo parts ready
+  uint64_t* slot_empty = full_split + SLOTS; // [SLOTS] MMAs have consumed the split A
+  uint64_t* acc_full = slot_empty + SLOTS;   // [ACC] accumulator complete
+  uint64_t* acc_empty = acc_full + ACC;      // [ACC] accumulator read back by the four epilogue warps
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + ACC);
 
   unsigned char* item_table = reinterpret_cast<unsigned char*>(bars) + 1024 - ITEM_TABLE;   // behind the barriers
   const unsigned char* item_g = tab.n_items <= ITEM_TABLE ? item_table : nullptr;
@@ -133,7 +133,7 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) { mbar_init(&full_raw[s], 1); mbar_init(&empty[s], 1); }
     for (int s = 0; s < SLOTS; ++s) { mbar_init(&full_split[s], 4); mbar_init(&slot_empty[s], 1); }
-    for (int b = 0; b < 2; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 4); }
+    for (int b = 0; b < ACC; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 4); }
     mbar_fence_init();
   }
   if (warp == 1) {
@@ -145,7 +145,7 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   wait_for_previous_kernel();
   const uint32_t tmem_base = *tmem_slot;
-  const uint32_t tmem_a = tmem_base + (uint32_t)(4 * BN);     // A_TMEM: [SLOTS][hi 32 columns | lo 32 columns]
+  const uint32_t tmem_a = tmem_base + TMEM_A;     // [SLOTS][hi 32 columns | lo 32 columns]
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
@@ -181,8 +181,8 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
     uint32_t lt = 0;
     for (long long tile = blockIdx.x; tile < n_tiles_total; tile += gridDim.x, ++lt) {
       const int n_kb = (int)uniform((uint32_t)decode_tile(tab, item_g, tile, m_tiles, n_tiles, kb_per_seg, BN).n_kb);
-      const uint32_t buf = lt & 1u;
-      mbar_wait(&acc_empty[buf], ((lt >> 1) & 1u) ^ 1u, status);
+      const uint32_t buf = lt % ACC;
+      mbar_wait(&acc_empty[buf], ((lt / ACC) & 1u) ^ 1u, status);
       tc_fence_after();
       // columns [0, BN): hi x hi;  [BN, 2 BN): hi x lo + lo x hi (small terms, kept apart so that their
       // sum is not absorbed one rounding at a time into the large accumulator)
@@ -192,69 +192,49 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
         mbar_wait(&full_split[slot], (it / SLOTS) & 1u, status);
         __syncwarp();
         tc_fence_after();
-        const uint64_t a_hi = desc_at(desc0, (uint32_t)(s * C_::STAGE_BYTES));
-        const uint64_t a_lo = desc_at(a_hi, C_::A_BYTES), b_hi = desc_at(a_hi, C_::B_OFF);    // B_hi tile, B_lo tile right behind it
-        const uint32_t ta = tm + (uint32_t)(4 * BN) + (uint32_t)(slot * 2 * BK);
+        const uint64_t b_hi = desc_at(desc0, (uint32_t)(s * C_::STAGE_BYTES + C_::B_OFF));    // B_hi tile, B_lo tile right behind it
+        const uint32_t ta = tm + TMEM_A + (uint32_t)(slot * 2 * BK);
 #pragma unroll
         for (int kk = 0; kk < BK / 8; ++kk) {
           const uint32_t off = kk * 32;   // 8 TF32 values = 32 bytes along K inside the 128-byte swizzle row
-          if (A_TMEM) {
-            warp_mma_tf32_a_tmem(tmem_d, ta + kk * 8, desc_at(b_hi, off), idesc2, (kb | kk) ? 1u : 0u);
-            warp_mma_tf32_a_tmem(tmem_d + (uint32_t)BN, ta + (uint32_t)(BK + kk * 8), desc_at(b_hi, off), idesc1, 1u);
-          } else {
-            warp_mma_tf32(tmem_d, desc_at(a_hi, off), desc_at(b_hi, off), idesc2, (kb | kk) ? 1u : 0u);
-            warp_mma_tf32(tmem_d + (uint32_t)BN, desc_at(a_lo, off), desc_at(b_hi, off), idesc1, 1u);
-          }
+          warp_mma_tf32_a_tmem(tmem_d, ta + kk * 8, desc_at(b_hi, off), idesc2, (kb | kk) ? 1u : 0u);
+          warp_mma_tf32_a_tmem(tmem_d + (uint32_t)BN, ta + (uint32_t)(BK + kk * 8), desc_at(b_hi, off), idesc1, 1u);
         }
         warp_mma_commit(&empty[s]);            // the stage may be refilled once these MMAs have read it
-        if (A_TMEM) warp_mma_commit(&slot_empty[slot]);
+        warp_mma_commit(&slot_empty[slot]);
       }
       warp_mma_commit(&acc_full[buf]);
     }
   } else if (warp < 6) {
     // ------------------------------------------------------------------ split raw tiles into hi / lo
-    const int tid = threadIdx.x - 64;     // 0..127
+    // thread = row of the tile = its TMEM lane; 16-byte chunk j of row r sits at chunk position j ^ (r & 7)
+    const int row = (warp & 3) * 32 + lane;
     int it = 0;
     for (long long tile = blockIdx.x; tile < n_tiles_total; tile += gridDim.x) {
       const Tile tl = decode_tile(tab, item_g, tile, m_tiles, n_tiles, kb_per_seg, BN);
       for (int kb = 0; kb < tl.n_kb; ++kb, ++it) {
         const int s = it % STAGES, slot = it % SLOTS;
-        if (A_TMEM) mbar_wait(&slot_empty[slot], ((it / SLOTS) & 1u) ^ 1u, status);
+        mbar_wait(&slot_empty[slot], ((it / SLOTS) & 1u) ^ 1u, status);
         mbar_wait(&full_raw[s], (it / STAGES) & 1u, status);
-        unsigned char* st = stage_base + (size_t)s * C_::STAGE_BYTES;
-        float4* a_hi = reinterpret_cast<float4*>(st);
-        float4* a_lo = reinterpret_cast<float4*>(st + C_::A_BYTES);
-        auto split = [](float4 v, float4& hi, float4& lo) {
-          hi.x = __uint_as_float(__float_as_uint(v.x) & 0xffffe000u); lo.x = v.x - hi.x;
-          hi.y = __uint_as_float(__float_as_uint(v.y) & 0xffffe000u); lo.y = v.y - hi.y;
-          hi.z = __uint_as_float(__float_as_uint(v.z) & 0xffffe000u); lo.z = v.z - hi.z;
-          hi.w = __uint_as_float(__float_as_uint(v.w) & 0xffffe000u); lo.w = v.w - hi.w;
-        };
-        if (A_TMEM) {
-          // thread = row of the tile = its TMEM lane; 16-byte chunk j of row r sits at chunk position j ^ (r & 7)
-          const int row = (warp & 3) * 32 + lane;
-          uint32_t hi_bits[32], lo_bits[32];
+        const unsigned char* st = stage_base + (size_t)s * C_::STAGE_BYTES;
+        uint32_t hi[32], lo[32];
 #pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            float4 hi, lo; split(*reinterpret_cast<const float4*>(st + row * 128 + ((j ^ (row & 7)) << 4)), hi, lo);
-            hi_bits[4 * j] = __float_as_uint(hi.x); hi_bits[4 * j + 1] = __float_as_uint(hi.y);
-            hi_bits[4 * j + 2] = __float_as_uint(hi.z); hi_bits[4 * j + 3] = __float_as_uint(hi.w);
-            lo_bits[4 * j] = __float_as_uint(lo.x); lo_bits[4 * j + 1] = __float_as_uint(lo.y);
-            lo_bits[4 * j + 2] = __float_as_uint(lo.z); lo_bits[4 * j + 3] = __float_as_uint(lo.w);
-          }
-          const uint32_t ta = tmem_a + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(slot * 2 * BK);
-          tc_fence_after();
-          tmem_st_32(ta, hi_bits);
-          tmem_st_32(ta + (uint32_t)BK, lo_bits);
-          tc_fence_before();
-        } else {
+        for (int j = 0; j < 8; ++j) {
+          const float4 v = *reinterpret_cast<const float4*>(st + row * 128 + ((j ^ (row & 7)) << 4));
+          const float part[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-          for (int i = 0; i < C_::A_BYTES / 16 / 128; ++i) {
-            float4 hi, lo; split(a_hi[tid + i * 128], hi, lo);
-            a_hi[tid + i * 128] = hi; a_lo[tid + i * 128] = lo;
+          for (int c = 0; c < 4; ++c) {
+            float h, l;
+            split_tf32(part[c], h, l);
+            hi[4 * j + c] = __float_as_uint(h);
+            lo[4 * j + c] = __float_as_uint(l);
           }
-          fence_async_smem();               // generic-proxy writes -> visible to the tensor core's async proxy
         }
+        const uint32_t ta = tmem_a + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(slot * 2 * BK);
+        tc_fence_after();
+        tmem_st_32_begin(ta, hi);
+        tmem_st_32(ta + (uint32_t)BK, lo);
+        tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(&full_split[slot]);
       }
@@ -269,25 +249,32 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
     int chunk_no = 0;
     for (long long tile = blockIdx.x; tile < n_tiles_total; tile += gridDim.x, ++lt) {
       const Tile tl = decode_tile(tab, item_g, tile, m_tiles, n_tiles, kb_per_seg, BN);
-      const uint32_t buf = lt & 1u;
-      mbar_wait(&acc_full[buf], (lt >> 1) & 1u, status);
+      const uint32_t buf = lt % ACC;
+      mbar_wait(&acc_full[buf], (lt / ACC) & 1u, status);
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const int c_row = tab.group_c_row[tl.g] + tl.t;
-#pragma unroll 1
-      for (int c = 0; c < BN / 32; ++c, ++chunk_no) {
+      float sum[BN];
+#pragma unroll
+      for (int c = 0; c < BN / 32; ++c) {
         uint32_t r[32], q[32];
         const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + buf * (uint32_t)(2 * BN) + (uint32_t)(c * 32);
         tmem_ld_32(taddr, r);                      // hi x hi
         tmem_ld_32(taddr + (uint32_t)BN, q);       // hi x lo + lo x hi
 #pragma unroll
-        for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) + __uint_as_float(q[j]));
+        for (int j = 0; j < 32; ++j) sum[c * 32 + j] = __uint_as_float(r[j]) + __uint_as_float(q[j]);
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&acc_empty[buf]);
+#pragma unroll
+      for (int c = 0; c < BN / 32; ++c, ++chunk_no) {
         unsigned char* sl = slab + (size_t)(chunk_no & 1) * 4096;
         if (lane == 0) bulk_wait_read<1>();     // the slab used two chunks ago has been read by its store
         __syncwarp();
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
           *reinterpret_cast<float4*>(sl + lane * 128 + ((j ^ (lane & 7)) << 4)) =
-              make_float4(__uint_as_float(r[4 * j]), __uint_as_float(r[4 * j + 1]), __uint_as_float(r[4 * j + 2]), __uint_as_float(r[4 * j + 3]));
+              make_float4(sum[c * 32 + 4 * j], sum[c * 32 + 4 * j + 1], sum[c * 32 + 4 * j + 2], sum[c * 32 + 4 * j + 3]);
         }
         fence_async_smem();
         __syncwarp();
@@ -301,9 +288,6 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
           bulk_commit();
         }
       }
-      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&acc_empty[buf]);
     }
     if (lane == 0) bulk_wait_read<0>();
   }
@@ -968,8 +952,7 @@ static int launch_bn(const TcTable& tab, const CUtensorMap& ma, const CUtensorMa
   int* st = nullptr;
   cudaError_t e = cudaGetSymbolAddress((void**)&st, g_tc_status);
   if (e != cudaSuccess) return cuda_fail(e);
-  constexpr bool A_TMEM = (BN == 64);
-  e = cudaFuncSetAttribute(gemm_tf32x3_kernel<BN, A_TMEM>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<BN>::SMEM_BYTES);
+  e = cudaFuncSetAttribute(gemm_tf32x3_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<BN>::SMEM_BYTES);
   if (e != cudaSuccess) return cuda_fail(e);
   const long long m_tiles = (M + BM - 1) / BM;
   const int n_tiles = (N + BN - 1) / BN;
@@ -977,7 +960,7 @@ static int launch_bn(const TcTable& tab, const CUtensorMap& ma, const CUtensorMa
   const int sms = sm_count();
   if (sms < 1) return FASTEQ_CUDA_ERROR;
   const unsigned grid = (unsigned)(total < sms ? total : sms);     // one persistent CTA per SM
-  e = launch_dependent(gemm_tf32x3_kernel<BN, A_TMEM>, grid, NT_P, Cfg<BN>::SMEM_BYTES, s, ma, mbh, mbl, mc, tab, M, N, K, total, (int)m_tiles, n_tiles, st);
+  e = launch_dependent(gemm_tf32x3_kernel<BN>, grid, NT_P, Cfg<BN>::SMEM_BYTES, s, ma, mbh, mbl, mc, tab, M, N, K, total, (int)m_tiles, n_tiles, st);
   return e == cudaSuccess ? FASTEQ_OK : cuda_fail(e);
 }
 
