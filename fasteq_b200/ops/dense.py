@@ -6,7 +6,8 @@ not a multiple of four, operands that are not 16-byte aligned) and every weight 
 the SO3Linear family: a plain GEMM is its one-path, one-row case (``fasteq_eqlinear_forward`` / ``_dgrad`` /
 ``_wgrad`` with ``u = K``, ``v = N``), so no library GEMM is called on CUDA tensors.  FP64 forward and grad_x with
 even extents run on the FP64 tensor cores (DMMA, as the reference's FP64 back-end does:
-fasteq/cuda/src/eqlinear/backends/fp64/direct_gemm_f64_tma.cu:204); the rest run on FMA tile kernels.
+fasteq/cuda/src/eqlinear/backends/fp64/direct_gemm_f64_tma.cu:204), FP32 weight gradients of more than 128 rows on tcgen05 in three bf16
+parts per operand (FP32 accuracy); the rest run on FMA tile kernels.
 CPU tensors (the oracle's territory) fall through to ``torch.matmul``.
 """
 from __future__ import annotations

@@ -6,7 +6,8 @@ elements (viewed ``[P, U, V]``), the result is ``[B, J*V]``.  Precision routing 
 (fasteq/ops/eqlinear.py:24-41): float64 -> FP64; float32 -> ``compute_precision`` ``None`` /
 ``"tf32"`` / ``"tf32x3"`` (error bound of 3xTF32) or ``"fp32"``; anything else raises ``ValueError``.
 The reference returns no gradient for ``w`` (eqlinear_runtime.py:104); here ``w`` gets one when it
-requires grad (``fasteq_eqlinear_wgrad``, FP32 / FP64 FMA arithmetic), so the mixing weights can be trained.
+requires grad (``fasteq_eqlinear_wgrad``: FP32 on the tensor cores in three bf16 parts per operand, short batches and FP64 on FMA tiles),
+so the mixing weights can be trained.
 Unsupported descriptors raise; there is no fallback path.
 """
 from __future__ import annotations
