@@ -14,7 +14,7 @@
 // Structure of one CTA (persistent: one CTA per SM walks 128 x BN output tiles round-robin, the stage ring
 // and two TMEM accumulators carry over from tile to tile so that loads, splits, MMAs and stores of
 // neighbouring tiles overlap):
-//   warp 0       : TMA producer -- 3-D tiled loads (SWIZZLE_128B) of the raw A and Bt k-blocks
+//   warps 0, 10  : TMA producers -- 3-D tiled loads (SWIZZLE_128B) of the raw A k-blocks (0) and of the weights' (10)
 //   warp 1       : allocates TMEM, issues tcgen05.mma (kind::tf32, M = 128, N = BN, K = 8) from one lane,
 //                  releases ring stages and signals the epilogue with tcgen05.commit
 //   warps 2..5   : split each raw A k-block into hi / lo parts in tensor memory (thread = row = TMEM
@@ -41,18 +41,24 @@ namespace tc {
 
 constexpr int BM = 128, BK = 32;
 constexpr int NT = 192;     // A-stationary kernel: 6 warps
-constexpr int NT_P = 320;   // persistent grouped kernel: 10 warps
+constexpr int NT_P = 352;   // persistent grouped kernel: 11 warps
+
+constexpr int ITEM_TABLE = 768;       // entries of the table from item to group (see decode_tile)
 
 template <int BN> struct Cfg {
   static constexpr int A_BYTES = BM * BK * 4;          // 16 KB
   static constexpr int B_BYTES = BN * BK * 4;
-  static constexpr int B_OFF = A_BYTES;                // raw A, then B hi and lo
-  static constexpr int STAGE_BYTES = B_OFF + 2 * B_BYTES;
-  static constexpr int STAGES = (BN <= 64) ? 6 : 4;     // ring depth that fits the 227 KB of one CTA
+  // raw A and the weights' hi | lo tiles each have their own ring: A comes from HBM and is free again once split, the weights come from
+  // L2 and stay until the MMAs have read them.  Together they fill 192 KB.  Measured: 6 + 3 stages at 128 columns 85.0 us where 4 + 4 take 82.7
+  // (12,288 nodes, see below), 17.8 -> 18.4 at 1,536; 6 + 6 at 64 columns 9.4 us where 8 + 4 take 9.0 (192 nodes).
+  static constexpr int A_STAGES = (BN <= 64) ? 8 : 4, B_STAGES = 4;
+  static constexpr int RING_BYTES = A_STAGES * A_BYTES + B_STAGES * 2 * B_BYTES;
   static constexpr int SLOTS = 4;                       // split A: 4 x 64 tensor-memory columns
   static constexpr int ACCUMULATORS = 256 / (2 * BN);   // in the other 256: two tiles of 64 columns, one of 128
   static constexpr int STORE_BYTES = 4 * 2 * 4096;     // per epilogue warp: two 32 x 32 FP32 slabs for the TMA stores
-  static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + STORE_BYTES + 1024 /* barriers */ + 1024 /* alignment slack */;
+  static constexpr int BARRIER_BYTES = (2 * (A_STAGES + B_STAGES + SLOTS + ACCUMULATORS) + 1) * 8;
+  static constexpr int SMEM_BYTES = RING_BYTES + STORE_BYTES + BARRIER_BYTES + ITEM_TABLE + 1024 /* alignment slack */;
+  static_assert(SMEM_BYTES <= 227 * 1024, "shared memory of one CTA");
 };
 
 // one output tile of the persistent loop
@@ -64,20 +70,29 @@ struct Tile {
 // Every role of the CTA decodes every tile, in line with its other work: a short tile (K = 64: two k-blocks) spent more on three
 // 64-bit divisions and a walk over up to 64 groups than on its MMAs.  Hence 32-bit divisions where the tile count allows
 // and a shared-memory table from item to group (`item_g`, null when there are more items than it holds).
-constexpr int ITEM_TABLE = 768;
-
+//
+// Order of the tiles.  With many rounds of tiles the items of a row tile follow one another, turned by one from row tile to row tile (a CTA's
+// stride through them then meets long and short items alike): neighbouring CTAs read neighbouring rows of the same entries, whole DRAM
+// pages, and different weights.  With items outermost they read 128 bytes out of every entry, and the same weights at once: 12,288 nodes
+// (see below) 90.2 -> 85.0 us, 20,011 nodes 142.9 -> 131.8 (6 + 3 stages).  Up to four rounds (`m_tiles` > 0, else 0) items stay outermost: the short ones, which
+// come last, fill the last round (1,536 nodes 18.4 us, the other way 19.1).
 __device__ __forceinline__ Tile decode_tile(const TcTable& tab, const unsigned char* item_g, long long tile, int m_tiles, int n_tiles,
                                             int kb_per_seg, int BN) {
   Tile r;
   int mx, ny, z;
-  if (tile <= 0xffffffffLL) {
+  if (m_tiles > 0) {
     const unsigned t32 = (unsigned)tile, rest = t32 / (unsigned)m_tiles;
     mx = (int)(t32 - rest * (unsigned)m_tiles);
     z = (int)(rest / (unsigned)n_tiles);
     ny = (int)(rest - (unsigned)z * (unsigned)n_tiles);
+  } else if (tile <= 0xffffffffLL) {
+    const unsigned t32 = (unsigned)tile, rest = t32 / (unsigned)n_tiles, m = rest / (unsigned)tab.n_items;
+    ny = (int)(t32 - rest * (unsigned)n_tiles);
+    mx = (int)m;
+    z = (int)((rest - m * (unsigned)tab.n_items + m % (unsigned)tab.n_items) % (unsigned)tab.n_items);
   } else {
-    const long long rest = tile / m_tiles;
-    mx = (int)(tile % m_tiles); ny = (int)(rest % n_tiles); z = (int)(rest / n_tiles);
+    const long long rest = tile / n_tiles, m = rest / tab.n_items;
+    ny = (int)(tile % n_tiles); mx = (int)m; z = (int)((rest - m * tab.n_items + m) % tab.n_items);
   }
   int g = 0;
   if (item_g) g = item_g[z];
@@ -92,7 +107,8 @@ __device__ __forceinline__ Tile decode_tile(const TcTable& tab, const unsigned c
 // Shared memory bounds a k-block: TMA fills, the split's reads and the MMAs' operand reads share its 128 bytes per clock.  With the
 // split A in tensor memory (thread = row = TMEM lane, tcgen05.st) that is 112 KB at 128 columns, 875 clocks beside 773 of MMAs; split in
 // place in shared memory it was 176 KB.  SO3Linear after the tensor product (40 rows of 128 channels to 16): 12,288 nodes 112.7 -> 95.5 us a
-// direction (3.7 TB/s of features, 744 MB through L2 with the weights), 1,536 nodes 21.0 -> 17.9.
+// direction, 1,536 nodes 21.0 -> 17.9; with the two rings and the order of tiles above 82.7 (4.3 TB/s of features) and 17.8.  A second set of
+// split warps on alternate k-blocks changes nothing (93.3 where 90.2).
 // The price at 128 columns is a single accumulator (256 columns with its cross terms): the epilogue takes it to registers whole and
 // hands it back before it stores.
 template <int BN>
@@ -104,21 +120,23 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   using C_ = Cfg<BN>;
-  constexpr int STAGES = C_::STAGES, SLOTS = C_::SLOTS, ACC = C_::ACCUMULATORS;
+  constexpr int A_STAGES = C_::A_STAGES, B_STAGES = C_::B_STAGES, SLOTS = C_::SLOTS, ACC = C_::ACCUMULATORS;
   constexpr uint32_t TMEM_COLS = 512, TMEM_A = 256;
   static_assert(ACC * 2 * BN == (int)TMEM_A && SLOTS * 2 * BK <= 256, "tensor memory: accumulators + A ring");
-  unsigned char* stage_base = smem;
-  unsigned char* store_base = smem + STAGES * C_::STAGE_BYTES;     // [4 warps][2 slabs][32 rows x 128 B]
+  unsigned char* b_base = smem + A_STAGES * C_::A_BYTES;
+  unsigned char* store_base = smem + C_::RING_BYTES;               // [4 warps][2 slabs][32 rows x 128 B]
   uint64_t* bars = reinterpret_cast<uint64_t*>(store_base + C_::STORE_BYTES);
-  uint64_t* full_raw = bars;                 // [STAGES] TMA landed
-  uint64_t* empty = bars + STAGES;           // [STAGES] MMAs have consumed the stage
-  uint64_t* full_split = empty + STAGES;     // [SLOTS] hi / lo parts ready
+  uint64_t* a_full = bars;                   // [A_STAGES] TMA landed
+  uint64_t* a_empty = a_full + A_STAGES;     // [A_STAGES] the four split warps have read it
+  uint64_t* b_full = a_empty + A_STAGES;     // [B_STAGES] TMA landed
+  uint64_t* b_empty = b_full + B_STAGES;     // [B_STAGES] MMAs have read it
+  uint64_t* full_split = b_empty + B_STAGES; // [SLOTS] hi / lo parts ready
   uint64_t* slot_empty = full_split + SLOTS; // [SLOTS] MMAs have consumed the split A
   uint64_t* acc_full = slot_empty + SLOTS;   // [ACC] accumulator complete
   uint64_t* acc_empty = acc_full + ACC;      // [ACC] accumulator read back by the four epilogue warps
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + ACC);
 
-  unsigned char* item_table = reinterpret_cast<unsigned char*>(bars) + 1024 - ITEM_TABLE;   // behind the barriers
+  unsigned char* item_table = reinterpret_cast<unsigned char*>(bars) + C_::BARRIER_BYTES;
   const unsigned char* item_g = tab.n_items <= ITEM_TABLE ? item_table : nullptr;
   if (item_g) {
     for (int z = threadIdx.x; z < tab.n_items; z += NT_P) {
@@ -131,7 +149,8 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
   const int kb_per_seg = (K + BK - 1) / BK;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < STAGES; ++s) { mbar_init(&full_raw[s], 1); mbar_init(&empty[s], 1); }
+    for (int s = 0; s < A_STAGES; ++s) { mbar_init(&a_full[s], 1); mbar_init(&a_empty[s], 4); }
+    for (int s = 0; s < B_STAGES; ++s) { mbar_init(&b_full[s], 1); mbar_init(&b_empty[s], 1); }
     for (int s = 0; s < SLOTS; ++s) { mbar_init(&full_split[s], 4); mbar_init(&slot_empty[s], 1); }
     for (int b = 0; b < ACC; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 4); }
     mbar_fence_init();
@@ -147,8 +166,8 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
   const uint32_t tmem_base = *tmem_slot;
   const uint32_t tmem_a = tmem_base + TMEM_A;     // [SLOTS][hi 32 columns | lo 32 columns]
 
-  if (warp == 0) {
-    // ------------------------------------------------------------------ TMA producer
+  if (warp == 0 || warp == 10) {
+    // ------------------------------------------------------------------ TMA producers: warp 0 of A, warp 10 of the weights
     if (lane == 0) {
       int it = 0;
       for (long long tile = blockIdx.x; tile < n_tiles_total; tile += gridDim.x) {
@@ -156,17 +175,23 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
         // each tile starts its walk over the k-blocks at a different one, so that the CTAs do not all fetch the same
         // weight lines from L2 at the same moment (the terms of a sum are the same, their order depends on the tile)
         const int kb_start = (int)(tile % tl.n_kb);
+        int seg = tl.seg0 + kb_start / kb_per_seg, k_in = kb_start % kb_per_seg;
         for (int kbi = 0; kbi < tl.n_kb; ++kbi, ++it) {
-          const int kb = kbi + kb_start < tl.n_kb ? kbi + kb_start : kbi + kb_start - tl.n_kb;
-          const int s = it % STAGES;
-          mbar_wait(&empty[s], ((it / STAGES) & 1u) ^ 1u, status);
-          unsigned char* st = stage_base + (size_t)s * C_::STAGE_BYTES;
-          const int seg = tl.seg0 + kb / kb_per_seg;
-          const int k0 = (kb % kb_per_seg) * BK;
-          mbar_arrive_expect_tx(&full_raw[s], (uint32_t)(C_::A_BYTES + 2 * C_::B_BYTES));
-          tma_load_3d(st, &tmA, k0, tab.path_a_row[seg] + tl.t, (int)tl.m0, &full_raw[s]);
-          tma_load_3d(st + C_::B_OFF, &tmBhi, k0, tl.n0, tab.path_w[seg], &full_raw[s]);
-          tma_load_3d(st + C_::B_OFF + C_::B_BYTES, &tmBlo, k0, tl.n0, tab.path_w[seg], &full_raw[s]);
+          if (warp == 0) {
+            const int s = it % A_STAGES;
+            mbar_wait(&a_empty[s], ((it / A_STAGES) & 1u) ^ 1u, status);
+            mbar_arrive_expect_tx(&a_full[s], (uint32_t)C_::A_BYTES);
+            tma_load_3d(smem + (size_t)s * C_::A_BYTES, &tmA, k_in * BK, tab.path_a_row[seg] + tl.t, (int)tl.m0, &a_full[s]);
+          } else {
+            const int s = it % B_STAGES;
+            unsigned char* st = b_base + (size_t)s * (2 * C_::B_BYTES);
+            mbar_wait(&b_empty[s], ((it / B_STAGES) & 1u) ^ 1u, status);
+            mbar_arrive_expect_tx(&b_full[s], (uint32_t)(2 * C_::B_BYTES));
+            tma_load_3d(st, &tmBhi, k_in * BK, tl.n0, tab.path_w[seg], &b_full[s]);
+            tma_load_3d(st + C_::B_BYTES, &tmBlo, k_in * BK, tl.n0, tab.path_w[seg], &b_full[s]);
+          }
+          if (++k_in == kb_per_seg) { k_in = 0; ++seg; }
+          if (seg == tl.seg0 + tl.n_kb / kb_per_seg) seg = tl.seg0;
         }
       }
     }
@@ -175,7 +200,7 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
     // instruction descriptors: D = F32, A = B = TF32, both K-major, M = 128; N = 2 BN for the product of
     // A_hi with the stacked [B_hi; B_lo] tile, N = BN for A_lo x B_hi
     const uint32_t idesc2 = idesc_tf32_m128(2 * BN), idesc1 = idesc_tf32_m128(BN);
-    const uint32_t tm = uniform(tmem_base), ring = uniform(smem_u32(stage_base));
+    const uint32_t tm = uniform(tmem_base), ring = uniform(smem_u32(b_base));
     const uint64_t desc0 = make_desc(ring);
     int it = 0;
     uint32_t lt = 0;
@@ -188,11 +213,12 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
       // sum is not absorbed one rounding at a time into the large accumulator)
       const uint32_t tmem_d = tm + buf * (uint32_t)(2 * BN);
       for (int kb = 0; kb < n_kb; ++kb, ++it) {
-        const int s = it % STAGES, slot = it % SLOTS;
+        const int s = it % B_STAGES, slot = it % SLOTS;
+        mbar_wait(&b_full[s], (it / B_STAGES) & 1u, status);
         mbar_wait(&full_split[slot], (it / SLOTS) & 1u, status);
         __syncwarp();
         tc_fence_after();
-        const uint64_t b_hi = desc_at(desc0, (uint32_t)(s * C_::STAGE_BYTES + C_::B_OFF));    // B_hi tile, B_lo tile right behind it
+        const uint64_t b_hi = desc_at(desc0, (uint32_t)(s * 2 * C_::B_BYTES));    // B_hi tile, B_lo tile right behind it
         const uint32_t ta = tm + TMEM_A + (uint32_t)(slot * 2 * BK);
 #pragma unroll
         for (int kk = 0; kk < BK / 8; ++kk) {
@@ -200,7 +226,7 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
           warp_mma_tf32_a_tmem(tmem_d, ta + kk * 8, desc_at(b_hi, off), idesc2, (kb | kk) ? 1u : 0u);
           warp_mma_tf32_a_tmem(tmem_d + (uint32_t)BN, ta + (uint32_t)(BK + kk * 8), desc_at(b_hi, off), idesc1, 1u);
         }
-        warp_mma_commit(&empty[s]);            // the stage may be refilled once these MMAs have read it
+        warp_mma_commit(&b_empty[s]);          // the stage may be refilled once these MMAs have read it
         warp_mma_commit(&slot_empty[slot]);
       }
       warp_mma_commit(&acc_full[buf]);
@@ -213,10 +239,9 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
     for (long long tile = blockIdx.x; tile < n_tiles_total; tile += gridDim.x) {
       const Tile tl = decode_tile(tab, item_g, tile, m_tiles, n_tiles, kb_per_seg, BN);
       for (int kb = 0; kb < tl.n_kb; ++kb, ++it) {
-        const int s = it % STAGES, slot = it % SLOTS;
-        mbar_wait(&slot_empty[slot], ((it / SLOTS) & 1u) ^ 1u, status);
-        mbar_wait(&full_raw[s], (it / STAGES) & 1u, status);
-        const unsigned char* st = stage_base + (size_t)s * C_::STAGE_BYTES;
+        const int s = it % A_STAGES, slot = it % SLOTS;
+        mbar_wait(&a_full[s], (it / A_STAGES) & 1u, status);
+        const unsigned char* st = smem + (size_t)s * C_::A_BYTES;
         uint32_t hi[32], lo[32];
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
@@ -230,6 +255,10 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
             lo[4 * j + c] = __float_as_uint(l);
           }
         }
+        fence_async_smem();                 // these reads precede the TMA write that refills the stage
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&a_empty[s]);
+        mbar_wait(&slot_empty[slot], ((it / SLOTS) & 1u) ^ 1u, status);
         const uint32_t ta = tmem_a + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(slot * 2 * BK);
         tc_fence_after();
         tmem_st_32_begin(ta, hi);
@@ -971,7 +1000,7 @@ static int launch_bn(const TcTable& tab, const CUtensorMap& ma, const CUtensorMa
   const int sms = sm_count();
   if (sms < 1) return FASTEQ_CUDA_ERROR;
   const unsigned grid = (unsigned)(total < sms ? total : sms);     // one persistent CTA per SM
-  e = launch_dependent(gemm_tf32x3_kernel<BN>, grid, NT_P, Cfg<BN>::SMEM_BYTES, s, ma, mbh, mbl, mc, tab, M, N, K, total, (int)m_tiles, n_tiles, st);
+  e = launch_dependent(gemm_tf32x3_kernel<BN>, grid, NT_P, Cfg<BN>::SMEM_BYTES, s, ma, mbh, mbl, mc, tab, M, N, K, total, total > 4LL * sms ? 0 : (int)m_tiles, n_tiles, st);
   return e == cudaSuccess ? FASTEQ_OK : cuda_fail(e);
 }
 
