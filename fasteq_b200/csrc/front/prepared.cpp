@@ -1,9 +1,10 @@
 // Cache of prepared (split / packed) weight forms for the tensor-core kernels, shared by the SO3Linear, dense and radial-chain
-// operators.  Keyed on the weight tensors' storage address and version, so an in-place update or a new tensor invalidates the entry; an
-// entry keeps the weights' storages alive (through detached aliases: a parameter object can be given another storage,
-// `module.double()` or `p.data = ...`) so the address cannot be reused while it exists.  An entry remembers the stream it was built
-// on and an event recorded behind the build: a later call on another stream waits for that event (and tells the allocator about the
-// new reader) before it uses the entry.  Plays the part of the reference's plan LRU
+// operators.  Keyed on the weight tensors' storage address, version, type, extents and strides, so that an in-place update, a new tensor or
+// another view from the same address (a transposed weight) is another entry; an entry keeps the weights' storages alive (through
+// detached aliases: a parameter object can be given another storage, `module.double()` or `p.data = ...`) so the address cannot be
+// reused while it exists.  An entry remembers the stream it was built on and an event recorded behind the build: a later call on
+// another stream waits for that event (and tells the allocator about the new reader) before it uses the entry.  Plays the part of
+// the reference's plan LRU
 // (fasteq/ops/auto_schedule/eqlinear_plan.py:38-41, :81-100, :167-187).
 //
 // Inside CUDA-graph capture a prepared form would be baked into the graph and go stale when the weights change, so the cache is bypassed
@@ -42,7 +43,9 @@ std::optional<Tensor> prepared(const std::vector<Tensor>& weights, const std::st
   std::string key = tag;
   append(key, weights[0].device().index());
   for (const Tensor& w : weights) {
-    append(key, (int64_t)w.const_data_ptr()); append(key, w._version()); append(key, w.numel());
+    append(key, (int64_t)w.const_data_ptr()); append(key, w._version()); append(key, (int64_t)w.scalar_type()); append(key, w.dim());
+    for (int64_t n : w.sizes()) append(key, n);
+    for (int64_t n : w.strides()) append(key, n);
   }
   const bool in_capture = capturing();
   {

@@ -133,3 +133,23 @@ def test_prepared_weights_survive_a_storage_swap():
         assert _rel(out.detach().cpu(), x.cpu().double() @ w.detach().cpu().double().t()) <= 2e-6
         w.data = w.data.double()
         del w, out
+
+
+def test_weight_views_that_begin_at_one_address():
+    """Prepared weight forms belong to a view, not to an address: a transposed or strided view of a weight is another matrix."""
+    from fasteq_b200 import descriptors
+    from fasteq_b200.irreps import Irreps
+    from fasteq_b200.ops import fast_equi_linear
+    from fasteq_b200.ops.dense import dense
+    g = torch.Generator().manual_seed(11)
+    x, big = torch.randn(70, 64, generator=g).cuda(), torch.randn(128, 128, generator=g).cuda()
+    w = big[:64, :64].contiguous()
+    flat = w.view(-1)
+    # [64, 64] and [32, 128] of equal size, rows apart by 64 or 128, columns apart by 1 or 64
+    views = [w, w.t(), flat.as_strided((64, 64), (63, 1)), big[:64, :64], big[:128:2, :64], w]
+    for v in views:
+        assert _rel(dense(x, v), x.double() @ v.double().t()) <= 2e-6
+    assert _rel(dense(x[:, :32], w.view(128, 32)), x[:, :32].double() @ w.view(128, 32).double().t()) <= 2e-6
+    d = descriptors.linear(Irreps("64x0e"), Irreps("64x0e"))
+    for v in (w, w.t()):
+        assert _rel(fast_equi_linear(d, v, x), x.double() @ v.reshape(64, 64).double() / 8) <= 2e-6
