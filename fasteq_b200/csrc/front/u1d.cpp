@@ -66,25 +66,35 @@ struct Plan : torch::CustomClassHolder {
   std::unordered_map<U1DModule*, std::pair<Module, Shares>> shares;
   std::vector<std::pair<cudaStream_t, std::shared_ptr<at::cuda::CUDAEvent>>> built;
   std::set<cudaStream_t> ordered;      // streams already behind every event in `built`
+  uint64_t marks = 0;                  // changes of `built`
 
   Plan(Tensor s, std::optional<Tensor> p, int64_t rows, int64_t edges, py::object r)
       : seg_ptr(std::move(s)), n_rows(rows), n_edges(edges), rule(std::move(r)) {
     if (p) perm = *p;
   }
-  void mark_built() {
-    if (capturing()) return;
+  // `publish` (under the lock) makes what the current stream has just been told to build visible; the event behind it comes first
+  template <typename Publish> void mark(Publish publish) {
     const auto cur = c10::cuda::getCurrentCUDAStream(seg_ptr.device().index());
-    auto e = std::make_shared<at::cuda::CUDAEvent>();
-    e->record(cur);
+    std::shared_ptr<at::cuda::CUDAEvent> e;
+    if (!capturing()) {
+      e = std::make_shared<at::cuda::CUDAEvent>();
+      e->record(cur);
+    }
     std::lock_guard<std::mutex> g(lock);
+    publish();
+    if (!e) return;
     built.erase(std::remove_if(built.begin(), built.end(), [&](const auto& b) { return b.first == cur.stream(); }), built.end());
     built.emplace_back(cur.stream(), std::move(e));
     ordered.clear();
+    ++marks;
   }
+  void mark_built() { mark([] {}); }
+  // A stream counts as ordered once its waits are issued: another thread may launch on it at any moment.
   void order_current_stream() {
     const auto cur = c10::cuda::getCurrentCUDAStream(seg_ptr.device().index());
     std::vector<std::shared_ptr<at::cuda::CUDAEvent>> wait;
     std::vector<Tensor> read;
+    uint64_t seen;
     {
       std::lock_guard<std::mutex> g(lock);
       if (built.empty() || ordered.count(cur.stream())) return;
@@ -97,10 +107,12 @@ struct Plan : torch::CustomClassHolder {
         if (perm.defined()) read.push_back(perm);
         for (const auto& p : parts) read.push_back(p.second);
       }
-      ordered.insert(cur.stream());
+      seen = marks;
     }
     for (const auto& e : wait) e->block(cur);
     for (const Tensor& t : read) c10::cuda::CUDACachingAllocator::recordStream(t.storage().data_ptr(), cur);
+    std::lock_guard<std::mutex> g(lock);
+    if (seen == marks) ordered.insert(cur.stream());     // otherwise something was built meanwhile: the next call waits for that too
   }
   // first row of each share [1, n + 1]; with `split` shares are cut between edges and a second row holds their first edges
   Tensor partition(int64_t n, bool split) {
@@ -116,8 +128,7 @@ struct Plan : torch::CustomClassHolder {
     cudaStream_t s = stream_of(p);
     if (split) check(core.graph_partition_edges(seg_ptr.const_data_ptr<int32_t>(), n_rows, n_edges, (int32_t)n, d, d + n + 1, s), "fasteq_graph_partition_edges", core.last_cuda_error);
     else check(core.graph_partition(seg_ptr.const_data_ptr<int32_t>(), n_rows, n_edges, (int32_t)n, d, s), "fasteq_graph_partition", core.last_cuda_error);
-    { std::lock_guard<std::mutex> g(lock); parts.emplace(std::make_pair(n, split), p); }
-    mark_built();
+    mark([&] { p = parts.emplace(std::make_pair(n, split), p).first->second; });     // another thread's, if it was first
     return p;
   }
   Shares shares_of(const Module& m) {

@@ -66,3 +66,47 @@ def test_operators_launch_on_the_current_stream():
         y = dense(x, w)                  # must see the filled values
     side.synchronize()
     assert float(y.min()) == 3.0 and float(y.max()) == 3.0
+
+
+def _operator(n=600, e=5000, seed=0):
+    from fasteq_b200 import descriptors
+    from fasteq_b200.irreps import Irreps
+    sh = Irreps.spherical_harmonics(2)
+    io, ins = descriptors.full_channelwise_instructions("32x0e+32x1o", sh, 2)
+    d = descriptors.channelwise_tensor_product("32x0e+32x1o", sh, io, ins)
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    src, dst = (torch.randint(0, n, (e,), generator=g, device="cuda", dtype=torch.int32) for _ in range(2))
+    w, x, y = (torch.randn(*s, generator=g, device="cuda") for s in ((e, d.w_seg_num * 32), (n, d.x_seg_num * 32), (e, d.y_seg_num)))
+    return src, dst, w, x, y, d.meta(torch.float32, "cuda")
+
+
+def test_threads_share_a_plan_on_their_own_streams():
+    """The partitions of a graph are built by whichever thread comes first and used by all: each stream waits for what others built."""
+    import threading
+    from fasteq_b200.ops import fast_uniform1d_jit, uniform1d_jit as u1d
+    src, dst, w, x, y, meta = _operator()
+
+    def step(index):
+        ops = [t.detach().requires_grad_(True) for t in (w, x, y)]
+        out = fast_uniform1d_jit(*ops, {1: src}, {0: index}, meta)
+        return [out.detach(), *torch.autograd.grad(out, ops, torch.ones_like(out))]
+    want = step(dst)
+    for _ in range(10):
+        index, got = dst.clone(), {}              # a plan of its own, whose partitions nobody has built
+        u1d.graph_plan(index, x.shape[0])
+        start = threading.Barrier(4)
+
+        def work(k):
+            with torch.cuda.stream(torch.cuda.Stream()) as _:
+                torch.cuda.current_stream().wait_stream(torch.cuda.default_stream())
+                start.wait()
+                got[k] = step(index)
+                torch.cuda.current_stream().synchronize()
+        threads = [threading.Thread(target=work, args=(k,)) for k in range(4)]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+        for k in range(4):
+            for a, b in zip(got[k], want):         # the features' gradient is summed by atomics
+                assert (a - b).norm() <= 1e-6 * b.norm()
