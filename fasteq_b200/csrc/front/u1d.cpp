@@ -75,20 +75,16 @@ struct Plan : torch::CustomClassHolder {
   // `publish` (under the lock) makes what the current stream has just been told to build visible; the event behind it comes first
   template <typename Publish> void mark(Publish publish) {
     const auto cur = c10::cuda::getCurrentCUDAStream(seg_ptr.device().index());
-    std::shared_ptr<at::cuda::CUDAEvent> e;
-    if (!capturing()) {
-      e = std::make_shared<at::cuda::CUDAEvent>();
-      e->record(cur);
-    }
+    auto e = std::make_shared<at::cuda::CUDAEvent>();
+    e->record(cur);
     std::lock_guard<std::mutex> g(lock);
     publish();
-    if (!e) return;
     built.erase(std::remove_if(built.begin(), built.end(), [&](const auto& b) { return b.first == cur.stream(); }), built.end());
     built.emplace_back(cur.stream(), std::move(e));
     ordered.clear();
     ++marks;
   }
-  void mark_built() { mark([] {}); }
+  void mark_built() { if (!capturing()) mark([] {}); }
   // A stream counts as ordered once its waits are issued: another thread may launch on it at any moment.
   void order_current_stream() {
     const auto cur = c10::cuda::getCurrentCUDAStream(seg_ptr.device().index());
@@ -114,7 +110,8 @@ struct Plan : torch::CustomClassHolder {
     std::lock_guard<std::mutex> g(lock);
     if (seen == marks) ordered.insert(cur.stream());     // otherwise something was built meanwhile: the next call waits for that too
   }
-  // first row of each share [1, n + 1]; with `split` shares are cut between edges and a second row holds their first edges
+  // first row of each share [1, n + 1]; with `split` shares are cut between edges and a second row holds their first edges.  One that
+  // a capture needs first belongs to that capture: its kernel has not run and its memory is the graph's, so the plan does not keep it
   Tensor partition(int64_t n, bool split) {
     {
       std::lock_guard<std::mutex> g(lock);
@@ -128,7 +125,7 @@ struct Plan : torch::CustomClassHolder {
     cudaStream_t s = stream_of(p);
     if (split) check(core.graph_partition_edges(seg_ptr.const_data_ptr<int32_t>(), n_rows, n_edges, (int32_t)n, d, d + n + 1, s), "fasteq_graph_partition_edges", core.last_cuda_error);
     else check(core.graph_partition(seg_ptr.const_data_ptr<int32_t>(), n_rows, n_edges, (int32_t)n, d, s), "fasteq_graph_partition", core.last_cuda_error);
-    mark([&] { p = parts.emplace(std::make_pair(n, split), p).first->second; });     // another thread's, if it was first
+    if (!capturing()) mark([&] { p = parts.emplace(std::make_pair(n, split), p).first->second; });     // another thread's, if it was first
     return p;
   }
   Shares shares_of(const Module& m) {
@@ -144,6 +141,7 @@ struct Plan : torch::CustomClassHolder {
       s.n = got[0].cast<int32_t>(); s.split = got[1].cast<bool>();
     }
     s.part = partition(s.n, s.split);
+    if (capturing()) return s;
     std::lock_guard<std::mutex> g(lock);
     shares.emplace(m.get(), std::make_pair(m, s));
     return s;

@@ -332,6 +332,7 @@ class _Call:
             g.perm = self.plan.perm.data_ptr() if self.plan.perm is not None else None
             part, g.n_parts, split = self.plan.shares(mod.desc)
             g.part_ptr, part_edge = part.data_ptr(), part[1].data_ptr() if split else None
+            g.part = part               # under capture nobody else holds it
             self.plan.ready_on_current_stream()
             self.plan.record()
         return g, part_edge

@@ -110,3 +110,36 @@ def test_threads_share_a_plan_on_their_own_streams():
         for k in range(4):
             for a, b in zip(got[k], want):         # the features' gradient is summed by atomics
                 assert (a - b).norm() <= 1e-6 * b.norm()
+
+
+def test_a_partition_first_needed_under_capture_stays_with_the_capture():
+    """Its kernel is recorded, not run: a call outside, before any replay, must not find it."""
+    from fasteq_b200.ops import fast_uniform1d_jit, uniform1d_jit as u1d
+    src, dst, w, x, y, meta = _operator(e=1500)       # few edges a row: forwards keep whole receivers, backwards cut them
+    ops = [t.requires_grad_(True) for t in (w, x, y)]
+    go = torch.randn_like(fast_uniform1d_jit(*ops, {1: src}, {0: dst}, meta))
+
+    def step(index):
+        return torch.autograd.grad(fast_uniform1d_jit(*ops, {1: src}, {0: index}, meta), ops, go)
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        want = step(dst)                               # modules loaded, first-use allocations made
+    index = dst.clone()
+    with torch.no_grad():
+        fast_uniform1d_jit(*ops, {1: src}, {0: index}, meta)
+    plan = u1d.graph_plan(index, x.shape[0])
+    kept = dict(plan._parts)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with u1d.record_plans() as plans, torch.cuda.graph(graph, stream=side):
+        captured = step(index)
+    assert plans == [plan] and plan._parts.keys() == kept.keys()
+    for _ in range(2):
+        for a, b in zip(step(index), want):
+            assert (a - b).norm() <= 1e-6 * b.norm()   # the features' gradient is summed by atomics
+        assert len(plan._parts) > len(kept)
+        graph.replay()
+        torch.cuda.synchronize()
+        for a, b in zip(captured, want):
+            assert (a - b).norm() <= 1e-6 * b.norm()
