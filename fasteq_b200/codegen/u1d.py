@@ -862,6 +862,11 @@ __global__ void __launch_bounds__(NTHREADS, {tun.min_blocks})
 fasteq_u1d_bwd_kernel(const Graph g, const T* __restrict__ go, const T* __restrict__ w, const T* __restrict__ x,
                       const T* __restrict__ y, T* __restrict__ gw, T* __restrict__ gx, T* __restrict__ gy{dual_params}) {{
   extern __shared__ __align__(128) unsigned char smem_all[];
+  const int warp_all = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // tensor-memory gradient rows: warp 0 allocates (before the next kernel is let in, which may want columns too), everyone reads
+  // the base address from the last word of the first barrier block (free when no gradient tile lives in shared memory)
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem_all + BAR_BYTES - 4);
+  if (GO_TMEM && warp_all == 0) scratch_tmem_alloc(tmem_slot, TMEM_COLS);
   if (threadIdx.x == 0) {{
     for (int p = 0; p < cfg::PIPES; ++p) {{
       uint64_t* f = reinterpret_cast<uint64_t*>(smem_all + (size_t)p * PIPE_BYTES);
@@ -871,18 +876,10 @@ fasteq_u1d_bwd_kernel(const Graph g, const T* __restrict__ go, const T* __restri
     }}
     mbar_fence_init();
   }}
+  if (GO_TMEM) asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
+  if (GO_TMEM) asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   wait_for_previous_kernel();
-  const int warp_all = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // tensor-memory gradient rows: warp 0 allocates, everyone reads the base address from the last word of the first
-  // barrier block (free when no gradient tile lives in shared memory)
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem_all + BAR_BYTES - 4);
-  if (GO_TMEM) {{
-    if (warp_all == 0) scratch_tmem_alloc(tmem_slot, TMEM_COLS);
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  }}
   const uint32_t tmem_base = GO_TMEM ? *tmem_slot : 0u;
   const bool is_producer = warp_all >= cfg::PIPES * cfg::NCONS_WARPS;
   const int pipe = is_producer ? warp_all - cfg::PIPES * cfg::NCONS_WARPS : warp_all / cfg::NCONS_WARPS;

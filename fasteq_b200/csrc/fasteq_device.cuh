@@ -104,7 +104,8 @@ __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wa
 
 // Programmatic dependent launch.  A kernel started by launch_dependent (launch.cuh) may begin while the one before it in the stream is
 // still running: it sets up its barriers and tensor memory, then every thread waits here for the end of that kernel, before it touches
-// global memory.  Every thread of such a kernel has to pass here, so that its end means the end of all earlier ones too.
+// global memory.  The first thread of a CTA to pass lets the next kernel in as far as that CTA goes: what the CTA allocates it has
+// allocated by then, with a barrier between, or the next one might hold the tensor memory it still needs.  Every thread of such a kernel has to pass here, so that its end means the end of all earlier ones too.
 __device__ __forceinline__ void wait_for_previous_kernel() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

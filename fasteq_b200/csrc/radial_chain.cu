@@ -113,14 +113,15 @@ radial_chain_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
     mbar_fence_init();
   }
   if (warp == 1) tmem_alloc(tmem_slot, TMEM_COLUMNS);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
   wait_for_previous_kernel();
   for (int i = threadIdx.x; i < H * NB; i += NT) {
     const int j = i / NB, k = i % NB;
     w1s[i] = k < a.nb ? *reinterpret_cast<const volatile float*>(a.w1 + j * a.nb + k) : 0.f;
   }
-  tc_fence_before();
   __syncthreads();
-  tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
   if (warp < GROUPS) {

@@ -30,7 +30,7 @@ from ..codegen import u1d as _emit
 from ..codegen.u1d_common import U1DSpec, make_spec
 from ._needs import asked
 
-_EMITTER_VERSION = "u1d-v8"
+_EMITTER_VERSION = "u1d-v9"
 _MODULES: Dict[Tuple, _cabi.U1DModule] = {}
 _TUNING_OVERRIDE: Dict[str, _emit.Tuning] = {}
 _lock = threading.Lock()
