@@ -675,8 +675,8 @@ __global__ void __launch_bounds__(WG_THREADS) eqlinear_wgrad_f32_kernel(const __
 // sits on the N side.  A path's chunks are numbered irrep row by irrep row, `chunks_per_row` = ceil(batch / 32) to each.
 template <int TN>
 __global__ void __launch_bounds__(wg::THREADS, 1) eqlinear_wgrad_tc_kernel(const __grid_constant__ CUtensorMap tmM,
-    const __grid_constant__ CUtensorMap tmN, const __grid_constant__ WgradTable tab, const float* __restrict__ X,
-    const float* __restrict__ G, float* __restrict__ partial, long long batch, int in_rows, int out_rows, int u, int v, int num_paths,
+    const __grid_constant__ CUtensorMap tmN, const __grid_constant__ WgradTable tab, const float* X,
+    const float* G, float* partial, long long batch, int in_rows, int out_rows, int u, int v, int num_paths,
     int chunks_per_row, int chunks_per_split, int swap, int* status) {
   using namespace fasteq::wg;
   using namespace fasteq::tc;

@@ -1,7 +1,8 @@
 // Launch of a kernel that calls wait_for_previous_kernel(): it may begin before the kernel ahead of it in the stream has ended, so that its
-// launch and set-up (barriers, tensor memory, descriptors: 1 to 2 us) lie beside the other's tail.  Only for kernels that read and write
-// global memory after that wait alone, and through addresses no compiler can load from ahead of it (bulk and tensor copies, loads that
-// depend on them).  Captured into CUDA graphs as programmatic edges.
+// launch and set-up (barriers, tensor memory, descriptors: 1 to 2 us) lie beside the other's tail.  Only for kernels that write global
+// memory after that wait alone.  Ahead of it they read only what was complete before the kernel ahead could begin (a graph's plan); the rest
+// after it, in a way no compiler can move ahead of it: bulk and tensor copies, loads whose addresses depend on those, volatile
+// loads, plain ones through pointers without __restrict__.  Captured into CUDA graphs as programmatic edges.
 #pragma once
 #include <cuda_runtime.h>
 

@@ -72,6 +72,18 @@ __device__ __forceinline__ void silu_and_derivative(float z, float& h, float& d)
   d = s * (1.0f + z * (1.0f - s));
 }
 
+// Loads from addresses known when the kernel begins: volatile, so that no compiler moves them ahead of wait_for_previous_kernel()
+__device__ __forceinline__ float load_after_wait(const float* p) {
+  float v;
+  asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ float4 load4_after_wait(const float* p) {
+  float4 v;
+  asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+  return v;
+}
+
 // 16-byte chunk c of row r of a 128-byte-row tile sits at chunk position c ^ (r & 7) (SWIZZLE_128B)
 __device__ __forceinline__ float4* swz(unsigned char* tile, int r, int c) {
   return reinterpret_cast<float4*>(tile + r * 128 + ((c ^ (r & 7)) << 4));
@@ -119,7 +131,7 @@ radial_chain_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
   wait_for_previous_kernel();
   for (int i = threadIdx.x; i < H * NB; i += NT) {
     const int j = i / NB, k = i % NB;
-    w1s[i] = k < a.nb ? *reinterpret_cast<const volatile float*>(a.w1 + j * a.nb + k) : 0.f;
+    w1s[i] = k < a.nb ? load_after_wait(a.w1 + j * a.nb + k) : 0.f;
   }
   __syncthreads();
   const uint32_t tmem_base = *tmem_slot;
@@ -192,12 +204,12 @@ radial_chain_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
       if (a.rows_in_vectors) {
 #pragma unroll
         for (int k = 0; k < NB; k += 4) {
-          const float4 q = mine ? __ldg(reinterpret_cast<const float4*>(a.basis + r * NB + k)) : make_float4(0.f, 0.f, 0.f, 0.f);
+          const float4 q = mine ? load4_after_wait(a.basis + r * NB + k) : make_float4(0.f, 0.f, 0.f, 0.f);
           bb[k] = q.x; bb[k + 1] = q.y; bb[k + 2] = q.z; bb[k + 3] = q.w;
         }
       } else {
 #pragma unroll
-        for (int k = 0; k < NB; ++k) bb[k] = (mine && k < a.nb) ? __ldg(a.basis + r * a.nb + k) : 0.f;
+        for (int k = 0; k < NB; ++k) bb[k] = (mine && k < a.nb) ? load_after_wait(a.basis + r * a.nb + k) : 0.f;
       }
     };
     auto first_layer = [&](const float (&bb)[NB], int j, float& h, float& d) {

@@ -1,5 +1,6 @@
 """Kernels that may start beside the one before them: what a CTA allocates of tensor memory it has before its first thread lets the next
-kernel begin.  Read from the sources: the other order can hang a GPU."""
+kernel begin (the other order can hang a GPU), and it reads no operand in a way a compiler may move ahead of its wait.  Both are read from
+the sources."""
 import dataclasses
 import os
 import re
@@ -31,3 +32,13 @@ def test_tensor_memory_is_allocated_before_the_next_kernel_may_begin(name, text)
         enter = re.search(r"wait_for_previous_kernel\(\)|let_next_kernel_begin\(\)", kernel)
         if alloc and enter:
             assert "__syncthreads()" in kernel[alloc.start():enter.start()]
+
+
+@pytest.mark.parametrize("name", [n for n in _build.CORE_SOURCES])
+def test_operands_are_read_after_the_wait(name):
+    with open(os.path.join(_build.CSRC, name)) as f:
+        text = f.read()
+    for kernel in re.split(r"__global__", text)[1:]:
+        body = kernel[:kernel.find("\n}\n")]
+        if "wait_for_previous_kernel()" in body:
+            assert "__ldg" not in body and "__restrict__" not in body[:body.find("{")]
