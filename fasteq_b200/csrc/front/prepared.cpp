@@ -18,21 +18,24 @@ struct Entry {
   std::string key;
   std::vector<Tensor> weights;
   Tensor value;
-  at::cuda::CUDAEvent built;
+  std::shared_ptr<at::cuda::CUDAEvent> built;
   std::set<cudaStream_t> ordered;      // streams already behind the build
 };
 
 constexpr int64_t kDefaultBudget = 256LL << 20;
+// Nothing that may take the GIL happens under it (an entry's tensors may carry Python objects, whose release does; so do hooks on
+// stream waits): a thread that holds the GIL may be waiting for it.
 std::mutex lock;
 std::list<Entry> entries;              // most recently used first
 std::unordered_map<std::string, std::list<Entry>::iterator> index_of;
 int64_t bytes = 0, budget = kDefaultBudget;
 int frozen = 0;
 
-void drop_last() {
-  bytes -= entries.back().value.nbytes();
-  index_of.erase(entries.back().key);
-  entries.pop_back();
+// moves an entry to `dropped`, which lets it go after the lock
+void drop(std::list<Entry>::iterator e, std::list<Entry>& dropped) {
+  bytes -= e->value.nbytes();
+  index_of.erase(e->key);
+  dropped.splice(dropped.end(), entries, e);
 }
 
 void append(std::string& key, int64_t v) { key.append(reinterpret_cast<const char*>(&v), sizeof v); }
@@ -49,44 +52,57 @@ std::optional<Tensor> prepared(const std::vector<Tensor>& weights, const std::st
   }
   const bool in_capture = capturing();
   {
-    std::lock_guard<std::mutex> g(lock);
+    std::unique_lock<std::mutex> g(lock);
     if (budget <= 0 || (in_capture && !frozen)) return std::nullopt;
     auto hit = index_of.find(key);
     if (hit != index_of.end()) {
       entries.splice(entries.begin(), entries, hit->second);
-      Entry& e = entries.front();
+      const Entry& e = entries.front();
+      Tensor value = e.value;
       if (!in_capture) {
-        auto cur = c10::cuda::getCurrentCUDAStream(e.value.device().index());
-        if (e.ordered.insert(cur.stream()).second) {
-          e.built.block(cur);
-          c10::cuda::CUDACachingAllocator::recordStream(e.value.storage().data_ptr(), cur);
+        const auto cur = c10::cuda::getCurrentCUDAStream(value.device().index());
+        if (!e.ordered.count(cur.stream())) {
+          const auto built = e.built;
+          g.unlock();
+          built->block(cur);
+          c10::cuda::CUDACachingAllocator::recordStream(value.storage().data_ptr(), cur);
+          g.lock();
+          hit = index_of.find(key);
+          if (hit != index_of.end() && hit->second->built == built) hit->second->ordered.insert(cur.stream());   // once the wait is issued
+          g.unlock();
         }
       }
-      return e.value;
+      return value;
     }
     if (in_capture) return std::nullopt;             // nothing persistent may be allocated inside a capture
   }
   Tensor value = build();
   if (!value.defined()) return std::nullopt;
   auto cur = c10::cuda::getCurrentCUDAStream(value.device().index());
-  Entry e;
+  std::list<Entry> fresh(1), dropped;
+  Entry& e = fresh.front();
   e.key = key; e.value = value; e.ordered.insert(cur.stream());
   for (const Tensor& w : weights) e.weights.push_back(w.detach());
-  e.built.record(cur);
-  std::lock_guard<std::mutex> g(lock);
-  auto hit = index_of.find(key);                      // another thread may have built it meanwhile
-  if (hit != index_of.end()) { bytes -= hit->second->value.nbytes(); entries.erase(hit->second); index_of.erase(hit); }
-  while (!entries.empty() && bytes + (int64_t)value.nbytes() > budget) drop_last();
-  entries.push_front(std::move(e));
-  index_of[key] = entries.begin();
-  bytes += value.nbytes();
+  e.built = std::make_shared<at::cuda::CUDAEvent>();
+  e.built->record(cur);
+  {
+    std::lock_guard<std::mutex> g(lock);
+    auto hit = index_of.find(key);                    // another thread may have built it meanwhile
+    if (hit != index_of.end()) drop(hit->second, dropped);
+    while (!entries.empty() && bytes + (int64_t)value.nbytes() > budget) drop(std::prev(entries.end()), dropped);
+    entries.splice(entries.begin(), fresh);
+    index_of[key] = entries.begin();
+    bytes += value.nbytes();
+  }
   return value;
 }
 
 void bind_prepared(py::module_& m) {
   auto clear = [] {
+    std::list<Entry> dropped;
     std::lock_guard<std::mutex> g(lock);
-    entries.clear(); index_of.clear(); bytes = 0;
+    dropped.swap(entries);
+    index_of.clear(); bytes = 0;
   };
   m.def("prepared_clear", clear);
   m.def("prepared_set_budget", [clear](std::optional<int64_t> most) {

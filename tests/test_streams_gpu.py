@@ -143,3 +143,34 @@ def test_a_partition_first_needed_under_capture_stays_with_the_capture():
         torch.cuda.synchronize()
         for a, b in zip(captured, want):
             assert (a - b).norm() <= 1e-6 * b.norm()
+
+
+def test_prepared_weights_are_evicted_beside_threads_that_hold_the_gil():
+    """A cached form that Python has seen takes the GIL when it goes, on autograd's thread too; other threads wait for the cache with the
+    GIL in hand."""
+    import threading
+    from fasteq_b200.ops import _prepared
+    from fasteq_b200.ops.dense import dense
+    _prepared.set_budget(6 * 64 * 64 * 4)                 # three weights' forms
+    done = []
+
+    def work(seed):
+        g = torch.Generator(device="cuda").manual_seed(seed)
+        x = torch.randn(40, 64, device="cuda", generator=g, requires_grad=True)
+        for _ in range(60):
+            w = torch.randn(64, 64, device="cuda", generator=g)
+            out = dense(x, w)
+            _prepared.snapshot()
+            (gx,) = torch.autograd.grad(out, x, torch.ones_like(out))     # prepares the transposed form: evicts
+        want = w.double().sum(0)
+        done.append(bool((gx.double() - want).abs().max() <= 2e-6 * want.abs().max() * 8))
+    try:
+        threads = [threading.Thread(target=work, args=(k,), daemon=True) for k in range(4)]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join(60)
+        assert done == [True] * 4
+    finally:
+        _prepared.set_budget(None)
+        _prepared.clear()
