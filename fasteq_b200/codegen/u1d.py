@@ -120,6 +120,10 @@ def untuned(spec: U1DSpec, direction: str) -> Tuning:
         # second order: two rows of every operand in a stage leave no room for the gradient tile beside a ring of any depth
         fit = (_SMEM_BUDGET // base.pipes - 256) // _stage_bytes(spec, base.ct, base.ct // base.vec // 32 * spec.y_segs * spec.elem_bytes)
         return replace(base, stages=max(2, min(4, fit)), min_blocks=1, go_smem=False, go_tmem=True)
+    if direction == "fwd" and spec.dual and smem_bytes(spec, base, "fwd") > _SMEM_BUDGET:
+        # ... and a single pipeline's default ring may be longer than an SM holds (128 channels, l <= 3 by l <= 3: 252 KB at five stages)
+        fit = (_SMEM_BUDGET // base.pipes - 256) // _stage_bytes(spec, base.ct, 0)
+        return replace(base, stages=max(2, min(base.stages, fit)))
     if direction != "bwd" or not (spec.scattered and base.vec == 2 and base.ct == 64 and 32 <= spec.out_segs <= 64):
         return base
     fit = (_SMEM_BUDGET // 8 - 256) // _stage_bytes(spec, 64, spec.y_segs * spec.elem_bytes)
@@ -129,6 +133,24 @@ def untuned(spec: U1DSpec, direction: str) -> Tuning:
 
 
 _SMEM_BUDGET = 220 * 1024
+SMEM_LIMIT = 227 * 1024        # what a CTA can have
+
+
+def smem_bytes(spec: U1DSpec, tun: Tuning, direction: str, need_gy: bool = True) -> int:
+    """Dynamic shared memory of one CTA (mirrors the layout constants of the generated source)."""
+    e = spec.elem_bytes
+    tpg = tun.ct // tun.vec
+    if direction == "fwd":
+        return tun.pipes * (256 + tun.stages * _stage_bytes(spec, tun.ct, 0))
+    warps = tun.groups * tpg // 32
+    extra = (warps * spec.y_segs * e + 15) // 16 * 16 if (need_gy and not spec.y_vec) else 0
+    go = ((spec.out_segs * tun.ct * e + 127) // 128 * 128) if tun.go_smem else 0
+    return tun.pipes * (256 + tun.stages * _stage_bytes(spec, tun.ct, extra) + go)
+
+
+def second_order_fits(spec: U1DSpec) -> bool:
+    """Whether both second-order modules of a signature fit an SM: with tangents beside them the rows of the widest do not, two stages deep."""
+    return all(smem_bytes(spec, untuned(spec, d), d) <= SMEM_LIMIT for d in ("fwd", "bwd"))
 
 
 def _stage_bytes(spec: U1DSpec, ct: int, extra: int) -> int:

@@ -22,12 +22,13 @@ using Module = c10::intrusive_ptr<U1DModule>;
 struct Signature : torch::CustomClassHolder {
   int64_t u, w_segs, x_segs, y_segs, out_segs;
   bool y_sh;
-  PyKeep load;                 // (direction, needs, tangents or None, odd address) -> (module, {name: address})
+  PyKeep load;                 // (direction, needs, tangents or None, odd address) -> (module, {name: address}), None: too wide for second-order ones
   std::mutex lock;
   std::unordered_map<int, Module> modules;
   Signature(int64_t u_, int64_t w, int64_t x, int64_t y, int64_t o, bool sh, py::object l)
       : u(u_), w_segs(w), x_segs(x), y_segs(y), out_segs(o), y_sh(sh), load(std::move(l)) {}
   int64_t y_cols() const { return y_sh ? 3 : y_segs; }
+  // null where the signature has no second-order modules
   Module module(bool backward, Flags needs, const Flags* tangents, bool odd) {
     int key = backward | odd << 1;
     for (int i = 0; i < 3; ++i) key |= needs[i] << (2 + i) | (tangents && (*tangents)[i]) << (5 + i);
@@ -40,7 +41,9 @@ struct Signature : torch::CustomClassHolder {
     auto m = c10::make_intrusive<U1DModule>();
     {
       py::gil_scoped_acquire gil;
-      py::tuple got = load.get()(backward ? "bwd" : "fwd", needs, tangents ? py::cast(*tangents) : py::none(), odd);
+      py::object loaded = load.get()(backward ? "bwd" : "fwd", needs, tangents ? py::cast(*tangents) : py::none(), odd);
+      if (loaded.is_none()) return Module();
+      py::tuple got = loaded;
       auto d = got[1].cast<std::unordered_map<std::string, uint64_t>>();
 #define F(name) m->name = reinterpret_cast<decltype(m->name)>(d.at("fasteq_u1d_" #name));
       F(forward) F(forward_split) F(backward) F(backward_split) F(tangent_forward) F(tangent_backward)
@@ -184,11 +187,13 @@ bool odd(std::initializer_list<Tensor> ts) {
   return false;
 }
 
-Tensor forward_launch(const Call& c, const Tensor& w, const Tensor& x, const Tensor& y, const Tensor* t, const Flags* has) {
+// `t`, `has`: tangents of w, x and y.  Undefined where the signature has no second-order modules.
+Tensor forward_launch(const Call& c, const Tensor& w, const Tensor& x, const Tensor& y, const Tensor* t = nullptr, const Flags* has = nullptr) {
   c10::cuda::CUDAGuard guard(x.device());
   const int64_t cols = c.sig->out_segs * c.sig->u;
   Tensor out = at::empty({c.plan->n_rows, cols}, x.options());
   const Module m = c.sig->module(false, {false, false, false}, has, odd({w, x, y, out}) || (t && odd({t[0], t[1], t[2]})));
+  if (!m) return Tensor();
   fasteq_u1d_graph g;
   Plan::Shares s;
   const int32_t* edge = graph_of(c, m, &g, &s);
@@ -201,10 +206,13 @@ Tensor forward_launch(const Call& c, const Tensor& w, const Tensor& x, const Ten
   return out;
 }
 
-variable_list backward_launch(const Call& c, const Tensor& go, const Tensor& w, const Tensor& x, const Tensor& y, Flags needs, const Tensor* t, const Flags* has) {
+// empty where the signature has no second-order modules
+variable_list backward_launch(const Call& c, const Tensor& go, const Tensor& w, const Tensor& x, const Tensor& y, Flags needs, const Tensor* t = nullptr,
+                              const Flags* has = nullptr) {
   c10::cuda::CUDAGuard guard(x.device());
   variable_list d = {needs[0] ? at::empty_like(w) : Tensor(), needs[1] ? at::empty_like(x) : Tensor(), needs[2] ? at::empty_like(y) : Tensor()};
   const Module m = c.sig->module(true, needs, has, odd({go, w, x, y, d[0], d[1], d[2]}) || (t && odd({t[0], t[1], t[2]})));
+  if (!m) return {};
   fasteq_u1d_graph g;
   Plan::Shares s;
   const int32_t* edge = graph_of(c, m, &g, &s);
@@ -216,9 +224,29 @@ variable_list backward_launch(const Call& c, const Tensor& go, const Tensor& w, 
   return d;
 }
 
+// The gradients of <go, F(w', x, y) + F(w, x', y) + F(w, x, y')> from first-order launches, an operand in its tangent's place.
+// `wants`: of go, w, x, y
+variable_list second_order_composed(const Call& c, const Tensor& go, const Tensor (&operands)[3], const Tensor (&t)[3], const bool (&wants)[4]) {
+  variable_list out(6);
+  auto add = [](Tensor& sum, const Tensor& v) { sum = sum.defined() ? sum + v : v; };
+  for (int i = 0; i < 3; ++i) {
+    if (!t[i].defined()) continue;
+    Tensor o[3] = {operands[0], operands[1], operands[2]};
+    o[i] = t[i];
+    if (wants[0]) add(out[0], forward_launch(c, o[0], o[1], o[2]));
+    for (int k = 0; k < 3; ++k) {
+      if (k == i || !wants[1 + k]) continue;
+      Flags only{};
+      only[k] = true;
+      add(out[1 + k], backward_launch(c, go, o[0], o[1], o[2], only)[k]);
+    }
+  }
+  return out;
+}
+
 struct TensorProductBackward : torch::autograd::Function<TensorProductBackward> {
   static variable_list forward(AutogradContext* ctx, const Tensor& go, const Tensor& w, const Tensor& x, const Tensor& y, const CallPtr& c, Flags needs) {
-    auto d = backward_launch(*c, go, w, x, y, needs, nullptr, nullptr);
+    auto d = backward_launch(*c, go, w, x, y, needs);
     ctx->save_for_backward({go, w, x, y});
     ctx->saved_data["c"] = capsule(c);
     ctx->saved_data["n"] = (int64_t)(needs[0] | needs[1] << 1 | needs[2] << 2);
@@ -226,7 +254,8 @@ struct TensorProductBackward : torch::autograd::Function<TensorProductBackward> 
     for (int i = 0; i < 3; ++i) if (!needs[i]) d[i] = at::empty({0}, x.options());
     return d;
   }
-  // of <go, F(w', x, y) + F(w, x', y) + F(w, x, y')>: one pass over the edges for grad_out's gradient, one for the operands'
+  // of <go, F(w', x, y) + F(w, x', y) + F(w, x, y')>: one pass over the edges for grad_out's gradient, one for the operands', where the
+  // signature has modules for that
   static variable_list backward(AutogradContext* ctx, variable_list gg) {
     const auto saved = ctx->get_saved_variables();
     const CallPtr c = uncapsule<Call>(ctx->saved_data["c"]);
@@ -240,12 +269,16 @@ struct TensorProductBackward : torch::autograd::Function<TensorProductBackward> 
     variable_list out(6);
     if (!has[0] && !has[1] && !has[2]) return out;
     const Tensor &go = saved[0], &w = saved[1], &x = saved[2], &y = saved[3];
-    if (ctx->needs_input_grad(0)) out[0] = forward_launch(*c, w, x, y, t, &has);
+    const bool wants[4] = {ctx->needs_input_grad(0), ctx->needs_input_grad(1), ctx->needs_input_grad(2), ctx->needs_input_grad(3)};
+    if (wants[0]) {
+      out[0] = forward_launch(*c, w, x, y, t, &has);
+      if (!out[0].defined()) return second_order_composed(*c, go, {w, x, y}, t, wants);
+    }
     // a gradient needs a tangent on another operand
-    const Flags needs = {ctx->needs_input_grad(1) && (has[1] || has[2]), ctx->needs_input_grad(2) && (has[0] || has[2]),
-                         ctx->needs_input_grad(3) && (has[0] || has[1])};
+    const Flags needs = {wants[1] && (has[1] || has[2]), wants[2] && (has[0] || has[2]), wants[3] && (has[0] || has[1])};
     if (needs[0] || needs[1] || needs[2]) {
       auto d = backward_launch(*c, go, w, x, y, needs, t, &has);
+      if (d.empty()) return second_order_composed(*c, go, {w, x, y}, t, wants);
       for (int i = 0; i < 3; ++i) out[1 + i] = d[i];
     }
     return out;
@@ -256,7 +289,7 @@ struct TensorProduct : torch::autograd::Function<TensorProduct> {
   static Tensor forward(AutogradContext* ctx, const Tensor& w, const Tensor& x, const Tensor& y, const CallPtr& c) {
     ctx->save_for_backward({w, x, y});
     ctx->saved_data["c"] = capsule(c);
-    return forward_launch(*c, w, x, y, nullptr, nullptr);
+    return forward_launch(*c, w, x, y);
   }
   static variable_list backward(AutogradContext* ctx, variable_list gout) {
     const auto saved = ctx->get_saved_variables();
@@ -270,7 +303,7 @@ struct TensorProduct : torch::autograd::Function<TensorProduct> {
       // not trilinear in the edge vector: the second-order kernels do not apply
       if (at::GradMode::is_enabled() && (go.requires_grad() || w.requires_grad() || x.requires_grad() || y.requires_grad()))
         throw std::runtime_error("fast_uniform1d_jit: no second-order gradient with in-kernel spherical harmonics; pass the harmonics as the y operand instead");
-      d = backward_launch(*c, go, w, x, y, needs, nullptr, nullptr);
+      d = backward_launch(*c, go, w, x, y, needs);
     } else {
       d = TensorProductBackward::apply(go, w, x, y, c, needs);
     }

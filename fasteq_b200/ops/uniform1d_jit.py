@@ -445,19 +445,20 @@ def _run_bwd(call: _Call, grad_out, w, x, y, needs):
     return gw, gx, gy
 
 
-_DUAL_SPECS: Dict[Tuple[U1DSpec, Tuple[bool, bool, bool]], U1DSpec] = {}
+_DUAL_SPECS: Dict[Tuple[U1DSpec, Tuple[bool, bool, bool]], Optional[U1DSpec]] = {}
 
 
 def _dual_spec(spec: U1DSpec, has: Tuple[bool, bool, bool]) -> Optional[U1DSpec]:
-    """The second-order signature with tangents where ``has`` says so; ``None`` for the operand forms without such modules."""
+    """The second-order signature with tangents where ``has`` says so; ``None`` for the operand forms without such modules and for rows so
+    wide that the modules would not fit an SM."""
     if not (spec.scattered and spec.x_indexed) or spec.w_shared or spec.y_vec or spec.y_indexed or spec.y_sh:
         return None
-    hit = _DUAL_SPECS.get((spec, has))
-    if hit is None:
+    if (spec, has) not in _DUAL_SPECS:
         if len(_DUAL_SPECS) > 256:
             _DUAL_SPECS.clear()
-        hit = _DUAL_SPECS[(spec, has)] = dataclasses.replace(spec, dual=has)
-    return hit
+        dual = dataclasses.replace(spec, dual=has)
+        _DUAL_SPECS[(spec, has)] = dual if _emit.second_order_fits(dual) else None
+    return _DUAL_SPECS[(spec, has)]
 
 
 def _second_order(call: _Call, go, w, x, y, tangents, wants):
@@ -591,6 +592,8 @@ def _signature(meta, dtype):
 
         def load(direction, needs, tangents, odd):
             sp = spec if tangents is None else _dual_spec(spec, tuple(tangents))
+            if sp is None:
+                return None
             mod = get_module(sp, direction, tuple(needs), tuning=_tuning_at(sp, direction, odd, tuple(needs)))
             return mod, _front.addresses(mod.lib, _EXPORTS)
         made = (_front.lib().Signature(u, *segs, bool(y_sh), load), segs[1] * u)

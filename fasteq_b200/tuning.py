@@ -75,16 +75,7 @@ def _lookup(spec: U1DSpec, direction: str, needs) -> Optional[_emit.Tuning]:
     return None
 
 
-def smem_bytes(spec: U1DSpec, tun: _emit.Tuning, direction: str, need_gy: bool = True) -> int:
-    """Dynamic shared memory of one CTA (mirrors the layout constants of the generated source)."""
-    e = spec.elem_bytes
-    tpg = tun.ct // tun.vec
-    if direction == "fwd":
-        return tun.pipes * (256 + tun.stages * _emit._stage_bytes(spec, tun.ct, 0))
-    warps = tun.groups * tpg // 32
-    extra = (warps * spec.y_segs * e + 15) // 16 * 16 if (need_gy and not spec.y_vec) else 0
-    go = ((spec.out_segs * tun.ct * e + 127) // 128 * 128) if tun.go_smem else 0
-    return tun.pipes * (256 + tun.stages * _emit._stage_bytes(spec, tun.ct, extra) + go)
+smem_bytes = _emit.smem_bytes
 
 
 def candidates(spec: U1DSpec, direction: str, needs=(True, True, True)) -> List[_emit.Tuning]:

@@ -128,3 +128,27 @@ def test_sweep_times_what_a_missing_entry_runs_with(in1, lmax, direction):
     from fasteq_b200.prebuild import cwtp_spec
     spec = cwtp_spec(in1, lmax, lmax, "f32")
     assert gen.untuned(spec, direction) in tuning.candidates(spec, direction, (direction == "bwd",) * 3)
+
+
+@pytest.mark.parametrize("in1", ["{0}x0e+{0}x1o", "{0}x0e+{0}x1o+{0}x2e", "{0}x0e+{0}x1o+{0}x2e+{0}x3o", "{0}x0e+{0}x0o+{0}x1o+{0}x1e+{0}x2e+{0}x2o"])
+@pytest.mark.parametrize("u,dtype", [(33, "f32"), (64, "f32"), (96, "f32"), (128, "f32"), (256, "f32"), (64, "f64"), (128, "f64")])
+def test_second_order_modules_fit_one_sm(in1, u, dtype):
+    """Tangents double a stage: every subset of them has a configuration an SM can hold, or is composed of first-order launches."""
+    import itertools
+    from fasteq_b200.ops import uniform1d_jit as u1d
+    for lmax in (2, 3, 4):
+        spec = cwtp_spec(in1.format(u), lmax, 3, dtype)
+        for has in itertools.product([False, True], repeat=3):
+            dual = u1d._dual_spec(spec, has) if any(has) else None
+            if dual is None:
+                continue
+            for odd in (False, True):
+                fwd, bwd = (u1d._tuning_at(dual, d, odd, (True,) * 3) for d in ("fwd", "bwd"))
+                assert fwd.stages >= 2 and tuning.smem_bytes(dual, fwd, "fwd") <= 227 * 1024
+                assert bwd.stages >= 2 and tuning.smem_bytes(dual, bwd, "bwd") <= 227 * 1024
+
+
+def test_rows_too_wide_for_second_order_modules():
+    from fasteq_b200.ops import uniform1d_jit as u1d
+    widest = cwtp_spec("+".join(f"128x{l}{p}" for l in range(4) for p in "eo"), 4, 4, "f64")
+    assert u1d._dual_spec(widest, (True, True, True)) is None

@@ -9,9 +9,10 @@ from fasteq_b200.irreps import Irreps
 
 pytestmark = pytest.mark.gpu
 # 128 channels: packed, gradient row in tensor memory; 33: channel tail, element copies; 64 in FP64: one channel per thread; 55
-# output segments of 64 channels: one-warp pipelines
+# output segments of 64 channels: one-warp pipelines; l = 3 senders: the ring of one pipeline shortened to what an SM holds
 SIGNATURES = [("128x0e+128x1o", 3, "natural", torch.float32), ("128x0e", 3, "natural", torch.float32), ("33x0e+33x1o", 2, None, torch.float32),
-              ("64x0e+64x1o", 2, None, torch.float64), ("64x0e+64x1o", 3, None, torch.float32)]
+              ("64x0e+64x1o", 2, None, torch.float64), ("64x0e+64x1o", 3, None, torch.float32),
+              ("128x0e+128x1o+128x2e+128x3o", 3, None, torch.float32)]
 
 
 def _case(sig, n, e, ordered, shift=0):
