@@ -461,37 +461,11 @@ def _dual_spec(spec: U1DSpec, has: Tuple[bool, bool, bool]) -> Optional[U1DSpec]
     return _DUAL_SPECS[(spec, has)]
 
 
-def _second_order(call: _Call, go, w, x, y, tangents, wants):
-    """``(d_go, d_w, d_x, d_y)`` of ``<go, F(w', x, y) + F(w, x', y) + F(w, x, y')>``, ``tangents = (w', x', y')`` with ``None`` for those that
-    are zero: one pass over the edges for the first and one for the others."""
-    has = tuple(t is not None for t in tangents)
-    spec = _dual_spec(call.spec, has)
-    if spec is None:
-        return _second_order_composed(call, go, w, x, y, tangents, wants)
-    dev, ptr = x.device, lambda t: t.data_ptr() if t is not None else None
-    operands = tuple(ptr(t) for t in (w, x, y) + tangents)
-    out = [None] * 4
-    with _cabi.on_device(dev):
-        stream = _cabi.stream(dev)
-        if wants[0]:
-            out[0] = torch.empty((call.n_out_rows, call.out_segs * call.u), dtype=x.dtype, device=dev)
-            mod = get_module(spec, "fwd", tuning=_tuning_for(spec, "fwd", (w, x, y, out[0]) + tangents))
-            g, part_edge = call.graph(mod, dev)
-            carry = torch.empty((g.n_parts, call.out_segs * call.u), dtype=x.dtype, device=dev) if part_edge is not None else None
-            mod.tangent_forward(g, part_edge, ptr(carry), *operands, out[0].data_ptr(), stream)
-        # a gradient needs a tangent on another operand
-        needs = tuple(wants[1 + i] and any(has[j] for j in range(3) if j != i) for i in range(3))
-        if any(needs):
-            out[1:] = [torch.empty_like(t) if n else None for t, n in zip((w, x, y), needs)]
-            mod = get_module(spec, "bwd", needs, tuning=_tuning_for(spec, "bwd", (go, w, x, y, *out[1:]) + tangents, needs))
-            g, part_edge = call.graph(mod, dev)
-            mod.tangent_backward(g, part_edge, go.data_ptr(), *operands, *(ptr(t) for t in out[1:]), stream)
-    return tuple(out)
-
-
 def _second_order_composed(call: _Call, go, w, x, y, tangents, wants):
-    """The same from first-order launches.  The operator is trilinear in (w, x, y), so every term is a forward or a one-gradient backward of
-    the same signature with an operand swapped for its tangent:
+    """``(d_go, d_w, d_x, d_y)`` of ``<go, F(w', x, y) + F(w, x', y) + F(w, x, y')>``, ``tangents = (w', x', y')`` with ``None`` for those that
+    are zero, from first-order launches.  The operator is trilinear in (w, x, y), so every term is a forward or a one-gradient backward of
+    the same signature with an operand swapped for its tangent (the usual operand form has modules of its own for this, see
+    ``csrc/front/u1d.cpp``):
 
         d_go = F(w', x, y) + F(w, x', y) + F(w, x, y')
         d_w  = Bw(go; x', y) + Bw(go; x, y')      (Bw = gradient with respect to the weight slot)
@@ -516,7 +490,7 @@ def _second_order_composed(call: _Call, go, w, x, y, tangents, wants):
 
 class FastUniform1dBackwardFunction(torch.autograd.Function):
     """First backward as a differentiable function (reference: fasteq/ops/uniform1d_jit.py:3098-3188),
-    so that force losses can be trained; its own backward is ``_second_order``."""
+    so that force losses can be trained."""
 
     @staticmethod
     def forward(ctx, grad_out, w, x, y, call, needs):
@@ -534,7 +508,7 @@ class FastUniform1dBackwardFunction(torch.autograd.Function):
         if all(t is None for t in tangents):
             return (None,) * 6
         wants = tuple(asked(ctx, i) for i in range(4))
-        return _second_order(ctx.call, go, w, x, y, tangents, wants) + (None, None)
+        return _second_order_composed(ctx.call, go, w, x, y, tangents, wants) + (None, None)
 
 
 class FastUniform1dJITFunction(torch.autograd.Function):
