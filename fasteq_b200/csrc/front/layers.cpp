@@ -283,6 +283,19 @@ std::optional<Tensor> chain_prepared(const std::vector<Tensor>& ws, bool backwar
   });
 }
 
+// The chain's gradient as differentiable operations, layer by layer: what enters it (the gradient of the chain's value) and the basis may be
+// differentiated through in their turn, as where a loss on forces trains other layers behind frozen radial ones.
+Tensor chain_gradient(const Tensor& go, const Tensor& basis, const std::vector<Tensor>& ws) {
+  variable_list z;
+  Tensor h = basis, g = go;
+  for (const Tensor& w : ws) {
+    z.push_back(Dense::apply(h, w));
+    if (z.size() < ws.size()) h = SiLU::apply(z.back());
+  }
+  for (size_t l = ws.size(); l-- > 0;) g = Dense::apply(SiLUBackward::apply(g, z[l]), ws[l].t());
+  return g;
+}
+
 struct RadialChain : torch::autograd::Function<RadialChain> {
   static bool takes(const Tensor& basis, const std::vector<Tensor>& ws) {
     if (!basis.is_cuda() || basis.scalar_type() != at::kFloat || basis.dim() != 2 || basis.size(0) == 0) return false;
@@ -322,6 +335,10 @@ struct RadialChain : torch::autograd::Function<RadialChain> {
     const Tensor& basis = saved[0];
     c10::cuda::CUDAGuard guard(basis.device());
     const Tensor g = go[0].contiguous();
+    if (at::GradMode::is_enabled()) {
+      grads[0] = chain_gradient(g, basis, ws);
+      return grads;
+    }
     std::vector<const float*> hidden;
     for (size_t i = 1; i < ws.size(); ++i) hidden.push_back(ws[i].const_data_ptr<float>());
     hidden.push_back(nullptr);

@@ -71,3 +71,26 @@ def test_radial_mlp_module_uses_the_same_values_as_the_layered_path():
     xd = x.cpu().double().requires_grad_(True)
     (g2,) = torch.autograd.grad((_ref(xd, ws[:-1]) @ ws[-1].t()).sum(), xd)
     assert _rel(g1.cpu(), g2) <= 2e-5
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n_hidden,nb", [(3, 8), (2, 5), (1, 16)])
+def test_differentiable_backward(n_hidden, nb):
+    """Fine-tuning behind frozen radial layers: the loss on forces is differentiated through the chain's basis gradient, with respect to
+    the gradient that enters it and to the basis."""
+    from fasteq_b200.ops.radial_chain import radial_chain
+    g = torch.Generator().manual_seed(n_hidden)
+    dims = [nb] + [64] * n_hidden
+    ws = [torch.randn(o, i, generator=g) / i ** 0.5 for i, o in zip(dims[:-1], dims[1:])]
+    basis, r, t = torch.randn(301, nb, generator=g), torch.randn(301, 64, generator=g), torch.randn(301, nb, generator=g)
+
+    def second(f, basis, r, t):
+        basis, r = basis.requires_grad_(True), r.requires_grad_(True)
+        (gb,) = torch.autograd.grad(f(basis), basis, r, create_graph=True)
+        return [gb.detach()] + list(torch.autograd.grad((gb * t).sum() + (gb ** 2).sum(), (basis, r)))
+
+    want = second(lambda b: _ref(b, ws), basis.double(), r.double(), t.double())
+    cw = [w.cuda() for w in ws]
+    got = second(lambda b: radial_chain(b, cw), basis.cuda(), r.cuda(), t.cuda())
+    for a, b in zip(got, want):
+        assert _rel(a.cpu(), b) <= 2e-5       # the chain's 1e-5, forwards and backwards
