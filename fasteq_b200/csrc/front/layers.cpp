@@ -94,26 +94,7 @@ struct EqLinearBackward : torch::autograd::Function<EqLinearBackward> {
     Tensor dx = need_x ? eqlinear_apply(*g, precision, w, go, true, true).view(x.sizes()) : at::empty({0}, x.options());
     return {dw, dx};
   }
-  static variable_list backward(AutogradContext* ctx, variable_list gg) {
-    const auto saved = ctx->get_saved_variables();
-    const Tensor &go = saved[0], &w = saved[1], &x = saved[2];
-    const Geom g = uncapsule<Geometry>(ctx->saved_data["g"]);
-    const int64_t precision = ctx->saved_data["p"].toInt();
-    const Tensor ggw = ctx->saved_data["w"].toBool() ? defined_contiguous(gg[0]) : Tensor();
-    const Tensor ggx = ctx->saved_data["x"].toBool() ? defined_contiguous(gg[1]) : Tensor();
-    Tensor d_go, d_w, d_x;
-    if (ctx->needs_input_grad(0)) {
-      if (ggx.defined()) d_go = eqlinear_apply(*g, precision, w, ggx, false, true);
-      if (ggw.defined()) {
-        const Tensor t = eqlinear_apply(*g, precision, ggw, x, false, false);
-        d_go = d_go.defined() ? d_go + t : t;
-      }
-      if (d_go.defined()) d_go = d_go.view(go.sizes());
-    }
-    if (ctx->needs_input_grad(1) && ggx.defined()) d_w = eqlinear_wgrad(*g, precision, w, ggx, go);
-    if (ctx->needs_input_grad(2) && ggw.defined()) d_x = eqlinear_apply(*g, precision, ggw, go, true, false).view(x.sizes());
-    return {d_go, d_w, d_x, Tensor(), Tensor(), Tensor(), Tensor()};
-  }
+  static variable_list backward(AutogradContext* ctx, variable_list gg);
 };
 
 struct EqLinear : torch::autograd::Function<EqLinear> {
@@ -132,6 +113,34 @@ struct EqLinear : torch::autograd::Function<EqLinear> {
     return {need_w ? d[0] : Tensor(), need_x ? d[1] : Tensor(), Tensor(), Tensor()};
   }
 };
+
+// in grad mode (a third order may follow) from the nodes, else from launches
+variable_list EqLinearBackward::backward(AutogradContext* ctx, variable_list gg) {
+  const auto saved = ctx->get_saved_variables();
+  const Tensor &go = saved[0], &w = saved[1], &x = saved[2];
+  const Geom g = uncapsule<Geometry>(ctx->saved_data["g"]);
+  const int64_t precision = ctx->saved_data["p"].toInt();
+  const Tensor ggw = ctx->saved_data["w"].toBool() ? defined_contiguous(gg[0]) : Tensor();
+  const Tensor ggx = ctx->saved_data["x"].toBool() ? defined_contiguous(gg[1]) : Tensor();
+  const bool want_go = ctx->needs_input_grad(0), want_w = ctx->needs_input_grad(1), want_x = ctx->needs_input_grad(2);
+  const bool nodes = at::GradMode::is_enabled();
+  auto forward = [&](const Tensor& b, const Tensor& a, bool weight) {
+    return nodes ? Tensor(EqLinear::apply(b, a, g, precision)) : eqlinear_apply(*g, precision, b, a, false, weight);
+  };
+  Tensor d_go, d_w, d_x;
+  if (want_go) {
+    if (ggx.defined()) d_go = forward(w, ggx, true);
+    if (ggw.defined()) {
+      const Tensor t = forward(ggw, x, false);
+      d_go = d_go.defined() ? d_go + t : t;
+    }
+    if (d_go.defined()) d_go = d_go.view(go.sizes());
+  }
+  if (want_w && ggx.defined()) d_w = nodes ? EqLinearBackward::apply(go, w, ggx, g, precision, true, false)[0] : eqlinear_wgrad(*g, precision, w, ggx, go);
+  if (want_x && ggw.defined())
+    d_x = nodes ? EqLinearBackward::apply(go, ggw, x, g, precision, false, true)[1] : eqlinear_apply(*g, precision, ggw, go, true, false).view(x.sizes());
+  return {d_go, d_w, d_x, Tensor(), Tensor(), Tensor(), Tensor()};
+}
 
 Tensor eqlinear(const Geom& g, const Tensor& w, const Tensor& x, int64_t precision) {
   if (!x.is_cuda() || !w.is_cuda()) throw Failure("eqlinear: x and w must be CUDA tensors: fasteq_b200 has no CPU path");
@@ -199,24 +208,7 @@ struct DenseBackward : torch::autograd::Function<DenseBackward> {
     ctx->set_materialize_grads(false);
     return {need_x ? gemm(g, weight.t(), weight, true) : at::empty({0}, x.options()), need_w ? row_product(g, x) : at::empty({0}, weight.options())};
   }
-  // d_g = ggx W^T + x ggW^T,  d_x = g ggW,  d_W = g^T ggx
-  static variable_list backward(AutogradContext* ctx, variable_list gg) {
-    const auto saved = ctx->get_saved_variables();
-    const Tensor &g = saved[0], &x = saved[1], &weight = saved[2];
-    const Tensor ggx = ctx->saved_data["x"].toBool() ? defined_contiguous(gg[0]) : Tensor();
-    const Tensor ggw = ctx->saved_data["w"].toBool() ? defined_contiguous(gg[1]) : Tensor();
-    Tensor d_g, d_x, d_w;
-    if (ctx->needs_input_grad(0)) {
-      if (ggx.defined()) d_g = gemm(ggx, weight, weight, false);
-      if (ggw.defined()) {
-        const Tensor t = gemm(x, ggw, Tensor(), false);
-        d_g = d_g.defined() ? d_g + t : t;
-      }
-    }
-    if (ctx->needs_input_grad(1) && ggw.defined()) d_x = gemm(g, ggw.t(), Tensor(), false);
-    if (ctx->needs_input_grad(2) && ggx.defined()) d_w = row_product(g, ggx);
-    return {d_g, d_x, d_w, Tensor(), Tensor()};
-  }
+  static variable_list backward(AutogradContext* ctx, variable_list gg);
 };
 
 struct Dense : torch::autograd::Function<Dense> {
@@ -232,6 +224,27 @@ struct Dense : torch::autograd::Function<Dense> {
     return {need_x ? d[0] : Tensor(), need_w ? d[1] : Tensor()};
   }
 };
+
+// d_g = ggx W^T + x ggW^T,  d_x = g ggW,  d_W = g^T ggx: in grad mode (a third order may follow) from the nodes, else from launches
+variable_list DenseBackward::backward(AutogradContext* ctx, variable_list gg) {
+  const auto saved = ctx->get_saved_variables();
+  const Tensor &g = saved[0], &x = saved[1], &weight = saved[2];
+  const Tensor ggx = ctx->saved_data["x"].toBool() ? defined_contiguous(gg[0]) : Tensor();
+  const Tensor ggw = ctx->saved_data["w"].toBool() ? defined_contiguous(gg[1]) : Tensor();
+  const bool nodes = at::GradMode::is_enabled();
+  auto product = [&](const Tensor& a, const Tensor& bt, const Tensor& w) { return nodes ? Tensor(Dense::apply(a, bt)) : gemm(a, bt, w, false); };
+  Tensor d_g, d_x, d_w;
+  if (ctx->needs_input_grad(0)) {
+    if (ggx.defined()) d_g = product(ggx, weight, weight);
+    if (ggw.defined()) {
+      const Tensor t = product(x, ggw, Tensor());
+      d_g = d_g.defined() ? d_g + t : t;
+    }
+  }
+  if (ctx->needs_input_grad(1) && ggw.defined()) d_x = product(g, ggw.t(), Tensor());
+  if (ctx->needs_input_grad(2) && ggx.defined()) d_w = nodes ? DenseBackward::apply(g, ggx, weight, false, true)[1] : row_product(g, ggx);
+  return {d_g, d_x, d_w, Tensor(), Tensor()};
+}
 
 // ------------------------------------------------------------------------------------------------ SiLU
 variable_list silu_run(int order, const Tensor& z, const Tensor& g, const Tensor& h) {

@@ -224,26 +224,6 @@ variable_list backward_launch(const Call& c, const Tensor& go, const Tensor& w, 
   return d;
 }
 
-// The gradients of <go, F(w', x, y) + F(w, x', y) + F(w, x, y')> from first-order launches, an operand in its tangent's place.
-// `wants`: of go, w, x, y
-variable_list second_order_composed(const Call& c, const Tensor& go, const Tensor (&operands)[3], const Tensor (&t)[3], const bool (&wants)[4]) {
-  variable_list out(6);
-  auto add = [](Tensor& sum, const Tensor& v) { sum = sum.defined() ? sum + v : v; };
-  for (int i = 0; i < 3; ++i) {
-    if (!t[i].defined()) continue;
-    Tensor o[3] = {operands[0], operands[1], operands[2]};
-    o[i] = t[i];
-    if (wants[0]) add(out[0], forward_launch(c, o[0], o[1], o[2]));
-    for (int k = 0; k < 3; ++k) {
-      if (k == i || !wants[1 + k]) continue;
-      Flags only{};
-      only[k] = true;
-      add(out[1 + k], backward_launch(c, go, o[0], o[1], o[2], only)[k]);
-    }
-  }
-  return out;
-}
-
 struct TensorProductBackward : torch::autograd::Function<TensorProductBackward> {
   static variable_list forward(AutogradContext* ctx, const Tensor& go, const Tensor& w, const Tensor& x, const Tensor& y, const CallPtr& c, Flags needs) {
     auto d = backward_launch(*c, go, w, x, y, needs);
@@ -254,35 +234,7 @@ struct TensorProductBackward : torch::autograd::Function<TensorProductBackward> 
     for (int i = 0; i < 3; ++i) if (!needs[i]) d[i] = at::empty({0}, x.options());
     return d;
   }
-  // of <go, F(w', x, y) + F(w, x', y) + F(w, x, y')>: one pass over the edges for grad_out's gradient, one for the operands', where the
-  // signature has modules for that
-  static variable_list backward(AutogradContext* ctx, variable_list gg) {
-    const auto saved = ctx->get_saved_variables();
-    const CallPtr c = uncapsule<Call>(ctx->saved_data["c"]);
-    const int64_t needed = ctx->saved_data["n"].toInt();
-    Tensor t[3];
-    Flags has{};
-    for (int i = 0; i < 3; ++i) {
-      if ((needed >> i & 1) && gg[i].defined()) t[i] = gg[i].contiguous();
-      has[i] = t[i].defined();
-    }
-    variable_list out(6);
-    if (!has[0] && !has[1] && !has[2]) return out;
-    const Tensor &go = saved[0], &w = saved[1], &x = saved[2], &y = saved[3];
-    const bool wants[4] = {ctx->needs_input_grad(0), ctx->needs_input_grad(1), ctx->needs_input_grad(2), ctx->needs_input_grad(3)};
-    if (wants[0]) {
-      out[0] = forward_launch(*c, w, x, y, t, &has);
-      if (!out[0].defined()) return second_order_composed(*c, go, {w, x, y}, t, wants);
-    }
-    // a gradient needs a tangent on another operand
-    const Flags needs = {wants[1] && (has[1] || has[2]), wants[2] && (has[0] || has[2]), wants[3] && (has[0] || has[1])};
-    if (needs[0] || needs[1] || needs[2]) {
-      auto d = backward_launch(*c, go, w, x, y, needs, t, &has);
-      if (d.empty()) return second_order_composed(*c, go, {w, x, y}, t, wants);
-      for (int i = 0; i < 3; ++i) out[1 + i] = d[i];
-    }
-    return out;
-  }
+  static variable_list backward(AutogradContext* ctx, variable_list gg);
 };
 
 struct TensorProduct : torch::autograd::Function<TensorProduct> {
@@ -312,6 +264,57 @@ struct TensorProduct : torch::autograd::Function<TensorProduct> {
     return d;
   }
 };
+
+// The gradients of <go, F(w', x, y) + F(w, x', y) + F(w, x, y')> from first-order nodes, an operand in its tangent's place.
+// `wants`: of go, w, x, y
+variable_list second_order_composed(const CallPtr& c, const Tensor& go, const Tensor (&operands)[3], const Tensor (&t)[3], const bool (&wants)[4]) {
+  variable_list out(6);
+  auto add = [](Tensor& sum, const Tensor& v) { sum = sum.defined() ? sum + v : v; };
+  for (int i = 0; i < 3; ++i) {
+    if (!t[i].defined()) continue;
+    Tensor o[3] = {operands[0], operands[1], operands[2]};
+    o[i] = t[i];
+    if (wants[0]) add(out[0], TensorProduct::apply(o[0], o[1], o[2], c));
+    for (int k = 0; k < 3; ++k) {
+      if (k == i || !wants[1 + k]) continue;
+      Flags only{};
+      only[k] = true;
+      add(out[1 + k], TensorProductBackward::apply(go, o[0], o[1], o[2], c, only)[k]);
+    }
+  }
+  return out;
+}
+
+// of <go, F(w', x, y) + F(w, x', y) + F(w, x, y')>: one pass over the edges for grad_out's gradient, one for the operands', where the
+// signature has modules for that and no third order may follow (grad mode)
+variable_list TensorProductBackward::backward(AutogradContext* ctx, variable_list gg) {
+  const auto saved = ctx->get_saved_variables();
+  const CallPtr c = uncapsule<Call>(ctx->saved_data["c"]);
+  const int64_t needed = ctx->saved_data["n"].toInt();
+  Tensor t[3];
+  Flags has{};
+  for (int i = 0; i < 3; ++i) {
+    if ((needed >> i & 1) && gg[i].defined()) t[i] = gg[i].contiguous();
+    has[i] = t[i].defined();
+  }
+  variable_list out(6);
+  if (!has[0] && !has[1] && !has[2]) return out;
+  const Tensor &go = saved[0], &w = saved[1], &x = saved[2], &y = saved[3];
+  const bool wants[4] = {ctx->needs_input_grad(0), ctx->needs_input_grad(1), ctx->needs_input_grad(2), ctx->needs_input_grad(3)};
+  if (at::GradMode::is_enabled()) return second_order_composed(c, go, {w, x, y}, t, wants);
+  if (wants[0]) {
+    out[0] = forward_launch(*c, w, x, y, t, &has);
+    if (!out[0].defined()) return second_order_composed(c, go, {w, x, y}, t, wants);
+  }
+  // a gradient needs a tangent on another operand
+  const Flags needs = {wants[1] && (has[1] || has[2]), wants[2] && (has[0] || has[2]), wants[3] && (has[0] || has[1])};
+  if (needs[0] || needs[1] || needs[2]) {
+    auto d = backward_launch(*c, go, w, x, y, needs, t, &has);
+    if (d.empty()) return second_order_composed(c, go, {w, x, y}, t, wants);
+    for (int i = 0; i < 3; ++i) out[1 + i] = d[i];
+  }
+  return out;
+}
 
 }  // namespace
 

@@ -463,7 +463,7 @@ def _dual_spec(spec: U1DSpec, has: Tuple[bool, bool, bool]) -> Optional[U1DSpec]
 
 def _second_order_composed(call: _Call, go, w, x, y, tangents, wants):
     """``(d_go, d_w, d_x, d_y)`` of ``<go, F(w', x, y) + F(w, x', y) + F(w, x, y')>``, ``tangents = (w', x', y')`` with ``None`` for those that
-    are zero, from first-order launches.  The operator is trilinear in (w, x, y), so every term is a forward or a one-gradient backward of
+    are zero, from the first-order functions, so that autograd may go on differentiating.  The operator is trilinear in (w, x, y), so every term is a forward or a one-gradient backward of
     the same signature with an operand swapped for its tangent (the usual operand form has modules of its own for this, see
     ``csrc/front/u1d.cpp``):
 
@@ -481,8 +481,9 @@ def _second_order_composed(call: _Call, go, w, x, y, tangents, wants):
     for i, t in enumerate(tangents):
         if t is None:
             continue
-        terms = [(0, _run_fwd(call, *swapped(i)))] if wants[0] else []
-        terms += [(1 + k, _run_bwd(call, go, *swapped(i), tuple(n == k for n in range(3)))[k]) for k in range(3) if k != i and wants[1 + k]]
+        terms = [(0, FastUniform1dJITFunction.apply(*swapped(i), None, None, call))] if wants[0] else []
+        terms += [(1 + k, FastUniform1dBackwardFunction.apply(go, *swapped(i), call, tuple(n == k for n in range(3)))[k])
+                  for k in range(3) if k != i and wants[1 + k]]
         for k, v in terms:
             out[k] = v if out[k] is None else out[k] + v
     return tuple(out)
@@ -513,12 +514,12 @@ class FastUniform1dBackwardFunction(torch.autograd.Function):
 
 class FastUniform1dJITFunction(torch.autograd.Function):
     """Autograd wrapper (reference: fasteq/ops/uniform1d_jit.py:3194-3326).  The backward produces
-    exactly the gradients autograd asks for and is itself differentiable."""
+    exactly the gradients autograd asks for and is itself differentiable.  ``meta`` may be the resolved call."""
 
     @staticmethod
     def forward(ctx, w, x, y, input_indices, output_indices, meta):
         _validate(w, x, y)
-        call = _Call(w, x, y, input_indices, output_indices, meta)
+        call = meta if isinstance(meta, _Call) else _Call(w, x, y, input_indices, output_indices, meta)
         ctx.call = call
         ctx.save_for_backward(w, x, y)
         return _run_fwd(call, w, x, y)
