@@ -693,7 +693,7 @@ __global__ void __launch_bounds__(wg::THREADS, 1) eqlinear_wgrad_tc_kernel(const
   uint64_t* acc_full = empty + STAGES;                                        // [2]
   uint64_t* acc_empty = acc_full + 2;                                         // [2]
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
-  int* redo = reinterpret_cast<int*>(tmem_slot + 1);                          // [2]: a sum is not finite; the largest |sum|'s bits
+  int* redo = reinterpret_cast<int*>(tmem_slot + 1);                          // a sum is not finite
 
   int split, tile;
   decode_cta(tab, num_paths, &split, &tile);
@@ -709,7 +709,7 @@ __global__ void __launch_bounds__(wg::THREADS, 1) eqlinear_wgrad_tc_kernel(const
     for (int s = 0; s < STAGES; ++s) { mbar_init(&full[s], 8); mbar_init(&empty[s], 1); }
     for (int b = 0; b < 2; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 8); }
     mbar_fence_init();
-    redo[0] = 0; redo[1] = 0;
+    *redo = 0;
   }
   if (warp == 16) tmem_alloc(tmem_slot, 512);
   tc_fence_before();
@@ -832,7 +832,6 @@ __global__ void __launch_bounds__(wg::THREADS, 1) eqlinear_wgrad_tc_kernel(const
     }
     const int m = m0 + quarter * 32 + lane, nb = n0 + half * HALF;
     const size_t sm = swap ? 1 : (size_t)v, sn = swap ? (size_t)v : 1;
-    float top = 0.f;
     bool bad = false;
     if (m < M) {
 #pragma unroll
@@ -841,8 +840,7 @@ __global__ void __launch_bounds__(wg::THREADS, 1) eqlinear_wgrad_tc_kernel(const
         float o[4];
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-          o[k] = outer[(j + k) * 256 + t];
-          top = fmaxf(top, fabsf(o[k]));
+          o[k] = outer[(j + k) * 256 + t] * UNSCALE;
           bad = bad || !(fabsf(o[k]) <= 3.402823466e38f);
         }
         if (!swap) {
@@ -853,14 +851,12 @@ __global__ void __launch_bounds__(wg::THREADS, 1) eqlinear_wgrad_tc_kernel(const
         }
       }
     }
-    if (bad) atomicOr(&redo[0], 1);
-    atomicMax(&redo[1], __float_as_int(top));
+    if (bad) atomicOr(redo, 1);
   }
   tc_fence_before();
   __syncthreads();
   if (warp == 16) { tc_fence_after(); tmem_dealloc(tmem, 512); }
-  const float largest = __int_as_float(redo[1]);
-  if (redo[0] == 0 && !(largest > 0.f && largest < 1e-20f)) return;
+  if (*redo == 0) return;
   const float* Xq = X + (size_t)tab.in_row[q] * u;
   const float* Gq = G + (size_t)tab.out_row[q] * v;
   for (int e = threadIdx.x; e < TM * TN; e += THREADS) {

@@ -19,8 +19,9 @@
 // 12,288 nodes 365 -> 117 us, at 512 nodes 28 -> 22; [80000, 64]^T [80000, 1280] 309 -> 149; [80000, 128]^T [80000, 128] 65 -> 31; at
 // 200 rows 18.6 -> 14.4.  Errors against FP64 (2-norm) 2.26e-7 -> 1.24e-7, 2.11e-7 -> 1.35e-7, 1.66e-7 -> 1.42e-7, 1.12e-7 -> 0.74e-7.
 // About 13 us are the launch, the first chunk's way through the roles and the reduction.
-// Non-finite sums (an infinite or NaN operand, or one above bf16's largest value) and tiles of sums below 1e-20 (parts below
-// bf16's range) are recomputed by the CTA in FP32.
+// Range: a third part reaches 24 bits below its operand, and bf16's smallest numbers are 2^-133.  Operands are therefore split 2^24 times as
+// large, which holds every FP32 number in three parts and keeps every product's parts above FP32's smallest; the stored sums are scaled
+// back.  Sums that are not finite then (an infinite or NaN operand, one above 2^104, sums above 2^80) the CTA recomputes in FP32.
 #pragma once
 #include "tcgen05_util.cuh"
 
@@ -28,6 +29,7 @@ namespace fasteq {
 namespace wg {
 
 constexpr int TM = 128, ROWS = 32, RAW = 3, STAGES = 2, THREADS = 18 * 32, OUTER = 16;
+constexpr float SCALE = 16777216.f, UNSCALE = 1.f / (SCALE * SCALE);
 constexpr int A_COLS = 3 * ROWS / 2;                       // TMEM columns of one M-operand stage: three parts, two rows per column
 __host__ __device__ constexpr int b_part(int tn) { return tn * ROWS * 2; }
 __host__ __device__ constexpr int smem_bytes(int tn) { return 1024 + STAGES * 3 * b_part(tn) + RAW * ROWS * (TM + tn) * 4 + TM * tn * 4 + 256; }
@@ -58,6 +60,7 @@ __device__ __forceinline__ uint32_t bf16_pair(float lo, float hi) {
 }
 __device__ __forceinline__ void split_pair(float2 v, uint32_t& p1, uint32_t& p2, uint32_t& p3) {
   const float2 minus = make_float2(-1.f, -1.f);
+  v = vmul(v, make_float2(SCALE, SCALE));
   p1 = bf16_pair(v.x, v.y);
   v = vfma(make_float2(__uint_as_float(p1 << 16), __uint_as_float(p1 & 0xffff0000u)), minus, v);
   p2 = bf16_pair(v.x, v.y);

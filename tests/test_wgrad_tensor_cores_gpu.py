@@ -68,6 +68,36 @@ def test_small_and_large_operands(scale):
     assert (_grad(g, x).double() - want).norm() <= 3e-7 * want.norm() + (2.0 ** -149 * 700 * 64 if scale < 1e-18 else 0.0)
 
 
+@pytest.mark.parametrize("tiny", [1e-30, 1e-33, 1e-35, 1e-37, 1e-40])
+@pytest.mark.parametrize("side", [0, 1])
+def test_tiny_operands_against_large_ones(tiny, side):
+    """An operand whose third bf16 part is below bf16's numbers, times one that brings the sums back to ordinary size."""
+    ops = _operands(700, 64, 132)
+    ops[side], ops[1 - side] = ops[side] * tiny, ops[1 - side] * 1e30
+    g, x = ops
+    want = g.double().t() @ x.double()
+    assert (_grad(g, x).double() - want).norm() <= 3e-7 * want.norm()
+
+
+def test_a_tiny_channel_beside_ordinary_ones():
+    """One channel of one operand is tiny, and so small that its sums vanish beside the tile's others."""
+    g, x = _operands(700, 64, 132)
+    x[:, 5] *= 1e-34
+    want = g.double().t() @ x.double()
+    got = _grad(g, x).double()
+    for cols in (slice(5, 6), slice(0, 5), slice(6, None)):
+        assert (got[:, cols] - want[:, cols]).norm() <= 3e-7 * want[:, cols].norm()
+
+
+@pytest.mark.parametrize("m", [160, 5000, 100_003])
+def test_operands_of_one_sign(m):
+    """The tensor core truncates, always towards zero here, and no cancellation hides it: per chunk two truncated steps of at most 2^-23,
+    half of that on average, beside the roundings of the sums."""
+    g, x = (t.abs() for t in _operands(m, 68, 128))
+    want = g.double().t() @ x.double()
+    assert (_grad(g, x).double() - want).norm() <= 3e-7 * want.norm()
+
+
 def test_zero_and_repeat():
     g, x = _operands(4000, 128, 128)
     assert torch.equal(_grad(g, x), _grad(g, x))                     # fixed order of the sums
