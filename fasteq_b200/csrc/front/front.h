@@ -27,8 +27,6 @@ using at::Tensor;
 using torch::autograd::AutogradContext;
 using torch::autograd::variable_list;
 
-struct Failure : std::runtime_error { using std::runtime_error::runtime_error; };
-
 // the C interface of the core library
 struct Core {
 #define F(name) decltype(&fasteq_##name) name = nullptr;
@@ -40,6 +38,9 @@ struct Core {
 };
 extern Core core;
 
+// Raises the Python layer's error.  It travels as the Python error itself: a C++ type would reach the caller of a backward, whose nodes run
+// on autograd's threads, as a plain RuntimeError.
+[[noreturn]] void fail(const std::string& message);
 void check(int rc, const char* what, decltype(&fasteq_last_cuda_error) last_error = nullptr);
 
 // A Python object held by something autograd may free on a thread without the GIL.

@@ -3,13 +3,20 @@
 namespace front {
 
 Core core;
+static PyObject* raised = nullptr;
+
+void fail(const std::string& message) {
+  py::gil_scoped_acquire gil;
+  PyErr_SetString(raised, message.c_str());
+  throw py::error_already_set();
+}
 
 void check(int rc, const char* what, decltype(&fasteq_last_cuda_error) last_error) {
   if (rc == FASTEQ_OK) return;
   static const char* names[] = {"ok", "unsupported", "invalid argument", "CUDA error", "internal error", "device fault"};
   std::string detail;
   if (rc == FASTEQ_CUDA_ERROR && last_error) detail = std::string(": ") + last_error();
-  throw Failure(std::string(what) + " failed with status " + std::to_string(rc) + " (" + (rc > 0 && rc < 6 ? names[rc] : "?") + ")" + detail);
+  fail(std::string(what) + " failed with status " + std::to_string(rc) + " (" + (rc > 0 && rc < 6 ? names[rc] : "?") + ")" + detail);
 }
 
 }  // namespace front
@@ -24,11 +31,7 @@ PYBIND11_MODULE(fasteq_front, m) {
     F(radial_chain_prepare) F(radial_chain_forward) F(radial_chain_backward) F(edge_geometry_forward) F(edge_geometry_backward)
     F(silu) F(neighbors_work_bytes) F(neighbors_count) F(neighbors_fill) F(graph_partition) F(graph_partition_edges) F(last_cuda_error)
 #undef F
-    static PyObject* raised = failure.release().ptr();
-    py::register_exception_translator([](std::exception_ptr p) {
-      try { if (p) std::rethrow_exception(p); }
-      catch (const Failure& e) { PyErr_SetString(raised, e.what()); }
-    });
+    raised = failure.release().ptr();
   });
   bind_prepared(m);
   bind_layers(m);

@@ -94,3 +94,14 @@ def test_differentiable_backward(n_hidden, nb):
     got = second(lambda b: radial_chain(b, cw), basis.cuda(), r.cuda(), t.cuda())
     for a, b in zip(got, want):
         assert _rel(a.cpu(), b) <= 2e-5       # the chain's 1e-5, forwards and backwards
+
+
+@pytest.mark.gpu
+def test_a_failure_on_autograds_thread_keeps_its_type():
+    from fasteq_b200._cabi import FasteqError
+    from fasteq_b200.ops.radial_chain import radial_chain
+    basis = torch.randn(40, 8, device="cuda", requires_grad=True)
+    out = radial_chain(basis, [torch.randn(64, 8, device="cuda"), torch.randn(64, 64, device="cuda")])
+    odd = torch.zeros(40 * 64 + 1, device="cuda")[1:].view(40, 64)        # not on 16 bytes: refused by the launch
+    with pytest.raises(FasteqError, match="fasteq_radial_chain_backward failed with status 1"):
+        torch.autograd.grad(out, basis, odd)
