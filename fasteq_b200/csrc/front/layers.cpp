@@ -145,6 +145,7 @@ variable_list EqLinearBackward::backward(AutogradContext* ctx, variable_list gg)
 Tensor eqlinear(const Geom& g, const Tensor& w, const Tensor& x, int64_t precision) {
   if (!x.is_cuda() || !w.is_cuda()) fail("eqlinear: x and w must be CUDA tensors: fasteq_b200 has no CPU path");
   const int64_t cols = (int64_t)g->in_rows * g->u;
+  TORCH_CHECK_VALUE(cols > 0, "eqlinear: the descriptor has no input values (I*U = ", cols, ")");
   TORCH_CHECK_VALUE((x.dim() > 0 && x.size(-1) == cols) || x.numel() % cols == 0, "eqlinear: x has ", x.numel(), " elements, not a multiple of I*U = ", cols);
   TORCH_CHECK_VALUE(w.numel() == g->paths() * g->u * g->v, "eqlinear: w has ", w.numel(), " elements, expected P*U*V = ", g->paths() * g->u * g->v);
   return EqLinear::apply(w, x, g, precision);

@@ -187,3 +187,9 @@ def test_rows_without_a_path_are_zero(dtype, prec, tol):
     assert _rel_fro(o3, ref) <= tol and _rel_fro(g3, ref_gx) <= tol
     assert np.count_nonzero(o3[:, :7]) == 0 and np.count_nonzero(o3[:, 16:]) == 0           # 3o (rows 0-6) and 4e (rows 16-24)
     assert np.count_nonzero(g3[:, :3]) == 0 and np.count_nonzero(g3[:, 7:12]) == 0 and np.count_nonzero(g3[:, 17:]) == 0
+
+
+def test_a_descriptor_without_input_values_is_refused():
+    from fasteq_b200.ops.eqlinear import fast_equi_linear
+    with pytest.raises(ValueError, match="no input values"):
+        fast_equi_linear(_FakeDescriptor([1], 0, 4, [1.0]), torch.empty(0, device="cuda"), torch.empty(3, 0, device="cuda"))
