@@ -80,6 +80,13 @@ FRONT_SOURCES = ["module.cpp", "prepared.cpp", "layers.cpp", "edges.cpp", "u1d.c
 _front_lock = threading.Lock()
 
 
+def _loaded_runtime() -> List[str]:
+    """The C++ runtime torch brought into this process.  The extension is linked to it by path: a compiler whose own is an archive would
+    put a second one into the extension, and formatting a number with that one ends the process."""
+    with open("/proc/self/maps") as f:
+        return sorted({line.split()[-1] for line in f if os.path.basename(line.split()[-1]).startswith("libstdc++.so")})
+
+
 def build_front(force: bool = False) -> str:
     """The native host path: host code only, compiled with g++ against torch's headers."""
     import sysconfig
@@ -111,7 +118,7 @@ def build_front(force: bool = False) -> str:
                 list(ex.map(lambda so: run([cxx] + flags + ["-c", so[0], "-o", so[1]]), zip(srcs, objs)))
             out = os.path.join(tmp, "fasteq_front.so")
             libs = os.path.join(base, "lib")
-            run([cxx, "-shared", "-o", out] + objs + [f"-L{libs}", f"-Wl,-rpath,{libs}", f"-L{cuda}/lib64", "-ltorch", "-ltorch_cpu", "-ltorch_cuda",
+            run([cxx, "-shared", "-o", out] + objs + _loaded_runtime() + [f"-L{libs}", f"-Wl,-rpath,{libs}", f"-L{cuda}/lib64", "-ltorch", "-ltorch_cpu", "-ltorch_cuda",
                                                        "-ltorch_python", "-lc10", "-lc10_cuda", "-lcudart"])
             os.replace(out, FRONT_SO)
     return FRONT_SO

@@ -144,3 +144,9 @@ def test_device_status_helper_needs_no_gpu():
     from fasteq_b200.status import device_status
     if not torch.cuda.is_available():
         assert device_status() == {}
+
+
+def test_the_native_host_path_has_torchs_cpp_runtime():
+    from fasteq_b200 import _build
+    with open(_build.build_front(), "rb") as f:
+        assert b"libstdc++.so.6" in f.read()

@@ -193,3 +193,12 @@ def test_a_descriptor_without_input_values_is_refused():
     from fasteq_b200.ops.eqlinear import fast_equi_linear
     with pytest.raises(ValueError, match="no input values"):
         fast_equi_linear(_FakeDescriptor([1], 0, 4, [1.0]), torch.empty(0, device="cuda"), torch.empty(3, 0, device="cuda"))
+
+
+def test_wrong_extents_are_refused():
+    from fasteq_b200.ops.eqlinear import fast_equi_linear
+    d = _FakeDescriptor([1, 3], 4, 4, [1.0, 1.0])
+    with pytest.raises(ValueError, match="x has 15 elements"):
+        fast_equi_linear(d, torch.empty(32, device="cuda"), torch.empty(3, 5, device="cuda"))
+    with pytest.raises(ValueError, match="w has 31 elements, expected"):
+        fast_equi_linear(d, torch.empty(31, device="cuda"), torch.empty(3, 16, device="cuda"))
