@@ -551,9 +551,10 @@ def _signature(meta, dtype):
     """``(native signature, columns of x)`` of the usual operand form (per-edge weights, sender gather, receiver scatter, one y value per
     segment); ``None`` for the others."""
     y_sh = meta.get("y_sh")
+    # whole numbers may come as tensors, which would be another key each time they are taken out of their list
     key = tuple((id(meta[k]), getattr(meta[k], "_version", 0)) for k in _TABLES) + (
-        meta["w_seg_num"], meta["x_seg_num"], meta["y_seg_num"], meta["out_seg_num"], meta["u_dim"], meta["size_list"][2], dtype,
-        tuple(y_sh) if y_sh else ())
+        int(meta["w_seg_num"]), int(meta["x_seg_num"]), int(meta["y_seg_num"]), int(meta["out_seg_num"]), int(meta["u_dim"]),
+        int(meta["size_list"][2]), dtype, tuple(y_sh) if y_sh else ())
     hit = _SIGNATURES.get(key)
     if hit is not None:
         return hit[0]

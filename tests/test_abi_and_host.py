@@ -146,6 +146,18 @@ def test_device_status_helper_needs_no_gpu():
         assert device_status() == {}
 
 
+def test_signatures_of_tables_with_tensor_extents_are_found_again():
+    import torch
+    from fasteq_b200 import descriptors
+    from fasteq_b200.irreps import Irreps
+    from fasteq_b200.ops import uniform1d_jit as u1d
+    sh = Irreps.spherical_harmonics(1)
+    io, ins = descriptors.full_channelwise_instructions("8x0e+8x1o", sh, 1)
+    meta = descriptors.channelwise_tensor_product("8x0e+8x1o", sh, io, ins).meta(torch.float32, "cpu")
+    meta["size_list"] = torch.tensor([int(v) for v in meta["size_list"]])
+    assert u1d._signature(meta, torch.float32) is u1d._signature(meta, torch.float32)
+
+
 def test_the_native_host_path_has_torchs_cpp_runtime():
     from fasteq_b200 import _build
     with open(_build.build_front(), "rb") as f:
