@@ -75,7 +75,6 @@ def build_core(force: bool = False) -> str:
 
 
 FRONT = os.path.join(CSRC, "front")
-FRONT_SO = os.path.join(LIB, "fasteq_front.so")
 FRONT_SOURCES = ["module.cpp", "prepared.cpp", "layers.cpp", "edges.cpp", "u1d.cpp"]
 _front_lock = threading.Lock()
 
@@ -87,16 +86,24 @@ def _loaded_runtime() -> List[str]:
         return sorted({line.split()[-1] for line in f if os.path.basename(line.split()[-1]).startswith("libstdc++.so")})
 
 
+def front_so() -> str:
+    """Unlike the libraries behind the C interface the extension belongs to one torch, one interpreter and one ABI of the C++ runtime."""
+    import sys
+    import torch
+    return os.path.join(LIB, f"fasteq_front.torch{torch.__version__}.abi{int(torch._C._GLIBCXX_USE_CXX11_ABI)}.{sys.implementation.cache_tag}.so")
+
+
 def build_front(force: bool = False) -> str:
     """The native host path: host code only, compiled with g++ against torch's headers."""
     import sysconfig
     import tempfile
     from concurrent.futures import ThreadPoolExecutor
+    so = front_so()
     srcs = [os.path.join(FRONT, s) for s in FRONT_SOURCES]
     deps = srcs + [os.path.join(FRONT, "front.h"), os.path.join(INCLUDE, "fasteq_b200.h")]
     with _front_lock:
-        if not force and _newer(FRONT_SO, deps):
-            return FRONT_SO
+        if not force and _newer(so, deps):
+            return so
         import torch
         base = os.path.dirname(torch.__file__)
         cuda = os.path.dirname(os.path.dirname(nvcc_path()))
@@ -120,8 +127,8 @@ def build_front(force: bool = False) -> str:
             libs = os.path.join(base, "lib")
             run([cxx, "-shared", "-o", out] + objs + _loaded_runtime() + [f"-L{libs}", f"-Wl,-rpath,{libs}", f"-L{cuda}/lib64", "-ltorch", "-ltorch_cpu", "-ltorch_cuda",
                                                        "-ltorch_python", "-lc10", "-lc10_cuda", "-lcudart"])
-            os.replace(out, FRONT_SO)
-    return FRONT_SO
+            os.replace(out, so)
+    return so
 
 
 def build_generated(name: str, source: str, extra: Optional[List[str]] = None, force: bool = False) -> str:

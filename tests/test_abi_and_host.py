@@ -162,3 +162,12 @@ def test_the_native_host_path_has_torchs_cpp_runtime():
     from fasteq_b200 import _build
     with open(_build.build_front(), "rb") as f:
         assert b"libstdc++.so.6" in f.read()
+
+
+def test_the_native_host_path_is_built_for_one_torch(monkeypatch):
+    import torch
+    from fasteq_b200 import _build
+    here = _build.front_so()
+    assert here == _build.build_front()
+    monkeypatch.setattr(torch, "__version__", "0.0")
+    assert _build.front_so() != here
