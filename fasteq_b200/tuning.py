@@ -52,7 +52,8 @@ _LOOKUPS: Dict[Tuple, Optional[_emit.Tuning]] = {}
 
 def lookup(spec: U1DSpec, direction: str, needs=(False, False, False)) -> Optional[_emit.Tuning]:
     """The stored winner of this signature, or ``None``.  A signature with in-kernel spherical harmonics shares the
-    entry of the same signature without them (the consumer code is identical).  Answers are memoised: the database
+    entry of the same signature without them (the consumer code is identical), a backward of a gradient subset without an entry
+    that of all gradients (the same rows to move, a little less arithmetic).  Answers are memoised: the database
     key hashes the whole path table, which must not happen on every operator call."""
     memo = (spec, direction, tuple(bool(n) for n in needs))
     if memo in _LOOKUPS:
@@ -66,12 +67,13 @@ def _lookup(spec: U1DSpec, direction: str, needs) -> Optional[_emit.Tuning]:
     for sp in (spec, dataclasses.replace(spec, y_sh=()) if spec.y_sh else None):
         if sp is None:
             continue
-        hit = db.get(_key(sp, direction, needs))
-        if hit is not None:
-            try:
-                return _emit.Tuning(**{k: hit["tuning"][k] for k in _FIELDS if k in hit["tuning"]})
-            except (KeyError, TypeError):
-                return None
+        for subset in (needs, (True, True, True)) if direction == "bwd" else (needs,):
+            hit = db.get(_key(sp, direction, subset))
+            if hit is not None:
+                try:
+                    return _emit.Tuning(**{k: hit["tuning"][k] for k in _FIELDS if k in hit["tuning"]})
+                except (KeyError, TypeError):
+                    return None
     return None
 
 

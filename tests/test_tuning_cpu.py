@@ -152,3 +152,25 @@ def test_rows_too_wide_for_second_order_modules():
     from fasteq_b200.ops import uniform1d_jit as u1d
     widest = cwtp_spec("+".join(f"128x{l}{p}" for l in range(4) for p in "eo"), 4, 4, "f64")
     assert u1d._dual_spec(widest, (True, True, True)) is None
+
+
+def test_gradient_subsets_share_the_full_sets_entry():
+    db = tuning.load_db()
+    for label, spec, direction, needs in tuning.sweep_jobs():
+        if direction != "bwd" or tuning._key(spec, "bwd", (True, True, True)) not in db:
+            continue
+        full = tuning.lookup(spec, "bwd", (True, True, True))
+        for subset in ((True, True, False), (False, True, True), (True, False, False)):
+            if tuning._key(spec, "bwd", subset) not in db:
+                assert tuning.lookup(spec, "bwd", subset) == full
+                gen.emit_backward(spec, full, *subset)
+
+
+def test_a_training_steps_modules_are_prebuilt():
+    from fasteq_b200.prebuild import model_jobs
+    u1d, stc, _ = model_jobs("f32", "mace", channels=32)
+    first, second = ({(s.dual, d, n) for s, d, n in u1d if s.x_segs == k and not s.y_sh} for k in (1, 4))
+    want = lambda dual: {((), "fwd", (False,) * 3), ((), "bwd", (True, True, False)), (dual, "fwd", (False,) * 3), (dual, "bwd", (True, True, False))}
+    assert first >= want((True, False, True)) | {((), "bwd", (True, False, True))}
+    assert second >= want((True, True, True)) | {((), "bwd", (True, True, True))}
+    assert {(d, n) for _, d, n in stc} == {("fwd", False), ("bwd", False), ("dbwd", False), ("bwdsum", True)}
