@@ -6,16 +6,28 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
-def test_force_pass_skips_weight_gradients_and_loses_none(monkeypatch):
+def _weight_gradient_launches(call):
+    """``(result, launches of weight-gradient kernels)`` of a call."""
+    from torch.profiler import ProfilerActivity, profile
+    torch.cuda.synchronize()
+    with profile(activities=[ProfilerActivity.CPU, ProfilerActivity.CUDA]) as prof:
+        out = call()
+        torch.cuda.synchronize()
+    kernels = [e.name for e in prof.events() if e.device_type == torch.autograd.DeviceType.CUDA]
+    assert kernels                                 # the profiler saw the launches
+    return out, sum("wgrad" in k and "reduce" not in k for k in kernels)
+
+
+def test_force_pass_skips_weight_gradients_and_loses_none():
     from fasteq_b200.ops import dense as dense_mod
-    calls = []
-    inner = dense_mod._matmul_tn
-    monkeypatch.setattr(dense_mod, "_matmul_tn", lambda g, x: (calls.append(1), inner(g, x))[1])
     g = torch.Generator(device="cuda").manual_seed(0)
     x = torch.randn(40, 16, device="cuda", generator=g, requires_grad=True)
     w = torch.randn(8, 16, device="cuda", generator=g, requires_grad=True)
-    (f,) = torch.autograd.grad((dense_mod.dense(x, w) ** 3).sum(), x, create_graph=True)
-    assert not calls
+    y = (dense_mod.dense(x, w) ** 3).sum()
+    (f,), launched = _weight_gradient_launches(lambda: torch.autograd.grad(y, x, create_graph=True))
+    assert launched == 0
+    _, launched = _weight_gradient_launches(lambda: torch.autograd.grad((dense_mod.dense(x, w) ** 3).sum(), (x, w), create_graph=True))
+    assert launched == 1
     (gw,) = torch.autograd.grad((f ** 2).sum(), w)
     xd, wd = x.detach().double().requires_grad_(True), w.detach().double().requires_grad_(True)
     y = xd @ wd.t()
