@@ -473,12 +473,12 @@ def operator_extras(args, dev):
         torch.autograd.grad(o, x, ro)
     t_lb = timed(lb)
     # the two launches alone, replayed from a CUDA graph (no host work per launch): kernel time of the forward and of grad_x
+    from fasteq_b200 import _front
     from fasteq_b200.ops import eqlinear as eql
-    geom = eql._descriptor_problem(dl)
-    plan = eql._Plan(geom, eql._resolve_precision(x, w, None), N, w.shape)
+    geom, precision, launch = eql._geometry(dl), eql._resolve_precision(x, w, None), _front.lib().eqlinear_launch
     xd = x.detach()
-    t_fk = _graph_replay_ms(lambda: plan.forward(w, xd)) * 1e-3
-    t_dk = _graph_replay_ms(lambda: plan.dgrad(w, ro)) * 1e-3
+    t_fk = _graph_replay_ms(lambda: launch(geom, w, xd, precision, False)) * 1e-3
+    t_dk = _graph_replay_ms(lambda: launch(geom, w, ro, precision, True)) * 1e-3
     rows = sum(p_rows for p_rows in [irr_tp[p.indices[1]].ir.dim for p in dl.paths])
     lbytes = 4.0 * (N * irr_tp.dim + N * 16 * 128 + dl.num_weights)
     peak, _ = measured_peak()

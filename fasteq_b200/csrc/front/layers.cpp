@@ -382,6 +382,7 @@ void bind_layers(py::module_& m) {
     at::AutoGradMode no_grad(false);
     return eqlinear_apply(*g, precision, w, a, dgrad, true);
   });
+  m.def("radial_chain_takes", &RadialChain::takes);
   m.def("radial_chain", [](const Tensor& basis, std::vector<Tensor> weights) -> std::optional<Tensor> {
     if (!RadialChain::takes(basis, weights)) return std::nullopt;
     return RadialChain::apply(basis.contiguous(), at::TensorList(weights));

@@ -85,13 +85,6 @@ def _fma_wgrad(x: torch.Tensor, g: torch.Tensor) -> torch.Tensor:
     return out
 
 
-def _matmul_nt(a: torch.Tensor, bt: torch.Tensor) -> torch.Tensor:
-    """``a [M, K] @ bt[N, K]^T`` on this library's one-path SO3Linear kernels (CUDA) or torch (CPU)."""
-    if a.is_cuda and a.dtype in (torch.float32, torch.float64) and a.dtype == bt.dtype:
-        return _fma_gemm(a, bt.t())
-    return a @ bt.t()
-
-
 def _matmul_tn(g: torch.Tensor, x: torch.Tensor) -> torch.Tensor:
     """``g [M, N]^T @ x [M, K] -> [N, K]``."""
     if g.is_cuda and g.dtype in (torch.float32, torch.float64) and g.dtype == x.dtype:

@@ -158,17 +158,11 @@ def wgrad_into(prob, x, g, dw) -> None:
 
 
 class _Plan:
-    """One operator call resolved: geometry, precision and the three launches over the caller's tensors.
-    ``w`` always has the caller's layout ``[P, u, v]`` flattened; ``x`` is ``[batch, I * u]``, ``g`` ``[batch, J * v]``."""
+    """The weight gradient of one operator call: ``x`` is ``[batch, I * u]``, ``g`` ``[batch, J * v]``, the result shaped like the caller's
+    weights."""
 
     def __init__(self, geom, precision, batch, w_shape):
         self.geom, self.precision, self.batch, self.w_shape = geom, precision, batch, tuple(w_shape)
-
-    def forward(self, w, x):
-        return _front.lib().eqlinear_launch(_native(self.geom), w, x, self.precision, False)
-
-    def dgrad(self, w, g):
-        return _front.lib().eqlinear_launch(_native(self.geom), w, g, self.precision, True)
 
     def wgrad(self, x, g):
         mapping, coeff, u, v, I, J = self.geom

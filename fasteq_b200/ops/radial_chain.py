@@ -13,22 +13,10 @@ import torch
 
 from .. import _front
 
-WIDTH = 64
-MAX_BASIS = 16
-MAX_HIDDEN = 3
-
 
 def radial_chain_usable(basis: torch.Tensor, weights: Sequence[torch.Tensor]) -> bool:
-    if not (basis.is_cuda and basis.dtype == torch.float32 and basis.dim() == 2 and basis.shape[0] > 0):
-        return False
-    if not (1 <= len(weights) <= MAX_HIDDEN and 1 <= basis.shape[1] <= MAX_BASIS):
-        return False
-    if tuple(weights[0].shape) != (WIDTH, basis.shape[1]):
-        return False
-    for w in weights:
-        if w.dtype != torch.float32 or not w.is_cuda or (torch.is_grad_enabled() and w.requires_grad):
-            return False
-    return all(tuple(w.shape) == (WIDTH, WIDTH) for w in weights[1:])
+    """Whether the fused kernels take the arguments."""
+    return _front.lib().radial_chain_takes(basis, list(weights))
 
 
 def radial_chain(basis: torch.Tensor, weights: Sequence[torch.Tensor]) -> Optional[torch.Tensor]:
