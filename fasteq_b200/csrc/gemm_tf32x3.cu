@@ -11,11 +11,11 @@
 // keeps the relative error near 2^-21 (the reference's tf32x3 scheme,
 // fasteq/cuda/src/eqlinear/backends/tf32/shape_plan.cu:109-113: three MMAs, no lo*lo term).
 //
-// Structure of one CTA (persistent: one CTA per SM walks 128 x BN output tiles round-robin, the stage ring
-// and two TMEM accumulators carry over from tile to tile so that loads, splits, MMAs and stores of
+// Structure of one CTA (persistent: one CTA per SM walks 128 x BN output tiles round-robin, the rings and the TMEM
+// accumulators - two of 64 columns or one of 128 - carry over from tile to tile so that loads, splits, MMAs and stores of
 // neighbouring tiles overlap):
 //   warps 0, 10  : TMA producers -- 3-D tiled loads (SWIZZLE_128B) of the raw A k-blocks (0) and of the weights' (10)
-//   warp 1       : allocates TMEM, issues tcgen05.mma (kind::tf32, M = 128, N = BN, K = 8) from one lane,
+//   warp 1       : allocates TMEM, issues tcgen05.mma (kind::tf32, M = 128, N = BN and 2 BN, K = 8) as a whole warp that elects a lane,
 //                  releases ring stages and signals the epilogue with tcgen05.commit
 //   warps 2..5   : split each raw A k-block into hi / lo parts in tensor memory (thread = row = TMEM
 //                  lane, tcgen05.st), from where the MMAs take their A operand

