@@ -59,6 +59,28 @@ def test_values_beyond_bf16(value):
     assert (got.double() - want)[fine].abs().max() <= 1e-6 * want[fine].abs().max()
 
 
+@pytest.mark.parametrize("value", [float("inf"), float("nan"), 1e35])
+@pytest.mark.parametrize("u,v", [(64, 132), (132, 64), (200, 136)])
+def test_values_beyond_bf16_in_irrep_rows(value, u, v):
+    """The recomputation in FP32 over paths of several rows, either operand the wider one, tiles beyond the extents."""
+    from fasteq_b200 import descriptors
+    from fasteq_b200.irreps import Irreps
+    from fasteq_b200.ops import fast_equi_linear
+    d = descriptors.linear(Irreps(f"{u}x0e+{u}x2e"), Irreps(f"{v}x2e+{v}x0e"))
+    gen = torch.Generator(device="cuda").manual_seed(u)
+    x, go = (torch.randn(301, 6 * c, device="cuda", generator=gen) for c in (u, v))
+    x[300, u + 3] = value                 # the first of the l = 2 rows, channel 3, in the last chunk
+    w = torch.randn(d.num_weights, device="cuda", generator=gen).requires_grad_(True)
+    (gw,) = torch.autograd.grad(fast_equi_linear(d, w, x), w, go)
+    xr, gr, got = x.double().view(301, 6, u), go.double().view(301, 6, v), gw.double().view(2, u, v)
+    for q, (i, o, n) in enumerate([(0, 5, 1), (1, 0, 5)]):
+        want = torch.einsum("btu,btv->uv", xr[:, i:i + n], gr[:, o:o + n]) / u ** 0.5
+        assert torch.equal(got[q].isnan(), want.isnan()) and torch.equal(got[q].isposinf(), want.isposinf())
+        for rows in (slice(3, 4), slice(0, 3), slice(4, None)):
+            fine = want[rows].isfinite()
+            assert (got[q][rows] - want[rows])[fine].norm() <= 3e-7 * want[rows][fine].norm()
+
+
 @pytest.mark.parametrize("scale", [1e-36, 1e-19, 1e18])
 def test_small_and_large_operands(scale):
     g, x = _operands(700, 64, 64)
