@@ -1006,9 +1006,10 @@ __global__ void __launch_bounds__(NT) eqlinear_wgrad_kernel(const __grid_constan
 // loads: one thread per output walked hundreds of splits one after the other (28 us for a [64, 64] gradient in 313 splits), hence
 // Y = 8; a few rows make one split per path, and seven of eight threads would have none of it (ten-path SO3Linear of 128
 // channels, one node: 10.2 us with Y = 8, 6.9 with 1; general kernel in FP64 12.3 and 8.9).
+// `gain`: what the partial sums lost on average (see wgrad_bf16x6.cuh), given back with the coefficient in one rounding; 1 elsewhere.
 template <typename T, int Y>
 __global__ void __launch_bounds__(256) eqlinear_wgrad_reduce_kernel(const __grid_constant__ WgradTable tab, const T* partial, T* gw,
-                                                                    int num_paths, long long uv) {
+                                                                    int num_paths, long long uv, double gain) {
   wait_for_previous_kernel();
   constexpr int X = 256 / Y;
   __shared__ T share[Y][X + 1];
@@ -1025,7 +1026,7 @@ __global__ void __launch_bounds__(256) eqlinear_wgrad_reduce_kernel(const __grid
   if (threadIdx.y == 0 && i < total) {
 #pragma unroll
     for (int k = 1; k < Y; ++k) sum += share[k][threadIdx.x];
-    gw[i] = (T)tab.coeff[q] * sum;
+    gw[i] = gain == 1.0 ? (T)tab.coeff[q] * sum : (T)(tab.coeff[q] * gain * (double)sum);
   }
 }
 
@@ -1151,7 +1152,9 @@ int launch_wgrad(const fasteq_eqlinear_problem* p, const void* x, const void* go
   // The tensor cores from 129 rows on, in chunks of 32 batch entries of one irrep row (a batch below 16 would leave most of a chunk
   // empty).  Up to 128 rows every path is one share, and what counts is how many CTAs start and how little each stores: the
   // ten-path SO3Linear of 128 channels takes 9.7 us at 8 nodes and 18.5 on the tensor cores, at 33 nodes 22.9 and 18.9.
+  double gain = 1.0;
   if (quads && p->batch >= 16 && p->batch * max_rows > 128 && p->batch <= 0x7fffffffLL && (p->batch / 32 + 1) * max_rows < (1LL << 30)) {
+    gain = wg::GAIN;
     rc = std::min(p->u, p->v) <= 64 ? launch_wgrad_tc<64>(p, &tab, sms, xf, gf, pf, scratch, s)
                                     : launch_wgrad_tc<128>(p, &tab, sms, xf, gf, pf, scratch, s);
   } else if (quads && max_rows <= WG_MAX_ROWS) {
@@ -1169,9 +1172,9 @@ int launch_wgrad(const fasteq_eqlinear_problem* p, const void* x, const void* go
   }
   if (rc == FASTEQ_OK && partial) {
     if (tab.split_first[p->num_paths] == p->num_paths)
-      e = launch_dependent(eqlinear_wgrad_reduce_kernel<T, 1>, (unsigned)((total + 255) / 256), dim3(256, 1), 0, s, tab, partial, (T*)gw, p->num_paths, uv);
+      e = launch_dependent(eqlinear_wgrad_reduce_kernel<T, 1>, (unsigned)((total + 255) / 256), dim3(256, 1), 0, s, tab, partial, (T*)gw, p->num_paths, uv, gain);
     else
-      e = launch_dependent(eqlinear_wgrad_reduce_kernel<T, 8>, (unsigned)((total + 31) / 32), dim3(32, 8), 0, s, tab, partial, (T*)gw, p->num_paths, uv);
+      e = launch_dependent(eqlinear_wgrad_reduce_kernel<T, 8>, (unsigned)((total + 31) / 32), dim3(32, 8), 0, s, tab, partial, (T*)gw, p->num_paths, uv, gain);
     if (e != cudaSuccess) rc = cuda_fail(e);
   }
   if (scratch.own) cudaFreeAsync(scratch.own, s);

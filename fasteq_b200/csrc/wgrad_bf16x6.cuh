@@ -5,6 +5,7 @@
 // accuracy is the tensor core's accumulation, which truncates: 2^-24 or so per K step, toward zero.  Hence chunks of 32 rows, two K
 // steps at full magnitude (the small products go first), each added to registers with ordinary rounding, 16 chunks to a
 // second-level sum in shared memory.  Two TF32 parts would need lo x lo and TF32 runs at half the rate: no cheaper, less exact.
+// What the truncation costs on average, 0.75 x 2^-24 of a sum, the reduction multiplies back in, with the coefficient and in one rounding.
 //
 // One CTA of 18 warps per SM takes a share of one path's chunks, 32 batch
 // entries of one irrep row each, and a 128 x TN tile:
@@ -18,7 +19,9 @@
 // tensor cores are busy for 66 and issue for half (ncu).  Measured
 // with the reduction, against 8 x 8 register tiles on the FP32 pipe: the 128-channel SO3Linear after the tensor product at
 // 12,288 nodes 365 -> 117 us, at 512 nodes 28 -> 22; [80000, 64]^T [80000, 1280] 309 -> 149; [80000, 128]^T [80000, 128] 65 -> 31; at
-// 200 rows 18.6 -> 14.4.  Errors against FP64 (2-norm) 2.26e-7 -> 1.24e-7, 2.11e-7 -> 1.35e-7, 1.66e-7 -> 1.42e-7, 1.12e-7 -> 0.74e-7.
+// 200 rows 18.6 -> 14.4.  Errors against FP64 (2-norm, 1e-8; FP32 chunks of 32 rows, this without the gain, this) at 160, 2,000
+// and 100,003 rows of 128 x 128: normal operands 11.3, 7.3, 6.8; 12.8, 9.4, 9.1; 16.8, 13.7, 13.5; of one sign, where the losses do not cancel, 5.5, 6.6, 4.8;
+// 5.4, 7.4, 7.4; 4.4, 6.8, 4.6 (where the gain is less than half a step of the result it rounds away).
 // About 13 us are the launch, the first chunk's way through the roles and the reduction.
 // Range: a third part reaches 24 bits below its operand, and bf16's smallest numbers are 2^-133.  Operands are therefore split 2^24 times as
 // large, which holds every FP32 number in three parts and keeps every product's parts above FP32's smallest; the stored sums are scaled
@@ -30,6 +33,7 @@ namespace fasteq {
 namespace wg {
 
 constexpr int TM = 128, ROWS = 32, RAW = 3, STAGES = 2, THREADS = 18 * 32, OUTER = 16;
+constexpr double GAIN = 1.0 + 4.5e-8;
 constexpr float SCALE = 16777216.f, UNSCALE = 1.f / (SCALE * SCALE);
 constexpr int A_COLS = 3 * ROWS / 2;                       // TMEM columns of one M-operand stage: three parts, two rows per column
 __host__ __device__ constexpr int b_part(int tn) { return tn * ROWS * 2; }

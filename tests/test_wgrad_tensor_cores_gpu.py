@@ -114,10 +114,10 @@ def test_a_tiny_channel_beside_ordinary_ones():
 @pytest.mark.parametrize("m", [160, 5000, 100_003])
 def test_operands_of_one_sign(m):
     """The tensor core truncates, always towards zero here, and no cancellation hides it: per chunk two truncated steps of at most 2^-23,
-    half of that on average, beside the roundings of the sums."""
+    half of that on average, of which the reduction gives three quarters of 2^-24 back, beside the roundings of the sums."""
     g, x = (t.abs() for t in _operands(m, 68, 128))
     want = g.double().t() @ x.double()
-    assert (_grad(g, x).double() - want).norm() <= 3e-7 * want.norm()
+    assert (_grad(g, x).double() - want).norm() <= 1e-7 * want.norm()
 
 
 def test_zero_and_repeat():
